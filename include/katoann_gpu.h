@@ -223,17 +223,17 @@ int katoann_gpu_set_seed_rows(uint32_t rows);
 
 /* Knobs of the tensor-core ranking pass (process-wide; results never depend
  * on them): the largest work-item width (0 = by the prefix width, else 16,
- * 32 or 64 queries) and the cost weight of the split of tiles over the
- * persistent CTAs (0 = equal tile counts; 1 to 8 = a tile of an item of MMA
- * width w costs 64 + beta w, and the CTAs take equal cost). */
+ * 32 or 64 queries) and the cost weight of the split of the work over the
+ * persistent CTAs (0 = by the instructions a step takes; 1 to 8 = a step of
+ * an item of width w, 16, 32 or its most, costs 64 + beta w). */
 int katoann_gpu_set_rank_width(uint32_t width);
 int katoann_gpu_set_rank_schedule(uint32_t beta);
 /* The current knobs: h_out[3] = {seed rows (0 = default), split weight, item width}. */
 void katoann_gpu_rank_knobs(uint32_t *h_out);
 /* Every mbarrier wait of the tensor-core ranking pass gives up after this
  * many SM cycles (0 = the default, 4e9, about 2 s at 2 GHz); a CTA that gives
- * up sets its error flag, lets its copies and MMAs in flight finish, frees
- * its tensor memory and returns, and is counted in workspace statistic 3.
+ * up sets its error flag, lets its copies in flight finish and returns, and
+ * is counted in workspace statistic 3.
  * Process-wide. A limit far below a pipeline step makes searches fail with
  * KATO_ETIMEOUT (the host library checks the count after each pass); that is
  * its only use besides the default. */
@@ -257,12 +257,9 @@ int katoann_gpu_search_timed(const katoann_gpu_index *index, const float *d_quer
  * candidate buffer overflowed and were rescanned exactly, [7] the largest
  * number of candidates one query had (last batch pass), [16..29] SM cycles
  * of the tensor-core ranking pass's warp roles, summed over CTAs (first
- * thread of each role): converters waiting for raw tiles, for free A stages,
- * total; MMA waiting for query tiles, free accumulators, converted tiles,
- * total; epilogue waiting for query tiles, accumulators, total; TMA waiting
- * for free stages, total; query staging waiting for free query tiles, total;
- * [30] cycles the ranking pass's MMA thread spent issuing MMAs and commits;
- * [31] cycles of the longest ranking CTA (the slowest SM's share);
+ * thread of each role): [16] scoring warps waiting for rows, [17] for items,
+ * [18] total; [28] query staging waiting for a free buffer, [29] total
+ * ([19..27] and [30] are 0: the pass has no such roles); [31] cycles of the longest ranking CTA (the slowest SM's share);
  * [32..38] the same for the tensor-core coarse product: TMA waiting for free
  * stages, total; MMA waiting for accumulators, for stages, total; first
  * epilogue warp waiting for accumulators, total; [40..45] the ranking pass's

@@ -1,4 +1,4 @@
-// Ranking pass on the 5th-generation tensor cores.
+// Ranking pass on the tensor cores.
 //
 // The reference scores every row of every probed list against the queries
 // that probe it with the high bytes of the leading h rotated dimensions
@@ -8,29 +8,12 @@
 //      ranking l2: the S-th smallest one over the first rows of its nearest
 //      lists (any S of its candidates bound its S-th best from above), widened
 //      so that every l2 with the same float distance stays inside;
-//   2. rank_tc_kernel scores (row, query) pairs on the tensor cores. Work
-//      items are (list, up to N of the queries probing it); each of a list's
-//      128-row tiles is scored against the item's queries. One CTA per SM
-//      takes an equal share of all tiles and runs them through a pipeline of
-//      warp roles connected by mbarriers:
-//        - a TMA thread loads raw tiles of high bytes (128 rows x 128 bytes,
-//          128-byte swizzle) into a ring of stages;
-//        - two staging warps gather each item's query rows, re-centred to
-//          (byte - 128) as exact fp16, into a double-buffered B tile in the
-//          canonical K-major layout, with each query's bound;
-//        - eight converter warps (two threads per row) re-centre the raw tiles
-//          to fp16 and store them into tensor memory (the A operand, two
-//          stages) with tcgen05.st, and sum each row's centred norm xn';
-//        - one MMA thread issues tcgen05.mma (M = 128 rows, N queries, K = 16)
-//          into double-buffered fp32 TMEM accumulators. Products are at most
-//          128 * 128, so up to 1024 dimensions add up exactly;
-//        - eight epilogue warps (thread = row, each warpgroup half of the
-//          columns) test l2 = qn' + xn' - 2 dot' against the query's bound
-//          (translating both vectors by 128 leaves every squared distance
-//          unchanged) and append passing (query, l2, row) records to the
-//          CTA's list; tc_bucket_kernel then sorts the records into per-query
-//          buffers with their float distances;
-//   3. a query whose buffer overflowed is rescanned exactly (rescan_*
+//   2. rank_tc_kernel scores (row, query) pairs and appends those that may lie
+//      within the bound to per-CTA record lists (below);
+//   3. tc_bucket_kernel completes the records' l2, drops those beyond the
+//      bound and sorts the rest into per-query buffers with their float
+//      distances;
+//   4. a query whose buffer overflowed is rescanned exactly (rescan_*
 //      kernels), and the merge kernel takes the exact best S by (distance, id)
 //      from each buffer, so results never depend on the bound or the buffer
 //      size.
@@ -38,9 +21,9 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <type_traits>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "kcommon.cuh"
 #include "rank_tc.cuh"
@@ -52,505 +35,528 @@ namespace kato {
 namespace {
 
 constexpr uint32_t kSeedCap = 4096;  // rows a seed bound looks at, at most
-
-// Warp roles of rank_tc_kernel.
-constexpr int kConvWarps = 8, kEpiWarps = 8, kQueryWarps = 2;
-constexpr int kTmaWarp = kConvWarps + kEpiWarps;  // 16
-constexpr int kMmaWarp = kTmaWarp + 1;             // 17
-constexpr int kQueryWarp0 = kMmaWarp + 1;          // 18, 19
-constexpr int kTcThreads = (kQueryWarp0 + kQueryWarps) * 32;
 constexpr uint32_t kDropped = 0x80000000u;  // qcount flag: a record did not fit
 
-struct QInfo {
-  uint32_t qid;
-  int32_t qn;   // centred norm of the query's ranking bytes
-  int32_t qb;   // bound - qn: a row is a candidate iff xn' - 2 dot' <= qb
-  float qbf;    // qb as float (exact below 2^24; beyond, every row passes anyway)
+// rank_tc_kernel: one CTA per SM takes an equal share, by cost, of all 64-row
+// slabs of all work items (an item is a list and up to N of the queries
+// probing it).
+//
+// What bounds it is DRAM: each probed row's ranking bytes are read once per
+// item, and a row meets few queries (10M x 1,024, nlist 16,384, nprobe 72:
+// 8 to 18 per list), so the products are cheap for any matrix path. mma.sync
+// m16n8k16 is taken over tcgen05 because the work comes in groups of 8
+// queries and its operands stay in registers: 1,024 fp16 products per clock
+// per SM measured, against 54 to 108 cycles for each tcgen05.mma of 128 rows,
+// 16 to 64 queries and 16 dimensions, whose operands also had to pass through
+// tensor memory between five roles of warps.
+//
+//   - eight scoring warps, each with its own ring of stages of two TMA boxes
+//     (32 rows x `IN` bytes each: a slab's two halves, or two chunks of one
+//     half), filled by the warp's own lane 0 ahead of their use. A lane turns the bytes of its four
+//     rows into fp16 A fragments, sums each row's norm, and multiplies with
+//     the item's queries, eight at a time. A dot product is the same over any
+//     order of its dimensions, so the fragments take the dimensions in the
+//     order that 16-byte reads deliver them;
+//   - four staging warps, each with its own query buffer: every nB-th item's
+//     description, bounds and the fp16 rows of its queries, copied ahead of
+//     the scoring warps.
+// The products of 32 rows x 128 bytes with 16 queries take 109 cycles of an
+// SM when nothing else runs (157 when each step is guarded for four query
+// groups, so there is a body for two); the rest is what a slab costs besides:
+// with 32-row slabs, runtime divisions and 64-bit addresses it was 490 more.
+// Exactness. For h <= 256 a row byte b enters as the fp16 bit pattern 0x00bb,
+// the subnormal b 2^-24 (one byte permute makes two of them), and a query byte
+// as itself: sums of up to 256 * 255^2 < 2^24 such products are exact in fp32
+// (kScale undoes the 2^-24). Beyond 256 dimensions both are re-centred to
+// (byte - 128), which leaves every squared distance unchanged and bounds a
+// product by 2^14: up to 1,024 dimensions add up exactly.
+// A pair passes if l2 = qn + xn - 2 dot is at most the query's bound, that is
+// if dot - xn / 2 >= -(bound - qn) / 2; rounding is monotone, so no pair within
+// the bound fails the float compare, and tc_bucket_kernel drops the few beyond
+// it that pass.
+//
+// Filtered items: a squared distance over the leading f < h dimensions never
+// exceeds the one over h, so an item may be scored over its rows' first f
+// bytes alone; what passes is recorded with its partial l2 and completed by
+// tc_bucket_kernel. On rotated vectors the leading dimensions hold most of
+// the distance, and the pass then reads f instead of h bytes per row (10M x
+// 1,024, h = 256, f = 128: 0.50 against 0.71 ms). Data whose distance is spread
+// evenly would pass nearly everything, so each CTA watches the records its
+// slabs give and filters only while completing them costs less.
+constexpr int kScoreWarps = kTcScoreWarps, kStageWarps = 4;
+constexpr int kTcThreads = (kScoreWarps + kStageWarps) * 32;
+
+static_assert(kStageWarps >= static_cast<int>(kTcMaxBufs), "roles");
+
+// An item as the scoring warps see it: its slabs, rows, queries and chunks of
+// IN dimensions.
+struct __align__(16) Desc {
+  uint32_t s0, s1, row0, nrows;
+  uint32_t ne, nch, partial, pad;
 };
-static_assert(sizeof(QInfo) == kTcQInfo, "query slot size");
+static_assert(sizeof(Desc) == kTcDesc, "item slot size");
 
-struct Bars {
-  uint64_t *raw_full, *raw_empty, *a_full, *a_empty, *b_full, *b_empty, *acc_full, *acc_empty,
-      *xn_full, *done;
-};
-
-// Barrier slots in order: raw full/empty (4 each, at most), A full/empty,
-// query buffers full/empty (2 each, at most), accumulators full/empty, row
-// norms full, done.
-__device__ __forceinline__ Bars bars_at(unsigned char *sm, const TcSmem &L) {
-  uint64_t *b = reinterpret_cast<uint64_t *>(sm + L.bars);
-  uint64_t *a = b + 8, *q = a + 2 * kTcAStages, *c = q + 4;
-  return Bars{b, b + 4, a, a + kTcAStages, q, q + 2, c, c + kTcAcc, c + 2 * kTcAcc, c + 3 * kTcAcc};
+// Shared-memory accesses by 32-bit address.
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 lds_float2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
 }
 
-// sum over 16 bytes of (b - 128)^2 = sum b^2 - 256 sum b + 16 * 16384
-__device__ __forceinline__ int32_t centred_sq_sum16(uint4 v) {
-  const uint32_t s2 = dp4(v.x, v.x, dp4(v.y, v.y, dp4(v.z, v.z, dp4(v.w, v.w, 0))));
-  const uint32_t s1 =
-      dp4(v.x, 0x01010101u, dp4(v.y, 0x01010101u, dp4(v.z, 0x01010101u, dp4(v.w, 0x01010101u, 0))));
-  return static_cast<int32_t>(s2) - 256 * static_cast<int32_t>(s1) + 16 * 16384;
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                          uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Walk over this CTA's tiles [t0, t1) and the items they belong to; the next
-// item's description is loaded one item ahead.
-struct TileWalk {
-  const uint32_t *tile_off;
-  const TcItem *items;
-  uint32_t nitems, t0, t1, t, item, start, next, next2;
-  TcItem cur, nxt;
-  __device__ void init(const uint32_t *to, const TcItem *it, uint32_t n, uint32_t a, uint32_t b) {
-    tile_off = to;
-    items = it;
-    nitems = n;
-    t0 = a;
-    t1 = b;
-    t = a;
-    uint32_t lo = 0, hi = n;  // tile_off[lo] <= a < tile_off[hi]
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) / 2;
-      if (tile_off[mid] <= a) lo = mid;
-      else hi = mid;
-    }
-    item = lo;
-    start = tile_off[lo];
-    next = tile_off[lo + 1];
-    next2 = lo + 2 <= n ? tile_off[lo + 2] : 0xFFFFFFFFu;
-    cur = items[lo];
-    nxt = lo + 1 < n ? items[lo + 1] : cur;
-  }
-  // Called at the top of each tile.
-  __device__ void step() {
-    if (t == next) {
-      ++item;
-      start = next;
-      next = next2;
-      cur = nxt;
-      next2 = item + 2 <= nitems ? tile_off[item + 2] : 0xFFFFFFFFu;
-      nxt = item + 1 < nitems ? items[item + 1] : cur;
-    }
-  }
-  __device__ bool first() const { return t == t0 || t == start; }
-  __device__ bool last() const { return t + 1 == t1 || t + 1 == next; }
-};
-
-// The MMA width (queries) an item of ne queries uses: 16, 32 or N.
-template <uint32_t N>
-__device__ __forceinline__ uint32_t mma_width(uint32_t ne) {
-  return ne <= 16 ? 16u : (ne <= 32 && N > 32 ? 32u : N);
+// 16-byte asynchronous global -> shared copy (L2 only).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// A pipeline wait that also adds the cycles it took to `acc`.
-__device__ __forceinline__ bool timed_wait(uint64_t *b, uint32_t phase, volatile uint32_t *err,
-                                           unsigned long long &acc, long long limit) {
-  const long long t = clock64();
-  const bool ok = tc::mbar_wait_or(b, phase, err, limit);
-  acc += clock64() - t;
-  return ok;
+// One arrival on `bar` once this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_addr(bar))
+               : "memory");
 }
 
-template <uint32_t N, bool kFloat>
+// Two bytes of a word (selector) as fp16: the subnormals b 2^-24, or
+// (byte - 128) by way of 1024 + byte.
+template <bool kCentred>
+__device__ __forceinline__ uint32_t half2_of(uint32_t w, uint32_t selector) {
+  if (!kCentred) return __byte_perm(w, 0, selector);
+  const uint32_t a = __byte_perm(w, 0x64646464u, selector);
+  const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&a), __floats2half2_rn(1152.0f, 1152.0f));
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// sum over 16 bytes of b^2
+__device__ __forceinline__ uint32_t sq_sum16(const uint32_t *w, uint32_t acc) {
+  return dp4(w[0], w[0], dp4(w[1], w[1], dp4(w[2], w[2], dp4(w[3], w[3], acc))));
+}
+
+// IN: bytes of a row in one chunk, 128, or 64 where the pass has only 64.
+template <uint32_t IN, bool kCentred>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    rank_tc_kernel(const __grid_constant__ CUtensorMap tmap, const RankTcArgs A, const TcShape S) {
+    rank_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ RankTcArgs A,
+                   const __grid_constant__ TcShape S) {
+  constexpr uint32_t NI = IN / 64;        // 16-byte reads per row, lane and chunk
+    constexpr uint32_t kBox = kTcBoxRows * IN, kStage = 2 * kBox;
+  // row bytes enter as multiples of kScale
+  constexpr float kScale = kCentred ? 1.0f : 0x1p-24f;
   extern __shared__ __align__(1024) unsigned char sm[];
-  const uint32_t h = A.h;
+  const uint32_t h = A.h, N = S.N, nB = S.Bs, depth = S.Rs;
   const TcSmem L = tc_smem_layout(h, S);
-  const Bars bar = bars_at(sm, L);
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + L.bars);  // per scoring warp and stage
+  uint64_t *d_full = full + kScoreWarps * kTcMaxStages;        // per query buffer: described,
+  uint64_t *b_full = d_full + kTcMaxBufs;                      // copied,
+  uint64_t *b_empty = b_full + kTcMaxBufs;                     // used by every scoring warp
   volatile uint32_t *err = reinterpret_cast<volatile uint32_t *>(sm + L.err);
-  uint32_t *tbase = reinterpret_cast<uint32_t *>(sm + L.tbase);
   uint32_t *rcount = reinterpret_cast<uint32_t *>(sm + L.rcount);
-  int32_t *sxn = reinterpret_cast<int32_t *>(sm + L.sxn);
-  QInfo *qinfo = reinterpret_cast<QInfo *>(sm + L.qinfo);
-  uint32_t *swidth = reinterpret_cast<uint32_t *>(sm + L.width);  // per query buffer: queries
-  const uint32_t btile = N * h * 2, rtile = kTcRows * S.inner;
+  // slabs scored, and filtered ones staged before any were
+  volatile uint32_t *slabs = rcount + 1, *fstaged = rcount + 2;
+  uint32_t *qids = reinterpret_cast<uint32_t *>(sm + L.qids);
+  // -(bound - qn) / 2 of each query slot, in units of kScale
+  float *qbv = reinterpret_cast<float *>(sm + L.qbv);
+  Desc *desc = reinterpret_cast<Desc *>(sm + L.desc);
+  const uint32_t nkc = (h + IN - 1) / IN, brow = nkc * IN * 2, btile = N * brow;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    for (uint32_t s = 0; s < S.Rs; ++s) {
-      tc::mbar_init(bar.raw_full + s, 1);
-      tc::mbar_init(bar.raw_empty + s, kConvWarps);
+    for (uint32_t s = 0; s < kScoreWarps * kTcMaxStages; ++s) tc::mbar_init(full + s, 1);
+    for (uint32_t s = 0; s < kTcMaxBufs; ++s) {
+      tc::mbar_init(d_full + s, 1);
+      tc::mbar_init(b_full + s, 64);
+      tc::mbar_init(b_empty + s, kScoreWarps);
     }
-    for (uint32_t s = 0; s < kTcAStages; ++s) {
-      tc::mbar_init(bar.a_full + s, kConvWarps);
-      tc::mbar_init(bar.a_empty + s, 1);
-    }
-    for (uint32_t s = 0; s < kTcAcc; ++s) {
-      tc::mbar_init(bar.acc_full + s, 1);
-      tc::mbar_init(bar.acc_empty + s, kEpiWarps);
-      tc::mbar_init(bar.xn_full + s, kConvWarps);
-    }
-    for (uint32_t s = 0; s < S.Bs; ++s) {
-      tc::mbar_init(bar.b_full + s, kQueryWarps);
-      tc::mbar_init(bar.b_empty + s, 1 + kEpiWarps);
-    }
-    tc::mbar_init(bar.done, 1);
-    *rcount = 0;
+    rcount[0] = rcount[1] = rcount[2] = 0;
     // the TMA swizzle pattern repeats every 1024 bytes of shared address
     *err = (tc::smem_addr(sm + L.raw) & 1023u) ? 2u : 0u;
     tc::fence_barrier_init();
   }
-  if (warp == kMmaWarp) tc::tmem_alloc(tbase, S.tcols);
-  tc::fence_before();
   __syncthreads();
-  tc::fence_after();
-  const uint32_t tmem = *tbase;
-  const uint32_t acol = kTcAcc * N;  // TMEM columns of the A stages follow the accumulators
-  const uint32_t nitems = *A.nitems;
-  const uint32_t T = nitems ? A.tile_off[nitems] : 0;
-  uint32_t t0, t1;
-  if (A.cost_off && nitems) {
-    // an equal share of the cost; cost unit c lies in tile tile_at(c)
-    const uint32_t C = A.cost_off[nitems];
-    auto tile_at = [&](uint32_t c) -> uint32_t {
-      if (c >= C) return T;
-      uint32_t lo = 0, hi = nitems;  // cost_off[lo] <= c < cost_off[hi]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (A.cost_off[mid] <= c) lo = mid;
-        else hi = mid;
-      }
-      const uint32_t tiles = A.tile_off[lo + 1] - A.tile_off[lo];
-      const uint32_t per = (A.cost_off[lo + 1] - A.cost_off[lo]) / tiles;
-      return A.tile_off[lo] + (c - A.cost_off[lo]) / per;
-    };
-    t0 = tile_at(static_cast<uint32_t>(static_cast<uint64_t>(C) * blockIdx.x / gridDim.x));
-    t1 = tile_at(static_cast<uint32_t>(static_cast<uint64_t>(C) * (blockIdx.x + 1) / gridDim.x));
-  } else {
-    t0 = static_cast<uint32_t>(static_cast<uint64_t>(T) * blockIdx.x / gridDim.x);
-    t1 = static_cast<uint32_t>(static_cast<uint64_t>(T) * (blockIdx.x + 1) / gridDim.x);
-  }
-  const uint32_t nkc = (h + S.inner - 1) / S.inner;
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
+  // this CTA's slabs t0 .. t1 - 1 and items it0 .. it1
+  const uint2 share = A.share[blockIdx.x], upto = A.share[blockIdx.x + 1];
+  const uint32_t t0 = share.x, t1 = upto.x, it0 = share.y;
   // per-role cycle profile (first thread of each role): waits, then total
-  unsigned long long pw[3] = {0, 0, 0};
+  unsigned long long pw[2] = {0, 0};
   const long long tstart = clock64();
+  // a bounded wait by the whole warp on the barrier at shared address b
+  // calling meanwhile() between its tries
+  auto wait_for = [&](uint32_t b, uint32_t phase, unsigned long long &acc, auto meanwhile) -> bool {
+    if (__all_sync(0xffffffffu, tc::mbar_test(b, phase))) return true;
+    const long long t = clock64();
+    bool ok = false;
+    long long took = 0;
+    do {
+      ok = meanwhile(b, phase);
+      took = clock64() - t;
+    } while (!ok && !*err && took <= A.wait);
+    if (took > A.wait) *err = 1, ok = false;
+    acc += took;
+    return __all_sync(0xffffffffu, ok);
+  };
+  auto wait = [&](uint32_t b, uint32_t phase, unsigned long long &acc) -> bool {
+    return wait_for(b, phase, acc, [](uint32_t x, uint32_t p) { return tc::mbar_try(x, p); });
+  };
 
   if (t0 < t1 && !*err) {
-    TileWalk w;
-    w.init(A.tile_off, A.items, nitems, t0, t1);
-    if (warp < kConvWarps) {
-      // ---- converters: raw stage -> fp16 A stage and the row's centred
-      // norm; two threads per row, each half of every chunk's 16-byte columns
-      const uint32_t r = tid & (kTcRows - 1), hf = tid >> 7, swm = S.inner == 128 ? 7u : 3u;
-      const uint32_t nuh = S.inner / 32;  // 16-byte columns per half of a full chunk
-      uint32_t rs = 0, rph = 0, as = 0, aph = 0, ab = 0, abph = 0;
+    // the item after the last one may start inside the next share
+    const uint32_t n_li = upto.y - it0 + (A.tile_off[upto.y] < t1);
+    const uint32_t d_full_a = tc::smem_addr(d_full), b_full_a = tc::smem_addr(b_full);
+    const uint32_t b_empty_a = tc::smem_addr(b_empty), desc_a = tc::smem_addr(desc);
+    if (warp < kScoreWarps) {
+      // ---- scoring: slabs t0 + warp, t0 + warp + kScoreWarps, ...
+      const uint32_t g = lane >> 2, tig = lane & 3;
+      const uint32_t ring = tc::smem_addr(sm + L.raw) + warp * depth * kStage;
+      const uint32_t bar = tc::smem_addr(full + warp * kTcMaxStages);
+      const uint32_t qbv_a = tc::smem_addr(qbv) + tig * 8, qid_a = tc::smem_addr(qids) + tig * 8;
+      const uint32_t b_a = tc::smem_addr(sm + L.b) + g * brow;
+      uint4 *rec = A.rec + static_cast<size_t>(blockIdx.x) * A.rec_cap;
+      // fetch side: the next stage to fetch (slab tn, its cn-th), its item (the
+      // i_n-th, in buffer i_bf) and ring stage
+      uint32_t inflight = 0, tn = t0 + warp, cn = 0, is = 0;
+      uint32_t i_n = 0, i_bf = nB - 1, i_ph = 1, i_end = 0, i_row = 0, i_nch = 1, i_pairs = 1;
+      // score side: the item being scored (the c_n-th), ring stage and phase
+      uint32_t c_n = 0, c_bf = nB - 1, c_ph = 1, c_end = 0, cs = 0, cph = 0;
+      uint4 d0 = make_uint4(0, 0, 0, 0), d1 = d0;
+      // fetches ahead as far as the ring and the described items allow; the
+      // item of the chunk to be read next is always described
+      auto fetch = [&]() {
+        while (inflight < depth && tn < t1) {
+          while (tn >= i_end) {
+            const uint32_t bf = i_bf + 1 == nB ? 0 : i_bf + 1, ph = i_ph ^ (bf == 0);
+            if (!__all_sync(0xffffffffu, tc::mbar_test(d_full_a + bf * 8, ph))) return;
+            const uint4 n0 = lds128(desc_a + bf * kTcDesc);
+            i_nch = lds32(desc_a + bf * kTcDesc + 20);
+            i_end = n0.y, i_row = n0.z - n0.x * kTcSlab, i_pairs = (i_nch + 1) / 2;
+            ++i_n, i_bf = bf, i_ph = ph;
+          }
+          if (lane == 0) {
+            const uint32_t dst = ring + is * kStage, b = bar + is * 8;
+            const int32_t y = static_cast<int32_t>(i_row + tn * kTcSlab);
+            if (i_nch == 1) {  // the slab's two halves
+              tc::mbar_expect_tx(b, kStage);
+              tc::tma_load_2d(dst, &tmap, 0, y, b);
+              tc::tma_load_2d(dst + kBox, &tmap, 0, y + static_cast<int32_t>(kTcBoxRows), b);
+            } else {           // two chunks of the first, then of the second half
+              const uint32_t half = cn >= i_pairs, ch = 2 * (half ? cn - i_pairs : cn);
+              const int32_t yh = y + static_cast<int32_t>(half * kTcBoxRows);
+              const bool both = ch + 1 < i_nch;
+              tc::mbar_expect_tx(b, both ? kStage : kBox);
+              tc::tma_load_2d(dst, &tmap, static_cast<int32_t>(ch * IN), yh, b);
+              if (both) tc::tma_load_2d(dst + kBox, &tmap, static_cast<int32_t>((ch + 1) * IN), yh, b);
+            }
+          }
+          ++inflight;
+          if (++is == depth) is = 0;
+          if (i_nch == 1 || ++cn == 2 * i_pairs) cn = 0, tn += kScoreWarps;
+        }
+      };
+      uint32_t xa[4][4 * NI];             // raw words of the lane's rows g, g + 8, g + 16, g + 24
+      auto read = [&](uint32_t st) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+#pragma unroll
+          for (uint32_t i = 0; i < NI; ++i) {
+            // 16-byte unit of the row, where the TMA's swizzle put it
+            const uint32_t u = IN == 128 ? ((2 * tig + i) ^ g) : (tig ^ ((g >> 1) & 3));
+            const uint4 v = lds128(st + (g + 8 * q) * IN + u * 16);
+            xa[q][4 * i] = v.x, xa[q][4 * i + 1] = v.y, xa[q][4 * i + 2] = v.z, xa[q][4 * i + 3] = v.w;
+          }
+      };
+      // the stage has been read by every lane: on to the next, and refill
+      auto release = [&]() {
+        __syncwarp();
+        if (++cs == depth) cs = 0, cph ^= 1;
+        --inflight;
+        fetch();
+      };
+      // the lane's part of its rows' norms
+      auto norms = [&](uint32_t (&xn)[4]) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+#pragma unroll
+          for (uint32_t i = 0; i < NI; ++i) {
+            const uint32_t *w = xa[q] + 4 * i;
+            if (kCentred) xn[q] += static_cast<uint32_t>(tc::centred_sq_sum16(make_uint4(w[0], w[1], w[2], w[3])));
+            else xn[q] = sq_sum16(w, xn[q]);
+          }
+      };
+      // the rows' norms from their four lanes' parts, and -xn / 2; `left` rows
+      // of the list remain from the lane's first row on, those past its end
+      // never pass
+      auto finish = [&](uint32_t (&xn)[4], float (&xh)[4], int32_t left) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          xn[q] += __shfl_xor_sync(0xffffffffu, xn[q], 1);
+          xn[q] += __shfl_xor_sync(0xffffffffu, xn[q], 2);
+          xh[q] = static_cast<int32_t>(8 * q) < left
+                      ? static_cast<float>(static_cast<int32_t>(xn[q])) * (-0.5f * kScale)
+                      : -INFINITY;
+        }
+      };
+      // dimensions 32 s .. of the chunk times the kG query groups at bq
+      auto step = [&](auto kg, uint32_t s, uint32_t bq, float (&c)[decltype(kg)::value][2][4]) {
+        uint32_t a[2][2][4];
+#pragma unroll
+        for (uint32_t m = 0; m < 2; ++m)
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j) {
+            // A fragments of rows g + 16 m, g + 16 m + 8
+            a[m][j][0] = half2_of<kCentred>(xa[2 * m][2 * s + j], 0x4140);
+            a[m][j][1] = half2_of<kCentred>(xa[2 * m + 1][2 * s + j], 0x4140);
+            a[m][j][2] = half2_of<kCentred>(xa[2 * m][2 * s + j], 0x4342);
+            a[m][j][3] = half2_of<kCentred>(xa[2 * m + 1][2 * s + j], 0x4342);
+          }
+        // the B fragments of two 16-dimension steps: one 16-byte unit of the
+        // query's row, swizzled so that eight lanes meet eight banks
+        uint32_t u;
+        if (IN == 128) {
+          u = 4 * tig + s;
+          u = u ^ ((u >> 3) & 1) ^ ((g & 1) << 1);
+        } else {
+          u = (2 * tig + s) ^ (g & 1);
+        }
+#pragma unroll
+        for (uint32_t gr = 0; gr < decltype(kg)::value; ++gr) {
+          const uint4 b = lds128(bq + gr * 8 * brow + u * 16);
+#pragma unroll
+          for (uint32_t m = 0; m < 2; ++m) mma_16816(c[gr][m], a[m][0], b.x, b.y);
+#pragma unroll
+          for (uint32_t m = 0; m < 2; ++m) mma_16816(c[gr][m], a[m][1], b.z, b.w);
+        }
+      };
+      // tests a group's pairs (query slots at `slot`) and records those that pass
+      auto test = [&](const float (&c)[2][4], const float (&xh)[4], const uint32_t (&xn)[4],
+                      uint32_t slot, uint32_t row) {
+        const float2 th = lds_float2(qbv_a + slot * 4);
+        bool hit = false;
+#pragma unroll
+        for (uint32_t b = 0; b < 8; ++b)
+          hit |= c[b >> 2][b & 3] + xh[b >> 1] >= ((b & 1) ? th.y : th.x);
+        if (hit) {
+          uint32_t mask = 0;
+#pragma unroll
+          for (uint32_t b = 0; b < 8; ++b)
+            mask |= static_cast<uint32_t>(c[b >> 2][b & 3] + xh[b >> 1] >= ((b & 1) ? th.y : th.x)) << b;
+          // records (query, xn - 2 dot, row, partial) go to this CTA's list;
+          // few lanes have any, so each reserves its own places
+          uint32_t at = atomicAdd(rcount, __popc(mask));
+          do {
+            const uint32_t b = __ffs(mask) - 1;
+            mask &= mask - 1;
+            const float v0 = b & 4 ? c[1][0] : c[0][0], v1 = b & 4 ? c[1][1] : c[0][1];
+            const float v2 = b & 4 ? c[1][2] : c[0][2], v3 = b & 4 ? c[1][3] : c[0][3];
+            const float w0 = b & 2 ? v2 : v0, w1 = b & 2 ? v3 : v1;
+            const uint32_t x0 = b & 4 ? xn[2] : xn[0], x1 = b & 4 ? xn[3] : xn[1];
+            const uint32_t qid = lds32(qid_a + (slot + (b & 1)) * 4);
+            const int32_t l2 = static_cast<int32_t>(b & 2 ? x1 : x0) +
+                               __float2int_rn((b & 1 ? w1 : w0) * (-2.0f / kScale));
+            if (at < A.rec_cap) rec[at] = make_uint4(qid, static_cast<uint32_t>(l2), row + 8 * (b >> 1), d1.z);
+            else atomicOr(A.qcount + qid, kDropped);
+            ++at;
+          } while (mask);
+        }
+      };
       bool ok = true;
-      for (; ok && w.t < t1; ++w.t) {
-        int32_t xs = 0;
-        for (uint32_t kc = 0; kc < nkc; ++kc) {
-          // warp-uniform waits: a warp arrives once for all its lanes below
-          if (!__all_sync(0xffffffffu, timed_wait(bar.raw_full + rs, rph, err, pw[0], A.wait) &&
-                                           timed_wait(bar.a_empty + as, aph ^ 1, err, pw[1], A.wait))) {
+      for (uint32_t t = t0 + warp; ok && t < t1; t += kScoreWarps) {
+        while (t >= c_end) {  // on to the slab's item, handing back those before it
+          __syncwarp();       // every lane has done with the item's queries
+          if (c_n && lane == 0) tc::mbar_arrive(b_empty_a + c_bf * 8);
+          c_bf = c_bf + 1 == nB ? 0 : c_bf + 1;
+          c_ph ^= c_bf == 0;
+          ++c_n;
+          // rows are fetched as soon as their item is described
+          if (!wait_for(b_full_a + c_bf * 8, c_ph, pw[1], [&](uint32_t x, uint32_t p) {
+                fetch();
+                return __all_sync(0xffffffffu, tc::mbar_test(x, p)) != 0;
+              })) {
             ok = false;
             break;
           }
-          tc::fence_after();  // the MMAs that read A stage `as` before have completed
-          const unsigned char *raw = sm + L.raw + rs * rtile;
-          const uint32_t nu = min(S.inner, h - kc * S.inner) / 16;
-          // the row's half of the chunk as fp16 pairs: 16 dimensions = 8 columns
-          uint32_t cols[32];
-#pragma unroll
-          for (uint32_t i = 0; i < 4; ++i) {
-            const uint32_t u = hf * nuh + i;
-            uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-            if (i < nuh && u < nu) {
-              const uint32_t o = r * S.inner + u * 16;
-              const uint4 v = *reinterpret_cast<const uint4 *>(raw + (o ^ (((o >> 7) & swm) << 4)));
-              tc::bytes_to_half16(v, bias, lo, hi);
-              xs += centred_sq_sum16(v);
-            }
-            cols[8 * i + 0] = lo.x, cols[8 * i + 1] = lo.y, cols[8 * i + 2] = lo.z, cols[8 * i + 3] = lo.w;
-            cols[8 * i + 4] = hi.x, cols[8 * i + 5] = hi.y, cols[8 * i + 6] = hi.z, cols[8 * i + 7] = hi.w;
+          d0 = lds128(desc_a + c_bf * kTcDesc);
+          d1 = lds128(desc_a + c_bf * kTcDesc + 16);
+          c_end = d0.y;
+          // the fetch side never falls behind: a buffer handed back may
+          // already describe a later item
+          if (i_n < c_n) {
+            i_n = c_n, i_bf = c_bf, i_ph = c_ph, i_end = d0.y;
+            i_row = d0.z - d0.x * kTcSlab, i_nch = d1.y, i_pairs = (i_nch + 1) / 2;
           }
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(bar.raw_empty + rs);  // the raw stage has been read
-          // into this row's TMEM lane: A stage `as`, the half's columns
-          if (hf * nuh < nu) {
-            const uint32_t taddr =
-                tmem + (((warp & 3) * 32u) << 16) + acol + as * (S.inner / 2) + hf * nuh * 8;
-            if (nuh == 4) tc::tmem_st32(taddr, cols);
-            else tc::tmem_st16(taddr, *reinterpret_cast<const uint32_t(*)[16]>(cols));
-          }
-          tc::tmem_wait_st();
-          tc::fence_before();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(bar.a_full + as);
-          if (++rs == S.Rs) rs = 0, rph ^= 1;
-          if (++as == kTcAStages) as = 0, aph ^= 1;
         }
         if (!ok) break;
-        // the row norms of this tile's accumulator slot, once the epilogue
-        // has finished with the slot's previous tile
-        if (!__all_sync(0xffffffffu, timed_wait(bar.acc_empty + ab, abph ^ 1, err, pw[1], A.wait))) break;
-        sxn[(ab * 2 + hf) * kTcRows + r] = xs;
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar.xn_full + ab);
-        if (++ab == kTcAcc) ab = 0, abph ^= 1;
-      }
-    } else if (warp < kTmaWarp) {
-      // ---- epilogue: thread = row (its TMEM lane), warpgroup = column half
-      constexpr uint32_t CH = N / 2;  // columns per half
-      const uint32_t q4 = warp & 3, half = (warp - kConvWarps) >> 2;
-      const uint32_t row = q4 * 32 + lane;
-      uint32_t cph = CH, c0 = half * CH;  // columns per half and this half's first, per item
-      uint4 *rec = A.rec + static_cast<size_t>(blockIdx.x) * A.rec_cap;
-      uint32_t ab = 0, abph = 0, ib = 0, bph = 0;
-      unsigned long long tiles = 0, found = 0;
-      const uint32_t *qbv = reinterpret_cast<const uint32_t *>(sm + L.qbv);
-      for (; w.t < t1; ++w.t) {
-        w.step();
-        const QInfo *qi = qinfo + ib * N;
-        // waits are made warp-uniform: the warp-collective steps below need all lanes
-        if (w.first()) {
-          if (!__all_sync(0xffffffffu, timed_wait(bar.b_full + ib, bph, err, pw[0], A.wait))) break;
-          cph = mma_width<N>(swidth[ib]) / 2;
-          c0 = half * cph;
-        }
-        const uint32_t rin = (w.t - w.start) * kTcRows + row;
-        const bool valid = rin < w.cur.nrows;
-        const uint32_t grow = w.cur.row0 + rin;
-        if (!__all_sync(0xffffffffu, timed_wait(bar.acc_full + ab, abph, err, pw[1], A.wait) &&
-                                         timed_wait(bar.xn_full + ab, abph, err, pw[1], A.wait)))
-          break;
-        tc::fence_after();
-        const int32_t xn = sxn[ab * 2 * kTcRows + row] + sxn[(ab * 2 + 1) * kTcRows + row];
-        const uint32_t taddr = tmem + ((q4 * 32u) << 16) + ab * N;
-        const float xnf = static_cast<float>(xn);
-        // this warpgroup's columns: half of the item's MMA width. In groups
-        // of up to 16: load the group's accumulators and bounds, compare each
-        // pair (or-ed into one predicate), and resolve the columns only when
-        // the warp has a passing pair (rare)
-        auto process = [&](auto gsize, uint32_t g) {
-          constexpr uint32_t G = decltype(gsize)::value;
-          uint32_t d[G], qb[G];
-          if constexpr (G == 16) tc::tmem_ld16(taddr + c0 + g, d);
-          else tc::tmem_ld8(taddr + c0 + g, d);
+        if (inflight == 0) fetch();
+        const uint32_t ng = (d1.x + 7) / 8;
+        const uint32_t first = (t - d0.x) * kTcSlab, row = d0.z + first + g;
+        const int32_t left = static_cast<int32_t>(d0.w - first) - static_cast<int32_t>(g);
+        const uint32_t bq = b_a + c_bf * btile, slot = c_bf * N;
+        const uint32_t nch = d1.y;
+        const bool two = d0.w - first > kTcBoxRows;  // the slab's second half has rows
+        // one chunk: a stage is the slab's two halves, and the second is left
+        // out of a slab without it; several: two chunks of a half
+        const uint32_t halves = nch == 1 && !two ? 1 : 2;
+        uint32_t box = 0, half = 0;
+        uint32_t xn[4];
+        float xh[4];
+        // the half's 32 rows against groups g0 .. g0 + kG - 1. A group past the
+        // first ones meets the same rows again (one chunk then: N = 64 only
+        // with h <= 128)
+        auto score = [&](auto kg, uint32_t g0) -> bool {
+          constexpr uint32_t kG = decltype(kg)::value;
+          float c[kG][2][4];
 #pragma unroll
-          for (uint32_t j = 0; j < G; j += 4)
-            *reinterpret_cast<uint4 *>(qb + j) =
-                *reinterpret_cast<const uint4 *>(qbv + ib * N + c0 + g + j);
-          tc::tmem_wait_ld();
-          auto pass = [&](uint32_t j) -> bool {
-            if constexpr (kFloat)
-              return fmaf(-2.0f, __uint_as_float(d[j]), xnf) <= __uint_as_float(qb[j]);
-            else return xn - 2 * __float2int_rn(__uint_as_float(d[j])) <= static_cast<int32_t>(qb[j]);
-          };
-          bool hit = false;
+          for (uint32_t gr = 0; gr < kG; ++gr)
 #pragma unroll
-          for (uint32_t j = 0; j < G; ++j) hit |= pass(j);
-          hit = hit && valid;
-          if (__any_sync(0xffffffffu, hit)) {
-            uint32_t mask = 0;
+            for (uint32_t m = 0; m < 2; ++m)
 #pragma unroll
-            for (uint32_t j = 0; j < G; ++j) mask |= static_cast<uint32_t>(pass(j)) << j;
-            if (!valid) mask = 0;
-            // records (query, l2, row) go to this CTA's list: one shared slot
-            // reservation per warp (a warp scan of the lanes' hit counts),
-            // then each lane writes its own records; the per-query count is a
-            // fire-and-forget global add per record
-            const uint32_t mine = __popc(mask);
-            uint32_t incl = mine;
-#pragma unroll
-            for (uint32_t o = 1; o < 32; o <<= 1) {
-              const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-              if (lane >= o) incl += t;
+              for (uint32_t e = 0; e < 4; ++e) c[gr][m][e] = 0.0f;
+          for (uint32_t ch = 0;;) {
+            if (g0 == 0) {
+              if (box == 0 && !wait(bar + cs * 8, cph, pw[0])) return false;
+              read(ring + cs * kStage + box * kBox);
+              box = box || (nch == 1 ? halves == 1 : ch + 1 == nch) ? 0 : 1;
+              if (box == 0) release();
             }
-            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-            uint32_t at = 0;
-            if (lane == 0) {
-              at = atomicAdd(rcount, total);
-              found += total;
-            }
-            at = __shfl_sync(0xffffffffu, at, 0) + incl - mine;
-            while (mask) {
-              const uint32_t j = __ffs(mask) - 1;
-              mask &= mask - 1;
-              uint32_t dj = 0;
 #pragma unroll
-              for (uint32_t k = 0; k < G; ++k) dj = k == j ? d[k] : dj;
-              const QInfo q = qi[c0 + g + j];
-              atomicAdd(A.qcount + q.qid, 1u);
-              if (at < A.rec_cap) {
-                const int32_t l2 = q.qn + xn - 2 * __float2int_rn(__uint_as_float(dj));
-                rec[at] = make_uint4(q.qid, static_cast<uint32_t>(l2), grow, 0);
-              } else {
-                atomicOr(A.qcount + q.qid, kDropped);
-              }
-              ++at;
-            }
+            for (uint32_t s = 0; s < 2 * NI; ++s) step(kg, s, bq + g0 * 8 * brow + ch * IN * 2, c);
+            // the last chunk may hold 64 dimensions only
+            if (g0 == 0 && ((ch + 1) * IN <= h || ch * IN + tig * (IN / 4) < h)) norms(xn);
+            if (++ch == nch) break;
           }
+          if (g0 == 0) finish(xn, xh, left - static_cast<int32_t>(kTcBoxRows * half));
+#pragma unroll
+          for (uint32_t gr = 0; gr < kG; ++gr)
+            test(c[gr], xh, xn, slot + (g0 + gr) * 8, row + kTcBoxRows * half);
+          return true;
         };
-        if (cph == 8) {
-          process(std::integral_constant<uint32_t, 8>{}, 0);
-        } else if constexpr (CH >= 16) {
-          for (uint32_t g = 0; g < cph; g += 16) process(std::integral_constant<uint32_t, 16>{}, g);
-        }
-        // the slot's accumulators and row norms have been read: hand it back
-        tc::fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar.acc_empty + ab);
-        if (++ab == kTcAcc) ab = 0, abph ^= 1;
-        ++tiles;
-        if (w.last()) {
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(bar.b_empty + ib);
-          if (++ib == S.Bs) ib = 0, bph ^= 1;
-        }
-      }
-      if (lane == 0) {
-        if (half == 0 && q4 == 0) atomicAdd(A.counters, tiles);
-        if (found) atomicAdd(A.counters + 1, found);
-      }
-    } else if (warp == kTmaWarp) {
-      // ---- TMA producer
-      if (lane == 0) {
-        uint32_t rs = 0, rph = 0;
-        uint32_t issued = 0, last_par[4] = {0, 0, 0, 0};
-        for (; w.t < t1; ++w.t) {
-          w.step();
-          const int32_t y = static_cast<int32_t>(w.cur.row0 + (w.t - w.start) * kTcRows);
-          bool ok = true;
-          for (uint32_t kc = 0; kc < nkc; ++kc) {
-            if (!timed_wait(bar.raw_empty + rs, rph ^ 1, err, pw[0], A.wait)) {
-              ok = false;
-              break;
-            }
-            tc::mbar_expect_tx(bar.raw_full + rs, rtile);
-            tc::tma_load_2d(sm + L.raw + rs * rtile, &tmap, static_cast<int32_t>(kc * S.inner), y,
-                            bar.raw_full + rs);
-            issued |= 1u << rs;
-            last_par[rs] = rph;
-            if (++rs == S.Rs) rs = 0, rph ^= 1;
+#pragma unroll 1
+        for (; ok && half < halves; ++half) {
+          xn[0] = xn[1] = xn[2] = xn[3] = 0;
+          // a body for each count of groups: guarding every step of one for
+          // four costs 42 cycles of the 150 that two groups take
+#pragma unroll 1
+          for (uint32_t g0 = 0; ok && g0 < ng; g0 += 4) {
+            const uint32_t n = ng - g0;
+            ok = n >= 4   ? score(std::integral_constant<uint32_t, 4>{}, g0)
+                 : n == 1 ? score(std::integral_constant<uint32_t, 1>{}, g0)
+                 : n == 2 ? score(std::integral_constant<uint32_t, 2>{}, g0)
+                          : score(std::integral_constant<uint32_t, 3>{}, g0);
           }
-          if (!ok) break;
         }
-        if (*err)  // copies still in flight land before the CTA exits
-          for (uint32_t s = 0; s < S.Rs; ++s)
-            if (issued >> s & 1u) tc::mbar_wait(bar.raw_full + s, last_par[s]);
+        if (!ok) break;
+        if (lane == 0) atomicAdd(const_cast<uint32_t *>(slabs), 1u);
       }
+      // hand back the remaining items' buffers, so that the staging warps end
       __syncwarp();
-    } else if (warp == kMmaWarp) {
-      // ---- MMA issuer
-      if (lane == 0) {
-        uint32_t idesc = tc::idesc_f16(kTcRows, N);
-        uint32_t as = 0, aph = 0, ab = 0, abph = 0, ib = 0, bph = 0;
-        unsigned long long pi = 0;  // cycles issuing MMAs and commits
-        bool ok = true;
-        for (; ok && w.t < t1; ++w.t) {
-          w.step();
-          if (w.first()) {
-            if (!timed_wait(bar.b_full + ib, bph, err, pw[0], A.wait)) break;
-            idesc = tc::idesc_f16(kTcRows, mma_width<N>(swidth[ib]));  // the item's queries
-          }
-          if (!timed_wait(bar.acc_empty + ab, abph ^ 1, err, pw[1], A.wait)) break;
-          tc::fence_after();
-          const uint32_t bbase = tc::smem_addr(sm + L.b + ib * btile);
-          for (uint32_t kc = 0; kc < nkc; ++kc) {
-            if (!timed_wait(bar.a_full + as, aph, err, pw[2], A.wait)) {
-              ok = false;
-              break;
-            }
-            tc::fence_after();
-            const long long ti = clock64();
-            // A from TMEM (8 columns per 16-dimension step); B's descriptor
-            // advances 256 bytes (two core matrices), i.e. 16 encoded, per step
-            const uint32_t a0 = tmem + acol + as * (S.inner / 2);
-            const uint64_t bd0 = tc::desc(bbase + kc * S.inner * 16, 128, (h / 8) * 128);
-            const uint32_t steps = min(S.inner, h - kc * S.inner) / 16;
-            const uint32_t dcol = tmem + ab * N;
-#pragma unroll
-            for (uint32_t s = 0; s < 8; ++s)
-              if (s < steps) tc::mma_f16_ts(dcol, a0 + 8 * s, bd0 + 16 * s, idesc, (kc | s) != 0);
-            tc::commit(bar.a_empty + as);
-            pi += clock64() - ti;
-            if (++as == kTcAStages) as = 0, aph ^= 1;
-          }
-          if (!ok) break;
-          tc::commit(bar.acc_full + ab);
-          if (++ab == kTcAcc) ab = 0, abph ^= 1;
-          if (w.last()) {
-            tc::commit(bar.b_empty + ib);
-            if (++ib == S.Bs) ib = 0, bph ^= 1;
-          }
-        }
-        // every MMA issued has completed before tensor memory is released
-        tc::commit(bar.done);
-        tc::mbar_wait(bar.done, 0);
-        if (A.prof) atomicAdd(A.prof + 14, pi);
+      while (ok && !*err) {
+        if (c_n && lane == 0) tc::mbar_arrive(b_empty_a + c_bf * 8);
+        if (++c_n > n_li) break;
+        c_bf = c_bf + 1 == nB ? 0 : c_bf + 1;
+        c_ph ^= c_bf == 0;
+        ok = wait(b_full_a + c_bf * 8, c_ph, pw[1]);
       }
-      __syncwarp();
+      // copies still in flight land before the CTA exits
+      for (; inflight; --inflight) {
+        for (uint32_t i = 0; i < (1u << 26) && !tc::mbar_try(bar + cs * 8, cph); ++i) {
+        }
+        if (++cs == depth) cs = 0, cph ^= 1;
+      }
     } else {
-      // ---- query staging: thread j < N gathers query j of each item; each
-      // staging warp arrives once per item
-      const uint32_t j = tid - kQueryWarp0 * 32;
-      uint32_t ib = 0, bph = 0;
-      for (; w.t < t1; ++w.t) {
-        w.step();
-        if (!w.first()) continue;
-        if (!__all_sync(0xffffffffu, timed_wait(bar.b_empty + ib, bph ^ 1, err, pw[0], A.wait))) break;
-        if (j < N) {
-          const uint32_t e0 = A.off[w.cur.list] + w.cur.qfirst;
-          const uint32_t ne = min(N, A.off[w.cur.list + 1] - e0);
-          if (j == 0) swidth[ib] = ne;
-          unsigned char *b = sm + L.b + ib * btile;
-          QInfo q{0, 0, INT_MIN, -INFINITY};
-          if (j < ne) {
-            q.qid = A.entries[e0 + j] / A.nprobe;
-            const uint4 *src = reinterpret_cast<const uint4 *>(A.qhi + static_cast<size_t>(q.qid) * A.dc);
-            uint32_t s1 = 0;
-#pragma unroll 8
-            for (uint32_t u = 0; u < h / 16; ++u) {
-              const uint4 v = __ldg(src + u);
-              uint4 lo, hi;
-              tc::bytes_to_half16(v, bias, lo, hi);
-              *reinterpret_cast<uint4 *>(b + tc::canon_off(j, u * 16, h)) = lo;
-              *reinterpret_cast<uint4 *>(b + tc::canon_off(j, u * 16 + 8, h)) = hi;
-              s1 = dp4(v.x, 0x01010101u, dp4(v.y, 0x01010101u, dp4(v.z, 0x01010101u, dp4(v.w, 0x01010101u, s1))));
+      // ---- query staging: warp sw takes the CTA's items sw, sw + nB, ...
+      const uint32_t sw = warp - kScoreWarps;
+      const uint32_t b0 = tc::smem_addr(sm + L.b + sw * btile);
+      if (sw < nB) {
+        // loads run ahead: an item's queries while the one before it is
+        // copied, the description of the one after while both are
+        auto item_at = [&](uint32_t li) { return li < n_li ? A.items[it0 + li] : TcItem{0, 0, 0, 0}; };
+        auto slab_at = [&](uint32_t li) { return li <= n_li ? A.tile_off[it0 + li] : 0u; };
+        auto entry = [&](const TcItem &it, uint32_t j) { return j < it.ne ? A.entries[it.e0 + j] : 0u; };
+        TcItem cur = item_at(sw), nxt = item_at(sw + nB);
+        uint32_t s0 = slab_at(sw), s1 = slab_at(sw + 1);
+        uint32_t q0 = entry(cur, lane) / A.nprobe, q1 = entry(cur, lane + 32) / A.nprobe;
+        for (uint32_t li = sw, use = 0; li < n_li; li += nB, ++use) {
+          const uint32_t e0 = entry(nxt, lane), e1 = entry(nxt, lane + 32);
+          const uint32_t n0 = slab_at(li + nB), n1 = slab_at(li + nB + 1);
+          const TcItem nxt2 = item_at(li + 2 * nB);
+          const int2 cn0 = A.qcn[q0], cn1 = N > 32 ? A.qcn[q1] : make_int2(0, 0);
+          const int32_t bd0 = A.bound[q0], bd1 = N > 32 ? A.bound[q1] : 0;
+          if (!wait(b_empty_a + sw * 8, (use & 1) ^ 1, pw[0])) break;
+          // Filtered while few records come of it. A slab saves about 0.15 us
+          // of an SM against all of h = 256, and completing a record costs an
+          // SM about 5 ns (10M x 1,024: 3 records per slab), so: on while the
+          // CTA's slabs gave below 32 each, whatever their items were (a run
+          // of items that pass too much is paid back by the unfiltered ones
+          // after it). The first 8 slabs go ahead, the next await their count
+          bool filt = A.f < h;
+          if (filt) filt = *slabs >= 8 ? *reinterpret_cast<volatile uint32_t *>(rcount) <= 32 * *slabs : *fstaged < 8;
+          const uint32_t dims = filt ? A.f : h;
+          if (lane == 0) {
+            desc[sw] = Desc{s0, s1, cur.row0, cur.nrows, cur.ne, (dims + IN - 1) / IN, filt, 0};
+            tc::mbar_arrive(d_full + sw);
+            if (filt && *slabs < 8) atomicAdd(const_cast<uint32_t *>(fstaged), s1 - s0);
+          }
+          // the queries' fp16 rows, `per` 16-byte units each, the ids shuffled
+          const uint32_t per = (dims + IN - 1) / IN * (IN / 8), steps = (cur.ne * per + 31) / 32;
+          uint32_t j = lane / per, u = lane % per;
+          for (uint32_t i = 0; i < steps; ++i) {
+            const uint32_t ql = __shfl_sync(0xffffffffu, q0, j & 31);
+            const uint32_t qh = N > 32 ? __shfl_sync(0xffffffffu, q1, j & 31) : 0;
+            if (j < cur.ne) {
+              const uint32_t pos = IN == 128 ? (u ^ ((u >> 3) & 1) ^ ((j & 1) << 1)) : (u ^ (j & 1));
+              cp_async16(b0 + j * brow + pos * 16,
+                         A.qr16 + static_cast<size_t>(j < 32 ? ql : qh) * (brow / 2) + u * 8);
             }
-            // sum (q - 128)^2 = sum q^2 - 256 sum q + 16384 h
-            const int64_t qn = A.qnorm[q.qid] - 256 * static_cast<int64_t>(s1) + 16384ll * h;
-            q.qn = static_cast<int32_t>(qn);
-            q.qb = static_cast<int32_t>(static_cast<int64_t>(A.bound[q.qid]) - qn);
-            q.qbf = static_cast<float>(q.qb);
-          } else {
-            const uint4 zero = make_uint4(0, 0, 0, 0);  // fp16 zeros: a centred byte of 128
-            for (uint32_t u = 0; u < h / 16; ++u) {
-              *reinterpret_cast<uint4 *>(b + tc::canon_off(j, u * 16, h)) = zero;
-              *reinterpret_cast<uint4 *>(b + tc::canon_off(j, u * 16 + 8, h)) = zero;
+            for (u += 32; u >= per; u -= per) ++j;
+          }
+#pragma unroll
+          for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t slot = lane + 32 * k;
+            if (slot < N) {
+              // a slot without a query never passes (its row of the buffer may
+              // hold any bits, infinities among them)
+              const int2 cn = k ? cn1 : cn0;
+              const float qb = static_cast<float>(static_cast<int64_t>(filt ? cn.x : cn.y) - (k ? bd1 : bd0));
+              qids[sw * N + slot] = k ? q1 : q0;
+              qbv[sw * N + slot] = slot < cur.ne ? qb * (0.5f * kScale) : NAN;
             }
           }
-          qinfo[ib * N + j] = q;
-          reinterpret_cast<uint32_t *>(sm + L.qbv)[ib * N + j] =
-              kFloat ? __float_as_uint(q.qbf) : static_cast<uint32_t>(q.qb);
-          tc::fence_smem_to_async();
+          cp_async_arrive(b_full + sw);
+          tc::mbar_arrive(b_full + sw);
+          cur = nxt, nxt = nxt2, s0 = n0, s1 = n1;
+          q0 = e0 / A.nprobe, q1 = e1 / A.nprobe;
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar.b_full + ib);
-        if (++ib == S.Bs) ib = 0, bph ^= 1;
+        asm volatile("cp.async.wait_all;" ::: "memory");
       }
     }
   }
-  if (A.prof) {
-    // slots: converters 0-2, MMA 3-6, epilogue 7-9, TMA 10-11, staging 12-13
-    const int base = warp < kConvWarps ? 0 : warp < kTmaWarp ? 7 : warp == kTmaWarp ? 10
-                   : warp == kMmaWarp ? 3 : 12;
-    const int nw = base == 3 ? 3 : base == 10 || base == 12 ? 1 : 2;
-    const bool lead = tid == 0 || tid == kConvWarps * 32 || tid == kTmaWarp * 32 ||
-                      tid == kMmaWarp * 32 || tid == kQueryWarp0 * 32;
-    if (lead) {
-      for (int i = 0; i < nw; ++i) atomicAdd(A.prof + base + i, pw[i]);
-      atomicAdd(A.prof + base + nw, static_cast<unsigned long long>(clock64() - tstart));
-    }
+  if (A.prof && lane == 0 && (warp == 0 || warp == kScoreWarps)) {
+    // slots: first scoring warp's waits for rows, for items, its total; first
+    // staging warp's wait for a buffer, its total
+    const int base = warp == 0 ? 0 : 12;
+    atomicAdd(A.prof + base, pw[0]);
+    if (warp == 0) atomicAdd(A.prof + 1, pw[1]);
+    atomicAdd(A.prof + base + (warp == 0 ? 2 : 1), static_cast<unsigned long long>(clock64() - tstart));
   }
-  tc::fence_before();
   __syncthreads();
-  tc::fence_after();
   if (tid == 0) {
     if (*err) atomicAdd(A.timeouts, 1u);
     A.rec_n[blockIdx.x] = min(*rcount, A.rec_cap);
     // the longest CTA (cycles): against the average it shows the schedule's imbalance
     if (A.prof) atomicMax(A.prof + 15, static_cast<unsigned long long>(clock64() - tstart));
   }
-  if (warp == kMmaWarp) tc::tmem_dealloc(tmem, S.tcols);
 }
 
 // The squared L2 over the first h high bytes of a row and a query whose bytes
@@ -870,7 +876,7 @@ __device__ __forceinline__ void load_query_words(const uint8_t *qhi, uint32_t q,
 
 __global__ void __launch_bounds__(256) rescan_bound_kernel(
     const uint32_t *__restrict__ ids, uint32_t *__restrict__ qcount,
-    const uint32_t *__restrict__ qfill, const uint2 *__restrict__ qbuf, uint32_t cap, uint32_t S,
+    const uint2 *__restrict__ qbuf, uint32_t cap, uint32_t S,
     uint32_t round, uint32_t *__restrict__ list, unsigned long long *__restrict__ kbound,
     uint32_t *__restrict__ nlisted, unsigned long long *__restrict__ stats) {
   __shared__ uint32_t hist[256], sel[2];
@@ -879,10 +885,9 @@ __global__ void __launch_bounds__(256) rescan_bound_kernel(
   if (round == 0 && threadIdx.x == 0)
     atomicMax(stats + 1, static_cast<unsigned long long>(n & ~kDropped));
   if (n <= cap) return;
-  // entries actually in the buffer: the bucketing step's fill in round 0,
-  // the previous round's count after that
-  // (a subset's S-th smallest key is a bound as well: look at 2048 at most)
-  const uint32_t valid = min(min(round == 0 ? qfill[q] : n, cap), 2048u);
+  // entries actually in the buffer (a subset's S-th smallest key is a bound
+  // as well: look at 2048 at most)
+  const uint32_t valid = min(min(n & ~kDropped, cap), 2048u);
   const uint2 *buf = qbuf + static_cast<size_t>(q) * cap;
   const unsigned long long K =
       valid < S ? ~0ull
@@ -982,35 +987,35 @@ __global__ void __launch_bounds__(256) rescan_exact_kernel(
 }
 
 // -------------------------------------------------- work items and offsets
-// Per list: items = ceil(queries / N) (none for an empty list), tiles per
-// item = ceil(rows / 128); counts[c] = items, counts[L + 1 + c] = items x tiles.
-// MMA width of an item of ne queries (host and device, as mma_width<N>).
-__host__ __device__ __forceinline__ uint32_t item_width(uint32_t ne, uint32_t N) {
-  return ne <= 16 ? 16u : (ne <= 32 && N > 32 ? 32u : N);
+// The cost of a slab of an item of ne queries: by default in steps of about
+// 20 instructions (180 for the rows and 40 per group of 8 queries), or
+// 64 + beta * width (16, 32 or N queries).
+__device__ __forceinline__ uint32_t slab_cost(uint32_t ne, uint32_t N, uint32_t beta) {
+  if (beta == 0) return 9 + 2 * ((ne + 7) / 8);
+  return 64 + beta * (ne <= 16 ? 16u : (ne <= 32 && N > 32 ? 32u : N));
 }
 
+// Per list: items = ceil(queries / N) (none for an empty list), slabs per
+// item = ceil(rows / 64); counts[c] = items, counts[L + 1 + c] = items x slabs.
 // probed (optional, 2 counters): the distinct lists the batch probes (not
 // empty) and their rows, i.e. the rows the pass reads once each.
 __global__ void tc_count_kernel(const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ list_off,
-                                uint32_t L, uint32_t N, uint32_t B, uint32_t beta,
+                                uint32_t L, uint32_t N, uint32_t B, uint32_t beta, bool cost,
                                 uint32_t *__restrict__ counts, uint32_t *__restrict__ qcount,
-                                uint32_t *__restrict__ qfill, unsigned long long *__restrict__ probed) {
+                                unsigned long long *__restrict__ probed) {
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < B) {
-    qcount[c] = 0;
-    qfill[c] = 0;
-  }
+  if (c < B) qcount[c] = 0;
   uint32_t lists = 0, rows = 0;
   if (c < L) {
     const uint32_t n = list_off[c + 1] - list_off[c];
     const uint32_t items = n ? (cnt[c] + N - 1) / N : 0;
-    const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
+    const uint32_t slabs = (n + kTcSlab - 1) / kTcSlab;
     counts[c] = items;
-    counts[L + 1 + c] = items * tiles;
-    if (beta) {  // full items first, then the remainder
+    counts[L + 1 + c] = items * slabs;
+    if (cost) {  // full items first, then the remainder
       const uint32_t full = n ? cnt[c] / N : 0, rem = n ? cnt[c] % N : 0;
       counts[2 * (L + 1) + c] =
-          tiles * (full * (64 + beta * N) + (rem ? 64 + beta * item_width(rem, N) : 0));
+          slabs * (full * slab_cost(N, N, beta) + (rem ? slab_cost(rem, N, beta) : 0));
     }
     if (items) lists = 1, rows = n;
   }
@@ -1024,12 +1029,12 @@ __global__ void tc_count_kernel(const uint32_t *__restrict__ cnt, const uint32_t
   }
 }
 
-// Exclusive scans of the two count arrays by one CTA of 1024 threads (in
-// place); the totals go to *nitems and tile_off[*nitems].
+// Exclusive scans of the count arrays by one CTA of 1024 threads (in place),
+// with the totals after them; the totals also end the slab offsets and the
+// shares (tile_off[items] and share[ctas]).
 __global__ void __launch_bounds__(1024) tc_scan_kernel(uint32_t *__restrict__ counts, uint32_t L,
-                                                       uint32_t *__restrict__ nitems,
-                                                       uint32_t *__restrict__ tile_off,
-                                                       uint32_t *__restrict__ cost_off) {
+                                                       bool by_cost, uint32_t *__restrict__ tile_off,
+                                                       uint2 *__restrict__ share, uint32_t ctas) {
   uint32_t *ca = counts, *cb = counts + L + 1, *cc = counts + 2 * (L + 1);
   const uint2 tot = block_scan2(
       L, [&](uint32_t i) { return make_uint2(ca[i], cb[i]); },
@@ -1037,8 +1042,8 @@ __global__ void __launch_bounds__(1024) tc_scan_kernel(uint32_t *__restrict__ co
         ca[i] = a;
         cb[i] = b;
       });
-  uint32_t cost = 0;
-  if (cost_off) {
+  uint32_t cost = tot.y;
+  if (by_cost) {
     __syncthreads();
     cost = block_scan2(
                L, [&](uint32_t i) { return make_uint2(cc[i], 0u); },
@@ -1046,62 +1051,134 @@ __global__ void __launch_bounds__(1024) tc_scan_kernel(uint32_t *__restrict__ co
                .x;
   }
   if (threadIdx.x == 0) {
-    *nitems = tot.x;
+    ca[L] = tot.x;
+    cb[L] = tot.y;
+    cc[L] = cost;
     tile_off[tot.x] = tot.y;
-    if (cost_off) cost_off[tot.x] = cost;
   }
+  // no work: every share is empty (the shares' starts come with the items)
+  if (tot.x == 0)
+    for (uint32_t i = threadIdx.x; i <= ctas; i += blockDim.x) share[i] = make_uint2(0, 0);
+  else if (threadIdx.x == 0) share[ctas] = make_uint2(tot.y, tot.x);
 }
 
-// tile_hist (optional, 6 counters): the tiles of the items with 1-2, 3-4,
-// 5-8, 9-16, 17-32 and 33-64 queries.
+// tile_hist (optional, 6 counters): the 128-row tiles of the items with 1-2,
+// 3-4, 5-8, 9-16, 17-32 and 33-64 queries; all_tiles: their sum.
 __global__ void tc_expand_kernel(const uint32_t *__restrict__ list_off, const uint32_t *__restrict__ counts,
-                                 const uint32_t *__restrict__ cnt, uint32_t L, uint32_t N,
-                                 uint32_t beta, const uint32_t *__restrict__ nitems,
+                                 const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ off,
+                                 uint32_t L, uint32_t N, uint32_t beta, bool by_cost, uint32_t ctas,
                                  TcItem *__restrict__ items, uint32_t *__restrict__ tile_off,
-                                 uint32_t *__restrict__ cost_off,
-                                 unsigned long long *__restrict__ tile_hist) {
+                                 uint2 *__restrict__ share, unsigned long long *__restrict__ tile_hist,
+                                 unsigned long long *__restrict__ all_tiles) {
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t hist[6] = {0, 0, 0, 0, 0, 0};
+  const uint32_t *unit = counts + (by_cost ? 2 : 1) * (L + 1);  // a list's first unit
+  if (c < ctas && unit[L]) {
+    // share c starts at unit total * c / ctas: the list that holds it, then
+    // the item (every one before a list's last is full) and the slab
+    const uint32_t u = static_cast<uint32_t>(static_cast<uint64_t>(unit[L]) * c / ctas);
+    uint32_t lo = 0, hi = L;  // unit[lo] <= u < unit[hi]
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (unit[mid] <= u) lo = mid;
+      else hi = mid;
+    }
+    const uint32_t slabs = (list_off[lo + 1] - list_off[lo] + kTcSlab - 1) / kTcSlab;
+    const uint32_t full = slabs * (by_cost ? slab_cost(N, N, beta) : 1), in = u - unit[lo];
+    const uint32_t j = min(in / full, (cnt[lo] - 1) / N);
+    const uint32_t per = by_cost ? slab_cost(min(N, cnt[lo] - j * N), N, beta) : 1;
+    share[c] = make_uint2(counts[L + 1 + lo] + j * slabs + (in - j * full) / per, counts[lo] + j);
+  }
   if (c < L) {
-    const uint32_t i0 = counts[c], i1 = c + 1 < L ? counts[c + 1] : *nitems;
-    const uint32_t tiles = (list_off[c + 1] - list_off[c] + kTcRows - 1) / kTcRows;
+    const uint32_t i0 = counts[c], i1 = counts[c + 1];
+    const uint32_t row0 = list_off[c], rows = list_off[c + 1] - row0;
+    const uint32_t slabs = (rows + kTcSlab - 1) / kTcSlab, tiles = (rows + kTcRows - 1) / kTcRows;
     const uint32_t tb = counts[L + 1 + c];
     for (uint32_t j = 0; j < i1 - i0; ++j) {
-      items[i0 + j] = TcItem{c, j * N, list_off[c], list_off[c + 1] - list_off[c]};
-      tile_off[i0 + j] = tb + j * tiles;
-      // every item before the last of its list is full (width N)
-      if (cost_off) cost_off[i0 + j] = counts[2 * (L + 1) + c] + j * tiles * (64 + beta * N);
       const uint32_t ne = min(N, cnt[c] - j * N);
+      items[i0 + j] = TcItem{off[c] + j * N, ne, row0, rows};
+      tile_off[i0 + j] = tb + j * slabs;
       hist[ne <= 2 ? 0 : ne <= 4 ? 1 : ne <= 8 ? 2 : ne <= 16 ? 3 : ne <= 32 ? 4 : 5] += tiles;
     }
   }
   if (tile_hist) {  // whole warps take part: one add per warp and bin
+    uint32_t all = 0;
 #pragma unroll
     for (int b = 0; b < 6; ++b) {
       const uint32_t v = __reduce_add_sync(0xffffffffu, hist[b]);
       if ((threadIdx.x & 31) == 0 && v) atomicAdd(tile_hist + b, static_cast<unsigned long long>(v));
+      all += v;
     }
+    if ((threadIdx.x & 31) == 0 && all) atomicAdd(all_tiles, static_cast<unsigned long long>(all));
   }
 }
 
-// The pass's candidate records (query, l2, row) into per-query buffers of
-// (distance bits, row); one CTA per pass CTA.
-__global__ void __launch_bounds__(512) tc_bucket_kernel(const uint4 *__restrict__ rec,
-                                                        const uint32_t *__restrict__ rec_n,
-                                                        uint32_t rec_cap, uint32_t *__restrict__ qfill,
-                                                        uint2 *__restrict__ qbuf, uint32_t cap,
-                                                        DistScale scale) {
-  // gridDim.y CTAs share each ranking CTA's list, so that enough records
-  // (each a global atomic and a scattered store) are in flight per SM
+// The pass's candidate records (query, xn - 2 dot, row, partial) into per-query
+// buffers of (distance bits, row); gridDim.y CTAs share each ranking CTA's
+// list, so that enough records (each a global atomic and a scattered store)
+// are in flight per SM. A partial record covers the first f dimensions:
+// eight lanes add the rest, 16 bytes of the row and of the query each, with
+// the loads of a warp's 32 records in flight together.
+__global__ void __launch_bounds__(256) tc_bucket_kernel(
+    const uint4 *__restrict__ rec, const uint32_t *__restrict__ rec_n, uint32_t rec_cap,
+    const uint8_t *__restrict__ xhi, const uint8_t *__restrict__ qhi, const int2 *__restrict__ qcn,
+    const int32_t *__restrict__ bound, uint32_t dc, uint32_t f, uint32_t h,
+    uint32_t *__restrict__ qcount, uint2 *__restrict__ qbuf, uint32_t cap, DistScale scale,
+    unsigned long long *__restrict__ found) {
   const uint4 *r = rec + static_cast<size_t>(blockIdx.x) * rec_cap;
-  const uint32_t n = rec_n[blockIdx.x];
-  for (uint32_t i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x) {
-    const uint4 e = r[i];
-    const uint32_t at = atomicAdd(qfill + e.x, 1u);
-    if (at < cap)
-      qbuf[static_cast<size_t>(e.x) * cap + at] =
-          make_uint2(__float_as_uint(dist_value(static_cast<int32_t>(e.y), scale)), e.z);
+  const uint32_t n = rec_n[blockIdx.x], lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
+  const uint32_t nw = gridDim.y * (blockDim.x >> 5);
+  uint32_t kept = 0;
+  for (uint32_t i0 = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; i0 < n;
+       i0 += nw * 32) {
+    const bool valid = i0 + lane < n;
+    const uint4 e = valid ? r[i0 + lane] : make_uint4(0, 0, 0, 0);
+    const int2 cn = valid ? qcn[e.x] : make_int2(0, 0);
+    int32_t l2 = static_cast<int32_t>(e.y) + (e.w ? cn.x : cn.y);
+    if (__any_sync(0xffffffffu, e.w != 0)) {
+      uint32_t tail = 0;
+      for (uint32_t u0 = f / 16; u0 < h / 16; u0 += 8) {
+        const bool in = u0 + gl < h / 16;
+        uint4 x[8], q[8];
+#pragma unroll
+        for (uint32_t it = 0; it < 8; ++it) {
+          const uint32_t src = it * 4 + grp;
+          const uint32_t eq = __shfl_sync(0xffffffffu, e.x, src), er = __shfl_sync(0xffffffffu, e.z, src);
+          const bool on = __shfl_sync(0xffffffffu, e.w, src) != 0 && in;
+          x[it] = on ? __ldg(reinterpret_cast<const uint4 *>(xhi + static_cast<size_t>(er) * dc) + u0 + gl)
+                     : make_uint4(0, 0, 0, 0);
+          q[it] = on ? __ldg(reinterpret_cast<const uint4 *>(qhi + static_cast<size_t>(eq) * dc) + u0 + gl)
+                     : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (uint32_t it = 0; it < 8; ++it) {
+          const uint32_t a[4] = {x[it].x, x[it].y, x[it].z, x[it].w};
+          const uint32_t b[4] = {q[it].x, q[it].y, q[it].z, q[it].w};
+          uint32_t sq = 0, xq = 0;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            sq = dp4(a[w], a[w], dp4(b[w], b[w], sq));
+            xq = dp4(a[w], b[w], xq);
+          }
+          uint32_t d2 = sq - 2 * xq;
+#pragma unroll
+          for (uint32_t o = 1; o < 8; o <<= 1) d2 += __shfl_xor_sync(0xffffffffu, d2, o);
+          const uint32_t t = __shfl_sync(0xffffffffu, d2, (lane & 3) * 8);
+          if (lane >> 2 == it) tail += t;
+        }
+      }
+      l2 += static_cast<int32_t>(tail);
+    }
+    const bool keep = valid && l2 <= bound[e.x];
+    kept += __popc(__ballot_sync(0xffffffffu, keep));
+    if (keep) {
+      const uint32_t at = atomicAdd(qcount + e.x, 1u) & ~kDropped;
+      if (at < cap)
+        qbuf[static_cast<size_t>(e.x) * cap + at] =
+            make_uint2(__float_as_uint(dist_value(l2, scale)), e.z);
+    }
   }
+  if (lane == 0 && kept) atomicAdd(found, static_cast<unsigned long long>(kept));
 }
 
 }  // namespace
@@ -1118,23 +1195,23 @@ std::atomic<unsigned long long> g_tc_wait{0};
 bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s) {
   if (h == 0 || h % 64 || h > 1024 || h > dc || dc % 64) return false;
   TcShape t{};
-  t.N = h <= 256 ? 64 : (h <= 512 ? 32 : 16);
+  // items narrow as the queries' rows widen, so that several query buffers fit
+  t.N = h <= 128 ? 64 : (h <= 512 ? 32 : 16);
   const uint32_t cap = g_tc_width.load();
   if (cap >= 16 && cap < t.N) t.N = cap;
-  t.inner = dc >= 128 ? 128 : 64;
-  // accumulators (kTcAcc slots of N columns), then the A stages (inner / 2 columns each)
-  t.tcols = 32;
-  while (t.tcols < kTcAcc * t.N + kTcAStages * t.inner / 2) t.tcols <<= 1;
-  for (uint32_t bs = 2; bs >= 1; --bs)
-    for (uint32_t rs = 4; rs >= 2; --rs) {
-      t.Bs = bs;
-      t.Rs = rs;
-      t.smem = tc_smem_layout(h, t).total;
-      if (t.smem <= 227 * 1024) {
-        *s = t;
-        return true;
-      }
+  t.inner = h == 64 ? 64 : 128;
+  t.f = std::min(h, kTcFilterDims);
+  t.centred = h > 256;
+  constexpr uint32_t shapes[][2] = {{4, 4}, {4, 2}, {3, 2}, {2, 2}, {1, 2}};
+  for (const auto &b : shapes) {
+    t.Bs = b[0];
+    t.Rs = b[1];
+    t.smem = tc_smem_layout(h, t).total;
+    if (t.smem <= 227 * 1024) {
+      *s = t;
+      return true;
     }
+  }
   return false;
 }
 
@@ -1146,12 +1223,14 @@ int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShap
   CUtensorMap tmap;
   const cuuint64_t dims[2] = {A.dc, npts};
   const cuuint64_t strides[1] = {A.dc};
-  const cuuint32_t box[2] = {s.inner, kTcRows};
+  const cuuint32_t box[2] = {s.inner, kTcBoxRows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult cr = encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(xhi), dims,
                              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                              s.inner == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                             s.inner == 128 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B
+                                            : CU_TENSOR_MAP_L2_PROMOTION_L2_64B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (cr != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed for the high-byte plane (error " + std::to_string(cr) + ")");
     return KATO_ERUNTIME;
@@ -1165,16 +1244,16 @@ int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShap
     KATO_LAUNCHED("rank_tc_kernel");
     return KATO_OK;
   };
-  // the float comparison is exact while |xn' - 2 dot'| < 2^24: h <= 320
-  if (s.N == 64) return go(rank_tc_kernel<64, true>);
-  if (s.N == 32) return A.h <= 320 ? go(rank_tc_kernel<32, true>) : go(rank_tc_kernel<32, false>);
-  if (s.N == 16) return go(rank_tc_kernel<16, false>);
-  return invalid("unsupported ranking shape");
+  if (s.inner == 64) return go(rank_tc_kernel<64, false>);
+  return s.centred ? go(rank_tc_kernel<128, true>) : go(rank_tc_kernel<128, false>);
 }
 
-int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas,
-                   uint32_t *qfill, uint2 *qbuf, uint32_t cap, DistScale scale, cudaStream_t st) {
-  tc_bucket_kernel<<<dim3(ctas, 4), 512, 0, st>>>(rec, rec_n, rec_cap, qfill, qbuf, cap, scale);
+int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas, uint32_t nq,
+                   const uint8_t *xhi, const uint8_t *qhi, const int2 *qcn, const int32_t *bound,
+                   uint32_t dc, uint32_t f, uint32_t h, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
+                   DistScale scale, unsigned long long *found, cudaStream_t st) {
+  tc_bucket_kernel<<<dim3(ctas, nq < 512 ? 1 : 8), 256, 0, st>>>(rec, rec_n, rec_cap, xhi, qhi, qcn, bound, dc, f, h,
+                                                  qcount, qbuf, cap, scale, found);
   KATO_LAUNCHED("tc_bucket_kernel");
   return KATO_OK;
 }
@@ -1203,17 +1282,16 @@ int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, cons
   return KATO_OK;
 }
 
-int rank_tc_prepare(const uint32_t *cnt, const uint32_t *list_off, uint32_t L, uint32_t N,
-                    uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
-                    uint32_t *tile_off, uint32_t *cost_off, uint32_t *nitems, uint32_t *qcount,
-                    uint32_t *qfill, unsigned long long *tile_hist, cudaStream_t st) {
-  uint32_t *co = beta ? cost_off : nullptr;
+int rank_tc_prepare(const uint32_t *cnt, const uint32_t *off, const uint32_t *list_off, uint32_t L,
+                    uint32_t N, uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
+                    uint32_t *tile_off, bool by_cost, uint2 *share, uint32_t ctas, uint32_t *qcount,
+                    unsigned long long *tile_hist, unsigned long long *tiles, cudaStream_t st) {
   // the distinct probed lists and rows go to the two counters after the histogram
   tc_count_kernel<<<div_up(std::max(std::max(L, B), 1u), 256), 256, 0, st>>>(
-      cnt, list_off, L, N, B, beta, scratch, qcount, qfill, tile_hist ? tile_hist + 6 : nullptr);
-  tc_scan_kernel<<<1, 1024, 0, st>>>(scratch, L, nitems, tile_off, co);
-  tc_expand_kernel<<<div_up(L, 256), 256, 0, st>>>(list_off, scratch, cnt, L, N, beta, nitems,
-                                                   items, tile_off, co, tile_hist);
+      cnt, list_off, L, N, B, beta, by_cost, scratch, qcount, tile_hist ? tile_hist + 6 : nullptr);
+  tc_scan_kernel<<<1, 1024, 0, st>>>(scratch, L, by_cost, tile_off, share, ctas);
+  tc_expand_kernel<<<div_up(std::max(L, ctas), 256), 256, 0, st>>>(list_off, scratch, cnt, off, L, N, beta, by_cost,
+                                                   ctas, items, tile_off, share, tile_hist, tiles);
   KATO_LAUNCHED("ranking work preparation");
   return KATO_OK;
 }
@@ -1230,7 +1308,7 @@ int rank_overflow(const uint8_t *xhi, const int64_t *xnorm, const uint32_t *ids,
   const RowKey key{xhi, xnorm, ids, dc, h, scale};
   KATO_CUDA(cudaMemsetAsync(rb.nlisted, 0, kRescanRounds * sizeof(uint32_t), st));
   for (int r = 0; r < kRescanRounds; ++r) {
-    rescan_bound_kernel<<<B, 256, 0, st>>>(ids, qcount, rb.qfill, qbuf, cap, S, r, rb.list,
+    rescan_bound_kernel<<<B, 256, 0, st>>>(ids, qcount, qbuf, cap, S, r, rb.list,
                                            rb.kbound, rb.nlisted + r, stats);
     rescan_rows_kernel<<<4 * sms, 256, 0, st>>>(key, qhi, qnorm, probed, qprobes, list_off, p,
                                                 qcount, qbuf, cap, rb.list, rb.kbound,

@@ -2,6 +2,8 @@
 // search orchestration (search.cu).
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include <atomic>
 
 #include <cstdint>
@@ -10,43 +12,50 @@
 
 namespace kato {
 
-// One work item: a list and up to N of the queries that probe it (probe
-// entries [off[list] + qfirst, +N)); its tiles are the list's rows, 128 each.
+// One work item: a list's rows [row0, +nrows) and up to N of the queries that
+// probe it (probe entries [e0, +ne)); its slabs are the rows, 64 each.
 struct TcItem {
-  uint32_t list, qfirst, row0, nrows;
+  uint32_t e0, ne, row0, nrows;
 };
 
 struct RankTcArgs {
-  const uint8_t *qhi;        // B x dc query high bytes
-  const int64_t *qnorm;      // per query: sum of squared high bytes over the h ranking dimensions
+  const __half *qr16;        // B query rows of the ranking bytes in fp16, zero-padded to chunks
+  const int2 *qcn;           // per query: sums of its squared values over f and over h dimensions
   const uint32_t *entries;   // probe slots (query * nprobe + rank) grouped by list
-  const uint32_t *off;       // nlist + 1
   const TcItem *items;
-  const uint32_t *tile_off;  // per item: first global tile; [nitems] = total tiles
-  const uint32_t *cost_off;  // per item: first cost unit; [nitems] = total (null: split by tiles)
-  const uint32_t *nitems;
+  const uint32_t *tile_off;  // per item: first global slab; [nitems] = total slabs
+  const uint2 *share;        // per CTA and one more: its first slab and that slab's item
   const int32_t *bound;      // per query: rows with a larger l2 cannot be selected
-  uint32_t *qcount;          // per query: candidates found (bit 31: some were dropped)
-  uint4 *rec;                // per CTA: rec_cap candidate records (query, l2, row)
+  uint32_t *qcount;          // per query: bit 31 is set when a record was dropped
+  uint4 *rec;                // per CTA: rec_cap records (query, xn - 2 dot, row, partial)
   uint32_t *rec_n;           // per CTA: records written
   uint32_t rec_cap;
   uint32_t *timeouts;        // CTAs whose bounded pipeline wait ran out
-  unsigned long long *counters;  // [0] 128-row tiles scored, [1] candidates found
-  unsigned long long *prof;      // optional: 14 cycle counters of the warp roles
-  uint32_t dc, h, nprobe;
+  unsigned long long *prof;  // optional: cycle counters of the warp roles
+  // f: dimensions of a filtered item (h: no item is filtered)
+  uint32_t dc, h, f, nprobe;
   long long wait;            // cycles a pipeline wait may take before the CTA gives up
-  DistScale scale;
 };
 
-// Launch shape: N queries per item (the MMA's N), Bs query buffers, Rs
-// raw-tile stages of `inner` bytes per row, TMEM columns.
+// Launch shape: N queries per item, Bs query buffers, Rs ring stages per
+// scoring warp of `inner` bytes per row, f filter dimensions.
 struct TcShape {
-  uint32_t N, Bs, Rs, inner, smem, tcols;
+  uint32_t N, Bs, Rs, inner, f, smem;
+  uint32_t centred;  // values enter as (byte - 128), not as the byte
+};
+
+// What centre_planes also makes of a batch's queries for the ranking pass
+// (rows null: nothing): their first h high bytes as fp16, centred or not,
+// zero-padded to `width`, and the sums of the squared values over f and h.
+struct RankRows {
+  __half *rows;
+  int2 *norms;
+  uint32_t f, h, width, centred;
 };
 
 // Shared-memory carve-up of the ranking CTA.
 struct TcSmem {
-  uint32_t raw, a, b, qinfo, qbv, width, sxn, bars, tbase, err, rcount, total;
+  uint32_t raw, b, qids, qbv, desc, bars, err, rcount, total;
 };
 
 __host__ __device__ inline uint32_t tc_take(uint32_t &o, uint32_t bytes, uint32_t align) {
@@ -56,29 +65,33 @@ __host__ __device__ inline uint32_t tc_take(uint32_t &o, uint32_t bytes, uint32_
   return at;
 }
 
-constexpr uint32_t kTcRows = 128;                        // rows per tile (the MMA's M)
-// Two A stages and two accumulators: four A stages (TMEM has the columns)
-// measured no faster at 10M (1.234 against 1.221 ms for the pass).
-constexpr uint32_t kTcAStages = 2;                       // converted row chunks (TMEM)
-constexpr uint32_t kTcAcc = 2;                           // accumulator slots (TMEM)
-constexpr uint32_t kTcATile = kTcRows * 128 * 2;         // 128 rows x 128 dims of fp16
-constexpr uint32_t kTcQInfo = 16;                        // bytes per query slot
-constexpr uint32_t kTcBars = 8 + 2 * kTcAStages + 4 + 3 * kTcAcc + 1;  // barrier slots
+constexpr uint32_t kTcRows = 128;     // rows per tile of the statistics
+// Dimensions of a filtered item: one chunk of 128 bytes per row.
+constexpr uint32_t kTcFilterDims = 128;
+constexpr uint32_t kTcBoxRows = 32;   // rows per TMA box: two mma row tiles
+constexpr uint32_t kTcSlab = 64;      // rows per slab
+constexpr uint32_t kTcScoreWarps = 8;
+constexpr uint32_t kTcMaxStages = 4;  // ring stages per scoring warp, at most
+constexpr uint32_t kTcMaxBufs = 4;    // query buffers, at most
+constexpr uint32_t kTcDesc = 32;      // bytes per item description
+
+// fp16 values of a query's row in RankTcArgs::qr16.
+__host__ __device__ inline uint32_t tc_qrow(uint32_t h, const TcShape &s) {
+  return (h + s.inner - 1) / s.inner * s.inner;
+}
 
 __host__ __device__ inline TcSmem tc_smem_layout(uint32_t h, const TcShape &s) {
   TcSmem L{};
   uint32_t o = 0;
-  L.raw = tc_take(o, s.Rs * kTcRows * s.inner, 1024);
-  L.a = tc_take(o, 0, 1024);  // the A stages live in tensor memory
-  L.b = tc_take(o, s.Bs * s.N * h * 2, 128);
-  L.qinfo = tc_take(o, s.Bs * s.N * kTcQInfo, 16);
+  const uint32_t brow = tc_qrow(h, s) * 2;
+  L.raw = tc_take(o, kTcScoreWarps * s.Rs * kTcSlab * s.inner, 1024);
+  L.b = tc_take(o, s.Bs * s.N * brow, 128);
+  L.qids = tc_take(o, s.Bs * s.N * 4, 16);
   L.qbv = tc_take(o, s.Bs * s.N * 4, 16);
-  L.width = tc_take(o, 2 * 4, 16);
-  L.sxn = tc_take(o, kTcAcc * 2 * kTcRows * 4, 16);
-  L.bars = tc_take(o, kTcBars * 8, 8);
-  L.tbase = tc_take(o, 4, 4);
+  L.desc = tc_take(o, kTcMaxBufs * kTcDesc, 16);
+  L.bars = tc_take(o, (kTcScoreWarps * kTcMaxStages + 3 * kTcMaxBufs) * 8, 8);
   L.err = tc_take(o, 4, 4);
-  L.rcount = tc_take(o, 4, 4);
+  L.rcount = tc_take(o, 3 * 4, 4);
   L.total = (o + 127) / 128 * 128;
   return L;
 }
@@ -95,25 +108,30 @@ int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, cons
               const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off,
               uint32_t L, uint32_t B, uint32_t p, uint32_t dc, uint32_t h, uint32_t S,
               uint32_t rows, uint32_t *order, int32_t *bound, cudaStream_t st);
-// Work items of the pass (per list: groups of N queries) and their tile
-// offsets; also zeroes the B candidate counts and buffer fills. With
-// beta > 0, also per-item cost offsets: a tile of an item of MMA width w
-// costs 64 + beta * w, and the CTAs split the cost instead of the tiles.
-// scratch: 3 x (L + 1) words.
-int rank_tc_prepare(const uint32_t *cnt, const uint32_t *list_off, uint32_t L, uint32_t N,
-                    uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
-                    uint32_t *tile_off, uint32_t *cost_off, uint32_t *nitems, uint32_t *qcount,
-                    uint32_t *qfill, unsigned long long *tile_hist, cudaStream_t st);
+// Work items of the pass (per list: groups of N queries) and their slab
+// offsets, and each CTA's share: an equal count of slabs, or of their cost
+// (by_cost: what a slab's instructions do with beta 0, or 64 + beta * w for an
+// item of width w, 16, 32 or N queries). Also zeroes the B candidate counts.
+// off: the lists' first probe entries. scratch: 3 x (L + 1) words.
+// tile_hist (optional): 6 counters of 128-row tiles by item width, then the
+// distinct probed lists and their rows; tiles: all tiles.
+int rank_tc_prepare(const uint32_t *cnt, const uint32_t *off, const uint32_t *list_off, uint32_t L,
+                    uint32_t N, uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
+                    uint32_t *tile_off, bool by_cost, uint2 *share, uint32_t ctas, uint32_t *qcount,
+                    unsigned long long *tile_hist, unsigned long long *tiles, cudaStream_t st);
 // Process-wide knobs of the pass (0 = default): the largest item width and
 // the cost weight of the CTA split.
 extern std::atomic<uint32_t> g_tc_width, g_tc_beta;
 // The pass's bounded pipeline waits give up after this many cycles (0: the
 // default of 4e9, about 2 s); a CTA that gives up is counted in stats[3].
 extern std::atomic<unsigned long long> g_tc_wait;
-// Candidate records of the pass into per-query buffers of cap entries
-// (distance bits, row); qfill counts the entries each query was offered.
-int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas,
-                   uint32_t *qfill, uint2 *qbuf, uint32_t cap, DistScale scale, cudaStream_t st);
+// Candidate records of the pass, completed over dimensions [f, h) where they
+// are partial, into per-query buffers of cap entries (distance bits, row);
+// qcount counts the candidates of each query and *found all of them.
+int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas, uint32_t nq,
+                   const uint8_t *xhi, const uint8_t *qhi, const int2 *qcn, const int32_t *bound,
+                   uint32_t dc, uint32_t f, uint32_t h, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
+                   DistScale scale, unsigned long long *found, cudaStream_t st);
 // CTAs of rank_tc (one per SM).
 uint32_t rank_tc_ctas();
 
@@ -123,7 +141,6 @@ struct RescanBufs {
   uint32_t *list;
   unsigned long long *kbound;
   uint32_t *nlisted;
-  const uint32_t *qfill;  // entries the buffers were offered by the bucketing step
 };
 constexpr uint32_t kRescanCounters = 4;
 

@@ -676,7 +676,8 @@ int sq16_tiles(const uint8_t *qhi, const uint8_t *qlo, const uint8_t *xhi, const
                uint32_t dims, uint32_t qstride, uint32_t xstride, float *out, bool full,
                cudaStream_t st);
 int centre_planes(const uint8_t *hi, const uint8_t *lo, const int64_t *norm, uint32_t rows,
-                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, cudaStream_t st);
+                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, const RankRows &rr,
+                  cudaStream_t st);
 bool coarse_tc_ok(uint32_t dc);
 int coarse_tc(const __half *ch, const __half *cl, const int64_t *cterm, uint32_t n, const __half *qh,
               const __half *ql, const int64_t *qterm, uint32_t m, uint32_t dc, double step_sq,
@@ -720,11 +721,12 @@ struct Plan {
   bool coarse_tc;                   // tensor-core coarse product
   TcShape tcs;
   uint32_t tcitems, cap, seed_rows, ctas, rec_cap, beta;
+  bool cost;                        // the ranking CTAs split the slabs' cost, not their count
   size_t off_fq, off_qhi, off_qlo, off_qn, off_qhn, off_qh0, off_cd, off_probed, off_cnt, off_off,
       off_woff, off_cur, off_work, off_ent, off_slots, off_surv, off_nsurv, off_stats,
-      off_tcscratch, off_tcitems, off_tileoff, off_nitems, off_qcount, off_qfill, off_bound,
+      off_tcscratch, off_tcitems, off_tileoff, off_qcount,  off_bound,
       off_rec, off_recn, off_rlist, off_rkey, off_rcount, off_qh16, off_ql16, off_qterm, off_rot,
-      off_qprobes, off_z, off_costoff, off_seedorder, total;
+      off_qprobes, off_z, off_qcn, off_qr16, off_share, off_seedorder, total;
 };
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -767,9 +769,9 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
         std::max<size_t>(8192, static_cast<size_t>(B) * pl.S * 32 / pl.ctas));
     // the cost split, unless its 32-bit cost units could overflow
     pl.beta = g_tc_beta.load();
-    const uint64_t worst = static_cast<uint64_t>(pl.tcitems) * ((ix->max_list + 127) / 128) *
-                           (64 + static_cast<uint64_t>(pl.beta) * pl.tcs.N);
-    if (worst >= (1ull << 31)) pl.beta = 0;
+    const uint64_t worst = static_cast<uint64_t>(pl.tcitems) * div_up(ix->max_list, kTcSlab) *
+                           (pl.beta ? 64 + static_cast<uint64_t>(pl.beta) * pl.tcs.N : 32);
+    pl.cost = worst < (1ull << 31);
   } else {
     pl.ctas = 1;
     pl.rec_cap = 0;
@@ -797,18 +799,19 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_ent = take(bp * 4);
   pl.off_slots = take((pl.tc ? static_cast<size_t>(B) * pl.cap : bp * pl.SC) * sizeof(uint2));
   pl.off_tcscratch = take(3 * (static_cast<size_t>(L) + 1) * 4);
-  pl.off_costoff = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * 4 : 16);
+  pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);
   pl.off_tileoff = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * 4 : 16);
-  pl.off_nitems = take(16);
   pl.off_qcount = take(static_cast<size_t>(B) * 4);
-  pl.off_qfill = take(static_cast<size_t>(B) * 4);
   pl.off_bound = take(static_cast<size_t>(B) * 4);
   pl.off_rec = take(pl.tc ? static_cast<size_t>(pl.ctas) * pl.rec_cap * 16 : 16);
   pl.off_recn = take(static_cast<size_t>(pl.ctas) * 4);
   pl.coarse_tc = ix->d_chi16 && ix->d_clo16 && ix->d_cterm && coarse_tc_ok(ix->dc);
-  pl.off_qh16 = take(pl.coarse_tc ? static_cast<size_t>(B) * ix->dc * 2 : 16);
-  pl.off_ql16 = take(pl.coarse_tc ? static_cast<size_t>(B) * ix->dc * 2 : 16);
+  const bool planes = pl.coarse_tc || pl.tc;  // the queries' centred fp16 planes
+  pl.off_qh16 = take(planes ? static_cast<size_t>(B) * ix->dc * 2 : 16);
+  pl.off_ql16 = take(planes ? static_cast<size_t>(B) * ix->dc * 2 : 16);
+  pl.off_qr16 = take(pl.tc ? static_cast<size_t>(B) * tc_qrow(pl.dims, pl.tcs) * 2 : 16);
+  pl.off_qcn = take(planes ? static_cast<size_t>(B) * sizeof(int2) : 16);
   pl.off_qterm = take(static_cast<size_t>(B) * 8);
   pl.off_rot = take(ix->rotated ? rotate_scratch_bytes(B, ix->dim) : 16);
   pl.off_rlist = take(static_cast<size_t>(B) * 4);
@@ -862,13 +865,20 @@ int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
                              : 0) +
                 1 + 2;
   mark(tm, 1, st);
+  // the queries' centred planes, for both tensor-core passes
+  __half *qh16 = reinterpret_cast<__half *>(ws + pl.off_qh16);
+  __half *ql16 = reinterpret_cast<__half *>(ws + pl.off_ql16);
+  int64_t *qterm = reinterpret_cast<int64_t *>(ws + pl.off_qterm);
+  if (pl.coarse_tc || pl.tc) {
+    RankRows rr{};
+    if (pl.tc)
+      rr = RankRows{reinterpret_cast<__half *>(ws + pl.off_qr16),
+                    reinterpret_cast<int2 *>(ws + pl.off_qcn), pl.tcs.f, pl.dims,
+                    tc_qrow(pl.dims, pl.tcs), pl.tcs.centred};
+    if ((rc = centre_planes(qhi, qlo, qn, nq, dc, qh16, ql16, qterm, rr, st))) return rc;
+  }
   // 2. coarse product and top-nprobe (:846-877)
   if (pl.coarse_tc) {
-    // fp16 tensor cores: the queries' centred planes, then the exact product
-    __half *qh16 = reinterpret_cast<__half *>(ws + pl.off_qh16);
-    __half *ql16 = reinterpret_cast<__half *>(ws + pl.off_ql16);
-    int64_t *qterm = reinterpret_cast<int64_t *>(ws + pl.off_qterm);
-    if ((rc = centre_planes(qhi, qlo, qn, nq, dc, qh16, ql16, qterm, st))) return rc;
     kmark(tm, 1, false, st);
     if ((rc = coarse_tc(reinterpret_cast<const __half *>(ix->d_chi16),
                         reinterpret_cast<const __half *>(ix->d_clo16), ix->d_cterm, L, qh16, ql16,
@@ -960,8 +970,6 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     int32_t *bound = reinterpret_cast<int32_t *>(ws + pl.off_bound);
     TcItem *items = reinterpret_cast<TcItem *>(ws + pl.off_tcitems);
     uint32_t *tile_off = reinterpret_cast<uint32_t *>(ws + pl.off_tileoff);
-    uint32_t *nitems = reinterpret_cast<uint32_t *>(ws + pl.off_nitems);
-    uint32_t *qfill = reinterpret_cast<uint32_t *>(ws + pl.off_qfill);
     uint4 *rec = reinterpret_cast<uint4 *>(ws + pl.off_rec);
     uint32_t *rec_n = reinterpret_cast<uint32_t *>(ws + pl.off_recn);
     qcount = reinterpret_cast<uint32_t *>(ws + pl.off_qcount);
@@ -975,41 +983,39 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
       return rc;
     g_launches += L <= 16384 ? 1 : 0;  // the seed order
     mark(tm, 6, st);
-    uint32_t *cost_off = reinterpret_cast<uint32_t *>(ws + pl.off_costoff);
-    if ((rc = rank_tc_prepare(cnt, ix->d_list_off, L, pl.tcs.N, nq, pl.beta,
+    uint2 *share = reinterpret_cast<uint2 *>(ws + pl.off_share);
+    if ((rc = rank_tc_prepare(cnt, off, ix->d_list_off, L, pl.tcs.N, nq, pl.beta,
                               reinterpret_cast<uint32_t *>(ws + pl.off_tcscratch), items, tile_off,
-                              cost_off, nitems, qcount, qfill, stats + 40, st)))
+                              pl.cost, share, pl.ctas, qcount, stats + 40, stats + 4, st)))
       return rc;
     RankTcArgs T{};
-    T.qhi = qhi;
-    T.qnorm = qnorm;
+    T.qr16 = reinterpret_cast<const __half *>(ws + pl.off_qr16);
+    T.qcn = reinterpret_cast<const int2 *>(ws + pl.off_qcn);
     T.entries = ent;
-    T.off = off;
     T.items = items;
     T.tile_off = tile_off;
-    T.cost_off = pl.beta ? cost_off : nullptr;
-    T.nitems = nitems;
+    T.share = share;
     T.bound = bound;
     T.qcount = qcount;
     T.rec = rec;
     T.rec_n = rec_n;
     T.rec_cap = pl.rec_cap;
     T.timeouts = reinterpret_cast<uint32_t *>(stats + 3);
-    T.counters = stats + 4;
     T.prof = stats + 16;
     T.dc = dc;
     T.h = pl.dims;
+    T.f = pl.tcs.f;
     T.nprobe = p;
     T.wait = g_tc_wait.load() ? static_cast<long long>(g_tc_wait.load()) : 4000000000ll;
-    T.scale = scale;
     kmark(tm, 2, false, st);
     if ((rc = rank_tc(T, ix->d_hi, ix->npts, pl.tcs, st))) return rc;
     kmark(tm, 2, true, st);
-    if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, qfill, slots, pl.cap, scale, st)))
+    if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, nq, ix->d_hi, qhi, T.qcn, bound, dc,
+                             pl.tcs.f, pl.dims, qcount, slots, pl.cap, scale, stats + 5, st)))
       return rc;
     const RescanBufs rb{reinterpret_cast<uint32_t *>(ws + pl.off_rlist),
                         reinterpret_cast<unsigned long long *>(ws + pl.off_rkey),
-                        reinterpret_cast<uint32_t *>(ws + pl.off_rcount), qfill};
+                        reinterpret_cast<uint32_t *>(ws + pl.off_rcount)};
     if ((rc = rank_overflow(ix->d_hi, xnorm, ix->d_ids, qhi, qnorm, probed, qprobes, ix->d_list_off, nq, p,
                             dc, pl.dims, pl.S, scale, qcount, slots, pl.cap, rb, stats + 6, st)))
       return rc;

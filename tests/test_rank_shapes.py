@@ -1,0 +1,49 @@
+"""The ranking pass at the edges of its tiles, bit for bit against the oracle:
+list lengths around its 32- and 64-row steps, query counts per list around its
+groups of 8 and its items of 16, 32 and 64, prefixes of one to eight chunks,
+with values that decay over the dimensions (items scored over the leading 128
+alone), that do not (nearly every pair passes there) and at the ends of the
+byte range (the largest sums)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (0, 1, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 700)
+
+
+def _arrays(dim, head, kind, nq, seed):
+    rng = np.random.default_rng(seed)
+    scale = np.arange(1, dim + 1) ** (-0.6 if kind == "decaying" else 0.0)
+    n = sum(SIZES)
+    if kind == "ends":
+        x = rng.integers(0, 2, (n, dim)).astype(np.float32)
+        q = rng.integers(0, 2, (nq, dim)).astype(np.float32)
+        x[n // 2], q[0] = 1.0, 1.0
+        x[n // 3], q[-1] = 0.0, 0.0
+    else:
+        x = (rng.standard_normal((n, dim)) * scale).astype(np.float32)
+        q = (rng.standard_normal((nq, dim)) * scale).astype(np.float32)
+    cen = (rng.standard_normal((len(SIZES), dim)) * scale).astype(np.float32)
+    return dict(centroids=cen, list_sizes=np.array(SIZES, np.uint32),
+                ids=np.arange(n, dtype=np.uint32), vectors=x, rotation=None, head_dims=head), q
+
+
+@pytest.mark.parametrize("kind", ["decaying", "flat", "ends"])
+@pytest.mark.parametrize("dim,head", [(64, 64), (128, 64), (128, 128), (192, 192), (256, 256), (320, 320),
+                                      (448, 384), (1024, 1024)])
+def test_ranking_tiles(dim, head, kind):
+    import katoann
+    a, q = _arrays(dim, head, kind, 130, dim + head)
+    idx = katoann.Index()
+    idx.load_arrays(a["centroids"], a["list_sizes"], a["ids"], a["vectors"], head_dims=head)
+    ref = oracle.OracleIndex(None, arrays=a)
+    for nq, nprobe, ranking in ((130, len(SIZES), "prefix"), (65, len(SIZES), "high"), (33, 9, "prefix"),
+                                (9, len(SIZES), "prefix"), (1, len(SIZES), "prefix")):
+        kw = dict(k=10, nprobe=nprobe, ranking=ranking, survivors=24)
+        ids, dists = idx.search(q[-nq:], **kw)
+        rid, rd = ref.search(q[-nq:], **kw)
+        bad = np.nonzero((ids != rid).any(1) | (dists != rd).any(1))[0]
+        assert len(bad) == 0, (nq, kw, bad[:5])
