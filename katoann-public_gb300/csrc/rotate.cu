@@ -6,13 +6,13 @@
 // multiply-add in k order, the 16 lanes are added as (l, l+8), (l, l+4),
 // (l, l+2), (0, 1), and the last d % 16 dimensions follow one by one
 // (src/index.cpp:139-208). Here 16 consecutive threads of a warp play the 16
-// lanes: each thread keeps the lane sums of an 8 x 8 block of outputs, and the
-// lane reduction is a xor-butterfly of shuffles (8, 4, 2, 1), which adds the
-// same pairs in the same order, so every thread ends with the reference's
-// bits. The scalar parts are replayed with explicit rounding: the reference's
+// lanes: each thread keeps the lane sums of a block of outputs, and the lane
+// reduction is a butterfly of shuffles (8, 4, 2, 1), which adds the same pairs
+// in the same order, so every output ends with the reference's bits. The scalar parts are replayed with explicit rounding: the reference's
 // compiler evaluates those chains four products at a time with the products
 // rounded, then fuses the last (length % 4) terms.
 #include "kcommon.cuh"
+#include "tc.cuh"
 
 namespace kato {
 
@@ -43,26 +43,51 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src, uint32_t
                : "memory");
 }
 
-// 16-byte asynchronous global -> shared copy (L2 only).
-__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
+// Lane reduction as a reduce-scatter: at each step (lane distance 8, 4, 2, 1)
+// a lane keeps half of its NV outputs and adds its partner's partial sums of
+// them. Every output meets the same pairs in the same order as in the
+// reference's horizontal add (IEEE addition is commutative). Lane l ends with
+// the NV / 16 outputs from the returned one on: against an all-reduce a quarter
+// of the shuffles, and no spills.
+template <int NV>
+__device__ __forceinline__ int lane_scatter(float (&v)[NV], int l) {
+#pragma unroll
+  for (int step = 0, half = NV / 2, m = 8; step < 4; ++step, half >>= 1, m >>= 1) {
+    const bool hi = (l & m) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = hi ? v[i] : v[i + half];
+      const float keep = hi ? v[i + half] : v[i];
+      v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
+    }
+  }
+  return ((l >> 3) & 1) * (NV / 2) + ((l >> 2) & 1) * (NV / 4) + ((l >> 1) & 1) * (NV / 8) +
+         (l & 1) * (NV / 16);
 }
 
-// kMajor: the staged parts are read from k-major copies xt (d x ldx, rows
-// zero-padded to ldx) and rt (d x ldr, columns zero-padded), 16 bytes per
-// copy; otherwise from the row-major inputs, 4 bytes per copy.
-// Two CTAs per SM (118 registers, no spills): 4096 x 1024 queries in 0.32 ms.
-template <bool kMajor>
+// The four outputs of row i from column j on: the scalar tail, then the store.
+__device__ __forceinline__ void store_outputs(const float *v, uint32_t i, uint32_t j, uint32_t nrows,
+                                              uint32_t d, const float *in, const float *rot,
+                                              float *out) {
+  if (i >= nrows) return;
+  const uint32_t d4 = d & ~3u, d16 = d & ~15u;
+  const float *x = in + static_cast<size_t>(i) * d;
+  float *o = out + static_cast<size_t>(i) * d + j;
+  if (d16 == d && j + 4 <= d4 && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
+    *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (j + e < d4) o[e] = rot_tail(v[e], x, rot + static_cast<size_t>(j + e) * d, d16, d);
+  }
+}
+
+// Rows as they are (an index's rows at load): 32 x 32 outputs per CTA, 8 x 8
+// per thread, chunks of 64 dimensions copied 4 bytes at a time into a
+// double-buffered k-major staging.
 __global__ void __launch_bounds__(256, 2) rotate_lanes_kernel(const float *__restrict__ in,
                                                               uint32_t nrows, uint32_t d,
                                                               const float *__restrict__ rot,
-                                                              const float *__restrict__ xt,
-                                                              uint32_t ldx,
-                                                              const float *__restrict__ rt,
-                                                              uint32_t ldr,
                                                               float *__restrict__ out) {
   // two stages, each staged k-major (xs[k][row], rs[k][column]) so that a
   // thread reads its 8 rows and 8 columns at one k with four 128-bit loads;
@@ -80,28 +105,17 @@ __global__ void __launch_bounds__(256, 2) rotate_lanes_kernel(const float *__res
     for (int b = 0; b < 8; ++b) acc[a][b] = 0.0f;
 
   auto stage = [&](uint32_t k0, int buf) {
-    if constexpr (kMajor) {
-      // per k: 32 rows (8 copies) of x and 32 columns of r
-      const uint32_t kn = min(static_cast<uint32_t>(kRotK), d16 - k0);
-      for (uint32_t idx = t; idx < kn * 8; idx += 256) {
-        const uint32_t c = idx >> 3, q = (idx & 7) * 4;
-        cp_async16(&xs[buf][c * kRotStride + q], xt + static_cast<size_t>(k0 + c) * ldx + i0 + q);
-        cp_async16(&rs[buf][c * kRotStride + q], rt + static_cast<size_t>(k0 + c) * ldr + j0 + q);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    } else {
-      for (int idx = t; idx < kRotRows * kRotK; idx += 256) {
-        const int r = idx / kRotK, c = idx % kRotK;
-        const uint32_t gk = k0 + c;
-        const uint32_t gi = i0 + r, gj = j0 + r;
-        const bool okx = gi < nrows && gk < d16, okr = gj < d4 && gk < d16;
-        cp_async4(&xs[buf][c * kRotStride + r], okx ? in + static_cast<size_t>(gi) * d + gk : in,
-                  okx ? 4u : 0u);
-        cp_async4(&rs[buf][c * kRotStride + r], okr ? rot + static_cast<size_t>(gj) * d + gk : rot,
-                  okr ? 4u : 0u);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int idx = t; idx < kRotRows * kRotK; idx += 256) {
+      const int r = idx / kRotK, c = idx % kRotK;
+      const uint32_t gk = k0 + c;
+      const uint32_t gi = i0 + r, gj = j0 + r;
+      const bool okx = gi < nrows && gk < d16, okr = gj < d4 && gk < d16;
+      cp_async4(&xs[buf][c * kRotStride + r], okx ? in + static_cast<size_t>(gi) * d + gk : in,
+                okx ? 4u : 0u);
+      cp_async4(&rs[buf][c * kRotStride + r], okr ? rot + static_cast<size_t>(gj) * d + gk : rot,
+                okr ? 4u : 0u);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int buf = 0;
   if (d16) stage(0, 0);
@@ -134,41 +148,182 @@ __global__ void __launch_bounds__(256, 2) rotate_lanes_kernel(const float *__res
     }
     __syncthreads();  // the buffer is refilled by the next iteration's copies
   }
-  // Lane reduction as a reduce-scatter: at each step (lane distance 8, 4, 2,
-  // 1) a lane keeps half of its outputs and adds its partner's partial sums
-  // of them. Every output meets the same pairs in the same order as in the
-  // reference's horizontal add (IEEE addition is commutative), and lane l
-  // ends with the four outputs a = 4 b3 + 2 b2 + b1, b = 4 b0 .. 4 b0 + 3
-  // (b3 .. b0 the bits of l): 60 shuffles instead of 256, and no spills.
   float v[64];
 #pragma unroll
   for (int a = 0; a < 8; ++a)
 #pragma unroll
     for (int b = 0; b < 8; ++b) v[a * 8 + b] = acc[a][b];
-#pragma unroll
-  for (int step = 0, half = 32, m = 8; step < 4; ++step, half >>= 1, m >>= 1) {
-    const bool hi = (l & m) != 0;
-#pragma unroll
-    for (int i = 0; i < half; ++i) {
-      const float send = hi ? v[i] : v[i + half];
-      const float keep = hi ? v[i + half] : v[i];
-      v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
+  const int at = lane_scatter<64>(v, l);
+  store_outputs(v, i0 + rb + at / 8, j0 + cb + at % 8, nrows, d, in, rot, out);
+}
+
+// The queries of a search. What bounds it is the FP32 pipe: d^2 products per
+// row in the reference's order, so no tensor cores; the same inner loop over
+// data already in place reaches 113 of 128 FMA per clock and SM, and 92 with a
+// barrier every 32 dimensions. Copying the staged parts with 16-byte cp.async,
+// 64 dimensions at a time, left 65: its address arithmetic and the chunk's
+// hand-over each cost as much as a third of the products. So the parts come by
+// TMA, 128 dimensions to a chunk (64: 12% slower), from thread 0: 128-byte rows
+// of the k-major copies, in the 128-byte swizzle, which leaves the 16-byte
+// reads of eight consecutive lanes (eight consecutive k) free of bank
+// conflicts. Products are packed two columns to an fma.rn.f32x2, which halves
+// their issue slots and rounds each as the scalar one does.
+//   kRows false: tiles of 32 x 32 outputs, 8 x 16 per thread (96 bytes read per
+//     128 products instead of 64 per 64), the queries' k-major copy by TMA too;
+//     two CTAs of 128 threads per SM hide each other's hand-overs (one of 256
+//     over 32 x 64: 8% slower). With the transpose, 4096 x 1024: 171 us (262
+//     before), 4096 x 3072: 1,331 us (2,118);
+//   kRows true (few queries): tiles of 8 rows x 32 columns, so that one query
+//     spreads over d / 32 CTAs of 64 threads; the CTA transposes its 8 rows
+//     into shared memory itself.
+constexpr int kRotChunk = 128, kRotStages = 3, kRotAhead = kRotStages - 1;
+constexpr uint32_t kRotBox = kRotChunk * 128;  // kRotChunk dimensions x 32 floats
+constexpr uint32_t kSlabRows = 8, kSlabStride = 12;  // floats per k: 16-byte reads without conflicts
+
+template <bool kRows>
+__host__ __device__ constexpr uint32_t rot_stage_bytes() {
+  return kRows ? kRotBox : 2 * kRotBox;
+}
+
+template <bool kRows>
+__host__ __device__ constexpr int rot_threads() {
+  return kRows ? 64 : 128;
+}
+
+template <bool kRows>
+__global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
+    rotate_tma_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tr,
+                      const float *__restrict__ in, uint32_t nrows, uint32_t d,
+                      const float *__restrict__ rot, float *__restrict__ out,
+                      uint32_t *__restrict__ timeouts) {
+  constexpr int TB = kRows ? 8 : 16, CG = kRows ? 4 : 2;
+  constexpr uint32_t kStage = rot_stage_bytes<kRows>();
+  constexpr uint32_t kRowTile = kRows ? kSlabRows : 32, kColTile = 32;
+  constexpr int kWarps = rot_threads<kRows>() / 32;
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  unsigned char *sm = smraw + ((1024 - (tc::smem_addr(smraw) & 1023u)) & 1023u);
+  __shared__ uint64_t full[kRotStages], empty[kRotStages];
+  __shared__ volatile uint32_t err;
+  const uint32_t d16 = d & ~15u, nk = (d16 + kRotChunk - 1) / kRotChunk;
+  const uint32_t i0 = blockIdx.y * kRowTile, j0 = blockIdx.x * kColTile;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) {
+    for (int s = 0; s < kRotStages; ++s) {
+      tc::mbar_init(full + s, 1);
+      tc::mbar_init(empty + s, kWarps);
     }
+    err = 0;
+    tc::fence_barrier_init();
   }
-  // the scalar tail and the store of this lane's four outputs
-  const int a = 4 * ((l >> 3) & 1) + 2 * ((l >> 2) & 1) + ((l >> 1) & 1), b0 = 4 * (l & 1);
-  const uint32_t i = i0 + rb + a, j = j0 + cb + b0;
-  if (i < nrows) {
-    const float *x = in + static_cast<size_t>(i) * d;
-    float *o = out + static_cast<size_t>(i) * d + j;
-    if (d16 == d && j + 4 <= d4 && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
-      *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+  __syncthreads();
+  const int l = t & 15, g = t >> 4;
+  const uint32_t rb = kRows ? 0 : (g / CG) * 8, cb = (g % CG) * TB;
+  float *slab = reinterpret_cast<float *>(sm + kRotStages * kStage);  // [k][row], kRows only
+  // chunk c into its stage, once every warp has read the one before in it
+  auto issue = [&](uint32_t c) -> bool {
+    const uint32_t s = c % kRotStages, use = c / kRotStages;
+    if (use && !tc::mbar_test(tc::smem_addr(empty + s), (use & 1) ^ 1) &&
+        !tc::mbar_wait_or(empty + s, (use & 1) ^ 1, &err))
+      return false;
+    unsigned char *st = sm + s * kStage;
+    const int32_t k = static_cast<int32_t>(c * kRotChunk), j = static_cast<int32_t>(j0);
+    tc::mbar_expect_tx(full + s, kStage);
+    tc::tma_load_2d(st, &tr, j, k, full + s);
+    if (!kRows) tc::tma_load_2d(st + kRotBox, &tx, static_cast<int32_t>(i0), k, full + s);
+    return true;
+  };
+  uint32_t issued = 0;  // thread 0's
+  bool ok = true;
+  if (t == 0)
+    for (; issued < nk && issued < kRotAhead; ++issued) issue(issued);
+  if (kRows) {
+    // thread t takes row t % 8, four dimensions at a time
+    const uint32_t r = t % kSlabRows;
+    const bool in_rows = i0 + r < nrows;
+    const float *x = in + static_cast<size_t>(in_rows ? i0 + r : 0) * d;
+    const bool vec = d % 4 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
+#pragma unroll 16
+    for (uint32_t k = t / kSlabRows * 4; k < d16; k += kWarps * 16) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (in_rows) v = vec ? __ldg(reinterpret_cast<const float4 *>(x + k)) : make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+      float *o = slab + k * kSlabStride + r;
+      o[0] = v.x, o[kSlabStride] = v.y, o[2 * kSlabStride] = v.z, o[3 * kSlabStride] = v.w;
+    }
+    __syncthreads();
+  }
+  // this lane's dimension is l of every 16: its 128-byte row of a box, and
+  // its 16-byte units where the swizzle put them
+  const unsigned char *xo[2], *ro[TB / 4];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    xo[u] = kRows ? reinterpret_cast<const unsigned char *>(slab + l * kSlabStride + 4 * u)
+                  : sm + kRotBox + l * 128 + (((rb / 4 + u) ^ (l & 7)) << 4);
+#pragma unroll
+  for (int u = 0; u < TB / 4; ++u)
+    ro[u] = sm + l * 128 + (((cb / 4 + u) ^ (l & 7)) << 4);
+  unsigned long long acc[8][TB / 2];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < TB / 2; ++b) acc[a][b] = 0ull;
+  uint32_t s = 0, ph = 0;
+  for (uint32_t c = 0; c < nk; ++c) {
+    if (t == 0 && issued < nk && (ok = issue(issued))) ++issued;
+    if (ok && !tc::mbar_test(tc::smem_addr(full + s), ph))
+      ok = tc::mbar_wait_or(full + s, ph, &err);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    // one 16-dimension step: this lane's products of the 8 rows and TB columns
+    auto step = [&](uint32_t k) {
+      const uint32_t so = s * kStage + k * 128;
+      float xv[8];
+      unsigned long long rv[TB / 2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float4 v = *reinterpret_cast<const float4 *>(xo[u] + (kRows ? (c * kRotChunk + k) * kSlabStride * 4 : so));
+        xv[4 * u] = v.x, xv[4 * u + 1] = v.y, xv[4 * u + 2] = v.z, xv[4 * u + 3] = v.w;
+      }
+#pragma unroll
+      for (int u = 0; u < TB / 4; ++u) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(ro[u] + so);
+        rv[2 * u] = v.x, rv[2 * u + 1] = v.y;
+      }
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        unsigned long long xx;
+        asm("mov.b64 %0, {%1,%1};" : "=l"(xx) : "f"(xv[a]));
+#pragma unroll
+        for (int b = 0; b < TB / 2; ++b)
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[a][b]) : "l"(xx), "l"(rv[b]));
+      }
+    };
+    if ((c + 1) * kRotChunk <= d16) {  // whole chunks without a test per step
+#pragma unroll
+      for (uint32_t k = 0; k < kRotChunk; k += 16) step(k);
     } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (j + e < d4) o[e] = rot_tail(v[e], x, rot + static_cast<size_t>(j + e) * d, d16, d);
+#pragma unroll 1
+      for (uint32_t k = 0; c * kRotChunk + k < d16; k += 16) step(k);
     }
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(empty + s);
+    if (++s == kRotStages) s = 0, ph ^= 1;
   }
+  float v[8 * TB];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < TB / 2; ++b)
+      asm("mov.b64 {%0,%1}, %2;" : "=f"(v[a * TB + 2 * b]), "=f"(v[a * TB + 2 * b + 1]) : "l"(acc[a][b]));
+  const int at = lane_scatter<8 * TB>(v, l);
+  if (!err) {
+#pragma unroll
+    for (int e = 0; e < TB / 2; e += 4)
+      store_outputs(v + e, i0 + rb + at / TB, j0 + cb + at % TB + e, nrows, d, in, rot, out);
+  }
+  if (t == 0 && err)  // copies still in flight land before the CTA exits
+    for (uint32_t c = issued < kRotStages ? 0 : issued - kRotStages; c < issued; ++c)
+      tc::mbar_wait(full + c % kRotStages, (c / kRotStages) & 1);
+  __syncthreads();
+  if (t == 0 && err && timeouts) atomicAdd(timeouts, 1u);
 }
 
 // out[k * ld + r] = in[r * d + k] for r < rows (zero for rows <= r < ld),
@@ -311,7 +466,7 @@ int rotate_rows(const float *in, uint32_t nrows, uint32_t d, const float *rot, f
   const uint32_t d4 = d & ~3u;
   if (d4) {
     dim3 grid(div_up(nrows, kRotRows), div_up(d4, kRotCols));
-    rotate_lanes_kernel<false><<<grid, 256, 0, st>>>(in, nrows, d, rot, nullptr, 0, nullptr, 0, out);
+    rotate_lanes_kernel<<<grid, 256, 0, st>>>(in, nrows, d, rot, out);
     KATO_LAUNCHED("rotate_lanes_kernel");
   }
   if (d4 < d) {
@@ -341,28 +496,78 @@ int rotation_kmajor(const float *rot, uint32_t d, float *out, cudaStream_t st) {
   return KATO_OK;
 }
 
+// A k-major copy (k rows of ld floats) in boxes of 32 floats x kRotChunk k.
+static int encode_kmajor(CUtensorMap *map, const float *base, uint32_t ld, uint32_t k) {
+  const PFN_cuTensorMapEncodeTiled_v12000 encode = tc::tensor_map_encoder();
+  if (!encode) return cuda_status(cudaErrorNotSupported, "cuTensorMapEncodeTiled");
+  const cuuint64_t dims[2] = {ld, k};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
+  const cuuint32_t box[2] = {32, kRotChunk};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims,
+                            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed for the rotation (error " + std::to_string(r) + ")");
+    return KATO_ERUNTIME;
+  }
+  return KATO_OK;
+}
+
+// Up to 64 rows the tiles of 32 would leave most of a tile empty and, at
+// d = 1,024, use 32 SMs: 16 rows took 23 us, in tiles of 8 rows 17 us.
+constexpr uint32_t kRotFewRows = 64;
+
 int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float *rot,
-                       const float *rot_kmajor, void *scratch, float *out, cudaStream_t st) {
+                       const float *rot_kmajor, void *scratch, float *out, uint32_t *timeouts,
+                       uint32_t *launches, cudaStream_t st) {
   if (nrows == 0) return KATO_OK;
   const uint32_t d4 = d & ~3u, d16 = d & ~15u;
-  if (d16 == 0) return rotate_rows(in, nrows, d, rot, out, st);
+  if (d16 == 0) {
+    *launches += (d4 ? 1 : 0) + (d4 < d ? 1 : 0);
+    return rotate_rows(in, nrows, d, rot, out, st);
+  }
   const uint32_t ldx = div_up(nrows, 32) * 32, ldr = div_up(d4, 32) * 32;
   float *xt = static_cast<float *>(scratch);
   const float *rt = rot_kmajor;
-  transpose_pad(in, nrows, d, d16, xt, ldx, st);
+  // 1 KiB of slack: the stages start on a 1 KiB boundary
+  const size_t slab_smem =
+      kRotStages * rot_stage_bytes<true>() + static_cast<size_t>(d16) * kSlabStride * 4 + 1024;
+  const bool few = nrows <= kRotFewRows && slab_smem <= 224 * 1024;  // d16 up to 3,728
+  if (!few) {
+    transpose_pad(in, nrows, d, d16, xt, ldx, st);
+    ++*launches;
+  }
   if (!rt) {  // no copy made at load: transpose the rotation here
     float *t = xt + static_cast<size_t>(ldx) * d16;
     transpose_pad(rot, d4, d, d16, t, ldr, st);
+    ++*launches;
     rt = t;
   }
   KATO_LAUNCHED("transpose_pad_kernel");
-  dim3 grid(div_up(nrows, kRotRows), div_up(d4, kRotCols));
-  rotate_lanes_kernel<true><<<grid, 256, 0, st>>>(in, nrows, d, rot, xt, ldx, rt, ldr, out);
-  KATO_LAUNCHED("rotate_lanes_kernel");
+  CUtensorMap tx{}, tr;
+  int rc;
+  if ((rc = encode_kmajor(&tr, rt, ldr, d16)) || (!few && (rc = encode_kmajor(&tx, xt, ldx, d16)))) return rc;
+  auto go = [&](auto kern, uint32_t row_tile, uint32_t col_tile, int threads, size_t smem) -> int {
+    if (const int r = smem_limit(reinterpret_cast<const void *>(kern), static_cast<int>(smem),
+                                 "rotate_tma_kernel shared memory"))
+      return r;
+    kern<<<dim3(div_up(d4, col_tile), div_up(nrows, row_tile)), threads, smem, st>>>(
+        tx, tr, in, nrows, d, rot, out, timeouts);
+    KATO_LAUNCHED("rotate_tma_kernel");
+    return KATO_OK;
+  };
+  rc = few ? go(rotate_tma_kernel<true>, kSlabRows, 32, rot_threads<true>(), slab_smem)
+           : go(rotate_tma_kernel<false>, 32, 32, rot_threads<false>(),
+                kRotStages * rot_stage_bytes<false>() + 1024);
+  if (rc) return rc;
+  ++*launches;
   if (d4 < d) {
     const uint64_t n = static_cast<uint64_t>(nrows) * (d - d4);
     rotate_seq_kernel<<<static_cast<uint32_t>((n + 255) / 256), 256, 0, st>>>(in, nrows, d, rot, out);
     KATO_LAUNCHED("rotate_seq_kernel");
+    ++*launches;
   }
   return KATO_OK;
 }

@@ -684,7 +684,8 @@ int coarse_tc(const __half *ch, const __half *cl, const int64_t *cterm, uint32_t
               float *out, uint32_t *timeouts, unsigned long long *prof, cudaStream_t st);
 size_t rotate_scratch_bytes(uint32_t nrows, uint32_t d);
 int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float *rot,
-                       const float *rot_kmajor, void *scratch, float *out, cudaStream_t st);
+                       const float *rot_kmajor, void *scratch, float *out, uint32_t *timeouts,
+                       uint32_t *launches, cudaStream_t st);
 int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint32_t stride,
                    uint32_t *probed, unsigned long long *tie_count, const uint32_t *only,
                    uint32_t only_above, cudaStream_t st);
@@ -849,7 +850,8 @@ int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   if (ix->rotated) {
     kmark(tm, 0, false, st);
     if ((rc = rotate_rows_kmajor(queries, nq, ix->dim, ix->d_rotation, ix->d_rotation_t,
-                                 ws + pl.off_rot, fq, st)))
+                                 ws + pl.off_rot, fq, reinterpret_cast<uint32_t *>(stats + 3),
+                                 &g_launches, st)))
       return rc;
     kmark(tm, 0, true, st);
     src = fq;
@@ -857,13 +859,7 @@ int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   if ((rc = quantize_rows(src, nq, ix->dim, dc, ix->lo, ix->inv_step, ix->head_dims, qhi, qlo, qn,
                           qhn, qh0, st)))
     return rc;
-  // rotation (the queries' transpose, the rotation's unless the index holds
-  // its k-major copy, and the product, plus the d % 4 columns), quantize,
-  // coarse, select
-  g_launches += (ix->rotated ? ((ix->dim & ~15u) ? (ix->d_rotation_t ? 2 : 3) : 1) +
-                                   ((ix->dim & 3) ? 1 : 0)
-                             : 0) +
-                1 + 2;
+  g_launches += 1 + 2;  // quantize, coarse, select
   mark(tm, 1, st);
   // the queries' centred planes, for both tensor-core passes
   __half *qh16 = reinterpret_cast<__half *>(ws + pl.off_qh16);

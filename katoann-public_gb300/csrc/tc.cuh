@@ -91,19 +91,6 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t phase) {
   return ok != 0;
 }
 
-// As mbar_try, but a thread whose phase is not complete sleeps until it
-// completes or `hint_ns` nanoseconds pass, instead of returning at once.
-__device__ __forceinline__ bool mbar_try_sleep(uint64_t *bar, uint32_t phase, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(phase), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-
 // Bounded wait on an mbarrier phase; false if it did not complete in time.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, uint32_t limit = 1u << 26) {
   for (uint32_t i = 0; i < limit; ++i)
@@ -113,12 +100,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, uint32_
 
 // Bounded wait on a phase with a clock deadline, giving up early once *err is
 // set by another role of the CTA; a timeout sets *err.
-// Waiting threads sleep in the barrier (up to 50 us per try) rather than
-// spin, leaving the issue slots to the warps that have work.
+// The try has no suspend-time hint: with one, the compiler's loop sleeps in
+// steps of about a microsecond, more than a pipeline stage lasts.
 __device__ __forceinline__ bool mbar_wait_or(uint64_t *bar, uint32_t phase, volatile uint32_t *err,
                                              long long limit_cycles = 4000000000ll) {
+  if (mbar_test(smem_addr(bar), phase)) return true;
   const long long t0 = clock64();
-  while (!mbar_try_sleep(bar, phase, 50000)) {
+  while (!mbar_try(bar, phase)) {
     if (*err) return false;
     if (clock64() - t0 > limit_cycles) {
       *err = 1;
