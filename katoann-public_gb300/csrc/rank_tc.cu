@@ -13,10 +13,9 @@
 //   3. tc_bucket_kernel completes the records' l2, drops those beyond the
 //      bound and sorts the rest into per-query buffers with their float
 //      distances;
-//   4. a query whose buffer overflowed is rescanned exactly (rescan_*
-//      kernels), and the merge kernel takes the exact best S by (distance, id)
-//      from each buffer, so results never depend on the bound or the buffer
-//      size.
+//   4. finish_kernel (finish.cu) takes the exact best S by (distance, id) from
+//      each buffer, after an exact rescan of a query whose buffer overflowed,
+//      so results never depend on the bound or the buffer size.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -27,6 +26,7 @@
 
 #include "kcommon.cuh"
 #include "rank_tc.cuh"
+#include "rows.cuh"
 #include "scan.cuh"
 #include "tc.cuh"
 
@@ -35,7 +35,6 @@ namespace kato {
 namespace {
 
 constexpr uint32_t kSeedCap = 4096;  // rows a seed bound looks at, at most
-constexpr uint32_t kDropped = 0x80000000u;  // qcount flag: a record did not fit
 
 // rank_tc_kernel: one CTA per SM takes an equal share, by cost, of all 64-row
 // slabs of all work items (an item is a list and up to N of the queries
@@ -559,112 +558,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   }
 }
 
-// The squared L2 over the first h high bytes of a row and a query whose bytes
-// are in shared memory as words; dp4a over 16 bytes per step.
-__device__ __forceinline__ uint32_t row_dot(const uint8_t *row, const uint32_t *qw, uint32_t h) {
-  const uint4 *rv = reinterpret_cast<const uint4 *>(row);
-  uint32_t dot = 0;
-  uint32_t u = 0;
-  for (; u + 4 <= h / 16; u += 4) {  // four loads in flight
-    uint4 v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __ldg(rv + u + j);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t *w = qw + 4 * (u + j);
-      dot = dp4(v[j].x, w[0], dp4(v[j].y, w[1], dp4(v[j].z, w[2], dp4(v[j].w, w[3], dot))));
-    }
-  }
-  for (; u < h / 16; ++u) {
-    const uint4 v = __ldg(rv + u);
-    const uint32_t *w = qw + 4 * u;
-    dot = dp4(v.x, w[0], dp4(v.y, w[1], dp4(v.z, w[2], dp4(v.w, w[3], dot))));
-  }
-  return dot;
-}
-
-// Dot products of a query (its h bytes as words in shared memory) with rows
-// row(0) .. row(n - 1) of a byte plane, lanes split along each row: a group of
-// G = min(32, h / 16) lanes reads a row as one coalesced run of 16-byte
-// loads and sums over the group by shuffles. A warp takes 32 rows at a time
-// (G steps, all loads of the batch in flight together) and hands row
-// base + l of the batch to one lane, so f(i, dot) runs on all 32 lanes at
-// once. All threads of the CTA take part.
-//
-// pre(i) - a per-row value the callback needs (e.g. the row's norm) - is
-// loaded at the start of the batch by the lane that later calls
-// f(i, dot, pre(i)), so that it arrives with the rows instead of after them.
-
-template <uint32_t G, typename F, typename Pre, typename RowAt>
-__device__ __forceinline__ void rows_split(const uint8_t *__restrict__ x, uint32_t dc, uint32_t h,
-                                           const uint32_t *qw, RowAt row, uint32_t n, Pre pre,
-                                           F f) {
-  constexpr uint32_t RPW = 32 / G;  // rows per step
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t sub = lane / G, gl = lane % G, cpl = (h / 16) / G;
-  for (uint32_t base = warp * 32; base < n; base += nw * 32) {
-    uint32_t mine = 0;
-    const uint32_t my_row = base + gl * RPW + sub;
-    const int64_t pv = my_row < n ? pre(my_row) : 0;
-    if (G <= 16 && cpl == 1) {
-      // every load of the batch first, then the sums
-      uint4 v[G <= 16 ? G : 1];
-      const uint32_t *w = qw + 4 * gl;
-#pragma unroll
-      for (uint32_t it = 0; it < (G <= 16 ? G : 1); ++it) {
-        const uint32_t i = base + it * RPW + sub;
-        v[it] = i < n ? __ldg(reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row(i)) * dc) + gl)
-                      : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (uint32_t it = 0; it < (G <= 16 ? G : 1); ++it) {
-        uint32_t dot = dp4(v[it].x, w[0], dp4(v[it].y, w[1], dp4(v[it].z, w[2], dp4(v[it].w, w[3], 0))));
-#pragma unroll
-        for (uint32_t o = G / 2; o; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (gl == it) mine = dot;
-      }
-    } else {
-#pragma unroll
-      for (uint32_t it = 0; it < G; ++it) {
-        const uint32_t i = base + it * RPW + sub;
-        uint32_t dot = 0;
-        if (i < n) {
-          const uint4 *rv = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row(i)) * dc);
-          for (uint32_t c = 0; c < cpl; ++c) {
-            const uint32_t u = gl + c * G;
-            const uint4 vv = __ldg(rv + u);
-            const uint32_t *w = qw + 4 * u;
-            dot = dp4(vv.x, w[0], dp4(vv.y, w[1], dp4(vv.z, w[2], dp4(vv.w, w[3], dot))));
-          }
-        }
-#pragma unroll
-        for (uint32_t o = G / 2; o; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (gl == it) mine = dot;
-      }
-    }
-    if (my_row < n) f(my_row, mine, pv);
-  }
-}
-
-// rows_split with the group size for h.
-template <typename F, typename Pre, typename RowAt>
-__device__ __forceinline__ void for_rows_at(const uint8_t *__restrict__ x, uint32_t dc, uint32_t h,
-                                            const uint32_t *qw, RowAt row, uint32_t n, F f, Pre pre) {
-  const uint32_t g = min(32u, h / 16);
-  if (g == 16) rows_split<16>(x, dc, h, qw, row, n, pre, f);
-  else if (g == 32) rows_split<32>(x, dc, h, qw, row, n, pre, f);
-  else if (g == 8) rows_split<8>(x, dc, h, qw, row, n, pre, f);
-  else rows_split<4>(x, dc, h, qw, row, n, pre, f);
-}
-
-// The same over the contiguous rows r0 .. r0 + n - 1.
-template <typename F, typename Pre>
-__device__ __forceinline__ void for_rows_split(const uint8_t *__restrict__ x, uint32_t dc, uint32_t h,
-                                               const uint32_t *qw, uint32_t r0, uint32_t n, F f,
-                                               Pre pre) {
-  for_rows_at(x, dc, h, qw, [r0](uint32_t i) { return r0 + i; }, n, f, pre);
-}
-
 // ------------------------------------------------------------- seed bounds
 // One CTA per query. It looks at the first `want` rows of the query's probed
 // lists (probe order, nearest list first). When there are more than `full` of
@@ -811,179 +704,6 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const int32_t v = static_cast<int32_t>(L2);
     bound[q] = v + (v >> 22) + 1;
   }
-}
-
-// --------------------------------------------------------- overflow rescan
-// A query whose buffer overflowed (more than `cap` rows within its seed
-// bound; the buffer holds the first cap of them) is rescanned in rounds:
-//   * rescan_bound_kernel: K = the S-th smallest key (distance bits << 32 |
-//     id) among the rows in its buffer - an upper bound on the query's true
-//     S-th best key, as they are some of its candidates; the query is listed
-//     and its count reset;
-//   * rescan_rows_kernel: CTAs over (listed query, probed list) pairs put the
-//     rows with key <= K into the buffer. If they fit, the buffer holds every
-//     row that can be selected. Otherwise the next round's K comes from the
-//     new buffer and is strictly smaller (its cap > S distinct keys are all
-//     <= K), which shrinks the count by about cap / S per round;
-//   * rescan_exact_kernel, after kRescanRounds rounds: the S smallest keys by
-//     8-bit radix selection over all of a query's candidates, one CTA each.
-// Distances are recomputed from the codes; results never depend on the
-// buffer size.
-constexpr int kRescanRounds = 2;
-
-// The rank-th smallest 64-bit key produced by key(i), i < n, by 8-bit radix
-// digits; all threads of the CTA call it and get the key.
-template <typename KeyAt>
-__device__ unsigned long long block_select64(uint32_t n, uint32_t rank, KeyAt key, uint32_t *hist,
-                                             uint32_t *sel) {
-  __shared__ uint32_t wsum[8];
-  unsigned long long prefix = 0;
-  for (int shift = 56; shift >= 0; shift -= 8) {
-    for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    const unsigned long long hm = shift == 56 ? 0ull : (~0ull << (shift + 8));
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const unsigned long long k = key(i);
-      if ((k & hm) == prefix) atomicAdd(&hist[(k >> shift) & 0xFFu], 1u);
-    }
-    __syncthreads();
-    block_pick_digit(hist, rank, sel, wsum);
-    rank -= sel[1];
-    prefix |= static_cast<unsigned long long>(sel[0]) << shift;
-    __syncthreads();
-  }
-  return prefix;
-}
-
-struct RowKey {
-  const uint8_t *xhi;
-  const int64_t *xnorm;
-  const uint32_t *ids;
-  uint32_t dc, h;
-  DistScale scale;
-  __device__ unsigned long long operator()(uint32_t row, const uint32_t *qw, int64_t qn) const {
-    const uint32_t dot = row_dot(xhi + static_cast<size_t>(row) * dc, qw, h);
-    const int64_t l2 = qn + xnorm[row] - 2 * static_cast<int64_t>(dot);
-    return (static_cast<unsigned long long>(__float_as_uint(dist_value(l2, scale))) << 32) | ids[row];
-  }
-};
-
-__device__ __forceinline__ void load_query_words(const uint8_t *qhi, uint32_t q, uint32_t dc,
-                                                 uint32_t h, uint32_t *qw) {
-  for (uint32_t i = threadIdx.x; i < h / 4; i += blockDim.x)
-    qw[i] = reinterpret_cast<const uint32_t *>(qhi + static_cast<size_t>(q) * dc)[i];
-}
-
-__global__ void __launch_bounds__(256) rescan_bound_kernel(
-    const uint32_t *__restrict__ ids, uint32_t *__restrict__ qcount,
-    const uint2 *__restrict__ qbuf, uint32_t cap, uint32_t S,
-    uint32_t round, uint32_t *__restrict__ list, unsigned long long *__restrict__ kbound,
-    uint32_t *__restrict__ nlisted, unsigned long long *__restrict__ stats) {
-  __shared__ uint32_t hist[256], sel[2];
-  const uint32_t q = blockIdx.x;
-  const uint32_t n = qcount[q];  // bit 31: records were dropped
-  if (round == 0 && threadIdx.x == 0)
-    atomicMax(stats + 1, static_cast<unsigned long long>(n & ~kDropped));
-  if (n <= cap) return;
-  // entries actually in the buffer (a subset's S-th smallest key is a bound
-  // as well: look at 2048 at most)
-  const uint32_t valid = min(min(n & ~kDropped, cap), 2048u);
-  const uint2 *buf = qbuf + static_cast<size_t>(q) * cap;
-  const unsigned long long K =
-      valid < S ? ~0ull
-                : block_select64(
-                      valid, S - 1,
-                      [&](uint32_t i) {
-                        const uint2 e = buf[i];
-                        return (static_cast<unsigned long long>(e.x) << 32) | ids[e.y];
-                      },
-                      hist, sel);
-  if (threadIdx.x == 0) {
-    kbound[q] = K;
-    qcount[q] = 0;
-    list[atomicAdd(nlisted, 1u)] = q;
-    if (round == 0) atomicAdd(stats, 1ull);
-  }
-}
-
-__global__ void __launch_bounds__(256) rescan_rows_kernel(
-    RowKey key, const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
-    const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
-    const uint32_t *__restrict__ list_off, uint32_t p, uint32_t *__restrict__ qcount,
-    uint2 *__restrict__ qbuf, uint32_t cap, const uint32_t *__restrict__ list,
-    const unsigned long long *__restrict__ kbound, const uint32_t *__restrict__ nlisted) {
-  __shared__ uint32_t qw[2048 / 4];
-  const size_t pairs = static_cast<size_t>(*nlisted) * p;
-  for (size_t pair = blockIdx.x; pair < pairs; pair += gridDim.x) {
-    const uint32_t q = list[pair / p];
-    if (qprobes && pair % p >= qprobes[q]) continue;  // beyond the query's budget
-    const uint32_t c = probed[static_cast<size_t>(q) * p + pair % p];
-    __syncthreads();
-    load_query_words(qhi, q, key.dc, key.h, qw);
-    __syncthreads();
-    const int64_t qn = qnorm[q];
-    const unsigned long long K = kbound[q];
-    uint2 *buf = qbuf + static_cast<size_t>(q) * cap;
-    const uint32_t r0 = list_off[c];
-    for_rows_split(
-        key.xhi, key.dc, key.h, qw, r0, list_off[c + 1] - r0,
-        [&](uint32_t i, uint32_t dot, int64_t xn) {
-      const uint32_t row = r0 + i;
-      const int64_t l2 = qn + xn - 2 * static_cast<int64_t>(dot);
-      const unsigned long long k =
-          (static_cast<unsigned long long>(__float_as_uint(dist_value(l2, key.scale))) << 32) |
-          key.ids[row];
-      if (k <= K) {
-        const uint32_t at = atomicAdd(qcount + q, 1u);
-        if (at < cap) buf[at] = make_uint2(static_cast<uint32_t>(k >> 32), row);
-      }
-    },
-        [&](uint32_t i) { return key.xnorm[r0 + i]; });
-  }
-}
-
-__global__ void __launch_bounds__(256) rescan_exact_kernel(
-    RowKey key, const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
-    const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
-    const uint32_t *__restrict__ list_off, uint32_t p, uint32_t S, uint32_t *__restrict__ qcount,
-    uint2 *__restrict__ qbuf, uint32_t cap) {
-  const uint32_t q = blockIdx.x, tid = threadIdx.x;
-  if (qcount[q] <= cap) return;
-  __shared__ uint32_t qw[2048 / 4];
-  __shared__ uint32_t hist[256], sel[2], taken;
-  load_query_words(qhi, q, key.dc, key.h, qw);
-  if (tid == 0) taken = 0;
-  __syncthreads();
-  const int64_t qn = qnorm[q];
-  const uint32_t *pq = probed + static_cast<size_t>(q) * p;
-  const uint32_t np = qprobes ? qprobes[q] : p;  // the query's own budget
-  uint32_t total = 0;
-  for (uint32_t r = 0; r < np; ++r) total += list_off[pq[r] + 1] - list_off[pq[r]];
-  // more than cap >= S candidates, so the S-th smallest key exists
-  const unsigned long long K = block_select64(
-      total, S - 1,
-      [&](uint32_t i) {
-        uint32_t r = 0;
-        for (;;) {
-          const uint32_t len = list_off[pq[r] + 1] - list_off[pq[r]];
-          if (i < len) break;
-          i -= len;
-          ++r;
-        }
-        return key(list_off[pq[r]] + i, qw, qn);
-      },
-      hist, sel);
-  uint2 *buf = qbuf + static_cast<size_t>(q) * cap;
-  for (uint32_t r = 0; r < np; ++r)
-    for (uint32_t row = list_off[pq[r]] + tid; row < list_off[pq[r] + 1]; row += blockDim.x) {
-      const unsigned long long k = key(row, qw, qn);
-      if (k <= K) {
-        const uint32_t at = atomicAdd(&taken, 1u);  // exactly S rows (distinct ids)
-        if (at < cap) buf[at] = make_uint2(static_cast<uint32_t>(k >> 32), row);
-      }
-    }
-  __syncthreads();
-  if (tid == 0) qcount[q] = min(taken, cap);
 }
 
 // -------------------------------------------------- work items and offsets
@@ -1293,30 +1013,6 @@ int rank_tc_prepare(const uint32_t *cnt, const uint32_t *off, const uint32_t *li
   tc_expand_kernel<<<div_up(std::max(L, ctas), 256), 256, 0, st>>>(list_off, scratch, cnt, off, L, N, beta, by_cost,
                                                    ctas, items, tile_off, share, tile_hist, tiles);
   KATO_LAUNCHED("ranking work preparation");
-  return KATO_OK;
-}
-
-int rank_overflow(const uint8_t *xhi, const int64_t *xnorm, const uint32_t *ids,
-                  const uint8_t *qhi, const int64_t *qnorm, const uint32_t *probed,
-                  const uint32_t *qprobes, const uint32_t *list_off, uint32_t B, uint32_t p,
-                  uint32_t dc, uint32_t h,
-                  uint32_t S, DistScale scale, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
-                  const RescanBufs &rb, unsigned long long *stats, cudaStream_t st) {
-  if (S > cap) return invalid("candidate buffer smaller than the survivor count");
-  if (B == 0) return KATO_OK;
-  const uint32_t sms = rank_tc_ctas();
-  const RowKey key{xhi, xnorm, ids, dc, h, scale};
-  KATO_CUDA(cudaMemsetAsync(rb.nlisted, 0, kRescanRounds * sizeof(uint32_t), st));
-  for (int r = 0; r < kRescanRounds; ++r) {
-    rescan_bound_kernel<<<B, 256, 0, st>>>(ids, qcount, qbuf, cap, S, r, rb.list,
-                                           rb.kbound, rb.nlisted + r, stats);
-    rescan_rows_kernel<<<4 * sms, 256, 0, st>>>(key, qhi, qnorm, probed, qprobes, list_off, p,
-                                                qcount, qbuf, cap, rb.list, rb.kbound,
-                                                rb.nlisted + r);
-  }
-  rescan_exact_kernel<<<B, 256, 0, st>>>(key, qhi, qnorm, probed, qprobes, list_off, p, S, qcount,
-                                         qbuf, cap);
-  KATO_LAUNCHED("overflow rescan kernels");
   return KATO_OK;
 }
 

@@ -65,6 +65,7 @@ __host__ __device__ inline uint32_t tc_take(uint32_t &o, uint32_t bytes, uint32_
   return at;
 }
 
+constexpr uint32_t kDropped = 0x80000000u;  // qcount flag: a record did not fit
 constexpr uint32_t kTcRows = 128;     // rows per tile of the statistics
 // Dimensions of a filtered item: one chunk of 128 bytes per row.
 constexpr uint32_t kTcFilterDims = 128;
@@ -134,24 +135,5 @@ int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, ui
                    DistScale scale, unsigned long long *found, cudaStream_t st);
 // CTAs of rank_tc (one per SM).
 uint32_t rank_tc_ctas();
-
-// Scratch of the overflow rescan: B listed queries, B 64-bit key bounds, and
-// one listed-query count per round.
-struct RescanBufs {
-  uint32_t *list;
-  unsigned long long *kbound;
-  uint32_t *nlisted;
-};
-constexpr uint32_t kRescanCounters = 4;
-
-// The queries whose candidate buffer overflowed are rescanned from the lists
-// (rare): afterwards their buffers hold every row that can be selected.
-// stats[0] counts them, stats[1] is the largest candidate count of a query.
-int rank_overflow(const uint8_t *xhi, const int64_t *xnorm, const uint32_t *ids,
-                  const uint8_t *qhi, const int64_t *qnorm, const uint32_t *probed,
-                  const uint32_t *qprobes, const uint32_t *list_off, uint32_t B, uint32_t p,
-                  uint32_t dc, uint32_t h,
-                  uint32_t S, DistScale scale, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
-                  const RescanBufs &rb, unsigned long long *stats, cudaStream_t st);
 
 }  // namespace kato

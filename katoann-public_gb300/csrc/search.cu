@@ -17,6 +17,7 @@
 
 #include <cuda_fp16.h>
 
+#include "finish.cuh"
 #include "kcommon.cuh"
 #include "probe.cuh"
 #include "rank_tc.cuh"
@@ -317,352 +318,6 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
   }
 }
 
-// ---------------------------------------------------- block selection helper
-// Chooses the `p` smallest of n entries by (key, id), where entry i gives
-// key = K(i) and id = I(i); keys == kEmpty are never chosen. Writes the chosen
-// (key << 32 | id, position) pairs into sel/pos (unsorted) and returns how
-// many were chosen (min(p, non-empty)). Radix selection over 8-bit digits,
-// first of the key, then of the id among the entries tied at the boundary key.
-template <class KeyF, class IdF>
-__device__ uint32_t block_select(uint32_t n, uint32_t p, KeyF K, IdF I, unsigned long long *sel,
-                                 uint32_t *pos, uint32_t *hist, uint32_t *scratch, uint32_t *wsum,
-                                 bool *boundary_tie) {
-  const uint32_t tid = threadIdx.x, nt = blockDim.x;
-  // count non-empty
-  if (tid == 0) scratch[0] = 0;
-  __syncthreads();
-  {
-    uint32_t m = 0;
-    for (uint32_t i = tid; i < n; i += nt) m += K(i) != kEmpty;
-    atomicAdd(&scratch[0], m);
-  }
-  __syncthreads();
-  const uint32_t valid = scratch[0];
-  __syncthreads();
-  const uint32_t want = min(p, valid);
-  *boundary_tie = false;
-  if (want == 0) return 0;
-  uint32_t T = kEmpty, idmax = 0xFFFFFFFFu;
-  if (want < valid) {
-    // radix select of the want-th key
-    uint32_t prefix = 0, rank = want - 1;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      for (uint32_t i = tid; i < 256; i += nt) hist[i] = 0;
-      __syncthreads();
-      const uint32_t hm = shift == 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      for (uint32_t i = tid; i < n; i += nt) {
-        const uint32_t k = K(i);
-        if (k != kEmpty && (k & hm) == prefix) atomicAdd(&hist[(k >> shift) & 0xFFu], 1u);
-      }
-      __syncthreads();
-      block_pick_digit(hist, rank, scratch + 1, wsum);
-      rank -= scratch[2];
-      prefix |= scratch[1] << shift;
-      __syncthreads();
-    }
-    T = prefix;
-    const uint32_t need = rank + 1;
-    if (tid == 0) scratch[3] = 0;
-    __syncthreads();
-    {
-      uint32_t m = 0;
-      for (uint32_t i = tid; i < n; i += nt) m += K(i) == T;
-      atomicAdd(&scratch[3], m);
-    }
-    __syncthreads();
-    const uint32_t neq = scratch[3];
-    *boundary_tie = neq > need;
-    if (neq > need) {
-      uint32_t ip = 0, ir = need - 1;
-      for (int shift = 24; shift >= 0; shift -= 8) {
-        for (uint32_t i = tid; i < 256; i += nt) hist[i] = 0;
-        __syncthreads();
-        const uint32_t hm = shift == 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-        for (uint32_t i = tid; i < n; i += nt) {
-          if (K(i) != T) continue;
-          const uint32_t id = I(i);
-          if ((id & hm) == ip) atomicAdd(&hist[(id >> shift) & 0xFFu], 1u);
-        }
-        __syncthreads();
-        block_pick_digit(hist, ir, scratch + 1, wsum);
-        ir -= scratch[2];
-        ip |= scratch[1] << shift;
-        __syncthreads();
-      }
-      idmax = ip;
-    }
-  }
-  if (tid == 0) scratch[4] = 0;
-  __syncthreads();
-  for (uint32_t i = tid; i < n; i += nt) {
-    const uint32_t k = K(i);
-    if (k == kEmpty) continue;
-    bool take = k < T;
-    uint32_t id = 0;
-    if (!take && k == T) {
-      id = I(i);
-      take = id <= idmax;
-    } else if (take) {
-      id = I(i);
-    }
-    if (take) {
-      const uint32_t at = atomicAdd(&scratch[4], 1u);
-      if (at < want) {
-        sel[at] = (static_cast<unsigned long long>(k) << 32) | id;
-        pos[at] = i;
-      }
-    }
-  }
-  __syncthreads();
-  return want;
-}
-
-// In-shared-memory bitonic sort of n (key, payload) pairs, ascending by key.
-__device__ void block_sort_pairs(unsigned long long *key, uint32_t *val, uint32_t n) {
-  uint32_t np2 = 1;
-  while (np2 < n) np2 <<= 1;
-  for (uint32_t i = n + threadIdx.x; i < np2; i += blockDim.x) {
-    key[i] = ~0ull;
-    val[i] = 0;
-  }
-  __syncthreads();
-  for (uint32_t size = 2; size <= np2; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = threadIdx.x; i < np2; i += blockDim.x) {
-        const uint32_t jx = i ^ stride;
-        if (jx > i) {
-          const bool up = (i & size) == 0;
-          const unsigned long long a = key[i], b = key[jx];
-          if ((a > b) == up) {
-            key[i] = b;
-            key[jx] = a;
-            const uint32_t tv = val[i];
-            val[i] = val[jx];
-            val[jx] = tv;
-          }
-        }
-      }
-      __syncthreads();
-    }
-}
-
-// -------------------------------------------------------------------- merge
-// Per query: the best S of its nprobe * SC slot entries (or of the first
-// qcount[q] entries of its candidate buffer) by (distance, id).
-// Ranked modes write the survivors in descending (distance, id) order - the
-// order in which the reference pops its merged heap into the refinement
-// (:1088-1112). The full mode writes the final top-k, ascending, padded.
-__global__ void __launch_bounds__(kThreads) merge_kernel(
-    const uint2 *__restrict__ slots, uint32_t per_query, const uint32_t *__restrict__ qcount,
-    const uint32_t *__restrict__ qprobes, uint32_t per_probe, const uint32_t *__restrict__ ids,
-    uint32_t S, bool final_topk, uint32_t k, uint2 *__restrict__ surv, uint32_t *__restrict__ nsurv,
-    uint32_t *__restrict__ out_ids, float *__restrict__ out_dists,
-    unsigned long long *__restrict__ tie_count) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t hist[256], scratch[8], wsum[8];
-  __shared__ bool tie;
-  unsigned long long *sel = reinterpret_cast<unsigned long long *>(smem);
-  uint32_t np2 = 1;
-  while (np2 < S) np2 <<= 1;
-  uint32_t *pos = reinterpret_cast<uint32_t *>(sel + np2);
-  const uint32_t q = blockIdx.x;
-  const uint2 *e = slots + static_cast<size_t>(q) * per_query;
-  // the tensor-core pass counts each query's candidates; on the CUDA-core
-  // pass a query's slots are its probes' (rank-major), of which the first
-  // budget ones were written
-  const uint32_t n = qcount    ? min(qcount[q], per_query)
-                     : qprobes ? min(per_query, qprobes[q] * per_probe)
-                               : per_query;
-  auto K = [&](uint32_t i) { return e[i].x; };
-  auto I = [&](uint32_t i) { return ids[e[i].y]; };
-  const uint32_t got = block_select(n, S, K, I, sel, pos, hist, scratch, wsum, &tie);
-  if (threadIdx.x == 0 && tie && tie_count) atomicAdd(tie_count, 1ull);
-  block_sort_pairs(sel, pos, got);
-  if (final_topk) {
-    for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
-      uint32_t id = 0xFFFFFFFFu;
-      float dd = 3.402823466e+38f;
-      if (i < got) {
-        id = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
-        dd = __uint_as_float(static_cast<uint32_t>(sel[i] >> 32));
-      }
-      out_ids[static_cast<size_t>(q) * k + i] = id;
-      out_dists[static_cast<size_t>(q) * k + i] = dd;
-    }
-    return;
-  }
-  for (uint32_t i = threadIdx.x; i < got; i += blockDim.x) {
-    const uint32_t src = got - 1 - i;  // descending
-    surv[static_cast<size_t>(q) * S + i] = e[pos[src]];
-  }
-  if (threadIdx.x == 0) nsurv[q] = got;
-}
-
-// ------------------------------------------------------------------- refine
-// Per query: exact distances of the survivors (in the order given), then the
-// reference's top-k heap: the first k enter, later ones replace the largest
-// (distance, id) when their distance is strictly smaller (:1113-1124); output
-// ascending by (distance, id), padded (emit_topk, :384-398).
-__global__ void __launch_bounds__(kThreads, 4) refine_kernel(
-    const uint8_t *__restrict__ qhi, const uint8_t *__restrict__ qlo,
-    const int64_t *__restrict__ qnorm, const uint8_t *__restrict__ xhi,
-    const uint8_t *__restrict__ xlo, const int64_t *__restrict__ xnorm,
-    const uint32_t *__restrict__ ids, uint32_t npts, uint32_t dc, const uint2 *__restrict__ surv,
-    const uint32_t *__restrict__ nsurv, uint32_t S, uint32_t k, DistScale scale,
-    uint32_t *__restrict__ out_ids, float *__restrict__ out_dists) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const uint32_t q = blockIdx.x, ns = nsurv[q];
-  const uint32_t n16 = dc / 16;                        // 16-byte words of a plane row
-  uint4 *sq = reinterpret_cast<uint4 *>(smem);         // [2][n16]
-  float *ex = reinterpret_cast<float *>(sq + 2 * n16);  // [S]
-  uint32_t *eid = reinterpret_cast<uint32_t *>(ex + S);  // [S]
-  float *hd = reinterpret_cast<float *>(eid + S);      // [k]
-  uint32_t *hid = reinterpret_cast<uint32_t *>(hd + k);  // [k]
-  uint32_t *srow = hid + k;                             // [S] the survivors' rows
-  for (uint32_t i = threadIdx.x; i < n16; i += blockDim.x) {
-    sq[i] = reinterpret_cast<const uint4 *>(qhi + static_cast<size_t>(q) * dc)[i];
-    sq[n16 + i] = reinterpret_cast<const uint4 *>(qlo + static_cast<size_t>(q) * dc)[i];
-  }
-  for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x)
-    srow[i] = surv[static_cast<size_t>(q) * S + i].y;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t nwarps = blockDim.x / 32;
-  const int64_t qn = qnorm[q];
-  // one survivor per warp step, its row loads issued before the products (a
-  // smaller register set than two survivors per step: four CTAs per SM)
-  for (uint32_t s0 = warp; s0 < ns; s0 += nwarps) {
-    const uint32_t r0 = srow[s0];
-    uint32_t id0 = 0;
-    int64_t xn0 = 0;
-    if (lane == 0) {
-      id0 = ids[r0];
-      xn0 = xnorm[r0];
-    }
-    const uint4 *h0 = reinterpret_cast<const uint4 *>(xhi + static_cast<size_t>(r0) * dc);
-    const uint4 *l0 = reinterpret_cast<const uint4 *>(xlo + static_cast<size_t>(r0) * dc);
-    uint32_t hh0 = 0, mx0 = 0, ll0 = 0;
-#pragma unroll 2
-    for (uint32_t u = lane; u < n16; u += 32) {
-      const uint4 bh0 = h0[u], bl0 = l0[u];
-      const uint4 ah = sq[u], al = sq[n16 + u];
-      const uint32_t a_h[4] = {ah.x, ah.y, ah.z, ah.w}, a_l[4] = {al.x, al.y, al.z, al.w};
-      const uint32_t b_h0[4] = {bh0.x, bh0.y, bh0.z, bh0.w}, b_l0[4] = {bl0.x, bl0.y, bl0.z, bl0.w};
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        hh0 = dp4(a_h[w], b_h0[w], hh0);
-        mx0 = dp4(a_h[w], b_l0[w], mx0);
-        mx0 = dp4(a_l[w], b_h0[w], mx0);
-        ll0 = dp4(a_l[w], b_l0[w], ll0);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      hh0 += __shfl_xor_sync(0xffffffffu, hh0, o);
-      mx0 += __shfl_xor_sync(0xffffffffu, mx0, o);
-      ll0 += __shfl_xor_sync(0xffffffffu, ll0, o);
-    }
-    if (lane == 0) {
-      const int64_t dot0 = static_cast<int64_t>((static_cast<uint64_t>(hh0) << 16) +
-                                                (static_cast<uint64_t>(mx0) << 8) + ll0);
-      ex[s0] = dist_value(qn + xn0 - 2 * dot0, scale);
-      eid[s0] = id0;
-    }
-  }
-  __syncthreads();
-  // The reference's heap (:1113-1124), survivors in the given order: the
-  // first k enter; a later one replaces the largest (distance, id) when its
-  // distance is strictly smaller; then ascending by (distance, id).
-  if (k <= 32) {
-    // one warp holds the heap sorted descending by (distance, id) across its
-    // lanes - lane 0 is the largest, the one the reference evicts - so an
-    // insertion is one ballot and one shift; unused lanes sort below all
-    if (warp != 0) return;
-    const uint32_t u = static_cast<uint32_t>(lane);
-    float d = -1.0f;
-    uint32_t id = 0u, n = 0;
-    for (uint32_t s = 0; s < ns; ++s) {
-      const float dd = ex[s];
-      const uint32_t ii = eid[s];
-      if (ii >= npts) continue;  // ids without a row are skipped (:1091-1094)
-      const bool gt = d > dd || (d == dd && id > ii);  // this slot sorts above the new one
-      if (n < k) {
-        // enters after the g larger ones; the rest move up one lane
-        const uint32_t g = __popc(__ballot_sync(0xffffffffu, gt && u < n));
-        const float ud = __shfl_up_sync(0xffffffffu, d, 1);
-        const uint32_t uid = __shfl_up_sync(0xffffffffu, id, 1);
-        if (u == g) {
-          d = dd;
-          id = ii;
-        } else if (u > g && u <= n) {
-          d = ud;
-          id = uid;
-        }
-        ++n;
-        continue;
-      }
-      if (!(dd < __shfl_sync(0xffffffffu, d, 0))) continue;  // strictly below the largest
-      // the largest leaves; the g larger ones below it move down one lane
-      const uint32_t g = __popc(__ballot_sync(0xffffffffu, gt && u >= 1 && u < k));
-      const float nd = __shfl_down_sync(0xffffffffu, d, 1);
-      const uint32_t nid = __shfl_down_sync(0xffffffffu, id, 1);
-      if (u < g) {
-        d = nd;
-        id = nid;
-      } else if (u == g) {
-        d = dd;
-        id = ii;
-      }
-    }
-    if (u < n) {  // ascending: lane u is the (n - 1 - u)-th
-      out_ids[static_cast<size_t>(q) * k + (n - 1 - u)] = id;
-      out_dists[static_cast<size_t>(q) * k + (n - 1 - u)] = d;
-    } else if (u < k) {
-      out_ids[static_cast<size_t>(q) * k + u] = 0xFFFFFFFFu;
-      out_dists[static_cast<size_t>(q) * k + u] = 3.402823466e+38f;
-    }
-    return;
-  }
-  if (threadIdx.x == 0) {
-    uint32_t n = 0;
-    for (uint32_t s = 0; s < ns; ++s) {
-      const float dd = ex[s];
-      const uint32_t id = eid[s];
-      if (id >= npts) continue;  // ids without a row are skipped (:1091-1094)
-      if (n < k) {
-        hd[n] = dd;
-        hid[n] = id;
-        ++n;
-        continue;
-      }
-      uint32_t mi = 0;  // the largest (distance, id)
-      for (uint32_t i = 1; i < n; ++i)
-        if (hd[i] > hd[mi] || (hd[i] == hd[mi] && hid[i] > hid[mi])) mi = i;
-      if (dd < hd[mi]) {
-        hd[mi] = dd;
-        hid[mi] = id;
-      }
-    }
-    // ascending by (distance, id)
-    for (uint32_t i = 1; i < n; ++i) {
-      const float d0 = hd[i];
-      const uint32_t i0 = hid[i];
-      uint32_t m = i;
-      while (m > 0 && (hd[m - 1] > d0 || (hd[m - 1] == d0 && hid[m - 1] > i0))) {
-        hd[m] = hd[m - 1];
-        hid[m] = hid[m - 1];
-        --m;
-      }
-      hd[m] = d0;
-      hid[m] = i0;
-    }
-    for (uint32_t i = 0; i < k; ++i) {
-      out_ids[static_cast<size_t>(q) * k + i] = i < n ? hid[i] : 0xFFFFFFFFu;
-      out_dists[static_cast<size_t>(q) * k + i] = i < n ? hd[i] : 3.402823466e+38f;
-    }
-  }
-}
-
 }  // namespace
 
 // ------------------------------------------------------------ orchestration
@@ -724,9 +379,9 @@ struct Plan {
   uint32_t tcitems, cap, seed_rows, ctas, rec_cap, beta;
   bool cost;                        // the ranking CTAs split the slabs' cost, not their count
   size_t off_fq, off_qhi, off_qlo, off_qn, off_qhn, off_qh0, off_cd, off_probed, off_cnt, off_off,
-      off_woff, off_cur, off_work, off_ent, off_slots, off_surv, off_nsurv, off_stats,
+      off_woff, off_cur, off_work, off_ent, off_slots, off_stats,
       off_tcscratch, off_tcitems, off_tileoff, off_qcount,  off_bound,
-      off_rec, off_recn, off_rlist, off_rkey, off_rcount, off_qh16, off_ql16, off_qterm, off_rot,
+      off_rec, off_recn, off_qh16, off_ql16, off_qterm, off_rot,
       off_qprobes, off_z, off_qcn, off_qr16, off_share, off_seedorder, total;
 };
 
@@ -815,14 +470,9 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_qcn = take(planes ? static_cast<size_t>(B) * sizeof(int2) : 16);
   pl.off_qterm = take(static_cast<size_t>(B) * 8);
   pl.off_rot = take(ix->rotated ? rotate_scratch_bytes(B, ix->dim) : 16);
-  pl.off_rlist = take(static_cast<size_t>(B) * 4);
-  pl.off_rkey = take(static_cast<size_t>(B) * 8);
-  pl.off_rcount = take(kRescanCounters * 4);
   pl.off_qprobes = take(static_cast<size_t>(B) * 4);
   pl.off_seedorder = take(static_cast<size_t>(B) * 4);
   pl.off_z = take(static_cast<size_t>(B) * KATO_PROBE_FEATURES * 4);
-  pl.off_surv = take(static_cast<size_t>(B) * pl.S * sizeof(uint2));
-  pl.off_nsurv = take(static_cast<size_t>(B) * 4);
   pl.total = o;
   return KATO_OK;
 }
@@ -911,8 +561,6 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   Work *work = reinterpret_cast<Work *>(ws + pl.off_work);
   uint32_t *ent = reinterpret_cast<uint32_t *>(ws + pl.off_ent);
   uint2 *slots = reinterpret_cast<uint2 *>(ws + pl.off_slots);
-  uint2 *surv = reinterpret_cast<uint2 *>(ws + pl.off_surv);
-  uint32_t *nsurv = reinterpret_cast<uint32_t *>(ws + pl.off_nsurv);
   unsigned long long *stats = reinterpret_cast<unsigned long long *>(ws + pl.off_stats);
 
   // with a model, the selection first goes as deep as its features and then,
@@ -1009,13 +657,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, nq, ix->d_hi, qhi, T.qcn, bound, dc,
                              pl.tcs.f, pl.dims, qcount, slots, pl.cap, scale, stats + 5, st)))
       return rc;
-    const RescanBufs rb{reinterpret_cast<uint32_t *>(ws + pl.off_rlist),
-                        reinterpret_cast<unsigned long long *>(ws + pl.off_rkey),
-                        reinterpret_cast<uint32_t *>(ws + pl.off_rcount)};
-    if ((rc = rank_overflow(ix->d_hi, xnorm, ix->d_ids, qhi, qnorm, probed, qprobes, ix->d_list_off, nq, p,
-                            dc, pl.dims, pl.S, scale, qcount, slots, pl.cap, rb, stats + 6, st)))
-      return rc;
-    g_launches += 11;  // seed, 3 preparation, scan, bucket, 2 x 2 rescan rounds, exact rescan
+    g_launches += 6;  // seed, 3 preparation, scan, bucket
   }
   // 4. ranking pass (:998-1044 / :1167-1204)
   const bool full = pl.ranking == KATO_RANK_FULL;
@@ -1058,35 +700,49 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     ++g_launches;
   }
   mark(tm, 7, st);
-  // 5. per-query merge of the slot lists (:1058-1080 / :1205-1218)
-  uint32_t np2 = 1;
-  while (np2 < pl.S) np2 <<= 1;
-  const size_t msmem = static_cast<size_t>(np2) * 12;
-  if ((rc = smem_limit(reinterpret_cast<const void *>(merge_kernel), static_cast<int>(msmem),
-                       "merge_kernel shared memory")))
-    return rc;
-  merge_kernel<<<nq, kThreads, msmem, st>>>(slots, pl.tc ? pl.cap : p * pl.SC, qcount, qprobes,
-                                            pl.SC, ix->d_ids, pl.S, full, pl.k, surv, nsurv,
-                                            out_ids, out_dists, stats + 1);
-  ++g_launches;
-  KATO_LAUNCHED("merge_kernel");
-  mark(tm, 8, st);
+  // 5. the best of the slot lists: of the exact distances the top-k (:1205-1218),
+  // of the ranking distances the survivors, their exact distances and the
+  // top-k (:1058-1125)
   if (full) {
-    mark(tm, 9, st);
-    if (tm && tm->used < tm->max_passes) ++tm->used;
-    return KATO_OK;
+    rc = merge_topk(slots, p * pl.SC, pl.SC, qprobes, ix->d_ids, nq, pl.k, out_ids, out_dists, stats + 1, st);
+  } else {
+    FinishArgs F{};
+    F.slots = slots;
+    F.per_query = pl.tc ? pl.cap : p * pl.SC;
+    F.per_probe = pl.SC;
+    F.qcount = qcount;
+    F.qprobes = qprobes;
+    F.qhi = qhi;
+    F.qlo = qlo;
+    F.qnorm = qn;
+    F.xhi = ix->d_hi;
+    F.xlo = ix->d_lo;
+    F.xnorm = ix->d_norm;
+    F.ids = ix->d_ids;
+    F.npts = ix->npts;
+    F.dc = dc;
+    F.S = pl.S;
+    F.k = pl.k;
+    F.scale = make_dist_scale(ix->step_sq);
+    F.out_ids = out_ids;
+    F.out_dists = out_dists;
+    F.ties = stats + 1;
+    F.rescans = stats + 6;
+    if (pl.tc) {
+      const bool prefix_mode = pl.ranking == KATO_RANK_PREFIX;
+      F.rank_xnorm = prefix_mode ? ix->d_headnorm : ix->d_hinorm;
+      F.rank_qnorm = prefix_mode ? qh0 : qhn;
+      F.probed = probed;
+      F.list_off = ix->d_list_off;
+      F.h = pl.dims;
+      F.nprobe = p;
+    }
+    mark(tm, 8, st);  // the survivor merge is part of the refinement kernel
+    rc = finish(F, nq, st);
   }
-  // 6. exact refinement and top-k (:1081-1125)
-  const size_t rsmem = static_cast<size_t>(dc) * 2 + static_cast<size_t>(pl.S) * 12 +
-                       static_cast<size_t>(pl.k) * 8;
-  if ((rc = smem_limit(reinterpret_cast<const void *>(refine_kernel), static_cast<int>(rsmem),
-                       "refine_kernel shared memory")))
-    return rc;
-  refine_kernel<<<nq, kThreads, rsmem, st>>>(qhi, qlo, qn, ix->d_hi, ix->d_lo, ix->d_norm,
-                                             ix->d_ids, ix->npts, dc, surv, nsurv, pl.S, pl.k,
-                                             make_dist_scale(ix->step_sq), out_ids, out_dists);
-  KATO_LAUNCHED("refine_kernel");
+  if (rc) return rc;
   ++g_launches;
+  if (full) mark(tm, 8, st);
   mark(tm, 9, st);
   if (tm && tm->used < tm->max_passes) ++tm->used;
   return KATO_OK;
