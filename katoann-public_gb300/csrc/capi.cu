@@ -95,8 +95,7 @@ void graph_destroy(void *h);
 void *timer_create(uint32_t max_passes);
 uint32_t last_launches();
 int centre_planes(const uint8_t *hi, const uint8_t *lo, const int64_t *norm, uint32_t rows,
-                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, const RankRows &rr,
-                  cudaStream_t st);
+                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, cudaStream_t st);
 bool coarse_tc_ok(uint32_t dc);
 int kmeans_assign(const float *x, uint32_t n, uint32_t ld, const float *cen, const float *cnorm,
                   uint32_t L, uint32_t *assign, float *best, uint32_t *timeouts, cudaStream_t st);
@@ -196,7 +195,7 @@ int katoann_gpu_coarse(const katoann_gpu_index *ix, const uint8_t *d_qhi, const 
     auto *qterm = reinterpret_cast<int64_t *>(static_cast<unsigned char *>(scratch) + 2 * plane);
     auto *flag = reinterpret_cast<uint32_t *>(qterm + nq);
     rc = cudaMemsetAsync(flag, 0, 4, st) != cudaSuccess ? KATO_ERUNTIME : KATO_OK;
-    if (!rc) rc = kato::centre_planes(d_qhi, d_qlo, d_qnorm, nq, ix->dc, qh16, ql16, qterm, kato::RankRows{}, st);
+    if (!rc) rc = kato::centre_planes(d_qhi, d_qlo, d_qnorm, nq, ix->dc, qh16, ql16, qterm, st);
     if (!rc)
       rc = kato::coarse_tc(reinterpret_cast<const __half *>(ix->d_chi16),
                            reinterpret_cast<const __half *>(ix->d_clo16), ix->d_cterm, ix->nlist,
@@ -356,8 +355,7 @@ int katoann_gpu_centre_planes(const uint8_t *d_hi, const uint8_t *d_lo, const in
                               uint32_t rows, uint32_t dc, uint16_t *d_hi16, uint16_t *d_lo16,
                               int64_t *d_term, katoann_stream_t stream) {
   return kato::centre_planes(d_hi, d_lo, d_norm, rows, dc, reinterpret_cast<__half *>(d_hi16),
-                             reinterpret_cast<__half *>(d_lo16), d_term,
-                             kato::RankRows{}, as_stream(stream));
+                             reinterpret_cast<__half *>(d_lo16), d_term, as_stream(stream));
 }
 
 int katoann_gpu_set_seed_rows(uint32_t rows) {

@@ -147,8 +147,9 @@ __device__ __forceinline__ uint32_t block_scan_bins(uint32_t *hist, uint32_t ran
 // (8-bit radix digits of the p-th key, then of the tied indices, then the
 // gather). sel holds np2(p) 64-bit words, hist 256 counters, scal 4 words.
 __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uint32_t p,
-                              uint32_t *__restrict__ outp, unsigned long long *__restrict__ tie_count,
-                              unsigned long long *sel, uint32_t *hist, uint32_t *scal) {
+                              uint32_t *__restrict__ outp, uint32_t *__restrict__ cnt,
+                              unsigned long long *__restrict__ tie_count, unsigned long long *sel,
+                              uint32_t *hist, uint32_t *scal) {
   const uint32_t tid = threadIdx.x;
   // 1) the p-th smallest key (rank p-1), and how many keys are below it.
   uint32_t prefix = 0, rank = p - 1, below = 0;
@@ -202,6 +203,7 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
     const uint32_t k = keys[i];
     if (k < T || (k == T && i <= idmax)) {
       const uint32_t pos = atomicAdd(&scal[2], 1u);
+      if (cnt) atomicAdd(&cnt[i], 1u);
       if (sorted) sel[pos] = (static_cast<unsigned long long>(k) << 32) | i;
       else outp[pos] = i;
     }
@@ -232,19 +234,21 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
   for (uint32_t i = tid; i < p; i += kSelThreads) outp[i] = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
 }
 
-// Rows are written `stride` apart. With `only`, rows whose only[q] is at
+// Rows are written `stride` apart. With `cnt`, each selected list's counter
+// there is incremented (the inversion's counts). With `only`, rows whose only[q] is at
 // most only_above are skipped (a second, deeper selection for the queries
 // that need it).
 __global__ void __launch_bounds__(kSelThreads) select_topp_kernel(
     const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride,
-    uint32_t *__restrict__ probed, unsigned long long *__restrict__ tie_count,
-    const uint32_t *__restrict__ only, uint32_t only_above) {
+    uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
+    unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
+    uint32_t only_above) {
   extern __shared__ unsigned long long sel[];  // up to kSortMax (key << 32 | id)
   __shared__ uint32_t hist[256], scal[4];
   const uint32_t q = blockIdx.x;
   if (only && only[q] <= only_above) return;
   select_passes(reinterpret_cast<const uint32_t *>(dists) + static_cast<size_t>(q) * n, n, p,
-                probed + static_cast<size_t>(q) * stride, tie_count, sel, hist, scal);
+                probed + static_cast<size_t>(q) * stride, cnt, tie_count, sel, hist, scal);
 }
 
 // In-shared-memory bitonic sort of n 64-bit keys, ascending.
@@ -282,8 +286,9 @@ constexpr uint32_t kCand = 2048;
 
 __global__ void __launch_bounds__(kSelThreads) select_topp_hist_kernel(
     const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride,
-    uint32_t *__restrict__ probed, unsigned long long *__restrict__ tie_count,
-    const uint32_t *__restrict__ only, uint32_t only_above) {
+    uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
+    unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
+    uint32_t only_above) {
   extern __shared__ unsigned long long dyn[];
   unsigned long long *cand = dyn;          // kCand
   unsigned long long *sel = dyn + kCand;   // np2(p)
@@ -340,7 +345,7 @@ __global__ void __launch_bounds__(kSelThreads) select_topp_hist_kernel(
   __syncthreads();
   const uint32_t bstar = scal[0], below = scal[1], c = hist[bstar];
   if (c > kCand) {  // a crowded boundary bin: the radix passes instead
-    select_passes(keys, n, p, outp, tie_count, sel, hist, scal + 4);
+    select_passes(keys, n, p, outp, cnt, tie_count, sel, hist, scal + 4);
     return;
   }
   // 3) gather: bins below the boundary are in; the boundary bin is a candidate
@@ -368,7 +373,11 @@ __global__ void __launch_bounds__(kSelThreads) select_topp_hist_kernel(
   __syncthreads();
   // 5) the p selected in order
   sort_keys(sel, p);
-  for (uint32_t i = tid; i < p; i += kSelThreads) outp[i] = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
+  for (uint32_t i = tid; i < p; i += kSelThreads) {
+    const uint32_t c = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
+    outp[i] = c;
+    if (cnt) atomicAdd(&cnt[c], 1u);
+  }
 }
 
 __global__ void dist_values_kernel(const int64_t *l2, uint32_t n, DistScale s, float *out) {
@@ -395,8 +404,8 @@ int sq16_tiles(const uint8_t *qhi, const uint8_t *qlo, const uint8_t *xhi, const
 }
 
 int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint32_t stride,
-                   uint32_t *probed, unsigned long long *tie_count, const uint32_t *only,
-                   uint32_t only_above, cudaStream_t st) {
+                   uint32_t *probed, uint32_t *cnt, unsigned long long *tie_count,
+                   const uint32_t *only, uint32_t only_above, cudaStream_t st) {
   if (nq == 0) return KATO_OK;
   if (p == 0 || p > n || stride < p) return invalid("need 1 <= nprobe <= nlist");
   uint32_t np2 = 1;
@@ -410,20 +419,20 @@ int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint
   if (p <= kSortMax) {
     // candidates and the sorted selection (the bitonic sort pads to a power of two)
     const size_t smem = (kCand + std::max<uint32_t>(np2, 2)) * sizeof(unsigned long long);
-    select_topp_hist_kernel<<<nq, kSelThreads, smem, st>>>(dists, n, p, stride, probed, tie_count,
-                                                            only, only_above);
+    select_topp_hist_kernel<<<nq, kSelThreads, smem, st>>>(dists, n, p, stride, probed, cnt,
+                                                            tie_count, only, only_above);
     KATO_LAUNCHED("select_topp_hist_kernel");
     return KATO_OK;
   }
-  select_topp_kernel<<<nq, kSelThreads, 0, st>>>(dists, n, p, stride, probed, tie_count, only,
-                                                  only_above);
+  select_topp_kernel<<<nq, kSelThreads, 0, st>>>(dists, n, p, stride, probed, cnt, tie_count,
+                                                  only, only_above);
   KATO_LAUNCHED("select_topp_kernel");
   return KATO_OK;
 }
 
 int select_topp(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint32_t *probed,
                 unsigned long long *tie_count, cudaStream_t st) {
-  return select_topp_ex(dists, nq, n, p, p, probed, tie_count, nullptr, 0, st);
+  return select_topp_ex(dists, nq, n, p, p, probed, nullptr, tie_count, nullptr, 0, st);
 }
 
 int dist_values(const int64_t *l2, uint32_t n, double step_sq, float *out, cudaStream_t st) {

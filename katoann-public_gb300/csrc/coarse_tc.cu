@@ -36,7 +36,6 @@
 #include <algorithm>
 
 #include "kcommon.cuh"
-#include "rank_tc.cuh"
 #include "tc.cuh"
 
 namespace kato {
@@ -73,29 +72,16 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
 __global__ void __launch_bounds__(256) centre_planes_kernel(
     const uint8_t *__restrict__ hi, const uint8_t *__restrict__ lo, const int64_t *__restrict__ norm,
     uint32_t rows, uint32_t dc, __half *__restrict__ hi16, __half *__restrict__ lo16,
-    int64_t *__restrict__ term, const RankRows rr) {
+    int64_t *__restrict__ term) {
   const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
-  int32_t sh = 0, sl = 0, cf = 0, ch = 0;
+  int32_t sh = 0, sl = 0;
   for (uint32_t u = lane; u < dc / 16; u += 32) {
     const size_t at = static_cast<size_t>(row) * dc + u * 16;
     const uint4 vh = *reinterpret_cast<const uint4 *>(hi + at);
     const uint4 vl = *reinterpret_cast<const uint4 *>(lo + at);
     uint4 a, b;
-    if (rr.rows && u * 16 < rr.width) {  // f <= h <= width, multiples of 64
-      uint4 ra = make_uint4(0, 0, 0, 0), rb = ra;
-      if (u * 16 < rr.h) {
-        tc::bytes_to_half16(vh, rr.centred ? bias : __floats2half2_rn(1024.0f, 1024.0f), ra, rb);
-        const int32_t c = rr.centred ? tc::centred_sq_sum16(vh)
-                                     : static_cast<int32_t>(dp4(vh.x, vh.x, dp4(vh.y, vh.y, dp4(vh.z, vh.z, dp4(vh.w, vh.w, 0)))));
-        ch += c;
-        if (u * 16 < rr.f) cf += c;
-      }
-      __half *o = rr.rows + static_cast<size_t>(row) * rr.width + u * 16;
-      *reinterpret_cast<uint4 *>(o) = ra;
-      *reinterpret_cast<uint4 *>(o + 8) = rb;
-    }
     tc::bytes_to_half16(vh, bias, a, b);
     *reinterpret_cast<uint4 *>(hi16 + at) = a;
     *reinterpret_cast<uint4 *>(hi16 + at + 8) = b;
@@ -109,13 +95,9 @@ __global__ void __launch_bounds__(256) centre_planes_kernel(
   for (int o = 16; o; o >>= 1) {
     sh += __shfl_xor_sync(0xffffffffu, sh, o);
     sl += __shfl_xor_sync(0xffffffffu, sl, o);
-    cf += __shfl_xor_sync(0xffffffffu, cf, o);
-    ch += __shfl_xor_sync(0xffffffffu, ch, o);
   }
-  if (lane == 0) {
-    if (rr.rows) rr.norms[row] = make_int2(cf, ch);
+  if (lane == 0)
     term[row] = norm[row] - 256 * (65792ll * sh + 257ll * sl) - 16384ll * dc * 66049ll;
-  }
 }
 
 struct CoarseArgs {
@@ -338,11 +320,10 @@ int encode_plane(CUtensorMap *map, const __half *base, uint32_t rows, uint32_t d
 }  // namespace
 
 int centre_planes(const uint8_t *hi, const uint8_t *lo, const int64_t *norm, uint32_t rows,
-                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, const RankRows &rr,
-                  cudaStream_t st) {
+                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, cudaStream_t st) {
   if (rows == 0) return KATO_OK;
   if (dc == 0 || dc % 64) return invalid("dc must be a positive multiple of 64");
-  centre_planes_kernel<<<div_up(rows, 8), 256, 0, st>>>(hi, lo, norm, rows, dc, hi16, lo16, term, rr);
+  centre_planes_kernel<<<div_up(rows, 8), 256, 0, st>>>(hi, lo, norm, rows, dc, hi16, lo16, term);
   KATO_LAUNCHED("centre_planes_kernel");
   return KATO_OK;
 }

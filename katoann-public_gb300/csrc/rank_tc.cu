@@ -573,28 +573,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // and how many bytes it costs: 2,048 sketched rows (32 bytes each) and 3S
 // scored rows read 2.3 times fewer bytes than 1,024 scored rows of 256 bytes
 // and leave fewer candidates. Fewer than S rows: no bound.
-// The queries grouped by their nearest list: a counting sort by one CTA, so
-// that seed CTAs reading the same list's rows run together and share them
-// through L2. order[i] = the query the i-th seed CTA takes.
-constexpr uint32_t kOrderLists = 16384;  // lists the counting sort holds in shared memory
-
-__global__ void __launch_bounds__(1024) seed_order_kernel(const uint32_t *__restrict__ probed,
-                                                          uint32_t p, uint32_t B, uint32_t L,
-                                                          uint32_t *__restrict__ order) {
-  extern __shared__ uint32_t lh[];  // L counters, then offsets
-  for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) lh[i] = 0;
-  __syncthreads();
-  for (uint32_t q = threadIdx.x; q < B; q += blockDim.x)
-    atomicAdd(&lh[probed[static_cast<size_t>(q) * p]], 1u);
-  __syncthreads();
-  block_scan2(
-      L, [&](uint32_t i) { return make_uint2(lh[i], 0u); },
-      [&](uint32_t i, uint32_t a, uint32_t) { lh[i] = a; });
-  __syncthreads();
-  for (uint32_t q = threadIdx.x; q < B; q += blockDim.x)
-    order[atomicAdd(&lh[probed[static_cast<size_t>(q) * p]], 1u)] = q;
-}
-
 constexpr uint32_t kSketchBytes = 32;  // head bytes of a row the sketch reads
 
 __device__ __forceinline__ uint32_t sq_diff4(uint32_t a, uint32_t b, uint32_t acc) {
@@ -606,14 +584,14 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint8_t *__restrict__ xhi, const int64_t *__restrict__ xnorm,
     const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
     const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
-    const uint32_t *__restrict__ list_off, const uint32_t *__restrict__ order, uint32_t p,
+    const uint32_t *__restrict__ list_off, uint32_t p,
     uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, int32_t *__restrict__ bound) {
   // rowof: the rows looked at; val: their sketch keys. After the pick the
   // scored rows are in val and their l2 go to rowof.
   __shared__ uint32_t rowof[kSeedCap], val[kSeedCap];
   __shared__ __align__(16) uint32_t qw[2048 / 4];
   __shared__ uint32_t hist[256], sel[2], wsum[8], npick;
-  const uint32_t q = order ? order[blockIdx.x] : blockIdx.x, tid = threadIdx.x;
+  const uint32_t q = blockIdx.x, tid = threadIdx.x;
   for (uint32_t i = tid; i < h / 4; i += blockDim.x)
     qw[i] = reinterpret_cast<const uint32_t *>(qhi + static_cast<size_t>(q) * dc)[i];
   const uint32_t pq = qprobes ? qprobes[q] : p;  // the query's own budget
@@ -703,133 +681,6 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
   if (tid == 0) {
     const int32_t v = static_cast<int32_t>(L2);
     bound[q] = v + (v >> 22) + 1;
-  }
-}
-
-// -------------------------------------------------- work items and offsets
-// The cost of a slab of an item of ne queries: by default in steps of about
-// 20 instructions (180 for the rows and 40 per group of 8 queries), or
-// 64 + beta * width (16, 32 or N queries).
-__device__ __forceinline__ uint32_t slab_cost(uint32_t ne, uint32_t N, uint32_t beta) {
-  if (beta == 0) return 9 + 2 * ((ne + 7) / 8);
-  return 64 + beta * (ne <= 16 ? 16u : (ne <= 32 && N > 32 ? 32u : N));
-}
-
-// Per list: items = ceil(queries / N) (none for an empty list), slabs per
-// item = ceil(rows / 64); counts[c] = items, counts[L + 1 + c] = items x slabs.
-// probed (optional, 2 counters): the distinct lists the batch probes (not
-// empty) and their rows, i.e. the rows the pass reads once each.
-__global__ void tc_count_kernel(const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ list_off,
-                                uint32_t L, uint32_t N, uint32_t B, uint32_t beta, bool cost,
-                                uint32_t *__restrict__ counts, uint32_t *__restrict__ qcount,
-                                unsigned long long *__restrict__ probed) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < B) qcount[c] = 0;
-  uint32_t lists = 0, rows = 0;
-  if (c < L) {
-    const uint32_t n = list_off[c + 1] - list_off[c];
-    const uint32_t items = n ? (cnt[c] + N - 1) / N : 0;
-    const uint32_t slabs = (n + kTcSlab - 1) / kTcSlab;
-    counts[c] = items;
-    counts[L + 1 + c] = items * slabs;
-    if (cost) {  // full items first, then the remainder
-      const uint32_t full = n ? cnt[c] / N : 0, rem = n ? cnt[c] % N : 0;
-      counts[2 * (L + 1) + c] =
-          slabs * (full * slab_cost(N, N, beta) + (rem ? slab_cost(rem, N, beta) : 0));
-    }
-    if (items) lists = 1, rows = n;
-  }
-  if (probed) {  // whole warps take part: one add per warp and counter
-    const uint32_t wl = __reduce_add_sync(0xffffffffu, lists);
-    const uint32_t wr = __reduce_add_sync(0xffffffffu, rows);
-    if ((threadIdx.x & 31) == 0 && wl) {
-      atomicAdd(probed, static_cast<unsigned long long>(wl));
-      atomicAdd(probed + 1, static_cast<unsigned long long>(wr));
-    }
-  }
-}
-
-// Exclusive scans of the count arrays by one CTA of 1024 threads (in place),
-// with the totals after them; the totals also end the slab offsets and the
-// shares (tile_off[items] and share[ctas]).
-__global__ void __launch_bounds__(1024) tc_scan_kernel(uint32_t *__restrict__ counts, uint32_t L,
-                                                       bool by_cost, uint32_t *__restrict__ tile_off,
-                                                       uint2 *__restrict__ share, uint32_t ctas) {
-  uint32_t *ca = counts, *cb = counts + L + 1, *cc = counts + 2 * (L + 1);
-  const uint2 tot = block_scan2(
-      L, [&](uint32_t i) { return make_uint2(ca[i], cb[i]); },
-      [&](uint32_t i, uint32_t a, uint32_t b) {
-        ca[i] = a;
-        cb[i] = b;
-      });
-  uint32_t cost = tot.y;
-  if (by_cost) {
-    __syncthreads();
-    cost = block_scan2(
-               L, [&](uint32_t i) { return make_uint2(cc[i], 0u); },
-               [&](uint32_t i, uint32_t a, uint32_t) { cc[i] = a; })
-               .x;
-  }
-  if (threadIdx.x == 0) {
-    ca[L] = tot.x;
-    cb[L] = tot.y;
-    cc[L] = cost;
-    tile_off[tot.x] = tot.y;
-  }
-  // no work: every share is empty (the shares' starts come with the items)
-  if (tot.x == 0)
-    for (uint32_t i = threadIdx.x; i <= ctas; i += blockDim.x) share[i] = make_uint2(0, 0);
-  else if (threadIdx.x == 0) share[ctas] = make_uint2(tot.y, tot.x);
-}
-
-// tile_hist (optional, 6 counters): the 128-row tiles of the items with 1-2,
-// 3-4, 5-8, 9-16, 17-32 and 33-64 queries; all_tiles: their sum.
-__global__ void tc_expand_kernel(const uint32_t *__restrict__ list_off, const uint32_t *__restrict__ counts,
-                                 const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ off,
-                                 uint32_t L, uint32_t N, uint32_t beta, bool by_cost, uint32_t ctas,
-                                 TcItem *__restrict__ items, uint32_t *__restrict__ tile_off,
-                                 uint2 *__restrict__ share, unsigned long long *__restrict__ tile_hist,
-                                 unsigned long long *__restrict__ all_tiles) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t hist[6] = {0, 0, 0, 0, 0, 0};
-  const uint32_t *unit = counts + (by_cost ? 2 : 1) * (L + 1);  // a list's first unit
-  if (c < ctas && unit[L]) {
-    // share c starts at unit total * c / ctas: the list that holds it, then
-    // the item (every one before a list's last is full) and the slab
-    const uint32_t u = static_cast<uint32_t>(static_cast<uint64_t>(unit[L]) * c / ctas);
-    uint32_t lo = 0, hi = L;  // unit[lo] <= u < unit[hi]
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) / 2;
-      if (unit[mid] <= u) lo = mid;
-      else hi = mid;
-    }
-    const uint32_t slabs = (list_off[lo + 1] - list_off[lo] + kTcSlab - 1) / kTcSlab;
-    const uint32_t full = slabs * (by_cost ? slab_cost(N, N, beta) : 1), in = u - unit[lo];
-    const uint32_t j = min(in / full, (cnt[lo] - 1) / N);
-    const uint32_t per = by_cost ? slab_cost(min(N, cnt[lo] - j * N), N, beta) : 1;
-    share[c] = make_uint2(counts[L + 1 + lo] + j * slabs + (in - j * full) / per, counts[lo] + j);
-  }
-  if (c < L) {
-    const uint32_t i0 = counts[c], i1 = counts[c + 1];
-    const uint32_t row0 = list_off[c], rows = list_off[c + 1] - row0;
-    const uint32_t slabs = (rows + kTcSlab - 1) / kTcSlab, tiles = (rows + kTcRows - 1) / kTcRows;
-    const uint32_t tb = counts[L + 1 + c];
-    for (uint32_t j = 0; j < i1 - i0; ++j) {
-      const uint32_t ne = min(N, cnt[c] - j * N);
-      items[i0 + j] = TcItem{off[c] + j * N, ne, row0, rows};
-      tile_off[i0 + j] = tb + j * slabs;
-      hist[ne <= 2 ? 0 : ne <= 4 ? 1 : ne <= 8 ? 2 : ne <= 16 ? 3 : ne <= 32 ? 4 : 5] += tiles;
-    }
-  }
-  if (tile_hist) {  // whole warps take part: one add per warp and bin
-    uint32_t all = 0;
-#pragma unroll
-    for (int b = 0; b < 6; ++b) {
-      const uint32_t v = __reduce_add_sync(0xffffffffu, hist[b]);
-      if ((threadIdx.x & 31) == 0 && v) atomicAdd(tile_hist + b, static_cast<unsigned long long>(v));
-      all += v;
-    }
-    if ((threadIdx.x & 31) == 0 && all) atomicAdd(all_tiles, static_cast<unsigned long long>(all));
   }
 }
 
@@ -979,40 +830,17 @@ int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, ui
 }
 
 int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, const int64_t *qnorm,
-              const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off,
-              uint32_t L, uint32_t B, uint32_t p, uint32_t dc, uint32_t h, uint32_t S,
-              uint32_t rows, uint32_t *order, int32_t *bound, cudaStream_t st) {
+              const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off, uint32_t B,
+              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, int32_t *bound,
+              cudaStream_t st) {
   if (h > 2048 || h % 16) return invalid("seed bounds need h <= 2048, a multiple of 16");
   if (B == 0) return KATO_OK;
-  const uint32_t *ord = nullptr;
-  if (order && L <= kOrderLists) {
-    if (const int rc = smem_limit(reinterpret_cast<const void *>(seed_order_kernel),
-                                  static_cast<int>(kOrderLists * 4), "seed_order_kernel shared memory"))
-      return rc;
-    seed_order_kernel<<<1, 1024, L * 4, st>>>(probed, p, B, L, order);
-    KATO_LAUNCHED("seed_order_kernel");
-    ord = order;
-  }
   // rows the sketch picks to score in full: 3S (fewer loosen the bound, more
   // cost bytes)
   const uint32_t want = std::min(std::max(rows, S), kSeedCap);
-  rank_seed_kernel<<<B, 256, 0, st>>>(xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, ord, p, dc,
-                                      h, S, want, std::min(want, 3 * S), bound);
+  rank_seed_kernel<<<B, 256, 0, st>>>(xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
+                                      S, want, std::min(want, 3 * S), bound);
   KATO_LAUNCHED("rank_seed_kernel");
-  return KATO_OK;
-}
-
-int rank_tc_prepare(const uint32_t *cnt, const uint32_t *off, const uint32_t *list_off, uint32_t L,
-                    uint32_t N, uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
-                    uint32_t *tile_off, bool by_cost, uint2 *share, uint32_t ctas, uint32_t *qcount,
-                    unsigned long long *tile_hist, unsigned long long *tiles, cudaStream_t st) {
-  // the distinct probed lists and rows go to the two counters after the histogram
-  tc_count_kernel<<<div_up(std::max(std::max(L, B), 1u), 256), 256, 0, st>>>(
-      cnt, list_off, L, N, B, beta, by_cost, scratch, qcount, tile_hist ? tile_hist + 6 : nullptr);
-  tc_scan_kernel<<<1, 1024, 0, st>>>(scratch, L, by_cost, tile_off, share, ctas);
-  tc_expand_kernel<<<div_up(std::max(L, ctas), 256), 256, 0, st>>>(list_off, scratch, cnt, off, L, N, beta, by_cost,
-                                                   ctas, items, tile_off, share, tile_hist, tiles);
-  KATO_LAUNCHED("ranking work preparation");
   return KATO_OK;
 }
 

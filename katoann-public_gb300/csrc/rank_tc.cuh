@@ -44,14 +44,28 @@ struct TcShape {
   uint32_t centred;  // values enter as (byte - 128), not as the byte
 };
 
-// What centre_planes also makes of a batch's queries for the ranking pass
-// (rows null: nothing): their first h high bytes as fp16, centred or not,
-// zero-padded to `width`, and the sums of the squared values over f and h.
+// The ranking pass's copy of a batch's queries (rows null: none): their first
+// h high bytes as fp16, centred or not, zero-padded to `width`, and the sums of
+// the squared values over f and h.
 struct RankRows {
   __half *rows;
   int2 *norms;
   uint32_t f, h, width, centred;
 };
+
+// A batch's coded queries (rows of dc) and what is derived from them
+// (query_planes): byte planes, norms, and with hi16 the centred fp16 planes and
+// terms of the coarse product. `zeros` words at `zero` are cleared on the way.
+struct QueryPlanes {
+  uint8_t *hi, *lo;
+  int64_t *norm, *hinorm, *headnorm;
+  uint32_t dc, head;
+  __half *hi16, *lo16;
+  int64_t *term;
+  uint32_t *zero, zeros;
+};
+int query_planes(const float *x, uint32_t nrows, uint32_t d, float lo, double inv_step,
+                 const QueryPlanes &P, const RankRows &rr, cudaStream_t st);
 
 // Shared-memory carve-up of the ranking CTA.
 struct TcSmem {
@@ -106,20 +120,9 @@ int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShap
 // Per query, an upper bound on its final S-th ranking l2 from the first
 // `rows` rows (at most 4096) of its probed lists in probe order.
 int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, const int64_t *qnorm,
-              const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off,
-              uint32_t L, uint32_t B, uint32_t p, uint32_t dc, uint32_t h, uint32_t S,
-              uint32_t rows, uint32_t *order, int32_t *bound, cudaStream_t st);
-// Work items of the pass (per list: groups of N queries) and their slab
-// offsets, and each CTA's share: an equal count of slabs, or of their cost
-// (by_cost: what a slab's instructions do with beta 0, or 64 + beta * w for an
-// item of width w, 16, 32 or N queries). Also zeroes the B candidate counts.
-// off: the lists' first probe entries. scratch: 3 x (L + 1) words.
-// tile_hist (optional): 6 counters of 128-row tiles by item width, then the
-// distinct probed lists and their rows; tiles: all tiles.
-int rank_tc_prepare(const uint32_t *cnt, const uint32_t *off, const uint32_t *list_off, uint32_t L,
-                    uint32_t N, uint32_t B, uint32_t beta, uint32_t *scratch, TcItem *items,
-                    uint32_t *tile_off, bool by_cost, uint2 *share, uint32_t ctas, uint32_t *qcount,
-                    unsigned long long *tile_hist, unsigned long long *tiles, cudaStream_t st);
+              const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off, uint32_t B,
+              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, int32_t *bound,
+              cudaStream_t st);
 // Process-wide knobs of the pass (0 = default): the largest item width and
 // the cost weight of the CTA split.
 extern std::atomic<uint32_t> g_tc_width, g_tc_beta;

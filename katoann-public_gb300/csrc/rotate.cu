@@ -12,6 +12,7 @@
 // compiler evaluates those chains four products at a time with the products
 // rounded, then fuses the last (length % 4) terms.
 #include "kcommon.cuh"
+#include "rank_tc.cuh"
 #include "tc.cuh"
 
 namespace kato {
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
   __shared__ volatile uint32_t err;
   const uint32_t d16 = d & ~15u, nk = (d16 + kRotChunk - 1) / kRotChunk;
   const uint32_t i0 = blockIdx.y * kRowTile, j0 = blockIdx.x * kColTile;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, lane = t & 31;
   if (t == 0) {
     for (int s = 0; s < kRotStages; ++s) {
       tc::mbar_init(full + s, 1);
@@ -458,7 +459,101 @@ __global__ void quantize_rows_kernel(const float *__restrict__ x, uint32_t nrows
   }
 }
 
+// A query's codes and everything the search derives from them, one warp per
+// row, four dimensions per lane and step: the byte planes and their norms
+// (quantize_rows_kernel's), the centred fp16 planes and term of the coarse
+// product and the rows of the ranking pass (centre_planes_kernel's). Also
+// clears `zeros` words at `zero` (the inversion's and the candidates' counts).
+__global__ void __launch_bounds__(256) query_planes_kernel(const float *__restrict__ x, uint32_t nrows,
+                                                           uint32_t d, float lo, double inv_step,
+                                                           bool vec, const QueryPlanes P,
+                                                           const RankRows rr) {
+  const uint32_t lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.zeros; i += gridDim.x * blockDim.x)
+    P.zero[i] = 0;
+  if (row >= nrows) return;
+  const QuantScale qs = quant_scale(lo, inv_step);
+  const float *xr = x + static_cast<size_t>(row) * d;
+  uint64_t s = 0;
+  uint32_t sh = 0, s0 = 0;
+  int32_t ch = 0, cl = 0, rf = 0, rh = 0;  // centred byte sums; the ranking rows' norms
+  for (uint32_t k = lane * 4; k < P.dc; k += 128) {
+    float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (vec && k < d) {
+      const float4 v = *reinterpret_cast<const float4 *>(xr + k);
+      f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+    }
+    uint32_t hw = 0, lw = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      if (k + j >= d) break;  // padding dimensions are 0
+      const uint32_t v = quantize1(vec ? f[j] : xr[k + j], qs);
+      hw |= (v >> 8) << (8 * j);
+      lw |= (v & 0xFFu) << (8 * j);
+      s += static_cast<uint64_t>(v) * v;
+    }
+    const size_t at = static_cast<size_t>(row) * P.dc + k;
+    *reinterpret_cast<uint32_t *>(P.hi + at) = hw;
+    *reinterpret_cast<uint32_t *>(P.lo + at) = lw;
+    const uint32_t h2 = dp4(hw, hw, 0), h1 = dp4(hw, 0x01010101u, 0);
+    sh += h2;
+    if (k < P.head) s0 += h2;
+    if (P.hi16) {
+      auto halves = [](uint32_t w, uint32_t bias2) {  // four bytes as fp16 (byte - bias)
+        const uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
+        const __half2 bias = *reinterpret_cast<const __half2 *>(&bias2);
+        const __half2 ha = __hsub2(*reinterpret_cast<const __half2 *>(&a), bias);
+        const __half2 hb = __hsub2(*reinterpret_cast<const __half2 *>(&b), bias);
+        return make_uint2(*reinterpret_cast<const uint32_t *>(&ha), *reinterpret_cast<const uint32_t *>(&hb));
+      };
+      constexpr uint32_t k1152 = 0x64806480u, k1024 = 0x64006400u;  // pairs of fp16 1152 and 1024
+      *reinterpret_cast<uint2 *>(P.hi16 + at) = halves(hw, k1152);
+      *reinterpret_cast<uint2 *>(P.lo16 + at) = halves(lw, k1152);
+      ch += static_cast<int32_t>(h1) - 512;
+      cl += static_cast<int32_t>(dp4(lw, 0x01010101u, 0)) - 512;
+      if (rr.rows && k < rr.width) {  // f <= h <= width, multiples of 64
+        uint2 r = make_uint2(0, 0);
+        if (k < rr.h) {
+          r = halves(hw, rr.centred ? k1152 : k1024);
+          // sum (b - 128)^2 = sum b^2 - 256 sum b + 4 * 16384
+          const int32_t c = static_cast<int32_t>(h2) -
+                            (rr.centred ? 256 * static_cast<int32_t>(h1) - 4 * 16384 : 0);
+          rh += c;
+          if (k < rr.f) rf += c;
+        }
+        *reinterpret_cast<uint2 *>(rr.rows + static_cast<size_t>(row) * rr.width + k) = r;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    sh += __shfl_xor_sync(0xffffffffu, sh, o);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    ch += __shfl_xor_sync(0xffffffffu, ch, o);
+    cl += __shfl_xor_sync(0xffffffffu, cl, o);
+    rf += __shfl_xor_sync(0xffffffffu, rf, o);
+    rh += __shfl_xor_sync(0xffffffffu, rh, o);
+  }
+  if (lane == 0) {
+    P.norm[row] = static_cast<int64_t>(s);
+    P.hinorm[row] = sh;
+    P.headnorm[row] = s0;
+    if (P.hi16) P.term[row] = static_cast<int64_t>(s) - 256 * (65792ll * ch + 257ll * cl) - 16384ll * P.dc * 66049ll;
+    if (P.hi16 && rr.rows) rr.norms[row] = make_int2(rf, rh);
+  }
+}
+
 }  // namespace
+
+int query_planes(const float *x, uint32_t nrows, uint32_t d, float lo, double inv_step,
+                 const QueryPlanes &P, const RankRows &rr, cudaStream_t st) {
+  if (nrows == 0) return KATO_OK;
+  const bool vec = d % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+  query_planes_kernel<<<div_up(nrows, 8), 256, 0, st>>>(x, nrows, d, lo, inv_step, vec, P, rr);
+  KATO_LAUNCHED("query_planes_kernel");
+  return KATO_OK;
+}
 
 int rotate_rows(const float *in, uint32_t nrows, uint32_t d, const float *rot, float *out,
                 cudaStream_t st) {

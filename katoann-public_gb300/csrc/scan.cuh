@@ -1,59 +1,61 @@
-// Exclusive prefix sums of two sequences at once by one CTA of 1024 threads
-// (the list-sized scans of the search: nlist is at most a few 10^5).
+// Exclusive prefix sums of four sequences at once by one CTA of 1024 threads
+// (the list-sized scans of the search: nlist is at most a few 10^5), and a
+// radix-selection step.
 #pragma once
 
 #include <cstdint>
 
 namespace kato {
 
-// val(i) gives the pair of values at i < n; out(i, a, b) receives the pair of
-// exclusive prefix sums there. Tiles of 4096: each thread takes 4 consecutive
-// values (coalesced across the CTA), warps scan with shuffles. Returns the
-// totals; all threads of the CTA must call it.
+__device__ __forceinline__ uint4 add4(uint4 a, uint4 b) {
+  return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ uint4 warp_scan4(uint4 x, uint32_t lane) {  // inclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint4 y = make_uint4(__shfl_up_sync(0xffffffffu, x.x, o), __shfl_up_sync(0xffffffffu, x.y, o),
+                               __shfl_up_sync(0xffffffffu, x.z, o), __shfl_up_sync(0xffffffffu, x.w, o));
+    if (lane >= static_cast<uint32_t>(o)) x = add4(x, y);
+  }
+  return x;
+}
+
+// val(i) gives the values at i < n; out(i, sums) receives the exclusive prefix
+// sums there. Tiles of 4096: each thread takes 4 consecutive values (coalesced
+// across the CTA), warps scan with shuffles. Returns the totals; all threads
+// of the CTA must call it.
 template <typename Val, typename Out>
-__device__ uint2 block_scan2(uint32_t n, Val val, Out out) {
-  __shared__ uint2 wsum[32];
+__device__ uint4 block_scan4(uint32_t n, Val val, Out out) {
+  __shared__ uint4 wsum[32];
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  uint2 carry = make_uint2(0, 0);
+  uint4 carry = make_uint4(0, 0, 0, 0);
   for (uint32_t base = 0; base < n; base += 4096) {
     const uint32_t i0 = base + t * 4;
-    uint2 v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = i0 + k < n ? val(i0 + k) : make_uint2(0, 0);
-    const uint2 ts = make_uint2(v[0].x + v[1].x + v[2].x + v[3].x, v[0].y + v[1].y + v[2].y + v[3].y);
-    uint2 x = ts;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t ya = __shfl_up_sync(0xffffffffu, x.x, o), yb = __shfl_up_sync(0xffffffffu, x.y, o);
-      if (lane >= static_cast<uint32_t>(o)) x.x += ya, x.y += yb;
-    }
-    if (lane == 31) wsum[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      const uint2 w = wsum[lane];
-      uint2 z = w;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t ya = __shfl_up_sync(0xffffffffu, z.x, o), yb = __shfl_up_sync(0xffffffffu, z.y, o);
-        if (lane >= static_cast<uint32_t>(o)) z.x += ya, z.y += yb;
-      }
-      wsum[lane] = make_uint2(z.x - w.x, z.y - w.y);  // exclusive over warps
-    }
-    __syncthreads();
-    uint2 e = make_uint2(carry.x + wsum[warp].x + x.x - ts.x, carry.y + wsum[warp].y + x.y - ts.y);
+    uint4 v[4], ts = make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      if (i0 + k < n) out(i0 + k, e.x, e.y);
-      e.x += v[k].x;
-      e.y += v[k].y;
+      v[k] = i0 + k < n ? val(i0 + k) : make_uint4(0, 0, 0, 0);
+      ts = add4(ts, v[k]);
     }
-    // the tile's total: the last thread's inclusive sum
-    __shared__ uint2 tile_total;
-    if (t == blockDim.x - 1) tile_total = make_uint2(e.x - carry.x, e.y - carry.y);
+    const uint4 x = warp_scan4(ts, lane);
+    if (lane == 31) wsum[warp] = x;
     __syncthreads();
-    carry.x += tile_total.x;
-    carry.y += tile_total.y;
-    __syncthreads();
+    // every warp scans the warp totals: no second barrier round
+    const uint4 w = warp_scan4(wsum[lane], lane);
+    const int before = warp ? static_cast<int>(warp) - 1 : 0;
+    uint4 e = make_uint4(__shfl_sync(0xffffffffu, w.x, before), __shfl_sync(0xffffffffu, w.y, before),
+                         __shfl_sync(0xffffffffu, w.z, before), __shfl_sync(0xffffffffu, w.w, before));
+    const uint4 tile = make_uint4(__shfl_sync(0xffffffffu, w.x, 31), __shfl_sync(0xffffffffu, w.y, 31),
+                                  __shfl_sync(0xffffffffu, w.z, 31), __shfl_sync(0xffffffffu, w.w, 31));
+    if (warp == 0) e = make_uint4(0, 0, 0, 0);
+    e = add4(carry, add4(e, make_uint4(x.x - ts.x, x.y - ts.y, x.z - ts.z, x.w - ts.w)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k < n) out(i0 + k, e);
+      e = add4(e, v[k]);
+    }
+    carry = add4(carry, tile);
+    __syncthreads();  // wsum is written again
   }
   return carry;
 }

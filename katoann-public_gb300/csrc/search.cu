@@ -1,14 +1,13 @@
-// The batched search pipeline after the coarse step: inversion of the probe
-// lists, the ranking pass, the survivor merge and the exact refinement.
+// The batched search pipeline, from a batch's queries to its results.
 //
 // Reference: Index::search_sq16_ranked_ (src/index.cpp:909-1128) and
-// Index::search_sq16_full_ (:1131-1219). The reference inverts the probe
-// lists into a hash map (invert, :403-412) and scans each probed list once
-// for all the queries that probe it (:998-1044); here the inversion is a CSR
-// built with a histogram, a scan and an atomic scatter, and each CTA of the
-// ranking kernel takes one list and up to kQG of its queries, stages the
-// list's rows in shared memory tile by tile and keeps, per query, the best S
-// candidates by (distance, id) in shared memory. Selection by (distance, id)
+// Index::search_sq16_full_ (:1131-1219), which scan each probed list once for
+// all the queries that probe it (:998-1044). Here the prefix and high-byte
+// rankings run on the tensor cores (rank_tc.cu); rank_kernel below, for the
+// full ranking and shapes that pass does not take, scores on the CUDA cores:
+// each CTA takes one list and up to kQG of its queries, stages the list's rows
+// in shared memory tile by tile and keeps, per query, the best S candidates by
+// (distance, id) in shared memory. Selection by (distance, id)
 // is the reference's Selection::kLocal result (:101-135 then :1063-1069) and
 // its kThreshold result wherever that has no tie on the survivor boundary.
 #include <algorithm>
@@ -18,10 +17,10 @@
 #include <cuda_fp16.h>
 
 #include "finish.cuh"
+#include "invert.cuh"
 #include "kcommon.cuh"
 #include "probe.cuh"
 #include "rank_tc.cuh"
-#include "scan.cuh"
 
 namespace kato {
 
@@ -40,66 +39,6 @@ constexpr uint32_t kSelMax = 256;  // largest per-slot S kept in shared memory
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
 constexpr uint32_t kSortMax = 4096;
-
-struct Work {
-  uint32_t list, first;
-};
-
-// ---------------------------------------------------------------- inversion
-// A (query, rank) pair i = query * p + rank is probed when the query's
-// budget (if any) exceeds the rank: its p nearest lists are in order, so a
-// budget of b probes exactly the lists a fixed nprobe of b would.
-__device__ __forceinline__ bool probed_pair(uint32_t i, uint32_t p,
-                                            const uint32_t *__restrict__ qprobes) {
-  return !qprobes || i % p < qprobes[i / p];
-}
-
-__global__ void count_kernel(const uint32_t *__restrict__ probed, uint32_t total, uint32_t p,
-                             const uint32_t *__restrict__ qprobes, uint32_t *__restrict__ cnt) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < total && probed_pair(i, p, qprobes)) atomicAdd(&cnt[probed[i]], 1u);
-}
-
-// One CTA: exclusive scans of the per-list query counts (off) and of the
-// per-list work-item counts (woff); clears the scatter cursors.
-__global__ void __launch_bounds__(1024) scan_kernel(const uint32_t *__restrict__ cnt, uint32_t L,
-                                                    uint32_t *__restrict__ off,
-                                                    uint32_t *__restrict__ woff,
-                                                    uint32_t *__restrict__ cursor) {
-  const uint2 tot = block_scan2(
-      L,
-      [&](uint32_t c) {
-        const uint32_t v = cnt[c];
-        return make_uint2(v, (v + kQG - 1) / kQG);
-      },
-      [&](uint32_t c, uint32_t a, uint32_t b) {
-        off[c] = a;
-        woff[c] = b;
-        cursor[c] = 0;
-      });
-  if (threadIdx.x == 0) {
-    off[L] = tot.x;
-    woff[L] = tot.y;
-  }
-}
-
-__global__ void scatter_kernel(const uint32_t *__restrict__ probed, uint32_t total, uint32_t p,
-                               const uint32_t *__restrict__ qprobes,
-                               const uint32_t *__restrict__ off, uint32_t *__restrict__ cursor,
-                               uint32_t *__restrict__ entries) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total || !probed_pair(i, p, qprobes)) return;
-  const uint32_t c = probed[i];
-  entries[off[c] + atomicAdd(&cursor[c], 1u)] = i;  // i = query * nprobe + rank
-}
-
-__global__ void work_kernel(const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ woff,
-                            uint32_t L, Work *__restrict__ work) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L) return;
-  const uint32_t nw = (cnt[c] + kQG - 1) / kQG;
-  for (uint32_t j = 0; j < nw; ++j) work[woff[c] + j] = Work{c, j * kQG};
-}
 
 // ------------------------------------------------------------- ranking pass
 struct RankArgs {
@@ -323,16 +262,10 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
 // ------------------------------------------------------------ orchestration
 int rotate_rows(const float *in, uint32_t nrows, uint32_t d, const float *rot, float *out,
                 cudaStream_t st);
-int quantize_rows(const float *x, uint32_t nrows, uint32_t d, uint32_t dc, float lo,
-                  double inv_step, uint32_t head, uint8_t *hi, uint8_t *lop, int64_t *norm,
-                  int64_t *hinorm, int64_t *headnorm, cudaStream_t st);
 int sq16_tiles(const uint8_t *qhi, const uint8_t *qlo, const uint8_t *xhi, const uint8_t *xlo,
                const int64_t *qn, const int64_t *xn, double step_sq, uint32_t m, uint32_t n,
                uint32_t dims, uint32_t qstride, uint32_t xstride, float *out, bool full,
                cudaStream_t st);
-int centre_planes(const uint8_t *hi, const uint8_t *lo, const int64_t *norm, uint32_t rows,
-                  uint32_t dc, __half *hi16, __half *lo16, int64_t *term, const RankRows &rr,
-                  cudaStream_t st);
 bool coarse_tc_ok(uint32_t dc);
 int coarse_tc(const __half *ch, const __half *cl, const int64_t *cterm, uint32_t n, const __half *qh,
               const __half *ql, const int64_t *qterm, uint32_t m, uint32_t dc, double step_sq,
@@ -342,8 +275,8 @@ int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float 
                        const float *rot_kmajor, void *scratch, float *out, uint32_t *timeouts,
                        uint32_t *launches, cudaStream_t st);
 int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint32_t stride,
-                   uint32_t *probed, unsigned long long *tie_count, const uint32_t *only,
-                   uint32_t only_above, cudaStream_t st);
+                   uint32_t *probed, uint32_t *cnt, unsigned long long *tie_count,
+                   const uint32_t *only, uint32_t only_above, cudaStream_t st);
 
 // Per pass: the KATO_PHASES + 1 phase boundaries, then a start and an end
 // event around each timed kernel (KATO_TIMED_KERNELS: the query rotation,
@@ -379,10 +312,10 @@ struct Plan {
   uint32_t tcitems, cap, seed_rows, ctas, rec_cap, beta;
   bool cost;                        // the ranking CTAs split the slabs' cost, not their count
   size_t off_fq, off_qhi, off_qlo, off_qn, off_qhn, off_qh0, off_cd, off_probed, off_cnt, off_off,
-      off_woff, off_cur, off_work, off_ent, off_slots, off_stats,
-      off_tcscratch, off_tcitems, off_tileoff, off_qcount,  off_bound,
+      off_base, off_cur, off_work, off_ent, off_slots, off_stats,
+      off_tcitems, off_tileoff, off_qcount,  off_bound,
       off_rec, off_recn, off_qh16, off_ql16, off_qterm, off_rot,
-      off_qprobes, off_z, off_qcn, off_qr16, off_share, off_seedorder, total;
+      off_qprobes, off_z, off_qcn, off_qr16, off_share, total;
 };
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -447,18 +380,17 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_qh0 = take(static_cast<size_t>(B) * 8);
   pl.off_cd = take(static_cast<size_t>(B) * L * 4);
   pl.off_probed = take(bp * 4);
-  pl.off_cnt = take(static_cast<size_t>(L) * 4);
+  pl.off_cnt = take(static_cast<size_t>(L) * 4);  // cleared together with qcount after it
+  pl.off_qcount = take(static_cast<size_t>(B) * 4);
   pl.off_off = take((static_cast<size_t>(L) + 1) * 4);
-  pl.off_woff = take((static_cast<size_t>(L) + 1) * 4);
+  pl.off_base = take(3 * (static_cast<size_t>(L) + 1) * 4);
   pl.off_cur = take(static_cast<size_t>(L) * 4);
   pl.off_work = take(wmax * sizeof(Work));
   pl.off_ent = take(bp * 4);
   pl.off_slots = take((pl.tc ? static_cast<size_t>(B) * pl.cap : bp * pl.SC) * sizeof(uint2));
-  pl.off_tcscratch = take(3 * (static_cast<size_t>(L) + 1) * 4);
   pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);
   pl.off_tileoff = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * 4 : 16);
-  pl.off_qcount = take(static_cast<size_t>(B) * 4);
   pl.off_bound = take(static_cast<size_t>(B) * 4);
   pl.off_rec = take(pl.tc ? static_cast<size_t>(pl.ctas) * pl.rec_cap * 16 : 16);
   pl.off_recn = take(static_cast<size_t>(pl.ctas) * 4);
@@ -471,7 +403,6 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_qterm = take(static_cast<size_t>(B) * 8);
   pl.off_rot = take(ix->rotated ? rotate_scratch_bytes(B, ix->dim) : 16);
   pl.off_qprobes = take(static_cast<size_t>(B) * 4);
-  pl.off_seedorder = take(static_cast<size_t>(B) * 4);
   pl.off_z = take(static_cast<size_t>(B) * KATO_PROBE_FEATURES * 4);
   pl.total = o;
   return KATO_OK;
@@ -482,7 +413,7 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
 // query's p1 nearest lists in order (probed, rows pl.p apart) in the
 // workspace.
 int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *queries, uint32_t nq,
-                unsigned char *ws, uint32_t p1, cudaStream_t st, PhaseTimer *tm) {
+                unsigned char *ws, uint32_t p1, uint32_t *cnt, cudaStream_t st, PhaseTimer *tm) {
   int rc;
   const uint32_t L = ix->nlist, p = pl.p, dc = ix->dc;
   float *fq = reinterpret_cast<float *>(ws + pl.off_fq);
@@ -506,23 +437,23 @@ int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     kmark(tm, 0, true, st);
     src = fq;
   }
-  if ((rc = quantize_rows(src, nq, ix->dim, dc, ix->lo, ix->inv_step, ix->head_dims, qhi, qlo, qn,
-                          qhn, qh0, st)))
-    return rc;
-  g_launches += 1 + 2;  // quantize, coarse, select
-  mark(tm, 1, st);
-  // the queries' centred planes, for both tensor-core passes
+  // the queries' planes, for the exact distances and both tensor-core passes;
+  // the counts of the inversion and of the candidates start at 0
   __half *qh16 = reinterpret_cast<__half *>(ws + pl.off_qh16);
   __half *ql16 = reinterpret_cast<__half *>(ws + pl.off_ql16);
   int64_t *qterm = reinterpret_cast<int64_t *>(ws + pl.off_qterm);
-  if (pl.coarse_tc || pl.tc) {
-    RankRows rr{};
-    if (pl.tc)
-      rr = RankRows{reinterpret_cast<__half *>(ws + pl.off_qr16),
-                    reinterpret_cast<int2 *>(ws + pl.off_qcn), pl.tcs.f, pl.dims,
-                    tc_qrow(pl.dims, pl.tcs), pl.tcs.centred};
-    if ((rc = centre_planes(qhi, qlo, qn, nq, dc, qh16, ql16, qterm, rr, st))) return rc;
-  }
+  QueryPlanes P{qhi, qlo, qn, qhn, qh0, dc, ix->head_dims, nullptr, nullptr, nullptr,
+                reinterpret_cast<uint32_t *>(ws + pl.off_cnt),
+                static_cast<uint32_t>((pl.off_qcount - pl.off_cnt) / 4 + pl.B)};
+  RankRows rr{};
+  if (pl.coarse_tc || pl.tc) P.hi16 = qh16, P.lo16 = ql16, P.term = qterm;
+  if (pl.tc)
+    rr = RankRows{reinterpret_cast<__half *>(ws + pl.off_qr16),
+                  reinterpret_cast<int2 *>(ws + pl.off_qcn), pl.tcs.f, pl.dims,
+                  tc_qrow(pl.dims, pl.tcs), pl.tcs.centred};
+  if ((rc = query_planes(src, nq, ix->dim, ix->lo, ix->inv_step, P, rr, st))) return rc;
+  g_launches += 1 + 2;  // planes, coarse, select
+  mark(tm, 1, st);
   // 2. coarse product and top-nprobe (:846-877)
   if (pl.coarse_tc) {
     kmark(tm, 1, false, st);
@@ -532,13 +463,12 @@ int coarse_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
                         stats + 32, st)))
       return rc;
     kmark(tm, 1, true, st);
-    ++g_launches;
   } else if ((rc = sq16_tiles(qhi, qlo, ix->d_chi, ix->d_clo, qn, ix->d_cnorm, ix->step_sq, nq, L,
                               dc, dc, dc, cd, true, st))) {
     return rc;
   }
   mark(tm, 2, st);
-  if ((rc = select_topp_ex(cd, nq, L, p1, p, probed, stats + 0, nullptr, 0, st))) return rc;
+  if ((rc = select_topp_ex(cd, nq, L, p1, p, probed, cnt, stats + 0, nullptr, 0, st))) return rc;
   mark(tm, 3, st);
   return KATO_OK;
 }
@@ -556,7 +486,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   uint32_t *probed = reinterpret_cast<uint32_t *>(ws + pl.off_probed);
   uint32_t *cnt = reinterpret_cast<uint32_t *>(ws + pl.off_cnt);
   uint32_t *off = reinterpret_cast<uint32_t *>(ws + pl.off_off);
-  uint32_t *woff = reinterpret_cast<uint32_t *>(ws + pl.off_woff);
+  uint32_t *base = reinterpret_cast<uint32_t *>(ws + pl.off_base);
   uint32_t *cur = reinterpret_cast<uint32_t *>(ws + pl.off_cur);
   Work *work = reinterpret_cast<Work *>(ws + pl.off_work);
   uint32_t *ent = reinterpret_cast<uint32_t *>(ws + pl.off_ent);
@@ -567,7 +497,9 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   // for the queries whose budget is deeper, to the cap
   const bool model = bud.model && !bud.nprobe_in;
   const uint32_t p1 = model ? std::min(p, bud.model->depth) : p;
-  if ((rc = coarse_pass(ix, pl, queries, nq, ws, p1, st, tm))) return rc;
+  // without budgets the selection counts the inversion's lists on the way
+  const bool counted = !bud.active();
+  if ((rc = coarse_pass(ix, pl, queries, nq, ws, p1, counted ? cnt : nullptr, st, tm))) return rc;
   // 2'. per-query budgets: given, or from the model over the coarse distances
   uint32_t *qprobes = nullptr;
   if (bud.active()) {
@@ -581,7 +513,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
       if ((rc = probe_budget(*bud.model, z, nq, bud.cap, nullptr, qprobes, st))) return rc;
       g_launches += 2;
       if (p1 < p) {
-        if ((rc = select_topp_ex(cd, nq, L, p, p, probed, nullptr, qprobes, p1, st))) return rc;
+        if ((rc = select_topp_ex(cd, nq, L, p, p, probed, nullptr, nullptr, qprobes, p1, st))) return rc;
         ++g_launches;
       }
     }
@@ -594,17 +526,31 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   }
   mark(tm, 4, st);
   // 3. inversion (:403-412)
-  const uint32_t total = nq * p;
-  KATO_CUDA(cudaMemsetAsync(cnt, 0, static_cast<size_t>(L) * 4, st));
-  count_kernel<<<div_up(total, 256), 256, 0, st>>>(probed, total, p, qprobes, cnt);
-  scan_kernel<<<1, 1024, 0, st>>>(cnt, L, off, woff, cur);
-  scatter_kernel<<<div_up(total, 256), 256, 0, st>>>(probed, total, p, qprobes, off, cur, ent);
-  g_launches += 3;
-  if (!pl.tc) {
-    work_kernel<<<div_up(L, 256), 256, 0, st>>>(cnt, woff, L, work);
-    ++g_launches;
+  InvertArgs I{};
+  I.probed = probed;
+  I.qprobes = qprobes;
+  I.B = nq;
+  I.p = p;
+  I.L = L;
+  I.N = pl.tc ? pl.tcs.N : kQG;
+  I.list_off = ix->d_list_off;
+  I.cnt = cnt;
+  I.off = off;
+  I.cur = cur;
+  I.base = base;
+  I.entries = ent;
+  I.work = work;
+  if (pl.tc) {
+    I.items = reinterpret_cast<TcItem *>(ws + pl.off_tcitems);
+    I.tile_off = reinterpret_cast<uint32_t *>(ws + pl.off_tileoff);
+    I.share = reinterpret_cast<uint2 *>(ws + pl.off_share);
+    I.ctas = pl.ctas;
+    I.beta = pl.beta;
+    I.by_cost = pl.cost;
+    I.tile_hist = stats + 40;
+    I.tiles = stats + 4;
   }
-  KATO_LAUNCHED("inversion kernels");
+  if ((rc = invert(I, counted, &g_launches, st))) return rc;
   mark(tm, 5, st);
   uint32_t *qcount = nullptr;
   if (!pl.tc) mark(tm, 6, st);  // no seed-bound phase on the CUDA-core pass
@@ -612,8 +558,6 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     // 4'. ranking pass on the tensor cores: seed bounds, work items, the
     // scan, and the exact rescan of any query whose buffer overflowed
     int32_t *bound = reinterpret_cast<int32_t *>(ws + pl.off_bound);
-    TcItem *items = reinterpret_cast<TcItem *>(ws + pl.off_tcitems);
-    uint32_t *tile_off = reinterpret_cast<uint32_t *>(ws + pl.off_tileoff);
     uint4 *rec = reinterpret_cast<uint4 *>(ws + pl.off_rec);
     uint32_t *rec_n = reinterpret_cast<uint32_t *>(ws + pl.off_recn);
     qcount = reinterpret_cast<uint32_t *>(ws + pl.off_qcount);
@@ -621,24 +565,17 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     const int64_t *xnorm = prefix_mode ? ix->d_headnorm : ix->d_hinorm;
     const int64_t *qnorm = prefix_mode ? qh0 : qhn;
     const DistScale scale = make_dist_scale(ix->step_sq);
-    if ((rc = rank_seed(ix->d_hi, xnorm, qhi, qnorm, probed, qprobes, ix->d_list_off, L, nq, p, dc,
-                        pl.dims, pl.S, pl.seed_rows,
-                        reinterpret_cast<uint32_t *>(ws + pl.off_seedorder), bound, st)))
+    if ((rc = rank_seed(ix->d_hi, xnorm, qhi, qnorm, probed, qprobes, ix->d_list_off, nq, p, dc,
+                        pl.dims, pl.S, pl.seed_rows, bound, st)))
       return rc;
-    g_launches += L <= 16384 ? 1 : 0;  // the seed order
     mark(tm, 6, st);
-    uint2 *share = reinterpret_cast<uint2 *>(ws + pl.off_share);
-    if ((rc = rank_tc_prepare(cnt, off, ix->d_list_off, L, pl.tcs.N, nq, pl.beta,
-                              reinterpret_cast<uint32_t *>(ws + pl.off_tcscratch), items, tile_off,
-                              pl.cost, share, pl.ctas, qcount, stats + 40, stats + 4, st)))
-      return rc;
     RankTcArgs T{};
     T.qr16 = reinterpret_cast<const __half *>(ws + pl.off_qr16);
     T.qcn = reinterpret_cast<const int2 *>(ws + pl.off_qcn);
     T.entries = ent;
-    T.items = items;
-    T.tile_off = tile_off;
-    T.share = share;
+    T.items = I.items;
+    T.tile_off = I.tile_off;
+    T.share = I.share;
     T.bound = bound;
     T.qcount = qcount;
     T.rec = rec;
@@ -657,7 +594,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, nq, ix->d_hi, qhi, T.qcn, bound, dc,
                              pl.tcs.f, pl.dims, qcount, slots, pl.cap, scale, stats + 5, st)))
       return rc;
-    g_launches += 6;  // seed, 3 preparation, scan, bucket
+    g_launches += 3;  // seed, scan, bucket
   }
   // 4. ranking pass (:998-1044 / :1167-1204)
   const bool full = pl.ranking == KATO_RANK_FULL;
@@ -671,7 +608,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   A.qlo = qlo;
   A.qnorm = full ? qn : (pl.ranking == KATO_RANK_PREFIX ? qh0 : qhn);
   A.work = work;
-  A.woff_total = woff + L;
+  A.woff_total = base + L;
   A.off = off;
   A.entries = ent;
   A.dc = dc;
@@ -809,8 +746,8 @@ int probe_features_search(const katoann_gpu_index *ix, const float *queries, uin
   g_launches = 0;
   for (uint32_t q0 = 0; q0 < nq; q0 += max_batch) {
     const uint32_t b = std::min(max_batch, nq - q0);
-    if ((rc = coarse_pass(ix, pl, queries + static_cast<size_t>(q0) * ix->dim, b, w, depth, st,
-                          nullptr)))
+    if ((rc = coarse_pass(ix, pl, queries + static_cast<size_t>(q0) * ix->dim, b, w, depth,
+                          nullptr, st, nullptr)))
       return rc;
     if ((rc = probe_features(reinterpret_cast<float *>(w + pl.off_cd), ix->nlist,
                              reinterpret_cast<uint32_t *>(w + pl.off_probed), depth, rank, b,
