@@ -87,7 +87,7 @@ struct Index::State {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   mutable std::mutex mu;
-  mutable DevBuf ws, dq, dids, ddists, dnp_in, dnp_out;
+  mutable DevBuf ws, dq, dids, dnp_in, dnp_out;  // dids: a pass's ids, then its distances
   // captured searches of search_device (SearchParams::graph), most recent last
   struct Graph {
     std::vector<uint64_t> key;
@@ -147,8 +147,19 @@ struct Index::State {
     return hwait;
   }
 
+  // Pinned staging of a small host search (at most kStageBytes): its queries
+  // and results cross in one asynchronous copy each. Three copies to pageable
+  // memory took a third of a one-query search.
+  static constexpr size_t kStageBytes = 1u << 20;
+  mutable unsigned char *hstage = nullptr;
+  unsigned char *stage() const {
+    if (!hstage) cuda_check(cudaMallocHost(reinterpret_cast<void **>(&hstage), kStageBytes), "cudaMallocHost");
+    return hstage;
+  }
+
   ~State() {
     if (hwait) cudaFreeHost(hwait);
+    if (hstage) cudaFreeHost(hstage);
     drop_graphs();
     if (done) cudaEventDestroy(done);
     if (stream) cudaStreamDestroy(stream);
@@ -680,18 +691,26 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
     s.ws.ensure(need);
   }
   s.dq.ensure(static_cast<size_t>(b) * s.dim * 4);
-  s.dids.ensure(static_cast<size_t>(b) * p.k * 4);
-  s.ddists.ensure(static_cast<size_t>(b) * p.k * 4);
+  // ids, then dists
+  const size_t rbytes = static_cast<size_t>(b) * p.k * 4, qbytes = static_cast<size_t>(b) * s.dim * 4;
+  s.dids.ensure(2 * rbytes);
+  uint32_t *d_ids = s.dids.as<uint32_t>();
+  float *d_dists = reinterpret_cast<float *>(d_ids + static_cast<size_t>(b) * p.k);
   if (p.nprobe_per_query) s.dnp_in.ensure(static_cast<size_t>(b) * 4);
   if (p.nprobe_used) s.dnp_out.ensure(static_cast<size_t>(b) * 4);
   if (s.last_stream && s.last_stream != s.stream)
     cuda_check(cudaStreamWaitEvent(s.stream, s.done, 0), "cudaStreamWaitEvent");
   const uint32_t passes = (nq + mb - 1) / mb;
   uint64_t *waits = s.wait_counts(passes);
+  // a batch of one pass whose queries and results fit goes by the staging
+  unsigned char *staged =
+      passes == 1 && qbytes + 2 * rbytes <= State::kStageBytes ? s.stage() : nullptr;
+  if (staged) std::memcpy(staged, queries, qbytes);
   for (uint32_t q0 = 0; q0 < nq; q0 += mb) {
     const uint32_t nb = std::min(mb, nq - q0);
-    cuda_check(cudaMemcpyAsync(s.dq.p, queries + static_cast<size_t>(q0) * s.dim,
-                               static_cast<size_t>(nb) * s.dim * 4, cudaMemcpyHostToDevice, s.stream),
+    const void *src = queries + static_cast<size_t>(q0) * s.dim;
+    cuda_check(cudaMemcpyAsync(s.dq.p, staged ? staged : src, static_cast<size_t>(nb) * s.dim * 4,
+                               cudaMemcpyHostToDevice, s.stream),
                "copy queries");
     if (p.graph) {
       // the kernels as one captured graph of the index's own buffers; the
@@ -701,7 +720,7 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
                                    cudaMemcpyHostToDevice, s.stream),
                    "copy budgets");
       void *h = s.graph_of(s.dq.as<float>(), nb, p, rk, bp.use_model ? &bp.model : nullptr,
-                           s.dids.as<uint32_t>(), s.ddists.as<float>(),
+                           d_ids, d_dists,
                            p.nprobe_per_query ? s.dnp_in.as<uint32_t>() : nullptr,
                            p.nprobe_used ? s.dnp_out.as<uint32_t>() : nullptr, s.stream);
       gpu_check(katoann_gpu_graph_launch(h, reinterpret_cast<katoann_stream_t>(s.stream)));
@@ -717,8 +736,8 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
       gpu_check(katoann_gpu_search_budget(
           &s.view, s.dq.as<float>(), nb, p.k, p.nprobe, rk, p.survivors, mb,
           p.nprobe_per_query ? s.dnp_in.as<uint32_t>() : nullptr,
-          bp.use_model ? &bp.model : nullptr, s.ws.p, s.ws.n, s.dids.as<uint32_t>(),
-          s.ddists.as<float>(), p.nprobe_used ? s.dnp_out.as<uint32_t>() : nullptr,
+          bp.use_model ? &bp.model : nullptr, s.ws.p, s.ws.n, d_ids,
+          d_dists, p.nprobe_used ? s.dnp_out.as<uint32_t>() : nullptr,
           reinterpret_cast<katoann_stream_t>(s.stream), nullptr));
       if (p.nprobe_used)
         cuda_check(cudaMemcpyAsync(p.nprobe_used + q0, s.dnp_out.p, static_cast<size_t>(nb) * 4,
@@ -726,15 +745,20 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
                    "copy budgets");
     } else {
       gpu_check(katoann_gpu_search(&s.view, s.dq.as<float>(), nb, p.k, p.nprobe, rk, p.survivors,
-                                   mb, s.ws.p, s.ws.n, s.dids.as<uint32_t>(),
-                                   s.ddists.as<float>(), reinterpret_cast<katoann_stream_t>(s.stream)));
+                                   mb, s.ws.p, s.ws.n, d_ids, d_dists,
+                                   reinterpret_cast<katoann_stream_t>(s.stream)));
     }
-    cuda_check(cudaMemcpyAsync(ids + static_cast<size_t>(q0) * p.k, s.dids.p,
-                               static_cast<size_t>(nb) * p.k * 4, cudaMemcpyDeviceToHost, s.stream),
-               "copy ids");
-    cuda_check(cudaMemcpyAsync(dists + static_cast<size_t>(q0) * p.k, s.ddists.p,
-                               static_cast<size_t>(nb) * p.k * 4, cudaMemcpyDeviceToHost, s.stream),
-               "copy dists");
+    if (staged) {
+      cuda_check(cudaMemcpyAsync(staged + qbytes, d_ids, 2 * rbytes, cudaMemcpyDeviceToHost, s.stream),
+                 "copy results");
+    } else {
+      cuda_check(cudaMemcpyAsync(ids + static_cast<size_t>(q0) * p.k, d_ids,
+                                 static_cast<size_t>(nb) * p.k * 4, cudaMemcpyDeviceToHost, s.stream),
+                 "copy ids");
+      cuda_check(cudaMemcpyAsync(dists + static_cast<size_t>(q0) * p.k, d_dists,
+                                 static_cast<size_t>(nb) * p.k * 4, cudaMemcpyDeviceToHost, s.stream),
+                 "copy dists");
+    }
     cuda_check(cudaMemcpyAsync(waits + q0 / mb, static_cast<const char *>(s.ws.p) + 3 * sizeof(uint64_t),
                                sizeof(uint64_t), cudaMemcpyDeviceToHost, s.stream),
                "copy statistics");
@@ -742,6 +766,10 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
   cuda_check(cudaEventRecord(s.done, s.stream), "cudaEventRecord");
   s.last_stream = s.stream;
   cuda_check(cudaStreamSynchronize(s.stream), "search");
+  if (staged) {
+    std::memcpy(ids, staged + qbytes, rbytes);
+    std::memcpy(dists, staged + qbytes + rbytes, rbytes);
+  }
   for (uint32_t i = 0; i < passes; ++i)
     if (waits[i])
       throw timeout_error("search: a bounded pipeline wait in a tensor-core kernel ran out (" +
