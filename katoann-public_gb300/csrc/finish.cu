@@ -152,7 +152,8 @@ __device__ void block_sort_pairs(unsigned long long *key, uint32_t *val, uint32_
 // padded.
 __global__ void __launch_bounds__(kThreads) merge_kernel(
     const uint2 *__restrict__ slots, uint32_t per_query, uint32_t per_probe,
-    const uint32_t *__restrict__ qprobes, const uint32_t *__restrict__ ids, uint32_t k,
+    const uint32_t *__restrict__ qcount, const uint32_t *__restrict__ qprobes,
+    const uint32_t *__restrict__ ids, uint32_t k,
     uint32_t *__restrict__ out_ids, float *__restrict__ out_dists,
     unsigned long long *__restrict__ tie_count) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -164,9 +165,11 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(
   uint32_t *pos = reinterpret_cast<uint32_t *>(sel + np2);
   const uint32_t q = blockIdx.x;
   const uint2 *e = slots + static_cast<size_t>(q) * per_query;
-  // a query's slots are its probes' (rank-major), of which the first budget
-  // ones were written
-  const uint32_t n = qprobes ? min(per_query, qprobes[q] * per_probe) : per_query;
+  // counted entries, or its probes' slots (rank-major), of which the first
+  // budget ones were written
+  const uint32_t n = qcount    ? min(qcount[q], per_query)
+                     : qprobes ? min(per_query, qprobes[q] * per_probe)
+                               : per_query;
   auto K = [&](uint32_t i) { return e[i].x; };
   auto I = [&](uint32_t i) { return ids[e[i].y]; };
   const uint32_t got = block_select(n, k, K, I, sel, pos, hist, scratch, wsum, &tie);
@@ -568,8 +571,8 @@ int finish(const FinishArgs &A, uint32_t nq, cudaStream_t st) {
   return KATO_OK;
 }
 
-int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const uint32_t *qprobes,
-               const uint32_t *ids, uint32_t nq, uint32_t k, uint32_t *out_ids, float *out_dists,
+int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const uint32_t *qcount,
+               const uint32_t *qprobes, const uint32_t *ids, uint32_t nq, uint32_t k, uint32_t *out_ids, float *out_dists,
                unsigned long long *ties, cudaStream_t st) {
   uint32_t np2 = 1;
   while (np2 < k) np2 <<= 1;
@@ -577,7 +580,7 @@ int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const
   if (const int rc = smem_limit(reinterpret_cast<const void *>(merge_kernel), static_cast<int>(smem),
                                 "merge_kernel shared memory"))
     return rc;
-  merge_kernel<<<nq, kThreads, smem, st>>>(slots, per_query, per_probe, qprobes, ids, k, out_ids,
+  merge_kernel<<<nq, kThreads, smem, st>>>(slots, per_query, per_probe, qcount, qprobes, ids, k, out_ids,
                                            out_dists, ties);
   KATO_LAUNCHED("merge_kernel");
   return KATO_OK;

@@ -11,7 +11,7 @@ namespace kato {
 struct FinishArgs {
   uint2 *slots;             // per query: per_query candidates (distance bits, row)
   uint32_t per_query, per_probe;
-  const uint32_t *qcount;   // tensor-core pass: candidates per query (bit 31: some were dropped)
+  const uint32_t *qcount;   // candidates per query (bit 31: some were dropped), or null: fixed slots
   const uint32_t *qprobes;  // per-query budgets, or null
   const uint8_t *qhi, *qlo;
   const int64_t *qnorm;     // over all dimensions, 16-bit codes
@@ -33,9 +33,10 @@ struct FinishArgs {
 // Survivors, refinement and top-k of nq queries (ranked modes).
 int finish(const FinishArgs &A, uint32_t nq, cudaStream_t st);
 // Top-k of slots of exact distances (full ranking): per query per_query
-// entries, per_probe for each of its probes.
-int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const uint32_t *qprobes,
-               const uint32_t *ids, uint32_t nq, uint32_t k, uint32_t *out_ids, float *out_dists,
+// entries, of which qcount are used or, without it, per_probe for each of its
+// probes.
+int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const uint32_t *qcount,
+               const uint32_t *qprobes, const uint32_t *ids, uint32_t nq, uint32_t k, uint32_t *out_ids, float *out_dists,
                unsigned long long *ties, cudaStream_t st);
 
 }  // namespace kato

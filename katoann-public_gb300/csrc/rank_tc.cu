@@ -585,7 +585,8 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
     const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
     const uint32_t *__restrict__ list_off, uint32_t p,
-    uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, int32_t *__restrict__ bound) {
+    uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, SeedBound kind, DistScale scale,
+    int32_t *__restrict__ bound) {
   // rowof: the rows looked at; val: their sketch keys. After the pick the
   // scored rows are in val and their l2 go to rowof.
   __shared__ uint32_t rowof[kSeedCap], val[kSeedCap];
@@ -680,7 +681,18 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
   const uint32_t L2 = select(l2s, n, S - 1, h * 65025u < (1u << 24) ? 16 : 24, 0);
   if (tid == 0) {
     const int32_t v = static_cast<int32_t>(L2);
-    bound[q] = v + (v >> 22) + 1;
+    if (kind == SeedBound::kRanking) {
+      bound[q] = v + (v >> 22) + 1;
+    } else {
+      // as the bits of a distance. For exact distances over all h dimensions:
+      // codes whose high bytes differ by e differ by at most 256 e + 255, and
+      // the sum of e is at most sqrt(h sum e^2)
+      int64_t u = v;
+      if (kind == SeedBound::kExactKey)
+        u = 65536ll * v + 65025ll * h + 1 +
+            static_cast<int64_t>(130560.0 * sqrt(static_cast<double>(h) * static_cast<double>(v)));
+      bound[q] = __float_as_int(dist_value(u, scale));
+    }
   }
 }
 
@@ -831,15 +843,15 @@ int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, ui
 
 int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, const int64_t *qnorm,
               const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off, uint32_t B,
-              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, int32_t *bound,
-              cudaStream_t st) {
+              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, SeedBound kind,
+              DistScale scale, int32_t *bound, cudaStream_t st) {
   if (h > 2048 || h % 16) return invalid("seed bounds need h <= 2048, a multiple of 16");
   if (B == 0) return KATO_OK;
   // rows the sketch picks to score in full: 3S (fewer loosen the bound, more
   // cost bytes)
   const uint32_t want = std::min(std::max(rows, S), kSeedCap);
   rank_seed_kernel<<<B, 256, 0, st>>>(xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
-                                      S, want, std::min(want, 3 * S), bound);
+                                      S, want, std::min(want, 3 * S), kind, scale, bound);
   KATO_LAUNCHED("rank_seed_kernel");
   return KATO_OK;
 }

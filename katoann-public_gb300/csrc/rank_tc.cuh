@@ -117,12 +117,15 @@ bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s);
 // One CTA per SM walks an equal share of all tiles.
 int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShape &s,
             cudaStream_t st);
-// Per query, an upper bound on its final S-th ranking l2 from the first
-// `rows` rows (at most 4096) of its probed lists in probe order.
+// Per query, an upper bound on its final S-th ranking l2 over h <= 2048
+// dimensions, from the first `rows` rows (at most 4096) of its probed lists in
+// probe order: as an l2 that no row it could keep exceeds, or as the bits of
+// the distance value of the ranking l2 or of the exact one (h = dc).
+enum class SeedBound { kRanking, kRankingKey, kExactKey };
 int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, const int64_t *qnorm,
               const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off, uint32_t B,
-              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, int32_t *bound,
-              cudaStream_t st);
+              uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, SeedBound kind,
+              DistScale scale, int32_t *bound, cudaStream_t st);
 // Process-wide knobs of the pass (0 = default): the largest item width and
 // the cost weight of the CTA split.
 extern std::atomic<uint32_t> g_tc_width, g_tc_beta;

@@ -33,8 +33,11 @@ std::atomic<uint32_t> g_seed_rows{0};
 namespace {
 
 constexpr int kQG = 16;            // queries per ranking work item
-constexpr int kRT = 16;            // list rows per ranking tile
-constexpr uint32_t kChunk = 1024;  // bytes of a row staged at once
+constexpr int kRT = 32;            // list rows per ranking tile: two per thread
+constexpr uint32_t kChunk = 512;   // bytes of a row staged at once
+// Rows of a list per CTA: lists are skewed, and with a CTA for a whole list the
+// longest one was the kernel's time (200,000 rows in 512 lists: 0.27 ms).
+constexpr uint32_t kSplitRows = 256;
 constexpr uint32_t kSelMax = 256;  // largest per-slot S kept in shared memory
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
@@ -51,7 +54,11 @@ struct RankArgs {
   const uint32_t *woff_total;
   const uint32_t *off, *entries;
   uint32_t dc, dims, nprobe, S, SC;
-  uint2 *slots;  // (query * nprobe + rank) * SC entries of (key, row)
+  const uint32_t *bound;  // per query: no candidate with a larger key is needed (null: none)
+  // selecting: per query, `cap` entries of (key, row), of which qcount are
+  // used; otherwise SC of each probe slot (query * nprobe + rank), in row order
+  uint2 *slots;
+  uint32_t *qcount, cap, split;  // split: rows per CTA
   DistScale scale;
 };
 
@@ -61,7 +68,7 @@ __host__ __device__ inline size_t rank_smem_bytes(int planes, bool select, uint3
   size_t b = static_cast<size_t>(planes) * kQG * qw * 4 + static_cast<size_t>(planes) * kRT * rw * 4;
   b += kRT * 4 + 3 * kQG * 4;           // sids, ccount, bcount, query ids
   b = (b + 15) / 16 * 16;
-  b += kQG * 8;                         // query norms
+  b += kQG * 12;                        // query norms and bounds
   if (select) b += static_cast<size_t>(kQG) * S * 12 + static_cast<size_t>(kQG) * kRT * 12;
   return b;
 }
@@ -79,7 +86,9 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
   const uint32_t c = wk.list;
   const uint32_t e0 = A.off[c] + wk.first;
   const uint32_t ne = min(static_cast<uint32_t>(kQG), A.off[c + 1] - e0);
-  const uint32_t r0 = A.list_off[c], nrows = A.list_off[c + 1] - r0;
+  const uint32_t r0 = A.list_off[c], all_rows = A.list_off[c + 1] - r0;
+  const uint32_t first = blockIdx.y * A.split, nrows = min(all_rows, first + A.split);
+  if (first >= all_rows && (kSelect || blockIdx.y)) return;
   const uint32_t dims = A.dims, qw = dims / 4 + 1;
   const uint32_t kch = min(dims, kChunk), rw = kch / 4 + 1;
   constexpr int kPlanes = kFull ? 2 : 1;
@@ -93,7 +102,8 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
   uint32_t *sslot = bcount + kQG;                      // [kQG]
   size_t off = (reinterpret_cast<unsigned char *>(sslot + kQG) - smem + 15) / 16 * 16;
   int64_t *sqn = reinterpret_cast<int64_t *>(smem + off);                      // [kQG]
-  unsigned long long *bkid = reinterpret_cast<unsigned long long *>(sqn + kQG);  // [kQG][S]
+  uint32_t *sbound = reinterpret_cast<uint32_t *>(sqn + kQG);                  // [kQG]
+  unsigned long long *bkid = reinterpret_cast<unsigned long long *>(sbound + kQG);  // [kQG][S]
   unsigned long long *ckid = bkid + (kSelect ? kQG * S : 0);                   // [kQG][kRT]
   uint32_t *brow = reinterpret_cast<uint32_t *>(ckid + (kSelect ? kQG * kRT : 0));  // [kQG][S]
   uint32_t *crow = brow + (kSelect ? kQG * S : 0);                             // [kQG][kRT]
@@ -106,7 +116,11 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
     sslot[t] = t < static_cast<int>(ne) ? A.entries[e0 + t] : 0;
   }
   __syncthreads();
-  if (t < static_cast<int>(ne)) sqn[t] = A.qnorm[sslot[t] / A.nprobe];
+  if (t < static_cast<int>(ne)) {
+    const uint32_t q = sslot[t] / A.nprobe;
+    sqn[t] = A.qnorm[q];
+    sbound[t] = A.bound ? A.bound[q] : kEmpty;
+  }
   // Stage the queries' bytes (16-byte loads; dims is a multiple of 64).
   const uint32_t v16 = dims / 16;
   for (uint32_t idx = t; idx < ne * v16 * kPlanes; idx += kThreads) {
@@ -119,17 +133,17 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
     dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w;
   }
   // Slots of rows past the list end are padding (store-all mode writes every row).
-  if (!kSelect) {
-    for (uint32_t idx = t; idx < ne * (A.SC - min(nrows, A.SC)); idx += kThreads) {
-      const uint32_t jj = idx / (A.SC - nrows), pos = nrows + idx % (A.SC - nrows);
+  if (!kSelect && blockIdx.y == 0) {
+    for (uint32_t idx = t; idx < ne * (A.SC - min(all_rows, A.SC)); idx += kThreads) {
+      const uint32_t jj = idx / (A.SC - all_rows), pos = all_rows + idx % (A.SC - all_rows);
       A.slots[static_cast<size_t>(sslot[jj]) * A.SC + pos] = make_uint2(kEmpty, 0);
     }
   }
   __syncthreads();
 
-  for (uint32_t rt = 0; rt < nrows; rt += kRT) {
+  for (uint32_t rt = first; rt < nrows; rt += kRT) {
     const uint32_t nr = min(static_cast<uint32_t>(kRT), nrows - rt);
-    uint32_t hh = 0, mx = 0, ll = 0;
+    uint32_t hh[2] = {0, 0}, mx[2] = {0, 0}, ll[2] = {0, 0};  // rows rr and rr + 16
     for (uint32_t k0 = 0; k0 < dims; k0 += kch) {
       const uint32_t kc = min(kch, dims - k0), c16 = kc / 16;
       __syncthreads();
@@ -146,47 +160,59 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
       __syncthreads();
       if (j < static_cast<int>(ne) && rr < static_cast<int>(nr)) {
         const uint32_t *qa = sq + j * qw + k0 / 4;
-        const uint32_t *xa = sr + rr * rw;
+        const uint32_t *xa = sr + rr * rw, *xa2 = xa + 16 * rw;  // (rows past nr: stale, unused)
         const uint32_t nw = kc / 4;
         if (kFull) {
           const uint32_t *qb = sq + (kQG + j) * qw + k0 / 4;
-          const uint32_t *xb = sr + (kRT + rr) * rw;
+          const uint32_t *xb = sr + (kRT + rr) * rw, *xb2 = xb + 16 * rw;
 #pragma unroll 8
           for (uint32_t u = 0; u < nw; ++u) {
-            const uint32_t ah = qa[u], al = qb[u], bh = xa[u], bl = xb[u];
-            hh = dp4(ah, bh, hh);
-            mx = dp4(ah, bl, mx);
-            mx = dp4(al, bh, mx);
-            ll = dp4(al, bl, ll);
+            const uint32_t ah = qa[u], al = qb[u];
+            const uint32_t bh = xa[u], bl = xb[u], ch = xa2[u], cl = xb2[u];
+            hh[0] = dp4(ah, bh, hh[0]);
+            mx[0] = dp4(ah, bl, mx[0]);
+            mx[0] = dp4(al, bh, mx[0]);
+            ll[0] = dp4(al, bl, ll[0]);
+            hh[1] = dp4(ah, ch, hh[1]);
+            mx[1] = dp4(ah, cl, mx[1]);
+            mx[1] = dp4(al, ch, mx[1]);
+            ll[1] = dp4(al, cl, ll[1]);
           }
         } else {
 #pragma unroll 8
-          for (uint32_t u = 0; u < nw; ++u) hh = dp4(qa[u], xa[u], hh);
+          for (uint32_t u = 0; u < nw; ++u) {
+            hh[0] = dp4(qa[u], xa[u], hh[0]);
+            hh[1] = dp4(qa[u], xa2[u], hh[1]);
+          }
         }
       }
     }
-    // The candidate of (row rr, query j).
-    if (j < static_cast<int>(ne) && rr < static_cast<int>(nr)) {
-      const uint32_t row = r0 + rt + rr;
-      const int64_t dot = kFull ? static_cast<int64_t>((static_cast<uint64_t>(hh) << 16) +
-                                                       (static_cast<uint64_t>(mx) << 8) + ll)
-                                : static_cast<int64_t>(hh);
-      const float dist = dist_value(sqn[j] + A.xnorm[row] - 2 * dot, A.scale);
-      const uint32_t key = __float_as_uint(dist);
+    // The candidates of rows rr and rr + 16 with query j. The seed bound leaves
+    // few lists any: merging every tile's candidates took a fifth of the kernel
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = rr + 16 * i;
+      if (j >= static_cast<int>(ne) || r >= static_cast<int>(nr)) continue;
+      const uint32_t row = r0 + rt + r;
+      const int64_t dot = kFull ? static_cast<int64_t>((static_cast<uint64_t>(hh[i]) << 16) +
+                                                       (static_cast<uint64_t>(mx[i]) << 8) + ll[i])
+                                : static_cast<int64_t>(hh[i]);
+      const uint32_t key = __float_as_uint(dist_value(sqn[j] + A.xnorm[row] - 2 * dot, A.scale));
       if (kSelect) {
-        const unsigned long long kid = (static_cast<unsigned long long>(key) << 32) | sids[rr];
+        const unsigned long long kid = (static_cast<unsigned long long>(key) << 32) | sids[r];
         const unsigned long long thr = bcount[j] == S ? bkid[j * S + S - 1] : ~0ull;
-        if (kid < thr) {
+        if (kid < thr && key <= sbound[j]) {
+          found = true;
           const uint32_t pos = atomicAdd(&ccount[j], 1u);
           ckid[j * kRT + pos] = kid;
           crow[j * kRT + pos] = row;
         }
       } else {
-        A.slots[static_cast<size_t>(sslot[j]) * A.SC + rt + rr] = make_uint2(key, row);
+        A.slots[static_cast<size_t>(sslot[j]) * A.SC + rt + r] = make_uint2(key, row);
       }
     }
-    if (kSelect) {
-      __syncthreads();
+    if (kSelect && __syncthreads_or(found)) {
       // Merge each query's new candidates (at most kRT, unsorted) into its
       // sorted best list: one warp per query.
       for (int jj = warp; jj < static_cast<int>(ne); jj += kThreads / 32) {
@@ -248,11 +274,15 @@ __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
     }
   }
   if (kSelect) {
+    // append what was kept to the queries' candidates
+    __syncthreads();
+    if (t < static_cast<int>(ne)) ccount[t] = bcount[t] ? atomicAdd(&A.qcount[sslot[t] / A.nprobe], bcount[t]) : 0;
+    __syncthreads();
     for (uint32_t idx = t; idx < ne * S; idx += kThreads) {
       const uint32_t jj = idx / S, i = idx % S;
-      uint2 v = make_uint2(kEmpty, 0);
-      if (i < bcount[jj]) v = make_uint2(static_cast<uint32_t>(bkid[jj * S + i] >> 32), brow[jj * S + i]);
-      A.slots[static_cast<size_t>(sslot[jj]) * A.SC + i] = v;
+      if (i < bcount[jj])
+        A.slots[static_cast<size_t>(sslot[jj] / A.nprobe) * A.cap + ccount[jj] + i] =
+            make_uint2(static_cast<uint32_t>(bkid[jj * S + i] >> 32), brow[jj * S + i]);
     }
   }
 }
@@ -310,6 +340,7 @@ struct Plan {
   bool coarse_tc;                   // tensor-core coarse product
   TcShape tcs;
   uint32_t tcitems, cap, seed_rows, ctas, rec_cap, beta;
+  uint32_t split, per_query;        // CUDA-core pass: rows per CTA, candidate entries per query
   bool cost;                        // the ranking CTAs split the slabs' cost, not their count
   size_t off_fq, off_qhi, off_qlo, off_qn, off_qhn, off_qh0, off_cd, off_probed, off_cnt, off_off,
       off_base, off_cur, off_work, off_ent, off_slots, off_stats,
@@ -345,6 +376,15 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   // to a buffer of `cap` entries (an overflowing query is rescanned exactly)
   pl.cap = g_candidate_cap.load();
   pl.tc = ranking != KATO_RANK_FULL && pl.S <= pl.cap && rank_tc_plan(pl.dims, ix->dc, &pl.tcs);
+  // rows per CTA of the CUDA-core pass; each CTA keeps up to SC candidates per
+  // query, and up to 2 GiB of them the lists are split (a larger batch then
+  // still has at least that, so that its workspace serves a smaller one too)
+  constexpr uint64_t kSplitEntries = 1ull << 28;
+  pl.split = kSplitRows;
+  if (pl.select && !pl.tc && static_cast<uint64_t>(B) * p * div_up(ml, kSplitRows) * pl.SC > kSplitEntries) pl.split = ml;
+  const uint64_t per_query = static_cast<uint64_t>(p) * pl.SC * (pl.select ? div_up(ml, pl.split) : 1);
+  if (!pl.tc && per_query >= (1ull << 32)) return invalid("too many candidates per query");
+  pl.per_query = static_cast<uint32_t>(per_query);
   if (pl.tc) {
     pl.select = true;
     pl.SC = pl.S;
@@ -387,7 +427,9 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_cur = take(static_cast<size_t>(L) * 4);
   pl.off_work = take(wmax * sizeof(Work));
   pl.off_ent = take(bp * 4);
-  pl.off_slots = take((pl.tc ? static_cast<size_t>(B) * pl.cap : bp * pl.SC) * sizeof(uint2));
+  uint64_t entries = static_cast<uint64_t>(B) * (pl.tc ? pl.cap : pl.per_query);
+  if (pl.select && !pl.tc && pl.split != kSplitRows) entries = std::max(entries, kSplitEntries);
+  pl.off_slots = take(entries * sizeof(uint2));
   pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);
   pl.off_tileoff = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * 4 : 16);
@@ -552,21 +594,32 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   }
   if ((rc = invert(I, counted, &g_launches, st))) return rc;
   mark(tm, 5, st);
-  uint32_t *qcount = nullptr;
-  if (!pl.tc) mark(tm, 6, st);  // no seed-bound phase on the CUDA-core pass
+  // (the CUDA-core pass that keeps every candidate has them in fixed slots)
+  uint32_t *qcount = pl.select ? reinterpret_cast<uint32_t *>(ws + pl.off_qcount) : nullptr;
+  const bool full = pl.ranking == KATO_RANK_FULL;
+  const bool prefix_mode = pl.ranking == KATO_RANK_PREFIX;
+  int32_t *bound = reinterpret_cast<int32_t *>(ws + pl.off_bound);
+  const DistScale scale = make_dist_scale(ix->step_sq);
+  const bool seeded = pl.select && !pl.tc && pl.dims <= 2048;
+  if (seeded) {
+    // seed bounds of the CUDA-core pass, over the same high bytes
+    if ((rc = rank_seed(ix->d_hi, prefix_mode ? ix->d_headnorm : ix->d_hinorm, qhi,
+                        prefix_mode ? qh0 : qhn, probed, qprobes, ix->d_list_off, nq, p, dc, pl.dims,
+                        pl.S, std::max(2048u, 16 * pl.S),
+                        full ? SeedBound::kExactKey : SeedBound::kRankingKey, scale, bound, st)))
+      return rc;
+    ++g_launches;
+  }
+  if (!pl.tc) mark(tm, 6, st);
   if (pl.tc) {
     // 4'. ranking pass on the tensor cores: seed bounds, work items, the
     // scan, and the exact rescan of any query whose buffer overflowed
-    int32_t *bound = reinterpret_cast<int32_t *>(ws + pl.off_bound);
     uint4 *rec = reinterpret_cast<uint4 *>(ws + pl.off_rec);
     uint32_t *rec_n = reinterpret_cast<uint32_t *>(ws + pl.off_recn);
-    qcount = reinterpret_cast<uint32_t *>(ws + pl.off_qcount);
-    const bool prefix_mode = pl.ranking == KATO_RANK_PREFIX;
     const int64_t *xnorm = prefix_mode ? ix->d_headnorm : ix->d_hinorm;
     const int64_t *qnorm = prefix_mode ? qh0 : qhn;
-    const DistScale scale = make_dist_scale(ix->step_sq);
     if ((rc = rank_seed(ix->d_hi, xnorm, qhi, qnorm, probed, qprobes, ix->d_list_off, nq, p, dc,
-                        pl.dims, pl.S, pl.seed_rows, bound, st)))
+                        pl.dims, pl.S, pl.seed_rows, SeedBound::kRanking, scale, bound, st)))
       return rc;
     mark(tm, 6, st);
     RankTcArgs T{};
@@ -597,7 +650,6 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     g_launches += 3;  // seed, scan, bucket
   }
   // 4. ranking pass (:998-1044 / :1167-1204)
-  const bool full = pl.ranking == KATO_RANK_FULL;
   RankArgs A{};
   A.xhi = ix->d_hi;
   A.xlo = ix->d_lo;
@@ -616,10 +668,15 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   A.nprobe = p;
   A.S = pl.SC;  // a slot never holds more than min(S, largest list) candidates
   A.SC = pl.SC;
+  A.bound = seeded ? reinterpret_cast<const uint32_t *>(bound) : nullptr;
   A.slots = slots;
-  A.scale = make_dist_scale(ix->step_sq);
+  A.qcount = reinterpret_cast<uint32_t *>(ws + pl.off_qcount);
+  A.cap = pl.per_query;
+  A.split = pl.split;
+  A.scale = scale;
   const size_t bp = static_cast<size_t>(nq) * p;
-  const uint32_t grid = static_cast<uint32_t>(std::min<size_t>(L, bp) + bp / kQG + 1);
+  const dim3 grid(static_cast<uint32_t>(std::min<size_t>(L, bp) + bp / kQG + 1),
+                  std::max(1u, div_up(ix->max_list, pl.split)));
   const size_t smem = rank_smem_bytes(full ? 2 : 1, pl.select, pl.dims, pl.SC);
   if (!pl.tc && smem > 227 * 1024) return invalid("ranking tile does not fit in shared memory");
   auto launch = [&](auto kern) -> int {
@@ -641,11 +698,12 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
   // of the ranking distances the survivors, their exact distances and the
   // top-k (:1058-1125)
   if (full) {
-    rc = merge_topk(slots, p * pl.SC, pl.SC, qprobes, ix->d_ids, nq, pl.k, out_ids, out_dists, stats + 1, st);
+    rc = merge_topk(slots, pl.per_query, pl.SC, qcount, qprobes, ix->d_ids, nq, pl.k, out_ids, out_dists,
+                    stats + 1, st);
   } else {
     FinishArgs F{};
     F.slots = slots;
-    F.per_query = pl.tc ? pl.cap : p * pl.SC;
+    F.per_query = pl.tc ? pl.cap : pl.per_query;
     F.per_probe = pl.SC;
     F.qcount = qcount;
     F.qprobes = qprobes;
@@ -660,13 +718,12 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     F.dc = dc;
     F.S = pl.S;
     F.k = pl.k;
-    F.scale = make_dist_scale(ix->step_sq);
+    F.scale = scale;
     F.out_ids = out_ids;
     F.out_dists = out_dists;
     F.ties = stats + 1;
     F.rescans = stats + 6;
     if (pl.tc) {
-      const bool prefix_mode = pl.ranking == KATO_RANK_PREFIX;
       F.rank_xnorm = prefix_mode ? ix->d_headnorm : ix->d_hinorm;
       F.rank_qnorm = prefix_mode ? qh0 : qhn;
       F.probed = probed;

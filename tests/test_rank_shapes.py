@@ -47,3 +47,17 @@ def test_ranking_tiles(dim, head, kind):
         rid, rd = ref.search(q[-nq:], **kw)
         bad = np.nonzero((ids != rid).any(1) | (dists != rd).any(1))[0]
         assert len(bad) == 0, (nq, kw, bad[:5])
+
+
+def test_workspace_of_a_batch_serves_smaller_ones():
+    """katoann_gpu_search_workspace grows with the batch for every ranking: a
+    workspace sized for max_batch must do for any batch up to it."""
+    import ctypes as C
+
+    from _gpu import GpuIndex, gpu
+    view = GpuIndex(dim=128, dc=128, nlist=4096, npts=1 << 22, head_dims=128, max_list=9000)
+    for ranking in (0, 1, 2):
+        for k, survivors in ((10, 32), (200, 200), (300, 600)):
+            sizes = [gpu().katoann_gpu_search_workspace(C.byref(view), b, k, 512, ranking, survivors)
+                     for b in (1, 2, 7, 63, 64, 500, 1000, 2000, 4096)]
+            assert sizes[0] > 0 and sizes == sorted(sizes), (ranking, k, sizes)
