@@ -564,22 +564,41 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // them, a sketch picks the ones to score: the squared distance over the first
 // 32 head dimensions (the leading rotated dimensions, which carry most of the
 // variance), of which the `full` smallest, and any others in the last one's
-// bin of sketch distance / 16, are scored over all h dimensions.
+// bin, are scored over all h dimensions.
 // The bound is the S-th smallest scored l2, widened to L + (L >> 22) + 1: the
 // distance value is monotone in l2 and two l2 that far apart never round to
 // the same float, so every row whose distance can tie the S-th best is still
 // inside. Any S of a query's candidates bound its S-th best from above, so
 // the rows the sketch picks change no result, only how tight the bound is
-// and how many bytes it costs: 2,048 sketched rows (32 bytes each) and 3S
-// scored rows read 2.3 times fewer bytes than 1,024 scored rows of 256 bytes
-// and leave fewer candidates. Fewer than S rows: no bound.
-constexpr uint32_t kSketchBytes = 32;  // head bytes of a row the sketch reads
+// and how many bytes it costs: 1,024 sketched rows (32 bytes each) and 2S
+// scored rows read 4 times fewer bytes than 1,024 scored rows of 256 bytes. Fewer than S rows: no bound.
 
-__device__ __forceinline__ uint32_t sq_diff4(uint32_t a, uint32_t b, uint32_t acc) {
-  const uint32_t d = __vabsdiffu4(a, b);  // |a - b| per byte
-  return dp4(d, d, acc);
+// sum x (x - 2 q) over 16 bytes: the squared distance less the query's own sum
+__device__ __forceinline__ uint32_t sketch16(uint4 x, uint4 q) {
+  const uint32_t xx = dp4(x.x, x.x, dp4(x.y, x.y, dp4(x.z, x.z, dp4(x.w, x.w, 0))));
+  const uint32_t xq = dp4(x.x, q.x, dp4(x.y, q.y, dp4(x.z, q.z, dp4(x.w, q.w, 0))));
+  return xx - 2 * xq;
 }
 
+// The bin of half a sketch distance (32 255^2 < 2^21, so half of it is below
+// 2^20): 32 bins per power of two, so that one histogram of 512 bins resolves
+// every distance to 3%.
+constexpr uint32_t kSketchBins = 512;
+__device__ __forceinline__ uint32_t sketch_bin(uint32_t d) {
+  if (d < 32) return d;
+  const uint32_t e = 31 - __clz(d);
+  return (e - 4) * 32 + ((d >> (e - 5)) & 31);
+}
+
+//
+// The sketch loads bound it: 32-byte pieces of rows h or more bytes apart. Two
+// lanes to a row halve the L1's work (2,048 rows: 148 -> 127 us for 4096 queries
+// at 1M; the squares as x (x - 2 q) by dp4a instead of a byte-wise difference
+// among it), eight of them are in flight to a thread; at 10M it is the DRAM's, and
+// more CTAs on an SM than three slow it down (206, 254, 276 us at three, four,
+// five). The rest is a chain of latencies, kept short: offsets read 32 lists at a
+// time, keys kept in registers, one histogram for the picked bin, and a last
+// selection that ranks by counting where there are few.
 __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint8_t *__restrict__ xhi, const int64_t *__restrict__ xnorm,
     const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
@@ -587,99 +606,158 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint32_t *__restrict__ list_off, uint32_t p,
     uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, SeedBound kind, DistScale scale,
     int32_t *__restrict__ bound) {
-  // rowof: the rows looked at; val: their sketch keys. After the pick the
-  // scored rows are in val and their l2 go to rowof.
-  __shared__ uint32_t rowof[kSeedCap], val[kSeedCap];
+  // rowof: the rows looked at. Where all are scored, l2s gets their distances;
+  // where some are, l2s gets those rows and rowof their distances.
+  __shared__ __align__(16) uint32_t rowof[kSeedCap];
+  __shared__ __align__(16) uint32_t l2s[kSeedCap];
   __shared__ __align__(16) uint32_t qw[2048 / 4];
-  __shared__ uint32_t hist[256], sel[2], wsum[8], npick;
-  const uint32_t q = blockIdx.x, tid = threadIdx.x;
-  for (uint32_t i = tid; i < h / 4; i += blockDim.x)
+  __shared__ uint32_t hist[kSketchBins], sel[2], wsum[8], npick;
+  const uint32_t q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (uint32_t i = tid; i < h / 4; i += 256)
     qw[i] = reinterpret_cast<const uint32_t *>(qhi + static_cast<size_t>(q) * dc)[i];
+  for (uint32_t i = tid; i < kSketchBins; i += 256) hist[i] = 0;
+  if (tid == 0) npick = 0;
+  // the rows, 32 lists at a time: every warp reads their offsets, and writes
+  // the rows of every eighth
   const uint32_t pq = qprobes ? qprobes[q] : p;  // the query's own budget
   uint32_t count = 0;
-  for (uint32_t r = 0; r < pq && count < want; ++r) {
-    const uint32_t c = probed[static_cast<size_t>(q) * p + r];
-    const uint32_t r0 = list_off[c], n = min(list_off[c + 1] - r0, want - count);
-    for (uint32_t i = tid; i < n; i += blockDim.x) rowof[count + i] = r0 + i;
-    count += n;
+  for (uint32_t r = 0; r < pq && count < want; r += 32) {
+    uint32_t r0 = 0, n = 0;
+    if (r + lane < pq) {
+      const uint32_t c = probed[static_cast<size_t>(q) * p + r + lane];
+      r0 = list_off[c];
+      n = list_off[c + 1] - r0;
+    }
+    uint32_t incl = min(n, want);  // (sums stay below 32 want)
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const uint32_t at = count + incl - min(n, want), total = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t l = warp; l < 32; l += 8) {
+      const uint32_t first = __shfl_sync(0xffffffffu, at, l), row = __shfl_sync(0xffffffffu, r0, l);
+      const uint32_t rows = __shfl_sync(0xffffffffu, n, l);
+      if (first >= want) break;
+      const uint32_t m = min(rows, want - first);
+      for (uint32_t i = lane; i < m; i += 32) rowof[first + i] = row + i;
+    }
+    count = min(want, count + total);
   }
-  if (tid == 0) npick = 0;
   __syncthreads();
   if (count < S) {
     if (tid == 0) bound[q] = 0x7FFFFFFF;
     return;
   }
-  // radix selection of the rank-th smallest of v[0 .. n) by 8-bit digits,
-  // from the digit at bit `start` down to the one at bit `stop` (the lower
-  // bits of the result stay 0; digits above `start` must be 0 in every value)
-  auto select = [&](const uint32_t *v, uint32_t n, uint32_t rank, int start, int stop) {
-    uint32_t prefix = 0;
-    for (int shift = start; shift >= stop; shift -= 8) {
-      for (uint32_t i = tid; i < 256; i += blockDim.x) hist[i] = 0;
+  uint32_t n = count;
+  const uint32_t *rows = rowof;
+  uint32_t *l2 = l2s;
+  if (count > full) {
+    // Every row in or below the bin of the full-th smallest sketch distance is
+    // scored: at least `full`, a few more when the bin holds several. Two lanes
+    // read a row's 32 bytes, which is one line of a load's 32 for each pair
+    // instead of one for each lane; even lanes keep the rows of the even loads,
+    // odd lanes those of the odd ones: row 32 (8 j + warp) + 16 (lane & 1) +
+    // lane / 2 is key j.
+    constexpr uint32_t kPer = kSeedCap / 256;
+    const uint32_t odd = lane & 1;
+    const uint4 qv = reinterpret_cast<const uint4 *>(qw)[odd];
+    const uint32_t qq = dp4(qv.x, qv.x, dp4(qv.y, qv.y, dp4(qv.z, qv.z, dp4(qv.w, qv.w, 0))));
+    const uint32_t q2 = qq + __shfl_xor_sync(0xffffffffu, qq, 1);
+    const uint32_t r0 = 32 * warp + lane / 2, mine0 = r0 + 16 * odd;
+    uint32_t bins[kPer / 2];  // two 16-bit bins to a word
+#pragma unroll
+    for (uint32_t j0 = 0; j0 < kPer; j0 += 4) {
+      if (j0 * 256 >= count) break;
+      uint4 v[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j) {
+        const uint32_t i = (j0 + j / 2) * 256 + r0 + 16 * (j & 1);
+        v[j] = __ldg(reinterpret_cast<const uint4 *>(xhi + static_cast<size_t>(rowof[min(i, count - 1)]) * dc) + odd);
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t t0 = sketch16(v[2 * j], qv), t1 = sketch16(v[2 * j + 1], qv);
+        const uint32_t d2 = q2 + (odd ? t1 : t0) + __shfl_xor_sync(0xffffffffu, odd ? t0 : t1, 1);
+        const uint32_t bin = sketch_bin(d2 / 2);
+        if ((j0 + j) * 256 + mine0 < count) atomicAdd(&hist[bin], 1u);
+        if (j & 1) bins[(j0 + j) / 2] |= bin << 16;
+        else bins[(j0 + j) / 2] = bin;
+      }
+    }
+    __syncthreads();
+    // the bin of rank full - 1: thread t has bins 2 t and 2 t + 1
+    const uint32_t ha = hist[2 * tid], hb = hist[2 * tid + 1];
+    uint32_t incl = ha + hb;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t below = incl - ha - hb;
+    for (uint32_t w = 0; w < warp; ++w) below += wsum[w];
+    if (full - 1 >= below && full - 1 < below + ha + hb) sel[0] = 2 * tid + (full - 1 >= below + ha);
+    __syncthreads();
+    const uint32_t last = sel[0];
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j) {
+      if (j * 256 >= count) break;
+      const bool take = j * 256 + mine0 < count && ((bins[j / 2] >> (16 * (j & 1))) & 0xFFFFu) <= last;
+      const uint32_t votes = __ballot_sync(0xffffffffu, take);
+      uint32_t at = 0;
+      if (lane == 0 && votes) at = atomicAdd(&npick, __popc(votes));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1));
+      if (take) l2s[at] = rowof[j * 256 + mine0];
+    }
+    __syncthreads();
+    n = npick;
+    rows = l2s;
+    l2 = rowof;
+  }
+  const int64_t qn = qnorm[q];
+  for_rows_at(
+      xhi, dc, h, qw, [&](uint32_t i) { return rows[i]; }, n,
+      [&](uint32_t i, uint32_t dot, int64_t xn) {
+        l2[i] = static_cast<uint32_t>(qn + xn - 2 * static_cast<int64_t>(dot));
+      },
+      [&](uint32_t i) { return xnorm[rows[i]]; });
+  // the S-th smallest
+  uint32_t L2 = 0;
+  bool have = false;
+  if (n <= 256) {
+    if (tid >= n && tid < (n + 3) / 4 * 4) l2[tid] = 0xFFFFFFFFu;
+    __syncthreads();
+    const uint32_t v = l2[min(tid, n - 1)];
+    uint32_t lt = 0, le = 0;
+    for (uint32_t j = 0; j < n; j += 4) {
+      const uint4 o = *reinterpret_cast<const uint4 *>(l2 + j);
+      lt += (o.x < v) + (o.y < v) + (o.z < v) + (o.w < v);
+      le += (o.x <= v) + (o.y <= v) + (o.z <= v) + (o.w <= v);
+    }
+    L2 = v;
+    have = tid < n && lt < S && S <= le;  // equal values: each of them says the same
+  } else {
+    __syncthreads();
+    // radix selection by 8-bit digits (l2 < 255^2 h: no top digit for h up to 258)
+    uint32_t prefix = 0, rank = S - 1;
+    for (int shift = h * 65025u < (1u << 24) ? 16 : 24; shift >= 0; shift -= 8) {
+      if (tid < 256) hist[tid] = 0;
       __syncthreads();
       const uint32_t hm = shift == 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      for (uint32_t i = tid; i < n; i += blockDim.x)
-        if ((v[i] & hm) == prefix) atomicAdd(&hist[(v[i] >> shift) & 0xFFu], 1u);
+      for (uint32_t i = tid; i < n; i += 256)
+        if ((l2[i] & hm) == prefix) atomicAdd(&hist[(l2[i] >> shift) & 0xFFu], 1u);
       __syncthreads();
       block_pick_digit(hist, rank, sel, wsum);
       rank -= sel[1];
       prefix |= sel[0] << shift;
       __syncthreads();
     }
-    return prefix;
-  };
-  const uint32_t *rows = rowof;
-  uint32_t *l2s = val, n = count;
-  if (count > full) {
-    // keys (sketch distance, at most 20 bits) << 12 | i. Two digits find the
-    // 16-bit bin (sketch distance >> 4) of the full-th smallest key; every
-    // row in or below that bin is scored: at least `full`, a few more when
-    // the bin holds several
-    const uint32_t parts = min(kSketchBytes, h) / 16;  // lanes per row, 16 bytes each
-    const uint32_t part = tid % parts, per = blockDim.x / parts;
-    const uint4 qv = reinterpret_cast<const uint4 *>(qw)[part];
-    for (uint32_t base = 0; base < count; base += 4 * per) {
-      uint4 v[4];
-#pragma unroll
-      for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t i = base + j * per + tid / parts;
-        v[j] = i < count ? __ldg(reinterpret_cast<const uint4 *>(
-                               xhi + static_cast<size_t>(rowof[i]) * dc) + part)
-                         : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (uint32_t j = 0; j < 4; ++j) {
-        uint32_t d2 = sq_diff4(v[j].x, qv.x, sq_diff4(v[j].y, qv.y,
-                      sq_diff4(v[j].z, qv.z, sq_diff4(v[j].w, qv.w, 0))));
-        if (parts == 2) d2 += __shfl_xor_sync(0xffffffffu, d2, 1);
-        const uint32_t i = base + j * per + tid / parts;
-        if (part == 0 && i < count) val[i] = (min(d2, 0xFFFFFu) << 12) | i;
-      }
-    }
-    __syncthreads();
-    const uint32_t kth = select(val, count, full - 1, 24, 16) | 0xFFFFu;
-    uint32_t mine = 0;  // bit j: key tid + 256 j is picked (count <= 16 x 256)
-    for (uint32_t j = 0, i = tid; i < count; ++j, i += blockDim.x)
-      if (val[i] <= kth) mine |= 1u << j;
-    __syncthreads();
-    for (uint32_t j = 0, i = tid; i < count; ++j, i += blockDim.x)
-      if (mine >> j & 1u) val[atomicAdd(&npick, 1u)] = rowof[i];
-    __syncthreads();
-    rows = val;
-    l2s = rowof;
-    n = npick;
+    L2 = prefix;
+    have = tid == 0;
   }
-  const int64_t qn = qnorm[q];
-  for_rows_at(
-      xhi, dc, h, qw, [&](uint32_t i) { return rows[i]; }, n,
-      [&](uint32_t i, uint32_t dot, int64_t xn) {
-        l2s[i] = static_cast<uint32_t>(qn + xn - 2 * static_cast<int64_t>(dot));
-      },
-      [&](uint32_t i) { return xnorm[rows[i]]; });
-  __syncthreads();
-  // l2 < 255^2 h: below 2^24 (no top digit) for h up to 258
-  const uint32_t L2 = select(l2s, n, S - 1, h * 65025u < (1u << 24) ? 16 : 24, 0);
-  if (tid == 0) {
+  if (have) {
     const int32_t v = static_cast<int32_t>(L2);
     if (kind == SeedBound::kRanking) {
       bound[q] = v + (v >> 22) + 1;
@@ -845,13 +923,13 @@ int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, cons
               const uint32_t *probed, const uint32_t *qprobes, const uint32_t *list_off, uint32_t B,
               uint32_t p, uint32_t dc, uint32_t h, uint32_t S, uint32_t rows, SeedBound kind,
               DistScale scale, int32_t *bound, cudaStream_t st) {
-  if (h > 2048 || h % 16) return invalid("seed bounds need h <= 2048, a multiple of 16");
+  if (h > 2048 || h % 64) return invalid("seed bounds need h <= 2048, a multiple of 64");
   if (B == 0) return KATO_OK;
-  // rows the sketch picks to score in full: 3S (fewer loosen the bound, more
-  // cost bytes)
+  // rows the sketch picks to score in full: 2S (3S leaves 1% fewer candidates
+  // for 8 to 14 us more of every 4096 queries' seeds, 3S / 2 1 to 10% more)
   const uint32_t want = std::min(std::max(rows, S), kSeedCap);
   rank_seed_kernel<<<B, 256, 0, st>>>(xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
-                                      S, want, std::min(want, 3 * S), kind, scale, bound);
+                                      S, want, std::min(want, 2 * S), kind, scale, bound);
   KATO_LAUNCHED("rank_seed_kernel");
   return KATO_OK;
 }

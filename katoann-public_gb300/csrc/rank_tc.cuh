@@ -111,6 +111,13 @@ __host__ __device__ inline TcSmem tc_smem_layout(uint32_t h, const TcShape &s) {
   return L;
 }
 
+// Rows a seed bound looks at unless set otherwise: a looser bound costs the
+// ranking pass little (its time follows the tiles, not the candidates), so the
+// seed's own time decides. max(1024, 8 S) with 2 S of them scored takes 88 us
+// for 4096 queries at 1M x 1024 (S = 32) and 132 at 10M (S = 64), where
+// max(2048, 16 S) with 3 S took 127 and 206 for 2% and 14% fewer candidates; at 512
+// rows the 78% more candidates at 10M cost more than the seed saves.
+inline uint32_t default_seed_rows(uint32_t S) { return std::max(1024u, 8 * std::min(S, 1u << 20)); }
 // The shape for h ranking dimensions over rows of dc bytes, or false when h
 // does not suit the pass (the caller then uses the CUDA-core pass).
 bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s);

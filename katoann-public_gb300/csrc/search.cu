@@ -27,7 +27,7 @@ namespace kato {
 thread_local uint32_t g_launches = 0;  // kernel launches of the last search pass
 // Entries per query of the tensor-core ranking pass's candidate buffer.
 std::atomic<uint32_t> g_candidate_cap{32768};
-// Rows a query's seed bound looks at (0: max(2048, 16 survivors)).
+// Rows a query's seed bound looks at (0: default_seed_rows).
 std::atomic<uint32_t> g_seed_rows{0};
 
 namespace {
@@ -389,7 +389,7 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
     pl.select = true;
     pl.SC = pl.S;
     const uint32_t sr = g_seed_rows.load();
-    pl.seed_rows = sr ? std::max(sr, pl.S) : std::max(2048u, 16 * pl.S);
+    pl.seed_rows = sr ? std::max(sr, pl.S) : default_seed_rows(pl.S);
     pl.tcitems = static_cast<uint32_t>(bp / pl.tcs.N + std::min<size_t>(L, bp) + 1);
     // candidate records per CTA: room for 32 S per query of the batch, spread
     // over the CTAs (a CTA that runs out flags the queries it drops)
@@ -605,7 +605,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     // seed bounds of the CUDA-core pass, over the same high bytes
     if ((rc = rank_seed(ix->d_hi, prefix_mode ? ix->d_headnorm : ix->d_hinorm, qhi,
                         prefix_mode ? qh0 : qhn, probed, qprobes, ix->d_list_off, nq, p, dc, pl.dims,
-                        pl.S, std::max(2048u, 16 * pl.S),
+                        pl.S, default_seed_rows(pl.S),
                         full ? SeedBound::kExactKey : SeedBound::kRankingKey, scale, bound, st)))
       return rc;
     ++g_launches;

@@ -49,6 +49,25 @@ def test_ranking_tiles(dim, head, kind):
         assert len(bad) == 0, (nq, kw, bad[:5])
 
 
+@pytest.mark.parametrize("kind", ["decaying", "ends"])
+@pytest.mark.parametrize("S", [1, 31, 128, 129, 300, 511, 1300])
+def test_seed_bounds(S, kind):
+    """Survivor counts around the seed bound's own edges: all of the probed rows
+    scored or a sketch's pick of 2 S, the last selection by counting (256 rows) or
+    by digits, fewer rows than S, and every sketch distance in a few bins."""
+    import katoann
+    a, q = _arrays(128, 64, kind, 17, S)
+    idx = katoann.Index()
+    idx.load_arrays(a["centroids"], a["list_sizes"], a["ids"], a["vectors"], head_dims=64)
+    ref = oracle.OracleIndex(None, arrays=a)
+    for nprobe, ranking in ((len(SIZES), "prefix"), (len(SIZES), "high"), (5, "prefix"), (len(SIZES), "full")):
+        kw = dict(k=min(S, 20), nprobe=nprobe, ranking=ranking, survivors=S)
+        ids, dists = idx.search(q, **kw)
+        rid, rd = ref.search(q, **kw)
+        bad = np.nonzero((ids != rid).any(1) | (dists != rd).any(1))[0]
+        assert len(bad) == 0, (kw, bad[:5])
+
+
 def test_workspace_of_a_batch_serves_smaller_ones():
     """katoann_gpu_search_workspace grows with the batch for every ranking: a
     workspace sized for max_batch must do for any batch up to it."""
