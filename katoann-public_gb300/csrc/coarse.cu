@@ -154,10 +154,10 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
   // 1) the p-th smallest key (rank p-1), and how many keys are below it.
   uint32_t prefix = 0, rank = p - 1, below = 0;
   for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = tid; i < 256; i += kSelThreads) hist[i] = 0;
+    for (uint32_t i = tid; i < 256; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     const uint32_t hmask = shift == 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-    for (uint32_t i = tid; i < n; i += kSelThreads) {
+    for (uint32_t i = tid; i < n; i += blockDim.x) {
       const uint32_t k = keys[i];
       if ((k & hmask) == prefix) atomicAdd(&hist[(k >> shift) & 0xFFu], 1u);
     }
@@ -173,7 +173,7 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
   // 2) among keys == T, the need-th smallest list id (only when ties exceed need).
   if (tid == 0) scal[3] = 0;
   __syncthreads();
-  for (uint32_t i = tid; i < n; i += kSelThreads)
+  for (uint32_t i = tid; i < n; i += blockDim.x)
     if (keys[i] == T) atomicAdd(&scal[3], 1u);
   __syncthreads();
   const uint32_t neq = scal[3];
@@ -182,10 +182,10 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
     if (tid == 0 && tie_count) atomicAdd(tie_count, 1ull);
     uint32_t ip = 0, ir = need - 1;
     for (int shift = 24; shift >= 0; shift -= 8) {
-      for (int i = tid; i < 256; i += kSelThreads) hist[i] = 0;
+      for (uint32_t i = tid; i < 256; i += blockDim.x) hist[i] = 0;
       __syncthreads();
       const uint32_t hmask = shift == 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      for (uint32_t i = tid; i < n; i += kSelThreads)
+      for (uint32_t i = tid; i < n; i += blockDim.x)
         if (keys[i] == T && (i & hmask) == ip) atomicAdd(&hist[(i >> shift) & 0xFFu], 1u);
       __syncthreads();
       const uint32_t bin = block_scan_bins(hist, ir, scal, scal + 1);
@@ -199,7 +199,7 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
   if (tid == 0) scal[2] = 0;
   __syncthreads();
   const bool sorted = p <= kSortMax;
-  for (uint32_t i = tid; i < n; i += kSelThreads) {
+  for (uint32_t i = tid; i < n; i += blockDim.x) {
     const uint32_t k = keys[i];
     if (k < T || (k == T && i <= idmax)) {
       const uint32_t pos = atomicAdd(&scal[2], 1u);
@@ -213,11 +213,11 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
   // 4) bitonic sort of the p selected, padded to a power of two.
   uint32_t np2 = 1;
   while (np2 < p) np2 <<= 1;
-  for (uint32_t i = p + tid; i < np2; i += kSelThreads) sel[i] = ~0ull;
+  for (uint32_t i = p + tid; i < np2; i += blockDim.x) sel[i] = ~0ull;
   __syncthreads();
   for (uint32_t size = 2; size <= np2; size <<= 1) {
     for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = tid; i < np2; i += kSelThreads) {
+      for (uint32_t i = tid; i < np2; i += blockDim.x) {
         const uint32_t j = i ^ stride;
         if (j > i) {
           const bool up = (i & size) == 0;
@@ -231,7 +231,7 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
       __syncthreads();
     }
   }
-  for (uint32_t i = tid; i < p; i += kSelThreads) outp[i] = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
+  for (uint32_t i = tid; i < p; i += blockDim.x) outp[i] = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
 }
 
 // Rows are written `stride` apart. With `cnt`, each selected list's counter
@@ -275,108 +275,201 @@ __device__ void sort_keys(unsigned long long *key, uint32_t n) {
 }
 
 // Smallest p of a row of n non-negative float distances by (distance, list),
-// ascending, for p <= kSortMax, in two passes over the row: a histogram of
-// the top 12 bits below the sign (distances cluster in a narrow range, so
-// these bits still spread them), then a gather that takes every key of a bin
-// below the boundary bin and collects the boundary bin's keys, of which the
-// first (p - below) by (key, index) complete the selection. A boundary bin
-// with more than kCand keys falls back to select_passes.
-constexpr uint32_t kHistBins = 4096;
-constexpr uint32_t kCand = 2048;
+// ascending, for p <= kSortMax, in one pass over the row: it stays in registers
+// (V 16-byte loads per thread; V = 0: longer rows are read again).
+//
+//   1. The p-th smallest of the minima of disjoint groups of keys bounds the p-th
+//      smallest key from above, and closely: p of G minima leave about
+//      -G ln(1 - p / G) keys at or below it (84 for p = 72, G = 512). A group
+//      is what a thread holds (level 0), four neighbours (1) or one key (2).
+//   2. A histogram over the range of the minima finds the p-th to 1/1024 of
+//      that range, from above.
+//   3. Every key up to it is gathered. A few are ranked by counting the smaller
+//      ones of each; more by a histogram of their own range, whose prefix sums
+//      leave a handful of keys to compare in each bin. (Counting c keys reads
+//      shared memory c^2 / 32 times: 460 keys of 5,000 took 184 us for 2000 rows, 39
+//      with the bins.)
+//
+// More than `cap` gathered keys (many equal distances) fall back to
+// select_passes, crowded bins to a bitonic sort. The rows' DRAM reads and, between
+// them, the chain of barriers bound it: 4096 rows of 16,384 lists, p = 72, take
+// 78 us (HBM needs 41 for their 268 MB) where a histogram of all keys, a second
+// pass and the sort of its boundary bin took 127; 4,096 lists 25 us for 52.
+constexpr uint32_t kSelBins = 1024;
 
-__global__ void __launch_bounds__(kSelThreads) select_topp_hist_kernel(
-    const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride,
-    uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
+__device__ __forceinline__ uint32_t min4(uint4 x) { return min(min(x.x, x.y), min(x.z, x.w)); }
+
+template <uint32_t NT, uint32_t V>
+__global__ void __launch_bounds__(NT) select_topp_near_kernel(
+    const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride, uint32_t level,
+    uint32_t cap, uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
     unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
     uint32_t only_above) {
-  extern __shared__ unsigned long long dyn[];
-  unsigned long long *cand = dyn;          // kCand
-  unsigned long long *sel = dyn + kCand;   // np2(p)
-  __shared__ uint32_t hist[kHistBins];
-  __shared__ uint32_t scal[8];
-  __shared__ uint32_t wsum[kSelThreads / 32];
+  extern __shared__ unsigned long long cand[];  // cap keys (key << 32 | list)
+  uint16_t *order = reinterpret_cast<uint16_t *>(cand + cap);
+  __shared__ uint32_t hist[kSelBins], wlo[NT / 32], whi[NT / 32], wsum[NT / 32], scal[4];
+  constexpr uint32_t kNone = 0xFFFFFFFFu;  // no key: above every distance
+  constexpr uint32_t kPer = kSelBins / NT;
   const uint32_t q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (only && only[q] <= only_above) return;
   const uint32_t *keys = reinterpret_cast<const uint32_t *>(dists) + static_cast<size_t>(q) * n;
   uint32_t *outp = probed + static_cast<size_t>(q) * stride;
-  for (uint32_t i = tid; i < kHistBins; i += kSelThreads) hist[i] = 0;
-  if (tid < 8) scal[tid] = 0;
-  __syncthreads();
   const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
-  const uint32_t n4 = vec ? n / 4 : 0;
-  auto bin_of = [](uint32_t k) { return (k >> 19) & (kHistBins - 1); };
-  // 1) histogram
-#pragma unroll 4
-  for (uint32_t i = tid; i < n4; i += kSelThreads) {
-    const uint4 v = reinterpret_cast<const uint4 *>(keys)[i];
-    atomicAdd(&hist[bin_of(v.x)], 1u);
-    atomicAdd(&hist[bin_of(v.y)], 1u);
-    atomicAdd(&hist[bin_of(v.z)], 1u);
-    atomicAdd(&hist[bin_of(v.w)], 1u);
-  }
-  for (uint32_t i = n4 * 4 + tid; i < n; i += kSelThreads) atomicAdd(&hist[bin_of(keys[i])], 1u);
-  __syncthreads();
-  // 2) the bin holding rank p - 1: each thread owns 16 consecutive bins
-  constexpr uint32_t kPer = kHistBins / kSelThreads;
-  uint32_t tsum = 0;
+  // keys 4 i .. 4 i + 3
+  auto load = [&](uint32_t i) -> uint4 {
+    const uint32_t i4 = 4 * i;
+    if (vec && i4 + 4 <= n) return reinterpret_cast<const uint4 *>(keys)[i];
+    return make_uint4(i4 < n ? keys[i4] : kNone, i4 + 1 < n ? keys[i4 + 1] : kNone,
+                      i4 + 2 < n ? keys[i4 + 2] : kNone, i4 + 3 < n ? keys[i4 + 3] : kNone);
+  };
+  uint4 held[V ? V : 1];
+  if constexpr (V > 0) {
 #pragma unroll
-  for (uint32_t j = 0; j < kPer; ++j) tsum += hist[tid * kPer + j];
-  uint32_t incl = tsum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= static_cast<uint32_t>(o)) incl += y;
+    for (uint32_t v = 0; v < V; ++v) held[v] = load(v * NT + tid);
   }
-  if (lane == 31) wsum[warp] = incl;
-  __syncthreads();
-  uint32_t wbase = 0;
-  for (uint32_t w = 0; w < warp; ++w) wbase += wsum[w];
-  const uint32_t excl = wbase + incl - tsum, rank = p - 1;
-  if (rank >= excl && rank < excl + tsum) {
-    uint32_t acc = excl, j = 0;
-    for (; j < kPer; ++j) {
-      const uint32_t h = hist[tid * kPer + j];
-      if (rank < acc + h) break;
-      acc += h;
+  for (uint32_t i = tid; i < kSelBins; i += NT) hist[i] = 0;
+  if (tid < 4) scal[tid] = 0;
+  // f(four keys, the first one's index) over the thread's keys
+  auto each = [&](auto f) {
+    if constexpr (V > 0) {
+#pragma unroll
+      for (uint32_t v = 0; v < V; ++v) f(held[v], 4 * (v * NT + tid));
+    } else {
+      for (uint32_t i = tid; i < (n + 3) / 4; i += NT) f(load(i), 4 * i);
     }
-    scal[0] = tid * kPer + j;  // boundary bin
-    scal[1] = acc;             // keys below it
+  };
+  // 1) the range of the minima
+  uint32_t tmin = kNone, hi = 0;
+  auto top = [&](uint32_t k) { hi = k == kNone ? hi : max(hi, k); };
+  each([&](uint4 x, uint32_t) {
+    const uint32_t m = min4(x);
+    tmin = min(tmin, m);
+    if (level == 1) top(m);
+    if (level == 2) top(x.x), top(x.y), top(x.z), top(x.w);
+  });
+  if (level == 0) top(tmin);
+  const uint32_t wl = __reduce_min_sync(0xffffffffu, tmin), wh = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) wlo[warp] = wl, whi[warp] = wh;
+  __syncthreads();
+  const uint32_t lo = __reduce_min_sync(0xffffffffu, wlo[lane % (NT / 32)]);
+  const uint32_t range = __reduce_max_sync(0xffffffffu, whi[lane % (NT / 32)]) - lo;
+  const uint32_t shift = range < kSelBins ? 0 : 32 - __clz(range) - 10;
+  // 2) the bin of rank p - 1: each thread owns kPer consecutive bins
+  auto tally = [&](uint32_t k) {
+    if (k != kNone) atomicAdd(&hist[(k - lo) >> shift], 1u);
+  };
+  if (level == 0) {
+    tally(tmin);
+  } else {
+    each([&](uint4 x, uint32_t) {
+      if (level == 1) tally(min4(x));
+      else tally(x.x), tally(x.y), tally(x.z), tally(x.w);
+    });
   }
   __syncthreads();
-  const uint32_t bstar = scal[0], below = scal[1], c = hist[bstar];
-  if (c > kCand) {  // a crowded boundary bin: the radix passes instead
-    select_passes(keys, n, p, outp, cnt, tie_count, sel, hist, scal + 4);
+  // the keys in bins below the thread's own, and in them
+  uint32_t sum;
+  auto scan_bins = [&]() -> uint32_t {
+    sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j) sum += hist[tid * kPer + j];
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t below = incl - sum;
+#pragma unroll
+    for (uint32_t w = 0; w < NT / 32; ++w) below += w < warp ? wsum[w] : 0;
+    return below;
+  };
+  uint32_t below = scan_bins();
+  if (p - 1 >= below && p - 1 < below + sum) {
+    uint32_t j = 0;
+    for (; j < kPer - 1; ++j) {
+      below += hist[tid * kPer + j];
+      if (p - 1 < below) break;
+    }
+    scal[0] = min(lo + min(((tid * kPer + j + 1) << shift) - 1, ~lo), kNone - 1);
+  }
+  __syncthreads();
+  // 3) the keys up to it
+  const uint32_t T = scal[0];
+  for (uint32_t i = tid; i < kSelBins; i += NT) hist[i] = 0;
+  each([&](uint4 x, uint32_t i) {
+    if (min4(x) > T) return;
+    const uint32_t k[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      if (k[j] > T) continue;
+      const uint32_t at = atomicAdd(&scal[1], 1u);
+      if (at < cap) cand[at] = (static_cast<unsigned long long>(k[j]) << 32) | (i + j);
+    }
+  });
+  __syncthreads();
+  const uint32_t c = scal[1];
+  if (c > cap) {
+    select_passes(keys, n, p, outp, cnt, tie_count, cand, hist, scal);
     return;
   }
-  // 3) gather: bins below the boundary are in; the boundary bin is a candidate
-  auto take = [&](uint32_t k, uint32_t i) {
-    const uint32_t b = bin_of(k);
-    if (b < bstar) sel[atomicAdd(&scal[2], 1u)] = (static_cast<unsigned long long>(k) << 32) | i;
-    else if (b == bstar) cand[atomicAdd(&scal[3], 1u)] = (static_cast<unsigned long long>(k) << 32) | i;
+  // 4) the first p of them in order
+  auto put = [&](uint32_t at, uint32_t list) {
+    outp[at] = list;
+    if (cnt) atomicAdd(&cnt[list], 1u);
   };
-#pragma unroll 4
-  for (uint32_t i = tid; i < n4; i += kSelThreads) {
-    const uint4 v = reinterpret_cast<const uint4 *>(keys)[i];
-    take(v.x, 4 * i);
-    take(v.y, 4 * i + 1);
-    take(v.z, 4 * i + 2);
-    take(v.w, 4 * i + 3);
+  auto ranked = [&](uint32_t at, unsigned long long k) {
+    if (at < p) put(at, static_cast<uint32_t>(k));
+    if (at + 1 == p) scal[2] = static_cast<uint32_t>(k >> 32);
+    if (at == p) scal[3] = static_cast<uint32_t>(k >> 32);
+  };
+  if (c <= NT / 4) {
+    // 2^lg threads count the keys below each
+    uint32_t lg = 0;
+    while (lg < 5 && (c << (lg + 1)) <= NT) ++lg;
+    const uint32_t g = tid >> lg;
+    const unsigned long long mine = cand[min(g, c - 1)];
+    uint32_t less = 0;
+    for (uint32_t j = tid & ((1u << lg) - 1); j < c; j += 1u << lg) less += cand[j] < mine;
+    for (uint32_t o = 1; o < 1u << lg; o <<= 1) less += __shfl_xor_sync(0xffffffffu, less, o);
+    if (g < c && (tid & ((1u << lg) - 1)) == 0) ranked(less, mine);
+    __syncthreads();
+    if (tid == 0 && tie_count && c > p && scal[2] == scal[3]) atomicAdd(tie_count, 1ull);
+    return;
   }
-  for (uint32_t i = n4 * 4 + tid; i < n; i += kSelThreads) take(keys[i], i);
+  const uint32_t near = T - lo, shift2 = near < kSelBins ? 0 : 32 - __clz(near) - 10;
+  auto bin_of = [&](unsigned long long k) { return (static_cast<uint32_t>(k >> 32) - lo) >> shift2; };
+  for (uint32_t i = tid; i < c; i += NT) atomicAdd(&hist[bin_of(cand[i])], 1u);
   __syncthreads();
-  // 4) the boundary bin's keys in order; the first `need` complete the set
-  sort_keys(cand, c);
-  const uint32_t need = p - below;
-  for (uint32_t i = tid; i < need; i += kSelThreads) sel[below + i] = cand[i];
-  if (tid == 0 && tie_count && need < c && (cand[need] >> 32) == (cand[need - 1] >> 32))
-    atomicAdd(tie_count, 1ull);
-  __syncthreads();
-  // 5) the p selected in order
-  sort_keys(sel, p);
-  for (uint32_t i = tid; i < p; i += kSelThreads) {
-    const uint32_t c = static_cast<uint32_t>(sel[i] & 0xFFFFFFFFu);
-    outp[i] = c;
-    if (cnt) atomicAdd(&cnt[c], 1u);
+  below = scan_bins();
+  bool crowded = false;
+#pragma unroll
+  for (uint32_t j = 0; j < kPer; ++j) {
+    const uint32_t h = hist[tid * kPer + j];
+    crowded |= h > 32;
+    hist[tid * kPer + j] = below;
+    below += h;
+  }
+  if (!__syncthreads_or(crowded)) {
+    for (uint32_t i = tid; i < c; i += NT) order[atomicAdd(&hist[bin_of(cand[i])], 1u)] = static_cast<uint16_t>(i);
+    __syncthreads();
+    // bin b is now order[hist[b - 1]] .. order[hist[b] - 1]
+    for (uint32_t i = tid; i < c; i += NT) {
+      const unsigned long long mine = cand[i];
+      const uint32_t b = bin_of(mine), end = hist[b];
+      uint32_t less = b ? hist[b - 1] : 0;
+      if (less > p) continue;
+      for (uint32_t j = less; j < end; ++j) less += cand[order[j]] < mine;
+      ranked(less, mine);
+    }
+    __syncthreads();
+    if (tid == 0 && tie_count && c > p && scal[2] == scal[3]) atomicAdd(tie_count, 1ull);
+  } else {
+    sort_keys(cand, c);
+    for (uint32_t i = tid; i < p; i += NT) put(i, static_cast<uint32_t>(cand[i]));
+    if (tid == 0 && tie_count && c > p && (cand[p] >> 32) == (cand[p - 1] >> 32)) atomicAdd(tie_count, 1ull);
   }
 }
 
@@ -408,21 +501,33 @@ int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint
                    const uint32_t *only, uint32_t only_above, cudaStream_t st) {
   if (nq == 0) return KATO_OK;
   if (p == 0 || p > n || stride < p) return invalid("need 1 <= nprobe <= nlist");
-  uint32_t np2 = 1;
-  while (np2 < p) np2 <<= 1;
-  int rc;
-  if ((rc = smem_limit(reinterpret_cast<const void *>(select_topp_kernel), kSortMax * 8,
-                       "select_topp_kernel shared memory")) ||
-      (rc = smem_limit(reinterpret_cast<const void *>(select_topp_hist_kernel),
-                       (kCand + kSortMax) * 8, "select_topp_hist_kernel shared memory")))
-    return rc;
   if (p <= kSortMax) {
-    // candidates and the sorted selection (the bitonic sort pads to a power of two)
-    const size_t smem = (kCand + std::max<uint32_t>(np2, 2)) * sizeof(unsigned long long);
-    select_topp_hist_kernel<<<nq, kSelThreads, smem, st>>>(dists, n, p, stride, probed, cnt,
-                                                            tie_count, only, only_above);
-    KATO_LAUNCHED("select_topp_hist_kernel");
-    return KATO_OK;
+    uint32_t cap = 1024;
+    while (cap < p) cap <<= 1;
+    cap *= 2;
+    // A row in one thread block's registers where it fits: the smallest block
+    // that takes at most 8 loads a thread, as smaller blocks overlap one row's
+    // loads with another's ranking (4096 rows of 4,096 lists: 25 us with 256
+    // threads, 36 with 512; 2000 rows of 5,000, p = 384: 39 and 49). 16,384
+    // lists: 512 threads 78 us, 256 with 16 loads 96, 1024 with four 127, reading
+    // the row again 90; 2000 rows of 5,000 read again 41.
+    auto go = [&](auto kern, uint32_t threads) -> int {
+      if (const int rc = smem_limit(reinterpret_cast<const void *>(kern), 2 * kSortMax * 10,
+                                    "select_topp_near_kernel shared memory"))
+        return rc;
+      // the largest groups that still leave few keys below the bound: p of 3 p
+      // minima leave 1.2 p, p of 3 p / 2 leave 1.7 p
+      const uint32_t level = std::min(threads, div_up(n, 4)) >= 3 * p ? 0 : div_up(n, 4) >= 3 * p / 2 ? 1 : 2;
+      kern<<<nq, threads, cap * 10, st>>>(dists, n, p, stride, level, cap, probed,
+                                                                  cnt, tie_count, only, only_above);
+      KATO_LAUNCHED("select_topp_near_kernel");
+      return KATO_OK;
+    };
+    if (n <= 1024) return go(select_topp_near_kernel<128, 2>, 128);
+    if (n <= 4096) return go(select_topp_near_kernel<256, 4>, 256);
+    if (n <= 8192) return go(select_topp_near_kernel<256, 8>, 256);
+    if (n <= 16384) return go(select_topp_near_kernel<512, 8>, 512);
+    return go(select_topp_near_kernel<512, 0>, 512);
   }
   select_topp_kernel<<<nq, kSelThreads, 0, st>>>(dists, n, p, stride, probed, cnt, tie_count,
                                                   only, only_above);
