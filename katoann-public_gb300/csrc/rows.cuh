@@ -34,7 +34,8 @@ __device__ __forceinline__ uint32_t row_dot(const uint8_t *row, const uint32_t *
 
 // Dot products of a query (its h bytes as words in shared memory) with rows
 // row(0) .. row(n - 1) of a byte plane, lanes split along each row: a group of
-// G = min(32, h / 16) lanes reads a row as one coalesced run of 16-byte
+// G = 4, 8, 16 or 32 lanes (32 from h = 512 on, whose last step some sit out
+// where h / 16 is no multiple of it) reads a row as one coalesced run of 16-byte
 // loads and sums over the group by shuffles. A warp takes 32 rows at a time
 // (G steps, all loads of the batch in flight together) and hands row
 // base + l of the batch to one lane, so f(i, dot) runs on all 32 lanes at
@@ -50,12 +51,12 @@ __device__ __forceinline__ void rows_split(const uint8_t *__restrict__ x, uint32
                                            F f) {
   constexpr uint32_t RPW = 32 / G;  // rows per step
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t sub = lane / G, gl = lane % G, cpl = (h / 16) / G;
+  const uint32_t sub = lane / G, gl = lane % G, units = h / 16;
   for (uint32_t base = warp * 32; base < n; base += nw * 32) {
     uint32_t mine = 0;
     const uint32_t my_row = base + gl * RPW + sub;
     const int64_t pv = my_row < n ? pre(my_row) : 0;
-    if (G <= 16 && cpl == 1) {
+    if (G <= 16 && units == G) {
       // every load of the batch first, then the sums
       uint4 v[G <= 16 ? G : 1];
       const uint32_t *w = qw + 4 * gl;
@@ -79,8 +80,7 @@ __device__ __forceinline__ void rows_split(const uint8_t *__restrict__ x, uint32
         uint32_t dot = 0;
         if (i < n) {
           const uint4 *rv = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row(i)) * dc);
-          for (uint32_t c = 0; c < cpl; ++c) {
-            const uint32_t u = gl + c * G;
+          for (uint32_t u = gl; u < units; u += G) {
             const uint4 vv = __ldg(rv + u);
             const uint32_t *w = qw + 4 * u;
             dot = dp4(vv.x, w[0], dp4(vv.y, w[1], dp4(vv.z, w[2], dp4(vv.w, w[3], dot))));

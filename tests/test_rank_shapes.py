@@ -68,6 +68,29 @@ def test_seed_bounds(S, kind):
         assert len(bad) == 0, (kw, bad[:5])
 
 
+@pytest.mark.parametrize("dim,ranking", [(192, "prefix"), (512, "high"), (576, "prefix"), (640, "high"),
+                                         (832, "high"), (960, "prefix"), (1024, "prefix")])
+def test_rescans_over_every_dimension(dim, ranking):
+    """Candidate buffers of 16 rows: the queries are rescanned, over all of a
+    prefix whose 16-byte pieces need not divide among the lanes of a row."""
+    import katoann
+
+    from _gpu import gpu
+    a, q = _arrays(dim, dim, "flat", 20, dim)
+    idx = katoann.Index()
+    idx.load_arrays(a["centroids"], a["list_sizes"], a["ids"], a["vectors"], head_dims=dim)
+    ref = oracle.OracleIndex(None, arrays=a)
+    kw = dict(k=10, nprobe=len(SIZES), ranking=ranking, survivors=16)
+    rid, rd = ref.search(q, **kw)
+    try:
+        assert gpu().katoann_gpu_set_candidate_cap(16) == 0
+        ids, dists = idx.search(q, **kw)
+        assert idx.search_stats()["ranking_rescans"] > 0
+    finally:
+        assert gpu().katoann_gpu_set_candidate_cap(32768) == 0
+    assert np.array_equal(ids, rid) and np.array_equal(dists, rd)
+
+
 def test_workspace_of_a_batch_serves_smaller_ones():
     """katoann_gpu_search_workspace grows with the batch for every ranking: a
     workspace sized for max_batch must do for any batch up to it."""
