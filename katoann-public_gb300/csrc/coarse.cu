@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256) sq16_tile_kernel(
     const uint8_t *__restrict__ xhi, const uint8_t *__restrict__ xlo,
     const int64_t *__restrict__ qn, const int64_t *__restrict__ xn, DistScale scale, uint32_t m,
     uint32_t n, uint32_t dims, uint32_t qstride, uint32_t xstride, float *__restrict__ out) {
+  after_previous();
   __shared__ uint32_t sqh[kTile * kSw], sxh[kTile * kSw];
   __shared__ uint32_t sql[kFull ? kTile * kSw : 1], sxl[kFull ? kTile * kSw : 1];
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(kSelThreads) select_topp_kernel(
     uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
     unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
     uint32_t only_above) {
+  after_previous();
   extern __shared__ unsigned long long sel[];  // up to kSortMax (key << 32 | id)
   __shared__ uint32_t hist[256], scal[4];
   const uint32_t q = blockIdx.x;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(NT) select_topp_near_kernel(
     uint32_t cap, uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
     unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
     uint32_t only_above) {
+  after_previous();
   extern __shared__ unsigned long long cand[];  // cap keys (key << 32 | list)
   uint16_t *order = reinterpret_cast<uint16_t *>(cand + cap);
   __shared__ uint32_t hist[kSelBins], wlo[NT / 32], whi[NT / 32], wsum[NT / 32], scal[4];
@@ -490,8 +493,8 @@ int sq16_tiles(const uint8_t *qhi, const uint8_t *qlo, const uint8_t *xhi, const
   const DistScale s = make_dist_scale(step_sq);
   dim3 grid(div_up(n, kTile), div_up(m, kTile));
   if (grid.y > 65535) return invalid("too many query rows for one call");
-  if (full) sq16_tile_kernel<true><<<grid, 256, 0, st>>>(qhi, qlo, xhi, xlo, qn, xn, s, m, n, dims, qstride, xstride, out);
-  else sq16_tile_kernel<false><<<grid, 256, 0, st>>>(qhi, qlo, xhi, xlo, qn, xn, s, m, n, dims, qstride, xstride, out);
+  if (full) launch(sq16_tile_kernel<true>, grid, 256, 0, st, qhi, qlo, xhi, xlo, qn, xn, s, m, n, dims, qstride, xstride, out);
+  else launch(sq16_tile_kernel<false>, grid, 256, 0, st, qhi, qlo, xhi, xlo, qn, xn, s, m, n, dims, qstride, xstride, out);
   KATO_LAUNCHED("sq16_tile_kernel");
   return KATO_OK;
 }
@@ -518,7 +521,7 @@ int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint
       // the largest groups that still leave few keys below the bound: p of 3 p
       // minima leave 1.2 p, p of 3 p / 2 leave 1.7 p
       const uint32_t level = std::min(threads, div_up(n, 4)) >= 3 * p ? 0 : div_up(n, 4) >= 3 * p / 2 ? 1 : 2;
-      kern<<<nq, threads, cap * 10, st>>>(dists, n, p, stride, level, cap, probed,
+      launch(kern, nq, threads, cap * 10, st, dists, n, p, stride, level, cap, probed,
                                                                   cnt, tie_count, only, only_above);
       KATO_LAUNCHED("select_topp_near_kernel");
       return KATO_OK;
@@ -529,7 +532,7 @@ int select_topp_ex(const float *dists, uint32_t nq, uint32_t n, uint32_t p, uint
     if (n <= 16384) return go(select_topp_near_kernel<512, 8>, 512);
     return go(select_topp_near_kernel<512, 0>, 512);
   }
-  select_topp_kernel<<<nq, kSelThreads, 0, st>>>(dists, n, p, stride, probed, cnt, tie_count,
+  launch(select_topp_kernel, nq, kSelThreads, 0, st, dists, n, p, stride, probed, cnt, tie_count,
                                                   only, only_above);
   KATO_LAUNCHED("select_topp_kernel");
   return KATO_OK;

@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     coarse_tc_kernel(const __grid_constant__ CUtensorMap tch, const __grid_constant__ CUtensorMap tcl,
                      const __grid_constant__ CUtensorMap tqh, const __grid_constant__ CUtensorMap tql,
                      const CoarseArgs A) {
+  after_previous();
   extern __shared__ __align__(1024) unsigned char smraw[];
   // 1 KiB-aligned stages (the swizzle pattern repeats every 1024 bytes)
   unsigned char *sm = smraw + ((1024 - (tc::smem_addr(smraw) & 1023u)) & 1023u);
@@ -347,7 +348,7 @@ int coarse_tc(const __half *ch, const __half *cl, const int64_t *cterm, uint32_t
     return rc;
   const CoarseArgs A{cterm, qterm, out, m, n, dc, make_dist_scale(step_sq), timeouts, prof};
   const uint32_t ntiles = div_up(n, kCM) * div_up(m, kQN);
-  coarse_tc_kernel<<<std::min<uint32_t>(ntiles, sms), kThreads, kSmem, st>>>(mch, mcl, mqh, mql, A);
+  launch(coarse_tc_kernel, std::min<uint32_t>(ntiles, sms), kThreads, kSmem, st, mch, mcl, mqh, mql, A);
   KATO_LAUNCHED("coarse_tc_kernel");
   return KATO_OK;
 }

@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(
     const uint32_t *__restrict__ ids, uint32_t k,
     uint32_t *__restrict__ out_ids, float *__restrict__ out_dists,
     unsigned long long *__restrict__ tie_count) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t hist[256], scratch[8], wsum[8];
   __shared__ bool tie;
@@ -403,6 +404,7 @@ __device__ void tied_topk(const FinishArgs &A, uint32_t ns, unsigned long long *
 constexpr uint32_t kCount = 256;  // entries ranked by counting, one per thread
 
 __global__ void __launch_bounds__(kThreads, 4) finish_kernel(const __grid_constant__ FinishArgs A) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(16) uint32_t hist[256];
   __shared__ uint32_t scratch[8], wsum[8], nsel, bound[2];
@@ -566,7 +568,7 @@ int finish(const FinishArgs &A, uint32_t nq, cudaStream_t st) {
   if (const int rc = smem_limit(reinterpret_cast<const void *>(finish_kernel), static_cast<int>(smem),
                                 "finish_kernel shared memory"))
     return rc;
-  finish_kernel<<<nq, kThreads, smem, st>>>(A);
+  launch(finish_kernel, nq, kThreads, smem, st, A);
   KATO_LAUNCHED("finish_kernel");
   return KATO_OK;
 }
@@ -580,7 +582,7 @@ int merge_topk(const uint2 *slots, uint32_t per_query, uint32_t per_probe, const
   if (const int rc = smem_limit(reinterpret_cast<const void *>(merge_kernel), static_cast<int>(smem),
                                 "merge_kernel shared memory"))
     return rc;
-  merge_kernel<<<nq, kThreads, smem, st>>>(slots, per_query, per_probe, qcount, qprobes, ids, k, out_ids,
+  launch(merge_kernel, nq, kThreads, smem, st, slots, per_query, per_probe, qcount, qprobes, ids, k, out_ids,
                                            out_dists, ties);
   KATO_LAUNCHED("merge_kernel");
   return KATO_OK;

@@ -26,6 +26,7 @@ __device__ __forceinline__ bool probed_pair(uint32_t i, uint32_t p,
 
 __global__ void count_kernel(const uint32_t *__restrict__ probed, uint32_t total, uint32_t p,
                              const uint32_t *__restrict__ qprobes, uint32_t *__restrict__ cnt) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total && probed_pair(i, p, qprobes)) atomicAdd(&cnt[probed[i]], 1u);
 }
@@ -42,6 +43,7 @@ __device__ __forceinline__ uint32_t slab_cost(uint32_t ne, uint32_t N, uint32_t 
 // N); on the tensor-core pass none for an empty list), slabs and cost (base),
 // with the totals after them.
 __global__ void __launch_bounds__(1024) invert_scan_kernel(const InvertArgs A) {
+  after_previous();
   const uint32_t L = A.L, N = A.N;
   uint32_t *ci = A.base, *cs = ci + L + 1, *cc = cs + L + 1;
   const uint4 tot = block_scan4(
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(1024) invert_scan_kernel(const InvertArgs A) {
 // Thread i: scatters probe slot i, writes the items of list i and finds where
 // share i starts.
 __global__ void invert_expand_kernel(const InvertArgs A) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, L = A.L, N = A.N;
   const uint32_t *ci = A.base, *cs = ci + L + 1;
   if (i < A.B * A.p && probed_pair(i, A.p, A.qprobes))
@@ -136,11 +139,11 @@ __global__ void invert_expand_kernel(const InvertArgs A) {
 int invert(const InvertArgs &A, bool counted, uint32_t *launches, cudaStream_t st) {
   const uint32_t total = A.B * A.p;
   if (!counted) {
-    count_kernel<<<div_up(total, 256), 256, 0, st>>>(A.probed, total, A.p, A.qprobes, A.cnt);
+    launch(count_kernel, div_up(total, 256), 256, 0, st, A.probed, total, A.p, A.qprobes, A.cnt);
     ++*launches;
   }
-  invert_scan_kernel<<<1, 1024, 0, st>>>(A);
-  invert_expand_kernel<<<div_up(std::max(std::max(total, A.L), A.ctas + 1), 256), 256, 0, st>>>(A);
+  launch(invert_scan_kernel, 1, 1024, 0, st, A);
+  launch(invert_expand_kernel, div_up(std::max(std::max(total, A.L), A.ctas + 1), 256), 256, 0, st, A);
   *launches += 2;
   KATO_LAUNCHED("inversion kernels");
   return KATO_OK;

@@ -57,6 +57,7 @@ __host__ __device__ __forceinline__ uint16_t bf16_round(float f) {
 __global__ void __launch_bounds__(256) probe_features_kernel(
     const float *__restrict__ cd, uint32_t L, const uint32_t *__restrict__ probed, uint32_t P,
     const uint32_t *__restrict__ rank, uint32_t B, float *__restrict__ z) {
+  after_previous();
   const uint32_t q = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (q >= B) return;
   const float *row = cd + static_cast<size_t>(q) * L;
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(kH) probe_mlp_kernel(const float *__restrict__
                                                         MlpArgs m, uint32_t cap,
                                                         float *__restrict__ probs,
                                                         uint32_t *__restrict__ nprobe) {
+  after_previous();
   extern __shared__ __align__(16) float sm[];
   float *x0 = sm;                 // [kF][kAS]
   float *h1 = x0 + kF * kAS;      // [kH][kAS]
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(kH) probe_mlp_kernel(const float *__restrict__
 
 __global__ void clamp_budget_kernel(const uint32_t *__restrict__ in, uint32_t B, uint32_t cap,
                                     uint32_t *__restrict__ out) {
+  after_previous();
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < B) out[q] = in ? max(1u, min(in[q], cap)) : cap;
 }
@@ -468,7 +471,7 @@ int check_probe_model(const katoann_gpu_probe_model &m) {
 int probe_features(const float *cd, uint32_t L, const uint32_t *probed, uint32_t P,
                    const uint32_t *rank, uint32_t B, float *z, cudaStream_t st) {
   if (B == 0) return KATO_OK;
-  probe_features_kernel<<<div_up(B, 8), 256, 0, st>>>(cd, L, probed, P, rank, B, z);
+  launch(probe_features_kernel, div_up(B, 8), 256, 0, st, cd, L, probed, P, rank, B, z);
   KATO_LAUNCHED("probe_features_kernel");
   return KATO_OK;
 }
@@ -481,14 +484,14 @@ int probe_budget(const katoann_gpu_probe_model &m, const float *z, uint32_t B, u
     return rc;
   const MlpArgs a{m.d_shift, m.d_scale, m.d_w1, m.d_w2, m.d_w3, m.d_b1,
                   m.d_b2,    m.d_b3,    m.d_ladder, m.nclass, m.threshold};
-  probe_mlp_kernel<<<div_up(B, kQB), kH, kMlpSmem, st>>>(z, B, a, cap, probs, nprobe);
+  launch(probe_mlp_kernel, div_up(B, kQB), kH, kMlpSmem, st, z, B, a, cap, probs, nprobe);
   KATO_LAUNCHED("probe_mlp_kernel");
   return KATO_OK;
 }
 
 int clamp_budget(const uint32_t *in, uint32_t B, uint32_t cap, uint32_t *out, cudaStream_t st) {
   if (B == 0) return KATO_OK;
-  clamp_budget_kernel<<<div_up(B, 256), 256, 0, st>>>(in, B, cap, out);
+  launch(clamp_budget_kernel, div_up(B, 256), 256, 0, st, in, B, cap, out);
   KATO_LAUNCHED("clamp_budget_kernel");
   return KATO_OK;
 }

@@ -151,6 +151,7 @@ template <uint32_t IN, bool kCentred>
 __global__ void __launch_bounds__(kTcThreads, 1)
     rank_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ RankTcArgs A,
                    const __grid_constant__ TcShape S) {
+  after_previous();
   constexpr uint32_t NI = IN / 64;        // 16-byte reads per row, lane and chunk
     constexpr uint32_t kBox = kTcBoxRows * IN, kStage = 2 * kBox;
   // row bytes enter as multiples of kScale
@@ -606,6 +607,7 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint32_t *__restrict__ list_off, uint32_t p,
     uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, SeedBound kind, DistScale scale,
     int32_t *__restrict__ bound) {
+  after_previous();
   // rowof: the rows looked at. Where all are scored, l2s gets their distances;
   // where some are, l2s gets those rows and rowof their distances.
   __shared__ __align__(16) uint32_t rowof[kSeedCap];
@@ -786,6 +788,7 @@ __global__ void __launch_bounds__(256) tc_bucket_kernel(
     const int32_t *__restrict__ bound, uint32_t dc, uint32_t f, uint32_t h,
     uint32_t *__restrict__ qcount, uint2 *__restrict__ qbuf, uint32_t cap, DistScale scale,
     unsigned long long *__restrict__ found) {
+  after_previous();
   const uint4 *r = rec + static_cast<size_t>(blockIdx.x) * rec_cap;
   const uint32_t n = rec_n[blockIdx.x], lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
   const uint32_t nw = gridDim.y * (blockDim.x >> 5);
@@ -901,7 +904,7 @@ int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShap
     if (const int rc = smem_limit(reinterpret_cast<const void *>(kern), static_cast<int>(s.smem),
                                   "rank_tc_kernel shared memory"))
       return rc;
-    kern<<<ctas, kTcThreads, s.smem, st>>>(tmap, A, s);
+    launch(kern, ctas, kTcThreads, s.smem, st, tmap, A, s);
     KATO_LAUNCHED("rank_tc_kernel");
     return KATO_OK;
   };
@@ -913,7 +916,7 @@ int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, ui
                    const uint8_t *xhi, const uint8_t *qhi, const int2 *qcn, const int32_t *bound,
                    uint32_t dc, uint32_t f, uint32_t h, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
                    DistScale scale, unsigned long long *found, cudaStream_t st) {
-  tc_bucket_kernel<<<dim3(ctas, nq < 512 ? 1 : 8), 256, 0, st>>>(rec, rec_n, rec_cap, xhi, qhi, qcn, bound, dc, f, h,
+  launch(tc_bucket_kernel, dim3(ctas, nq < 512 ? 1 : 8), 256, 0, st, rec, rec_n, rec_cap, xhi, qhi, qcn, bound, dc, f, h,
                                                   qcount, qbuf, cap, scale, found);
   KATO_LAUNCHED("tc_bucket_kernel");
   return KATO_OK;
@@ -928,7 +931,7 @@ int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, cons
   // rows the sketch picks to score in full: 2S (3S leaves 1% fewer candidates
   // for 8 to 14 us more of every 4096 queries' seeds, 3S / 2 1 to 10% more)
   const uint32_t want = std::min(std::max(rows, S), kSeedCap);
-  rank_seed_kernel<<<B, 256, 0, st>>>(xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
+  launch(rank_seed_kernel, B, 256, 0, st, xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
                                       S, want, std::min(want, 2 * S), kind, scale, bound);
   KATO_LAUNCHED("rank_seed_kernel");
   return KATO_OK;

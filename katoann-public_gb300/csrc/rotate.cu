@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
                       const float *__restrict__ in, uint32_t nrows, uint32_t d,
                       const float *__restrict__ rot, float *__restrict__ out,
                       uint32_t *__restrict__ timeouts) {
+  after_previous();
   constexpr int TB = kRows ? 8 : 16, CG = kRows ? 4 : 2;
   constexpr uint32_t kStage = rot_stage_bytes<kRows>();
   constexpr uint32_t kRowTile = kRows ? kSlabRows : 32, kColTile = 32;
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
 __global__ void __launch_bounds__(256) transpose_pad_kernel(const float *__restrict__ in,
                                                             uint32_t rows, uint32_t d, uint32_t kn,
                                                             float *__restrict__ out, uint32_t ld) {
+  after_previous();
   __shared__ float tile[32][33];
   const uint32_t r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -352,6 +354,7 @@ __global__ void __launch_bounds__(256) transpose_pad_kernel(const float *__restr
 __global__ void __launch_bounds__(256) transpose_pad4_kernel(const float *__restrict__ in,
                                                              uint32_t rows, uint32_t d, uint32_t kn,
                                                              float *__restrict__ out, uint32_t ld) {
+  after_previous();
   __shared__ float tile[64][65];
   const uint32_t r0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
   const uint32_t t = threadIdx.x;
@@ -378,16 +381,17 @@ __global__ void __launch_bounds__(256) transpose_pad4_kernel(const float *__rest
 void transpose_pad(const float *in, uint32_t rows, uint32_t d, uint32_t kn, float *out, uint32_t ld,
                    cudaStream_t st) {
   if (d % 4 == 0 && ld % 32 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0)
-    transpose_pad4_kernel<<<dim3(div_up(ld, 64), div_up(kn, 64)), 256, 0, st>>>(in, rows, d, kn, out,
+    launch(transpose_pad4_kernel, dim3(div_up(ld, 64), div_up(kn, 64)), 256, 0, st, in, rows, d, kn, out,
                                                                                 ld);
   else
-    transpose_pad_kernel<<<dim3(ld / 32, div_up(kn, 32)), 256, 0, st>>>(in, rows, d, kn, out, ld);
+    launch(transpose_pad_kernel, dim3(ld / 32, div_up(kn, 32)), 256, 0, st, in, rows, d, kn, out, ld);
 }
 
 // The last d % 4 output columns: one chain over all d dimensions
 // (src/index.cpp:171-179, :247-257).
 __global__ void rotate_seq_kernel(const float *__restrict__ in, uint32_t nrows, uint32_t d,
                                   const float *__restrict__ rot, float *__restrict__ out) {
+  after_previous();
   const uint32_t d4 = d & ~3u, nc = d - d4;
   const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<uint64_t>(nrows) * nc) return;
@@ -468,6 +472,7 @@ __global__ void __launch_bounds__(256) query_planes_kernel(const float *__restri
                                                            uint32_t d, float lo, double inv_step,
                                                            bool vec, const QueryPlanes P,
                                                            const RankRows rr) {
+  after_previous();
   const uint32_t lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.zeros; i += gridDim.x * blockDim.x)
     P.zero[i] = 0;
@@ -550,7 +555,7 @@ int query_planes(const float *x, uint32_t nrows, uint32_t d, float lo, double in
                  const QueryPlanes &P, const RankRows &rr, cudaStream_t st) {
   if (nrows == 0) return KATO_OK;
   const bool vec = d % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
-  query_planes_kernel<<<div_up(nrows, 8), 256, 0, st>>>(x, nrows, d, lo, inv_step, vec, P, rr);
+  launch(query_planes_kernel, div_up(nrows, 8), 256, 0, st, x, nrows, d, lo, inv_step, vec, P, rr);
   KATO_LAUNCHED("query_planes_kernel");
   return KATO_OK;
 }
@@ -566,7 +571,7 @@ int rotate_rows(const float *in, uint32_t nrows, uint32_t d, const float *rot, f
   }
   if (d4 < d) {
     const uint64_t n = static_cast<uint64_t>(nrows) * (d - d4);
-    rotate_seq_kernel<<<static_cast<uint32_t>((n + 255) / 256), 256, 0, st>>>(in, nrows, d, rot, out);
+    launch(rotate_seq_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, st, in, nrows, d, rot, out);
     KATO_LAUNCHED("rotate_seq_kernel");
   }
   return KATO_OK;
@@ -648,7 +653,7 @@ int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float 
     if (const int r = smem_limit(reinterpret_cast<const void *>(kern), static_cast<int>(smem),
                                  "rotate_tma_kernel shared memory"))
       return r;
-    kern<<<dim3(div_up(d4, col_tile), div_up(nrows, row_tile)), threads, smem, st>>>(
+    launch(kern, dim3(div_up(d4, col_tile), div_up(nrows, row_tile)), threads, smem, st,
         tx, tr, in, nrows, d, rot, out, timeouts);
     KATO_LAUNCHED("rotate_tma_kernel");
     return KATO_OK;
@@ -660,7 +665,7 @@ int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float 
   ++*launches;
   if (d4 < d) {
     const uint64_t n = static_cast<uint64_t>(nrows) * (d - d4);
-    rotate_seq_kernel<<<static_cast<uint32_t>((n + 255) / 256), 256, 0, st>>>(in, nrows, d, rot, out);
+    launch(rotate_seq_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, st, in, nrows, d, rot, out);
     KATO_LAUNCHED("rotate_seq_kernel");
     ++*launches;
   }

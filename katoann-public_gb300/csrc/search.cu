@@ -79,6 +79,7 @@ __host__ __device__ inline size_t rank_smem_bytes(int planes, bool select, uint3
 // otherwise write every candidate to its slot (slot capacity >= list size).
 template <bool kFull, bool kSelect>
 __global__ void __launch_bounds__(kThreads) rank_kernel(RankArgs A) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t w = blockIdx.x;
   if (w >= *A.woff_total) return;
@@ -683,7 +684,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     if (const int rc2 = smem_limit(reinterpret_cast<const void *>(kern), static_cast<int>(smem),
                                    "rank_kernel shared memory"))
       return rc2;
-    kern<<<grid, kThreads, smem, st>>>(A);
+    kato::launch(kern, grid, kThreads, smem, st, A);
     KATO_LAUNCHED("rank_kernel");
     return KATO_OK;
   };
@@ -767,6 +768,7 @@ int search(const katoann_gpu_index *ix, const float *queries, uint32_t nq, uint3
   unsigned char *w = static_cast<unsigned char *>(ws);
   KATO_CUDA(cudaMemsetAsync(w + pl.off_stats, 0, 48 * sizeof(unsigned long long), st));
   g_launches = 0;
+  const Chain chain;
   for (uint32_t q0 = 0; q0 < nq; q0 += max_batch) {
     const uint32_t b = std::min(max_batch, nq - q0);
     Budget bud = budget;
