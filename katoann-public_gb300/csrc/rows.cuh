@@ -74,13 +74,15 @@ __device__ __forceinline__ void rows_split(const uint8_t *__restrict__ x, uint32
         if (gl == it) mine = dot;
       }
     } else {
-#pragma unroll
+#pragma unroll 4
       for (uint32_t it = 0; it < G; ++it) {
         const uint32_t i = base + it * RPW + sub;
         uint32_t dot = 0;
         if (i < n) {
           const uint4 *rv = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row(i)) * dc);
-          for (uint32_t u = gl; u < units; u += G) {
+          for (uint32_t c = 0; c < (units + G - 1) / G; ++c) {
+            const uint32_t u = gl + c * G;
+            if (u >= units) break;
             const uint4 vv = __ldg(rv + u);
             const uint32_t *w = qw + 4 * u;
             dot = dp4(vv.x, w[0], dp4(vv.y, w[1], dp4(vv.z, w[2], dp4(vv.w, w[3], dot))));
