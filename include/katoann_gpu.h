@@ -188,7 +188,7 @@ void katoann_gpu_timer_destroy(void *timer);
  * into h_ms[0..KATO_PHASES) and their count into *passes; synchronous. */
 int katoann_gpu_timer_read(void *timer, float *h_ms, uint32_t *passes);
 /* The timer also brackets single kernels with events: 0 the query rotation
- * (its transposes and rotate_lanes_kernel), 1 coarse_tc_kernel, 2
+ * (its transpose and kernels), 1 coarse_tc_kernel, 2
  * rank_tc_kernel. Their summed ms and launch counts over the passes of the
  * last katoann_gpu_timer_read (a kernel a pass did not run is not counted). */
 #define KATO_TIMED_KERNELS 3
@@ -214,9 +214,10 @@ uint32_t katoann_gpu_last_launches(void);
 int katoann_gpu_set_candidate_cap(uint32_t cap);
 
 /* Rows of each query's nearest lists that give it a bound before the
- * tensor-core ranking pass (0 = the default, max(2048, 16 x survivors); at
- * most 4096; process-wide). Beyond 3 x survivors rows, a sketch over their
- * first 32 head bytes picks the 3 x survivors that are scored in full. More
+ * tensor-core ranking pass (0 = the default, max(1024, 8 x survivors); at
+ * most 4096; process-wide; twice as many for a query that probes many rows,
+ * 65,536 by its nearest lists). Of more than 2 x survivors rows (3 x for such a
+ * query) a sketch over their first 32 head bytes picks as many to score in full. More
  * rows mean a tighter bound (fewer candidates to merge) for more work up
  * front. Results do not depend on it. */
 int katoann_gpu_set_seed_rows(uint32_t rows);
@@ -337,7 +338,7 @@ int katoann_gpu_search_budget(const katoann_gpu_index *index, const float *d_que
  * the legacy default one) and instantiated. Nothing runs at capture.
  * katoann_gpu_graph_launch replays it on any stream: the same pointers and
  * sizes, with whatever the buffers hold at replay, in one launch instead of
- * some thirty. The workspace, index, model and buffers must stay allocated
+ * ten to sixteen a pass. The workspace, index, model and buffers must stay allocated
  * while the graph lives. */
 int katoann_gpu_search_capture(const katoann_gpu_index *index, const float *d_queries,
                                uint32_t nq, uint32_t k, uint32_t nprobe, int ranking,

@@ -28,8 +28,16 @@ struct FinishArgs {
   const int64_t *rank_xnorm, *rank_qnorm;
   const uint32_t *probed, *list_off;
   uint32_t h, nprobe;
+  // where a query can probe more rows than its buffer holds: per query, whether
+  // it was rescanned by the whole grid before, and the key it was rescanned for;
+  // the number of those queries (accumulating)
+  uint32_t *over;
+  unsigned long long *over_key, *over_n;
 };
 
+// The first rescan of queries with more candidates than their buffers hold (with
+// `over`; writes qcount), by the whole grid.
+int rescan_overflows(const FinishArgs &A, uint32_t *qcount, uint32_t nq, cudaStream_t st);
 // Survivors, refinement and top-k of nq queries (ranked modes).
 int finish(const FinishArgs &A, uint32_t nq, cudaStream_t st);
 // Top-k of slots of exact distances (full ranking): per query per_query

@@ -35,6 +35,7 @@ namespace kato {
 namespace {
 
 constexpr uint32_t kSeedCap = 4096;  // rows a seed bound looks at, at most
+constexpr uint32_t kSeedMany = 65536;  // probed rows from which it looks at twice as many
 
 // rank_tc_kernel: one CTA per SM takes an equal share, by cost, of all 64-row
 // slabs of all work items (an item is a list and up to N of the queries
@@ -496,12 +497,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           if (!wait(b_empty_a + sw * 8, (use & 1) ^ 1, pw[0])) break;
           // Filtered while few records come of it. A slab saves about 0.15 us
           // of an SM against all of h = 256, and completing a record costs an
-          // SM about 5 ns (10M x 1,024: 3 records per slab), so: on while the
-          // CTA's slabs gave below 32 each, whatever their items were (a run
-          // of items that pass too much is paid back by the unfiltered ones
-          // after it). The first 8 slabs go ahead, the next await their count
+          // SM about 5 ns: on while the CTA's slabs gave below 16 each, whatever
+          // their items were (10M x 1,024 of one spread-out cloud: 3 per slab,
+          // 0.50 ms against 0.70; of tight clusters, 20 and more, 1.16 ms with
+          // its records for 1.30 with 32 as the line and 1.07 without a
+          // filter). The first 8 slabs go ahead, the next await their count.
+          // Partial records must leave the CTA's list room: whoever's records
+          // do not fit is rescanned
           bool filt = A.f < h;
-          if (filt) filt = *slabs >= 8 ? *reinterpret_cast<volatile uint32_t *>(rcount) <= 32 * *slabs : *fstaged < 8;
+          if (filt) {
+            const uint32_t have = *reinterpret_cast<volatile uint32_t *>(rcount);
+            filt = (*slabs >= 8 ? have <= 16 * *slabs : *fstaged < 8) && have <= A.rec_cap / 4;
+          }
           const uint32_t dims = filt ? A.f : h;
           if (lane == 0) {
             desc[sw] = Desc{s0, s1, cur.row0, cur.nrows, cur.ne, (dims + IN - 1) / IN, filt, 0};
@@ -605,7 +612,7 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
     const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
     const uint32_t *__restrict__ list_off, uint32_t p,
-    uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t full, SeedBound kind, DistScale scale,
+    uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t more, SeedBound kind, DistScale scale,
     int32_t *__restrict__ bound) {
   after_previous();
   // rowof: the rows looked at. Where all are scored, l2s gets their distances;
@@ -622,13 +629,22 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
   // the rows, 32 lists at a time: every warp reads their offsets, and writes
   // the rows of every eighth
   const uint32_t pq = qprobes ? qprobes[q] : p;  // the query's own budget
-  uint32_t count = 0;
+  uint32_t count = 0, full = min(want, 2 * S);
   for (uint32_t r = 0; r < pq && count < want; r += 32) {
     uint32_t r0 = 0, n = 0;
     if (r + lane < pq) {
       const uint32_t c = probed[static_cast<size_t>(q) * p + r + lane];
       r0 = list_off[c];
       n = list_off[c + 1] - r0;
+    }
+    if (r == 0) {
+      // rows that the query probes, by its nearest lists: of many the bound
+      // lets more through, and more rows are looked at (default_seed_rows)
+      const uint32_t lists = min(pq, 32u), rows = __reduce_add_sync(0xffffffffu, min(n, 1u << 20));
+      if (static_cast<uint64_t>(rows) * pq > static_cast<uint64_t>(kSeedMany) * lists) {
+        want = more;
+        full = min(want, 3 * S);
+      }
     }
     uint32_t incl = min(n, want);  // (sums stay below 32 want)
 #pragma unroll
@@ -928,11 +944,11 @@ int rank_seed(const uint8_t *xhi, const int64_t *xnorm, const uint8_t *qhi, cons
               DistScale scale, int32_t *bound, cudaStream_t st) {
   if (h > 2048 || h % 64) return invalid("seed bounds need h <= 2048, a multiple of 64");
   if (B == 0) return KATO_OK;
-  // rows the sketch picks to score in full: 2S (3S leaves 1% fewer candidates
-  // for 8 to 14 us more of every 4096 queries' seeds, 3S / 2 1 to 10% more)
+  // `rows` for a query of few rows, twice as many for one of many
   const uint32_t want = std::min(std::max(rows, S), kSeedCap);
+  const uint32_t more = std::min(std::max(2 * rows, S), kSeedCap);
   launch(rank_seed_kernel, B, 256, 0, st, xhi, xnorm, qhi, qnorm, probed, qprobes, list_off, p, dc, h,
-                                      S, want, std::min(want, 2 * S), kind, scale, bound);
+                                      S, want, more, kind, scale, bound);
   KATO_LAUNCHED("rank_seed_kernel");
   return KATO_OK;
 }

@@ -111,12 +111,13 @@ __host__ __device__ inline TcSmem tc_smem_layout(uint32_t h, const TcShape &s) {
   return L;
 }
 
-// Rows a seed bound looks at unless set otherwise: a looser bound costs the
-// ranking pass little (its time follows the tiles, not the candidates), so the
-// seed's own time decides. max(1024, 8 S) with 2 S of them scored takes 88 us
-// for 4096 queries at 1M x 1024 (S = 32) and 132 at 10M (S = 64), where
-// max(2048, 16 S) with 3 S took 127 and 206 for 2% and 14% fewer candidates; at 512
-// rows the 78% more candidates at 10M cost more than the seed saves.
+// Rows a seed bound looks at unless set otherwise, for a query that probes few
+// rows; one that probes many (65,536 by its nearest lists) looks at twice as many
+// and scores 3 S instead of 2 S. A looser bound costs the ranking pass little where
+// the candidates stay few, so there the seed's own time decides: 1,024 rows and
+// 2 S take 88 us for 4096 queries at 1M x 1024 (S = 32), 2,048 and 3 S 127, for 2%
+// fewer candidates. In long lists of tight clusters (10M, S = 64, 72 lists) they
+// leave 2.4 times the candidates: 2.35 ms a search against 2.18.
 inline uint32_t default_seed_rows(uint32_t S) { return std::max(1024u, 8 * std::min(S, 1u << 20)); }
 // The shape for h ranking dimensions over rows of dc bytes, or false when h
 // does not suit the pass (the caller then uses the CUDA-core pass).

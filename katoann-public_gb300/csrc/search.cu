@@ -731,6 +731,14 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
       F.list_off = ix->d_list_off;
       F.h = pl.dims;
       F.nprobe = p;
+      if (static_cast<uint64_t>(p) * ix->max_list > pl.cap) {
+        // a buffer can overflow (the coarse product's terms have been read)
+        F.over = reinterpret_cast<uint32_t *>(bound);
+        F.over_key = reinterpret_cast<unsigned long long *>(ws + pl.off_qterm);
+        F.over_n = stats + 39;
+        if ((rc = rescan_overflows(F, qcount, nq, st))) return rc;
+        g_launches += 2;
+      }
     }
     mark(tm, 8, st);  // the survivor merge is part of the refinement kernel
     rc = finish(F, nq, st);
