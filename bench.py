@@ -349,23 +349,26 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------ roofline
-SEED_ROWS = 2048  # rows behind each query's seed bound (the library default for survivors <= 128)
+SEED_ROWS = 2048  # rows behind each query's seed bound, where no setting is given
+SCORED_ROWS = 2  # of which the sketch picks this many times the survivors, to score in full
 # the kernel the phase timer brackets inside each phase it can dominate
 PHASE_KERNEL = {"ranking pass": "rank_tc_kernel", "coarse product": "coarse_tc_kernel",
                 "rotate+quantize": "rotation"}
 SKETCH_BYTES = 32  # head bytes of a row the seed's sketch reads
 
 
-def seed_bytes(B: int, rows: int, S: int, head: int) -> float:
+def seed_bytes(B: int, rows: int, S: int, head: int, scored: int = 3) -> float:
     """Bytes the seed bounds read: every looked-at row's first SKETCH_BYTES
-    head bytes and the 3S rows the sketch picks in full; with at most 3S rows
-    every row in full."""
-    full = min(rows, 3 * S)
+    head bytes and the scored x S rows the sketch picks in full; with at most
+    that many rows every row in full."""
+    full = min(rows, scored * S)
     if rows > full:
         return float(B) * (rows * min(SKETCH_BYTES, head) + full * head)
     return float(B) * rows * head
 
-# DRAM bytes per 128-row tile of the tensor-core ranking kernel: one ncu
+# DRAM bytes per 128-row tile of a ranking pass that reads all of the prefix
+# (tiles scored over 128 dimensions alone read less than half: 12.7 KB, so the
+# figure is an upper one): one ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of this
 # 10M x 1024 search at nprobe 72 and 64 survivors moved 2,632.4 + 22.3 MB over
 # 96,108 tiles, about 27.6 KB per tile (1.09 x the 256 head bytes of each
@@ -374,7 +377,8 @@ RANK_TC_DRAM_BYTES_PER_TILE = (2632.4e6 + 22.3e6) / 96108
 
 
 def phase_work(phase: str, B: int, L: int, dc: int, d: int, nprobe: int, S: int, head: int,
-               probed_rows: float, probed_lists_rows: float):
+               probed_rows: float, probed_lists_rows: float, seed_rows: int = SEED_ROWS,
+               scored: int = 3):
     """(bound, algorithmic work per launch, unit) of one pipeline phase.
     Byte products of the exact integer products are counted as the BF16
     tensor-core MACs an exact split-byte product needs (four per code pair and
@@ -386,9 +390,9 @@ def phase_work(phase: str, B: int, L: int, dc: int, d: int, nprobe: int, S: int,
         # summed from the same bytes; ids are only read for the survivors)
         return "hbm", probed_lists_rows * head / 1e9, "GB/s"
     if phase == "seed bounds":
-        # the sketch over the first SEED_ROWS rows of each query's nearest
+        # the sketch over the first seed_rows rows of each query's nearest
         # lists, and the rows it picks
-        return "hbm", seed_bytes(B, SEED_ROWS, S, head) / 1e9, "GB/s"
+        return "hbm", seed_bytes(B, seed_rows, S, head, scored) / 1e9, "GB/s"
     if phase == "refine":
         return "hbm", B * S * (2 * dc + 8 + 4) / 1e9, "GB/s"
     if phase == "rotate+quantize":
@@ -715,7 +719,8 @@ def main():
             "p99_list": int(np.percentile(sizes, 99)), "empty_lists": int((sizes == 0).sum()),
             "lists_probed": int(search_stats.get("lists_probed") or probed.sum())}
     bound, work, unit = phase_work(dom, B, L, (d + 63) // 64 * 64, d, p, max(S, k), args.head,
-                                   probed_rows, probed_rows)
+                                   probed_rows, probed_rows,
+                                   (tuned or {}).get("seed_rows") or max(1024, 8 * max(S, k)), SCORED_ROWS)
     # the dominant phase's own kernel, timed by its events on the search stream
     # (the phase adds its preparation, bucketing and the like)
     kname = PHASE_KERNEL.get(dom)
