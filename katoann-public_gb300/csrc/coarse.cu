@@ -19,10 +19,10 @@ constexpr int kSw = kKw + 1;  // padded words per staged row
 
 template <bool kFull>
 __global__ void __launch_bounds__(256) sq16_tile_kernel(
-    const uint8_t *__restrict__ qhi, const uint8_t *__restrict__ qlo,
-    const uint8_t *__restrict__ xhi, const uint8_t *__restrict__ xlo,
-    const int64_t *__restrict__ qn, const int64_t *__restrict__ xn, DistScale scale, uint32_t m,
-    uint32_t n, uint32_t dims, uint32_t qstride, uint32_t xstride, float *__restrict__ out) {
+    const uint8_t *qhi, const uint8_t *qlo, const uint8_t *__restrict__ xhi,
+    const uint8_t *__restrict__ xlo, const int64_t *qn, const int64_t *__restrict__ xn,
+    DistScale scale, uint32_t m, uint32_t n, uint32_t dims, uint32_t qstride, uint32_t xstride,
+    float *out) {
   after_previous();
   __shared__ uint32_t sqh[kTile * kSw], sxh[kTile * kSw];
   __shared__ uint32_t sql[kFull ? kTile * kSw : 1], sxl[kFull ? kTile * kSw : 1];
@@ -147,9 +147,8 @@ __device__ __forceinline__ uint32_t block_scan_bins(uint32_t *hist, uint32_t ran
 // Smallest p keys of a row by (key, index) in up to six passes over the row
 // (8-bit radix digits of the p-th key, then of the tied indices, then the
 // gather). sel holds np2(p) 64-bit words, hist 256 counters, scal 4 words.
-__device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uint32_t p,
-                              uint32_t *__restrict__ outp, uint32_t *__restrict__ cnt,
-                              unsigned long long *__restrict__ tie_count, unsigned long long *sel,
+__device__ void select_passes(const uint32_t *keys, uint32_t n, uint32_t p, uint32_t *outp,
+                              uint32_t *cnt, unsigned long long *tie_count, unsigned long long *sel,
                               uint32_t *hist, uint32_t *scal) {
   const uint32_t tid = threadIdx.x;
   // 1) the p-th smallest key (rank p-1), and how many keys are below it.
@@ -240,10 +239,8 @@ __device__ void select_passes(const uint32_t *__restrict__ keys, uint32_t n, uin
 // most only_above are skipped (a second, deeper selection for the queries
 // that need it).
 __global__ void __launch_bounds__(kSelThreads) select_topp_kernel(
-    const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride,
-    uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
-    unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
-    uint32_t only_above) {
+    const float *dists, uint32_t n, uint32_t p, uint32_t stride, uint32_t *probed, uint32_t *cnt,
+    unsigned long long *tie_count, const uint32_t *only, uint32_t only_above) {
   after_previous();
   extern __shared__ unsigned long long sel[];  // up to kSortMax (key << 32 | id)
   __shared__ uint32_t hist[256], scal[4];
@@ -303,9 +300,8 @@ __device__ __forceinline__ uint32_t min4(uint4 x) { return min(min(x.x, x.y), mi
 
 template <uint32_t NT, uint32_t V>
 __global__ void __launch_bounds__(NT) select_topp_near_kernel(
-    const float *__restrict__ dists, uint32_t n, uint32_t p, uint32_t stride, uint32_t level,
-    uint32_t cap, uint32_t *__restrict__ probed, uint32_t *__restrict__ cnt,
-    unsigned long long *__restrict__ tie_count, const uint32_t *__restrict__ only,
+    const float *dists, uint32_t n, uint32_t p, uint32_t stride, uint32_t level, uint32_t cap,
+    uint32_t *probed, uint32_t *cnt, unsigned long long *tie_count, const uint32_t *only,
     uint32_t only_above) {
   after_previous();
   extern __shared__ unsigned long long cand[];  // cap keys (key << 32 | list)

@@ -151,11 +151,9 @@ __device__ void block_sort_pairs(unsigned long long *key, uint32_t *val, uint32_
 // Per query: the k smallest of its slot entries by (distance, id), ascending,
 // padded.
 __global__ void __launch_bounds__(kThreads) merge_kernel(
-    const uint2 *__restrict__ slots, uint32_t per_query, uint32_t per_probe,
-    const uint32_t *__restrict__ qcount, const uint32_t *__restrict__ qprobes,
-    const uint32_t *__restrict__ ids, uint32_t k,
-    uint32_t *__restrict__ out_ids, float *__restrict__ out_dists,
-    unsigned long long *__restrict__ tie_count) {
+    const uint2 *slots, uint32_t per_query, uint32_t per_probe, const uint32_t *qcount,
+    const uint32_t *qprobes, const uint32_t *__restrict__ ids, uint32_t k, uint32_t *out_ids,
+    float *out_dists, unsigned long long *tie_count) {
   after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint32_t hist[256], scratch[8], wsum[8];

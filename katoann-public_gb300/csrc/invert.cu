@@ -20,12 +20,12 @@ namespace {
 // budget (if any) exceeds the rank: its p nearest lists are in order, so a
 // budget of b probes exactly the lists a fixed nprobe of b would.
 __device__ __forceinline__ bool probed_pair(uint32_t i, uint32_t p,
-                                            const uint32_t *__restrict__ qprobes) {
+                                            const uint32_t *qprobes) {
   return !qprobes || i % p < qprobes[i / p];
 }
 
-__global__ void count_kernel(const uint32_t *__restrict__ probed, uint32_t total, uint32_t p,
-                             const uint32_t *__restrict__ qprobes, uint32_t *__restrict__ cnt) {
+__global__ void count_kernel(const uint32_t *probed, uint32_t total, uint32_t p,
+                             const uint32_t *qprobes, uint32_t *cnt) {
   after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total && probed_pair(i, p, qprobes)) atomicAdd(&cnt[probed[i]], 1u);

@@ -33,7 +33,11 @@ int cuda_status(cudaError_t e, const char *what);
 // CTAs may be placed while the one before it drains, and wait in
 // after_previous() until that one has ended and its writes are visible. Every
 // kernel launched this way calls after_previous() first, so each of them also
-// comes after all those before its predecessor. The ten kernels of a search of
+// comes after all those before its predecessor. What a kernel of the search
+// writes is read by the later ones through plain pointers: __restrict__ and
+// __ldg promise data that no kernel writes meanwhile, and may be loaded before
+// the wait, so they are for the index's arrays, the model's and the caller's
+// queries alone. The ten kernels of a search of
 // one query take 52 us of the device instead of 69, 4096 queries at 1M 580
 // instead of 604.
 inline thread_local bool chained = false;

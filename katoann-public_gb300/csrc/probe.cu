@@ -55,8 +55,8 @@ __host__ __device__ __forceinline__ uint16_t bf16_round(float f) {
 
 // ------------------------------------------------------------------ features
 __global__ void __launch_bounds__(256) probe_features_kernel(
-    const float *__restrict__ cd, uint32_t L, const uint32_t *__restrict__ probed, uint32_t P,
-    const uint32_t *__restrict__ rank, uint32_t B, float *__restrict__ z) {
+    const float *cd, uint32_t L, const uint32_t *probed, uint32_t P,
+    const uint32_t *__restrict__ rank, uint32_t B, float *z) {
   after_previous();
   const uint32_t q = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (q >= B) return;
@@ -118,10 +118,9 @@ __device__ __forceinline__ void dense_relu(const float *in, const uint16_t *__re
 constexpr size_t kMlpAct = (static_cast<size_t>(kF) + 2 * kH) * kAS * 4 + kQB * (kCMax + 1) * 4;
 constexpr size_t kMlpSmem = kMlpAct + (static_cast<size_t>(kF) * kH + kH * kCMax) * 2;
 
-__global__ void __launch_bounds__(kH) probe_mlp_kernel(const float *__restrict__ z, uint32_t B,
-                                                        MlpArgs m, uint32_t cap,
-                                                        float *__restrict__ probs,
-                                                        uint32_t *__restrict__ nprobe) {
+__global__ void __launch_bounds__(kH) probe_mlp_kernel(const float *z, uint32_t B, MlpArgs m,
+                                                        uint32_t cap, float *probs,
+                                                        uint32_t *nprobe) {
   after_previous();
   extern __shared__ __align__(16) float sm[];
   float *x0 = sm;                 // [kF][kAS]
@@ -198,8 +197,8 @@ __global__ void __launch_bounds__(kH) probe_mlp_kernel(const float *__restrict__
   }
 }
 
-__global__ void clamp_budget_kernel(const uint32_t *__restrict__ in, uint32_t B, uint32_t cap,
-                                    uint32_t *__restrict__ out) {
+__global__ void clamp_budget_kernel(const uint32_t *in, uint32_t B, uint32_t cap,
+                                    uint32_t *out) {
   after_previous();
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < B) out[q] = in ? max(1u, min(in[q], cap)) : cap;

@@ -612,11 +612,10 @@ __device__ __forceinline__ uint32_t sketch_bin(uint32_t d) {
 // selection that ranks by counting where there are few.
 __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
     const uint8_t *__restrict__ xhi, const int64_t *__restrict__ xnorm,
-    const uint8_t *__restrict__ qhi, const int64_t *__restrict__ qnorm,
-    const uint32_t *__restrict__ probed, const uint32_t *__restrict__ qprobes,
+    const uint8_t *qhi, const int64_t *qnorm, const uint32_t *probed, const uint32_t *qprobes,
     const uint32_t *__restrict__ list_off, uint32_t p,
     uint32_t dc, uint32_t h, uint32_t S, uint32_t want, uint32_t more, SeedBound kind, DistScale scale,
-    int32_t *__restrict__ bound) {
+    int32_t *bound) {
   after_previous();
   // rowof: the rows looked at. Where all are scored, l2s gets their distances;
   // where some are, l2s gets those rows and rowof their distances.
@@ -802,11 +801,9 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
 // eight lanes add the rest, 16 bytes of the row and of the query each, with
 // the loads of a warp's 32 records in flight together.
 __global__ void __launch_bounds__(256) tc_bucket_kernel(
-    const uint4 *__restrict__ rec, const uint32_t *__restrict__ rec_n, uint32_t rec_cap,
-    const uint8_t *__restrict__ xhi, const uint8_t *__restrict__ qhi, const int2 *__restrict__ qcn,
-    const int32_t *__restrict__ bound, uint32_t dc, uint32_t f, uint32_t h,
-    uint32_t *__restrict__ qcount, uint2 *__restrict__ qbuf, uint32_t cap, DistScale scale,
-    unsigned long long *__restrict__ found) {
+    const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, const uint8_t *__restrict__ xhi,
+    const uint8_t *qhi, const int2 *qcn, const int32_t *bound, uint32_t dc, uint32_t f, uint32_t h,
+    uint32_t *qcount, uint2 *qbuf, uint32_t cap, DistScale scale, unsigned long long *found) {
   after_previous();
   const uint4 *r = rec + static_cast<size_t>(blockIdx.x) * rec_cap;
   const uint32_t n = rec_n[blockIdx.x], lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
@@ -830,7 +827,7 @@ __global__ void __launch_bounds__(256) tc_bucket_kernel(
           const bool on = __shfl_sync(0xffffffffu, e.w, src) != 0 && in;
           x[it] = on ? __ldg(reinterpret_cast<const uint4 *>(xhi + static_cast<size_t>(er) * dc) + u0 + gl)
                      : make_uint4(0, 0, 0, 0);
-          q[it] = on ? __ldg(reinterpret_cast<const uint4 *>(qhi + static_cast<size_t>(eq) * dc) + u0 + gl)
+          q[it] = on ? reinterpret_cast<const uint4 *>(qhi + static_cast<size_t>(eq) * dc)[u0 + gl]
                      : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll

@@ -195,8 +195,7 @@ template <bool kRows>
 __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
     rotate_tma_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tr,
                       const float *__restrict__ in, uint32_t nrows, uint32_t d,
-                      const float *__restrict__ rot, float *__restrict__ out,
-                      uint32_t *__restrict__ timeouts) {
+                      const float *__restrict__ rot, float *out, uint32_t *timeouts) {
   after_previous();
   constexpr int TB = kRows ? 8 : 16, CG = kRows ? 4 : 2;
   constexpr uint32_t kStage = rot_stage_bytes<kRows>();
@@ -332,7 +331,7 @@ __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
 // k < kn: 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256) transpose_pad_kernel(const float *__restrict__ in,
                                                             uint32_t rows, uint32_t d, uint32_t kn,
-                                                            float *__restrict__ out, uint32_t ld) {
+                                                            float *out, uint32_t ld) {
   after_previous();
   __shared__ float tile[32][33];
   const uint32_t r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
@@ -353,7 +352,7 @@ __global__ void __launch_bounds__(256) transpose_pad_kernel(const float *__restr
 // float4 stores per thread.
 __global__ void __launch_bounds__(256) transpose_pad4_kernel(const float *__restrict__ in,
                                                              uint32_t rows, uint32_t d, uint32_t kn,
-                                                             float *__restrict__ out, uint32_t ld) {
+                                                             float *out, uint32_t ld) {
   after_previous();
   __shared__ float tile[64][65];
   const uint32_t r0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
@@ -390,7 +389,7 @@ void transpose_pad(const float *in, uint32_t rows, uint32_t d, uint32_t kn, floa
 // The last d % 4 output columns: one chain over all d dimensions
 // (src/index.cpp:171-179, :247-257).
 __global__ void rotate_seq_kernel(const float *__restrict__ in, uint32_t nrows, uint32_t d,
-                                  const float *__restrict__ rot, float *__restrict__ out) {
+                                  const float *__restrict__ rot, float *out) {
   after_previous();
   const uint32_t d4 = d & ~3u, nc = d - d4;
   const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -468,7 +467,7 @@ __global__ void quantize_rows_kernel(const float *__restrict__ x, uint32_t nrows
 // (quantize_rows_kernel's), the centred fp16 planes and term of the coarse
 // product and the rows of the ranking pass (centre_planes_kernel's). Also
 // clears `zeros` words at `zero` (the inversion's and the candidates' counts).
-__global__ void __launch_bounds__(256) query_planes_kernel(const float *__restrict__ x, uint32_t nrows,
+__global__ void __launch_bounds__(256) query_planes_kernel(const float *x, uint32_t nrows,
                                                            uint32_t d, float lo, double inv_step,
                                                            bool vec, const QueryPlanes P,
                                                            const RankRows rr) {
