@@ -126,6 +126,12 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// A word of shared memory that other warps write meanwhile, as lane 0 reads it:
+// the lanes of a warp must not differ in what they do next.
+__device__ __forceinline__ uint32_t warp_read(const volatile uint32_t *p) {
+  return __shfl_sync(0xffffffffu, *p, 0);
+}
+
 // One arrival on `bar` once this thread's copies so far have landed.
 __device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_addr(bar))
@@ -199,21 +205,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto wait_for = [&](uint32_t b, uint32_t phase, unsigned long long &acc, auto meanwhile) -> bool {
     if (__all_sync(0xffffffffu, tc::mbar_test(b, phase))) return true;
     const long long t = clock64();
-    bool ok = false;
+    bool ok = false, late = false;
     long long took = 0;
     do {
-      ok = meanwhile(b, phase);
+      ok = __all_sync(0xffffffffu, meanwhile(b, phase));
       took = clock64() - t;
-    } while (!ok && !*err && took <= A.wait);
-    if (took > A.wait) *err = 1, ok = false;
+      late = __any_sync(0xffffffffu, took > A.wait);
+    } while (!ok && !late && !warp_read(err));
+    if (late) *err = 1, ok = false;
     acc += took;
-    return __all_sync(0xffffffffu, ok);
+    return ok;
   };
   auto wait = [&](uint32_t b, uint32_t phase, unsigned long long &acc) -> bool {
     return wait_for(b, phase, acc, [](uint32_t x, uint32_t p) { return tc::mbar_try(x, p); });
   };
 
-  if (t0 < t1 && !*err) {
+  if (t0 < t1 && !warp_read(err)) {
     // the item after the last one may start inside the next share
     const uint32_t n_li = upto.y - it0 + (A.tile_off[upto.y] < t1);
     const uint32_t d_full_a = tc::smem_addr(d_full), b_full_a = tc::smem_addr(b_full);
@@ -462,7 +469,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       // hand back the remaining items' buffers, so that the staging warps end
       __syncwarp();
-      while (ok && !*err) {
+      while (ok && !warp_read(err)) {
         if (c_n && lane == 0) tc::mbar_arrive(b_empty_a + c_bf * 8);
         if (++c_n > n_li) break;
         c_bf = c_bf + 1 == nB ? 0 : c_bf + 1;
@@ -508,15 +515,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           // (400k searches/s at 10M: p99 8.4 -> 4.2 ms; with half the pairs, the
           // 384-probe batches' long lists went unfiltered, 245 -> 265 us)
           bool filt = A.f < h && cur.nrows * cur.ne <= 2 * A.rec_cap;
+          uint32_t scored = 0;
           if (filt) {
-            const uint32_t have = *reinterpret_cast<volatile uint32_t *>(rcount);
-            filt = (*slabs >= 8 ? have <= 16 * *slabs : *fstaged < 8) && have <= A.rec_cap / 4;
+            const uint32_t have = warp_read(rcount);
+            scored = warp_read(slabs);
+            const uint32_t ahead = warp_read(fstaged);
+            filt = (scored >= 8 ? have <= 16 * scored : ahead < 8) && have <= A.rec_cap / 4;
           }
           const uint32_t dims = filt ? A.f : h;
           if (lane == 0) {
             desc[sw] = Desc{s0, s1, cur.row0, cur.nrows, cur.ne, (dims + IN - 1) / IN, filt, 0};
             tc::mbar_arrive(d_full + sw);
-            if (filt && *slabs < 8) atomicAdd(const_cast<uint32_t *>(fstaged), s1 - s0);
+            if (filt && scored < 8) atomicAdd(const_cast<uint32_t *>(fstaged), s1 - s0);
           }
           // the queries' fp16 rows, `per` 16-byte units each, the ids shuffled
           const uint32_t per = (dims + IN - 1) / IN * (IN / 8), steps = (cur.ne * per + 31) / 32;
