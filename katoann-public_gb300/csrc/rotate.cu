@@ -529,6 +529,11 @@ __global__ void __launch_bounds__(256) query_planes_kernel(const float *x, uint3
       }
     }
   }
+  // a chunk that ends past the row meets zeros (the scan multiplies all of it, and
+  // the row bytes there are out of range: -128 when centred)
+  if (P.hi16 && rr.rows)
+    for (uint32_t k = P.dc + lane * 4; k < rr.width; k += 128)
+      *reinterpret_cast<uint2 *>(rr.rows + static_cast<size_t>(row) * rr.width + k) = make_uint2(0, 0);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     s += __shfl_xor_sync(0xffffffffu, s, o);
