@@ -38,6 +38,7 @@ constexpr uint32_t kChunk = 512;   // bytes of a row staged at once
 // Rows of a list per CTA: lists are skewed, and with a CTA for a whole list the
 // longest one was the kernel's time (200,000 rows in 512 lists: 0.27 ms).
 constexpr uint32_t kSplitRows = 256;
+constexpr uint32_t kMaxParts = 65535;  // CTAs of a list: the grid's second dimension
 constexpr uint32_t kSelMax = 256;  // largest per-slot S kept in shared memory
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
@@ -381,8 +382,9 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   // query, and up to 2 GiB of them the lists are split (a larger batch then
   // still has at least that, so that its workspace serves a smaller one too)
   constexpr uint64_t kSplitEntries = 1ull << 28;
-  pl.split = kSplitRows;
-  if (pl.select && !pl.tc && static_cast<uint64_t>(B) * p * div_up(ml, kSplitRows) * pl.SC > kSplitEntries) pl.split = ml;
+  const uint32_t least = std::max(kSplitRows, div_up(div_up(ml, kMaxParts), kRT) * kRT);
+  pl.split = least;
+  if (pl.select && !pl.tc && static_cast<uint64_t>(B) * p * div_up(ml, least) * pl.SC > kSplitEntries) pl.split = ml;
   const uint64_t per_query = static_cast<uint64_t>(p) * pl.SC * (pl.select ? div_up(ml, pl.split) : 1);
   if (!pl.tc && per_query >= (1ull << 32)) return invalid("too many candidates per query");
   pl.per_query = static_cast<uint32_t>(per_query);
@@ -429,7 +431,7 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_work = take(wmax * sizeof(Work));
   pl.off_ent = take(bp * 4);
   uint64_t entries = static_cast<uint64_t>(B) * (pl.tc ? pl.cap : pl.per_query);
-  if (pl.select && !pl.tc && pl.split != kSplitRows) entries = std::max(entries, kSplitEntries);
+  if (pl.select && !pl.tc && pl.split != least) entries = std::max(entries, kSplitEntries);
   pl.off_slots = take(entries * sizeof(uint2));
   pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);
