@@ -384,8 +384,13 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   constexpr uint64_t kSplitEntries = 1ull << 28;
   const uint32_t least = std::max(kSplitRows, div_up(div_up(ml, kMaxParts), kRT) * kRT);
   pl.split = least;
-  if (pl.select && !pl.tc && static_cast<uint64_t>(B) * p * div_up(ml, least) * pl.SC > kSplitEntries) pl.split = ml;
-  const uint64_t per_query = static_cast<uint64_t>(p) * pl.SC * (pl.select ? div_up(ml, pl.split) : 1);
+  // the candidates that `parts` CTAs keep of the probed lists: never more than
+  // the lists' rows, which is also what a pass that keeps them all has room for
+  auto kept = [&](uint32_t parts) {
+    return p * std::min<uint64_t>(ml, static_cast<uint64_t>(pl.SC) * (pl.select ? parts : 1));
+  };
+  if (pl.select && !pl.tc && B * kept(div_up(ml, least)) > kSplitEntries) pl.split = ml;
+  const uint64_t per_query = kept(div_up(ml, pl.split));
   if (!pl.tc && per_query >= (1ull << 32)) return invalid("too many candidates per query");
   pl.per_query = static_cast<uint32_t>(per_query);
   if (pl.tc) {

@@ -1,0 +1,34 @@
+"""Sizes of search workspaces, asked of the library without a GPU. A server sizes
+its slots once, for its largest batch, k and depth: no smaller search may need
+more."""
+import ctypes as C
+
+import pytest
+
+from _gpu import GpuIndex, gpu
+
+RANKINGS = {"full": 0, "high": 1, "prefix": 2}
+
+
+def _size(dim, max_list, batch, k, nprobe, ranking, survivors):
+    view = GpuIndex(dim=dim, dc=dim, nlist=4096, npts=1 << 24, head_dims=dim, max_list=max_list)
+    size = gpu().katoann_gpu_search_workspace(C.byref(view), batch, k, nprobe, RANKINGS[ranking], survivors)
+    assert size > 0
+    return size
+
+
+# ranking "high" and "prefix" over 1,152 bytes run on the CUDA cores too
+@pytest.mark.parametrize("dim,ranking", [(128, "full"), (1152, "full"), (1152, "high"), (1152, "prefix"),
+                                         (128, "prefix")])
+@pytest.mark.parametrize("max_list", [1, 200, 256, 257, 300, 513, 9000, 200_000])
+def test_workspace_grows_with_k_batch_and_probes(dim, ranking, max_list):
+    ks = (1, 2, 10, 31, 100, 199, 200, 201, 255, 256, 257, 299, 300, 301, 512, 1000, 4096)
+    for batch in (1, 64, 500, 4096):
+        for nprobe in (1, 32, 512):
+            sizes = [_size(dim, max_list, batch, k, nprobe, ranking, k) for k in ks]
+            assert sizes == sorted(sizes), (batch, nprobe, sizes)
+    for k in (10, 256, 300):
+        sizes = [_size(dim, max_list, batch, k, 64, ranking, k) for batch in (1, 7, 64, 500, 1000, 2000, 4096)]
+        assert sizes == sorted(sizes), (k, sizes)
+        sizes = [_size(dim, max_list, 256, k, p, ranking, k) for p in (1, 3, 10, 64, 200, 512, 2000, 4096)]
+        assert sizes == sorted(sizes), (k, sizes)
