@@ -39,6 +39,11 @@ constexpr uint32_t kChunk = 512;   // bytes of a row staged at once
 // longest one was the kernel's time (200,000 rows in 512 lists: 0.27 ms).
 constexpr uint32_t kSplitRows = 256;
 constexpr uint32_t kMaxParts = 65535;  // CTAs of a list: the grid's second dimension
+// Candidate places (8 bytes) up to which the lists are split: 128 MiB. Exact
+// ranking at 2M x 128, 512 lists, with 32 MiB, 128 MiB and 2 GiB: 256 queries of
+// 24 lists with k = 100 1.52, 1.04, 1.04 ms, 1024 of them 5.0, 2.7, 2.6 ms; 4096 of
+// 64 lists with k = 10 17.2, 16.5, 18.2 ms.
+constexpr uint64_t kSplitEntries = 1ull << 24;
 constexpr uint32_t kSelMax = 256;  // largest per-slot S kept in shared memory
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
@@ -378,19 +383,23 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   // to a buffer of `cap` entries (an overflowing query is rescanned exactly)
   pl.cap = g_candidate_cap.load();
   pl.tc = ranking != KATO_RANK_FULL && pl.S <= pl.cap && rank_tc_plan(pl.dims, ix->dc, &pl.tcs);
-  // rows per CTA of the CUDA-core pass; each CTA keeps up to SC candidates per
-  // query, and up to 2 GiB of them the lists are split (a larger batch then
-  // still has at least that, so that its workspace serves a smaller one too)
-  constexpr uint64_t kSplitEntries = 1ull << 28;
+  // rows per CTA of the CUDA-core pass: each of a list's parts keeps up to SC
+  // candidates per query. Within kSplitEntries places for them the parts are as
+  // short as they should be, beyond it so many as fit, and one per list at least.
+  // The places set aside are those of the shortest parts up to that bound (not
+  // those of the parts taken, which are fewer where a larger batch leaves fewer),
+  // so that a workspace also serves any smaller batch, k and nprobe.
   const uint32_t least = std::max(kSplitRows, div_up(div_up(ml, kMaxParts), kRT) * kRT);
-  pl.split = least;
-  // the candidates that `parts` CTAs keep of the probed lists: never more than
-  // the lists' rows, which is also what a pass that keeps them all has room for
-  auto kept = [&](uint32_t parts) {
-    return p * std::min<uint64_t>(ml, static_cast<uint64_t>(pl.SC) * (pl.select ? parts : 1));
+  const uint32_t most = pl.select ? div_up(ml, least) : 1;
+  auto kept = [&](uint32_t parts) {  // of a query: never more than the lists' rows
+    return p * std::min<uint64_t>(ml, static_cast<uint64_t>(pl.SC) * parts);
   };
-  if (pl.select && !pl.tc && B * kept(div_up(ml, least)) > kSplitEntries) pl.split = ml;
-  const uint64_t per_query = kept(div_up(ml, pl.split));
+  pl.split = least;
+  if (pl.select && !pl.tc && B * kept(most) > kSplitEntries) {
+    const uint64_t parts = std::max<uint64_t>(1, kSplitEntries / (static_cast<uint64_t>(B) * p * pl.SC));
+    pl.split = std::max(least, div_up(div_up(ml, static_cast<uint32_t>(parts)), kRT) * kRT);
+  }
+  const uint64_t per_query = kept(pl.select ? div_up(ml, pl.split) : 1);
   if (!pl.tc && per_query >= (1ull << 32)) return invalid("too many candidates per query");
   pl.per_query = static_cast<uint32_t>(per_query);
   if (pl.tc) {
@@ -435,8 +444,8 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_cur = take(static_cast<size_t>(L) * 4);
   pl.off_work = take(wmax * sizeof(Work));
   pl.off_ent = take(bp * 4);
-  uint64_t entries = static_cast<uint64_t>(B) * (pl.tc ? pl.cap : pl.per_query);
-  if (pl.select && !pl.tc && pl.split != least) entries = std::max(entries, kSplitEntries);
+  const uint64_t entries = pl.tc ? static_cast<uint64_t>(B) * pl.cap
+                                 : std::max(B * kept(1), std::min(B * kept(most), kSplitEntries));
   pl.off_slots = take(entries * sizeof(uint2));
   pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);

@@ -32,3 +32,12 @@ def test_workspace_grows_with_k_batch_and_probes(dim, ranking, max_list):
         assert sizes == sorted(sizes), (k, sizes)
         sizes = [_size(dim, max_list, 256, k, p, ranking, k) for p in (1, 3, 10, 64, 200, 512, 2000, 4096)]
         assert sizes == sorted(sizes), (k, sizes)
+
+
+@pytest.mark.parametrize("dim,ranking", [(128, "full"), (1152, "high")])
+@pytest.mark.parametrize("batch,k,nprobe", [(1, 10, 1), (4096, 10, 64), (4096, 10, 512), (4096, 100, 64), (4096, 1, 512)])
+def test_splitting_lists_takes_at_most_128_mib(dim, ranking, batch, k, nprobe):
+    """Lists of up to 256 rows have one part; longer ones may be split."""
+    whole = _size(dim, 256, batch, k, nprobe, ranking, k)
+    for max_list in (257, 6063, 30_000, 1_000_000):
+        assert _size(dim, max_list, batch, k, nprobe, ranking, k) <= whole + (128 << 20), max_list
