@@ -354,7 +354,11 @@ void katoann_gpu_graph_destroy(void *graph);
 /* The 64 raw features z (before standardization) of nq queries into d_z
  * (nq x 64, device): rotation, quantization, coarse product and selection of
  * the `depth` nearest lists, as in the search. The workspace is sized with
- * katoann_gpu_search_workspace(index, max_batch, 1, depth, KATO_RANK_FULL, 1). */
+ * katoann_gpu_probe_features_workspace (0 for a depth that does not suit); one of
+ * katoann_gpu_search_workspace(index, max_batch, 1, depth, KATO_RANK_FULL, 1)
+ * is large enough too. */
+size_t katoann_gpu_probe_features_workspace(const katoann_gpu_index *index, uint32_t max_batch,
+                                            uint32_t depth);
 int katoann_gpu_probe_features(const katoann_gpu_index *index, const float *d_queries,
                                uint32_t nq, const uint32_t *d_rank, uint32_t depth,
                                uint32_t max_batch, void *d_ws, size_t ws_bytes, float *d_z,

@@ -119,6 +119,7 @@ int timer_read(void *t, float *ms, uint32_t *passes);
 void timer_kernels(void *t, float *ms, uint32_t *launches);
 size_t search_workspace(const katoann_gpu_index *ix, uint32_t max_batch, uint32_t k, uint32_t p,
                         int ranking, uint32_t survivors);
+size_t features_workspace(const katoann_gpu_index *ix, uint32_t max_batch, uint32_t depth);
 
 }  // namespace kato
 
@@ -334,6 +335,12 @@ int katoann_gpu_graph_launch(void *graph, katoann_stream_t stream) {
 uint32_t katoann_gpu_graph_launches(const void *graph) { return kato::graph_launches(graph); }
 
 void katoann_gpu_graph_destroy(void *graph) { kato::graph_destroy(graph); }
+
+size_t katoann_gpu_probe_features_workspace(const katoann_gpu_index *ix, uint32_t max_batch,
+                                            uint32_t depth) {
+  if (!ix) return 0;
+  return kato::features_workspace(ix, max_batch, depth);
+}
 
 int katoann_gpu_probe_features(const katoann_gpu_index *ix, const float *d_queries, uint32_t nq,
                                const uint32_t *d_rank, uint32_t depth, uint32_t max_batch,

@@ -206,7 +206,7 @@ void ProbeModel::features(const Index &index, const float *queries, uint32_t nq,
   const auto *view = static_cast<const katoann_gpu_index *>(index.device_view());
   const std::vector<uint32_t> rank = probe_feature_ranks(depth);
   const uint32_t mb = std::min<uint32_t>(nq, 4096);
-  const size_t wsb = katoann_gpu_search_workspace(view, mb, 1, depth, KATO_RANK_FULL, 1);
+  const size_t wsb = katoann_gpu_probe_features_workspace(view, mb, depth);
   if (wsb == 0) gpu_check(KATO_EINVAL);
   const float *src = queries;  // normalized by the caller, as for Index::search
   Dev ws(wsb), dr(kF * 4), dq(static_cast<size_t>(mb) * index.dim() * 4),

@@ -358,8 +358,10 @@ struct Plan {
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
+// With `coarse_only` the plan ends with the selected lists (the feature pass):
+// it has no candidates.
 int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, int ranking,
-              uint32_t survivors, Plan *P) {
+              uint32_t survivors, Plan *P, bool coarse_only = false) {
   if (k == 0 || p == 0 || p > ix->nlist) return invalid("need k >= 1 and 1 <= nprobe <= nlist");
   if (ranking == KATO_RANK_PREFIX && ix->head_dims == 0)
     return invalid("prefix ranking needs the rotation file (.dimc)");
@@ -444,8 +446,9 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_cur = take(static_cast<size_t>(L) * 4);
   pl.off_work = take(wmax * sizeof(Work));
   pl.off_ent = take(bp * 4);
-  const uint64_t entries = pl.tc ? static_cast<uint64_t>(B) * pl.cap
-                                 : std::max(B * kept(1), std::min(B * kept(most), kSplitEntries));
+  const uint64_t entries = coarse_only ? 0
+                           : pl.tc     ? static_cast<uint64_t>(B) * pl.cap
+                                       : std::max(B * kept(1), std::min(B * kept(most), kSplitEntries));
   pl.off_slots = take(entries * sizeof(uint2));
   pl.off_share = take((static_cast<size_t>(pl.ctas) + 1) * sizeof(uint2));
   pl.off_tcitems = take(pl.tc ? (static_cast<size_t>(pl.tcitems) + 1) * sizeof(TcItem) : 16);
@@ -808,6 +811,17 @@ int search(const katoann_gpu_index *ix, const float *queries, uint32_t nq, uint3
   return KATO_OK;
 }
 
+static int features_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t depth, Plan *pl) {
+  if (depth == 0 || depth > ix->nlist || depth > kSortMax)
+    return invalid("feature depth must be 1 to min(nlist, 4096)");
+  return make_plan(ix, B, 1, depth, KATO_RANK_FULL, 1, pl, true);
+}
+
+size_t features_workspace(const katoann_gpu_index *ix, uint32_t max_batch, uint32_t depth) {
+  Plan pl{};
+  return features_plan(ix, max_batch, depth, &pl) ? 0 : pl.total;
+}
+
 // The probe-budget features of nq queries (phases 0-2, then the feature
 // kernel), max_batch at a time.
 int probe_features_search(const katoann_gpu_index *ix, const float *queries, uint32_t nq,
@@ -816,10 +830,8 @@ int probe_features_search(const katoann_gpu_index *ix, const float *queries, uin
   if (nq == 0) return KATO_OK;
   if (max_batch == 0) return invalid("max_batch must be positive");
   if (!rank) return invalid("null feature ranks");
-  if (depth == 0 || depth > ix->nlist || depth > kSortMax)
-    return invalid("feature depth must be 1 to min(nlist, 4096)");
   Plan pl{};
-  int rc = make_plan(ix, std::min(nq, max_batch), 1, depth, KATO_RANK_FULL, 1, &pl);
+  int rc = features_plan(ix, std::min(nq, max_batch), depth, &pl);
   if (rc) return rc;
   if (ws_bytes < pl.total) {
     set_error("feature workspace too small");

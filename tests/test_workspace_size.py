@@ -41,3 +41,18 @@ def test_splitting_lists_takes_at_most_128_mib(dim, ranking, batch, k, nprobe):
     whole = _size(dim, 256, batch, k, nprobe, ranking, k)
     for max_list in (257, 6063, 30_000, 1_000_000):
         assert _size(dim, max_list, batch, k, nprobe, ranking, k) <= whole + (128 << 20), max_list
+
+
+@pytest.mark.parametrize("batch,depth", [(1, 1), (64, 128), (4096, 512), (4096, 4096)])
+def test_features_take_no_candidate_places(batch, depth):
+    """The feature pass ends with the selected lists: its workspace does not depend
+    on the lists' lengths, and is no larger than a search's of that depth."""
+    gpu().katoann_gpu_probe_features_workspace.restype = C.c_size_t
+    gpu().katoann_gpu_probe_features_workspace.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32]
+    sizes = []
+    for max_list in (1, 300, 6063, 1_000_000):
+        view = GpuIndex(dim=128, dc=128, nlist=4096, npts=1 << 24, head_dims=128, max_list=max_list)
+        sizes.append(gpu().katoann_gpu_probe_features_workspace(C.byref(view), batch, depth))
+        assert 0 < sizes[-1] <= _size(128, max_list, batch, 1, depth, "full", 1)
+    assert len(set(sizes)) == 1, sizes
+    assert gpu().katoann_gpu_probe_features_workspace(C.byref(view), batch, 4097) == 0
