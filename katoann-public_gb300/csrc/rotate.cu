@@ -206,7 +206,9 @@ __global__ void __launch_bounds__(rot_threads<kRows>(), kRows ? 1 : 2)
   __shared__ uint64_t full[kRotStages], empty[kRotStages];
   __shared__ volatile uint32_t err;
   const uint32_t d16 = d & ~15u, nk = (d16 + kRotChunk - 1) / kRotChunk;
-  const uint32_t i0 = blockIdx.y * kRowTile, j0 = blockIdx.x * kColTile;
+  // one grid dimension: the second ends at 65,535, two million rows
+  const uint32_t across = div_up(d & ~3u, kColTile);
+  const uint32_t i0 = blockIdx.x / across * kRowTile, j0 = blockIdx.x % across * kColTile;
   const int t = threadIdx.x, lane = t & 31;
   if (t == 0) {
     for (int s = 0; s < kRotStages; ++s) {
@@ -653,17 +655,17 @@ int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float 
   CUtensorMap tx{}, tr;
   int rc;
   if ((rc = encode_kmajor(&tr, rt, ldr, d16)) || (!few && (rc = encode_kmajor(&tx, xt, ldx, d16)))) return rc;
-  auto go = [&](auto kern, uint32_t row_tile, uint32_t col_tile, int threads, size_t smem) -> int {
+  auto go = [&](auto kern, uint32_t row_tile, int threads, size_t smem) -> int {
     if (const int r = smem_limit(reinterpret_cast<const void *>(kern), static_cast<int>(smem),
                                  "rotate_tma_kernel shared memory"))
       return r;
-    launch(kern, dim3(div_up(d4, col_tile), div_up(nrows, row_tile)), threads, smem, st,
+    launch(kern, div_up(d4, 32) * div_up(nrows, row_tile), threads, smem, st,
         tx, tr, in, nrows, d, rot, out, timeouts);
     KATO_LAUNCHED("rotate_tma_kernel");
     return KATO_OK;
   };
-  rc = few ? go(rotate_tma_kernel<true>, kSlabRows, 32, rot_threads<true>(), slab_smem)
-           : go(rotate_tma_kernel<false>, 32, 32, rot_threads<false>(),
+  rc = few ? go(rotate_tma_kernel<true>, kSlabRows, rot_threads<true>(), slab_smem)
+           : go(rotate_tma_kernel<false>, 32, rot_threads<false>(),
                 kRotStages * rot_stage_bytes<false>() + 1024);
   if (rc) return rc;
   ++*launches;
