@@ -281,99 +281,118 @@ __device__ uint32_t rescan(const FinishArgs &A, uint32_t q, uint32_t n, uint2 *b
 // The first round for all overflowing queries at once, before finish_kernel,
 // where p times the longest list is above cap: a round by one CTA reads its
 // query's rows at some 30 GB/s (5 ms for 224 lists at 10M), the grid shares them.
-// With nothing to do the two kernels take 3 us.
+// What bounds the round is a chain of latencies for each query: the bound's
+// candidates are read once into shared memory (eight digits of a selection over
+// them in global memory took 95 us), a list of the queries is kept instead of
+// searching their flags, and the CTAs find their rows through the sums of 256
+// lists at a time, where walking list by list took 60 us. The phase with two queries
+// of 512 probes at 10M: 79 us, 680 before; with nothing to do 9 us, its events included.
+constexpr uint32_t kBoundLook = 2048;  // candidates a bound looks at (a subset's
+                                       // S-th smallest key is a bound as well)
+
 __global__ void __launch_bounds__(kThreads) overflow_bound_kernel(const __grid_constant__ FinishArgs A,
                                                                   uint32_t *qcount, uint32_t nq) {
   after_previous();
+  __shared__ unsigned long long keys[kBoundLook];
   __shared__ uint32_t hist[256], sel[2], list[kThreads], n_list;
-  const uint32_t tid = threadIdx.x, cap = A.per_query, mine = blockIdx.x * kThreads + tid;
-  if (tid == 0) n_list = 0;
-  __syncthreads();
-  if (mine < nq) {
-    const uint32_t n = qcount[mine];
-    A.over[mine] = n > cap;
-    if (n > cap) {
-      list[atomicAdd(&n_list, 1u)] = mine;
-      atomicMax(A.rescans + 1, static_cast<unsigned long long>(n & ~kDropped));
-      atomicAdd(A.rescans, 1ull);
-      atomicAdd(A.over_n, 1ull);
-    }
-  }
-  __syncthreads();
-  for (uint32_t i = 0; i < n_list; ++i) {
-    const uint32_t q = list[i];
-    const uint2 *buf = A.slots + static_cast<size_t>(q) * cap;
-    // (a subset's S-th smallest key is a bound as well: 2048 at most)
-    const uint32_t look = min(min(qcount[q] & ~kDropped, cap), 2048u);
-    const unsigned long long K = look < A.S ? ~0ull
-                                            : block_select64(
-                                                  look, A.S - 1,
-                                                  [&](uint32_t j) {
-                                                    const uint2 e = buf[j];
-                                                    return (static_cast<unsigned long long>(e.x) << 32) | A.ids[e.y];
-                                                  },
-                                                  hist, sel);
+  const uint32_t tid = threadIdx.x, cap = A.per_query;
+  // thread t looks at the CTA's t-th query
+  for (uint32_t q0 = blockIdx.x; q0 < nq; q0 += gridDim.x * kThreads) {
+    const uint32_t mine = q0 + tid * gridDim.x;
+    const bool full = mine < nq && qcount[mine] > cap;
+    if (mine < nq) A.over[mine] = full;
+    if (tid == 0) n_list = 0;
+    if (!__syncthreads_or(full)) continue;
+    if (full) list[atomicAdd(&n_list, 1u)] = mine;
     __syncthreads();
-    if (tid == 0) {
-      A.over_key[q] = K;
-      qcount[q] = 0;
+    for (uint32_t i = 0; i < n_list; ++i) {
+      const uint32_t q = list[i], n = qcount[q];
+      const uint2 *buf = A.slots + static_cast<size_t>(q) * cap;
+      const uint32_t look = min(min(n & ~kDropped, cap), kBoundLook);
+      unsigned long long K = ~0ull;
+      if (look >= A.S) {
+#pragma unroll
+        for (uint32_t j = 0; j < kBoundLook; j += kThreads)
+          if (j + tid < look) {
+            const uint2 e = buf[j + tid];
+            keys[j + tid] = (static_cast<unsigned long long>(e.x) << 32) | A.ids[e.y];
+          }
+        __syncthreads();
+        K = block_select64(look, A.S - 1, [&](uint32_t j) { return keys[j]; }, hist, sel);
+      }
+      __syncthreads();  // every thread has read the count
+      if (tid == 0) {
+        A.over_key[q] = K;
+        A.over_list[atomicAdd(A.over_n, 1u)] = q;
+        qcount[q] = 0;
+        atomicMax(A.rescans + 1, static_cast<unsigned long long>(n & ~kDropped));
+        atomicAdd(A.rescans, 1ull);
+      }
     }
+    __syncthreads();  // n_list is written again
   }
 }
 
 __global__ void __launch_bounds__(kThreads) overflow_rows_kernel(const __grid_constant__ FinishArgs A,
-                                                                 uint32_t *qcount, uint32_t nq) {
+                                                                 uint32_t *qcount) {
   after_previous();
-  if (*A.over_n == 0) return;
+  const uint32_t found = *A.over_n;
+  if (found == 0) return;
   __shared__ __align__(16) uint32_t qw[1024 / 4];
-  __shared__ uint32_t list[kThreads], n_list;
-  const uint32_t cap = A.per_query, tid = threadIdx.x, lane = tid & 31;
-  for (uint32_t q0 = 0; q0 < nq; q0 += kThreads) {
-    const bool over = q0 + tid < nq && A.over[q0 + tid];
-    if (tid == 0) n_list = 0;
-    if (!__syncthreads_or(over)) continue;
-    if (over) list[atomicAdd(&n_list, 1u)] = q0 + tid;
-    __syncthreads();
-    const uint32_t found = n_list;
-    for (uint32_t i = 0; i < found; ++i) {
-      const uint32_t q = list[i];
-      __syncthreads();
-      load_query_words(A.qhi, q, A.dc, A.h, qw);
-      __syncthreads();
-      const int64_t qn = A.rank_qnorm[q];
-      const unsigned long long K = A.over_key[q];
-      const uint32_t *pq = A.probed + static_cast<size_t>(q) * A.nprobe;
-      const uint32_t np = A.qprobes ? A.qprobes[q] : A.nprobe;
-      uint2 *buf = A.slots + static_cast<size_t>(q) * cap;
-      uint32_t turn = 0;  // whose turn the next 256 rows are
-      for (uint32_t rb = 0; rb < np; rb += 32) {
-        uint32_t first = 0, rows = 0;
-        if (rb + lane < np) {
-          first = A.list_off[pq[rb + lane]];
-          rows = A.list_off[pq[rb + lane] + 1] - first;
-        }
-        for (uint32_t l = 0; l < 32; ++l) {
-          const uint32_t r0 = __shfl_sync(0xffffffffu, first, l), n = __shfl_sync(0xffffffffu, rows, l);
-          for (uint32_t at0 = 0; at0 < n; at0 += kThreads) {
-            const bool ours = turn == blockIdx.x;
-            if (++turn == gridDim.x) turn = 0;
-            if (!ours) continue;
-            for_rows_split(
-                A.xhi, A.dc, A.h, qw, r0 + at0, min(n - at0, static_cast<uint32_t>(kThreads)),
-                [&](uint32_t j, uint32_t dot, int64_t xn) {
-                  const uint32_t row = r0 + at0 + j;
-                  const int64_t l2 = qn + xn - 2 * static_cast<int64_t>(dot);
-                  const uint32_t d = __float_as_uint(dist_value(l2, A.scale));
-                  if (((static_cast<unsigned long long>(d) << 32) | A.ids[row]) > K) return;
-                  const uint32_t at = atomicAdd(qcount + q, 1u);
-                  if (at < cap) buf[at] = make_uint2(d, row);
-                },
-                [&](uint32_t j) { return A.rank_xnorm[r0 + at0 + j]; });
-          }
-        }
+  __shared__ uint32_t first[kThreads], upto[kThreads], rows[kThreads], wsum[kThreads / 32];
+  const uint32_t cap = A.per_query, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t turn = blockIdx.x;  // pieces of 256 rows until this CTA's next one
+  for (uint32_t i = 0; i < found; ++i) {
+    const uint32_t q = A.over_list[i];
+    load_query_words(A.qhi, q, A.dc, A.h, qw);
+    const int64_t qn = A.rank_qnorm[q];
+    const unsigned long long K = A.over_key[q];
+    const uint32_t *pq = A.probed + static_cast<size_t>(q) * A.nprobe;
+    const uint32_t np = A.qprobes ? A.qprobes[q] : A.nprobe;
+    uint2 *buf = A.slots + static_cast<size_t>(q) * cap;
+    for (uint32_t rb = 0; rb < np; rb += kThreads) {
+      uint32_t at = 0, n = 0;
+      if (rb + tid < np) {
+        const uint32_t c = pq[rb + tid];
+        at = A.list_off[c];
+        n = A.list_off[c + 1] - at;
       }
+      uint32_t incl = div_up(n, kThreads);  // the list's pieces, then those up to its end
+#pragma unroll
+      for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) wsum[warp] = incl;
+      __syncthreads();  // (the query's words are there too)
+      for (uint32_t w = 0; w < warp; ++w) incl += wsum[w];
+      first[tid] = at;
+      rows[tid] = n;
+      upto[tid] = incl;
+      __syncthreads();
+      const uint32_t pieces = upto[kThreads - 1];
+      for (; turn < pieces; turn += gridDim.x) {
+        uint32_t lo = 0, hi = kThreads - 1;  // the first list that ends after piece `turn`
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) / 2;
+          if (upto[mid] > turn) hi = mid;
+          else lo = mid + 1;
+        }
+        const uint32_t at0 = (turn - (lo ? upto[lo - 1] : 0)) * kThreads, r0 = first[lo] + at0;
+        for_rows_split(
+            A.xhi, A.dc, A.h, qw, r0, min(rows[lo] - at0, static_cast<uint32_t>(kThreads)),
+            [&](uint32_t j, uint32_t dot, int64_t xn) {
+              const int64_t l2 = qn + xn - 2 * static_cast<int64_t>(dot);
+              const uint32_t d = __float_as_uint(dist_value(l2, A.scale));
+              if (((static_cast<unsigned long long>(d) << 32) | A.ids[r0 + j]) > K) return;
+              const uint32_t to = atomicAdd(qcount + q, 1u);
+              if (to < cap) buf[to] = make_uint2(d, r0 + j);
+            },
+            [&](uint32_t j) { return A.rank_xnorm[r0 + j]; });
+      }
+      turn -= pieces;
+      __syncthreads();  // the lists and the query's words are written again
     }
-    __syncthreads();  // n_list is written again
   }
 }
 
@@ -701,9 +720,10 @@ __global__ void __launch_bounds__(kThreads, 4) finish_kernel(const __grid_consta
 int rescan_overflows(const FinishArgs &A, uint32_t *qcount, uint32_t nq, cudaStream_t st) {
   int sms = 0;
   if (const int rc = current_sms(&sms)) return rc;
-  launch(overflow_bound_kernel, div_up(nq, kThreads), kThreads, 0, st, A, qcount, nq);
+  // (so few CTAs that the next kernel's are placed at once)
+  launch(overflow_bound_kernel, std::min(nq, kFewCtas - 1), kThreads, 0, st, A, qcount, nq);
   KATO_LAUNCHED("overflow_bound_kernel");
-  launch(overflow_rows_kernel, 4 * sms, kThreads, 0, st, A, qcount, nq);
+  launch(overflow_rows_kernel, 4 * sms, kThreads, 0, st, A, qcount);
   KATO_LAUNCHED("overflow_rows_kernel");
   return KATO_OK;
 }

@@ -30,9 +30,9 @@ struct FinishArgs {
   uint32_t h, nprobe;
   // where a query can probe more rows than its buffer holds: per query, whether
   // it was rescanned by the whole grid before, and the key it was rescanned for;
-  // the number of those queries (accumulating)
-  uint32_t *over;
-  unsigned long long *over_key, *over_n;
+  // those queries and their number (0 before the pass)
+  uint32_t *over, *over_list, *over_n;
+  unsigned long long *over_key;
 };
 
 // The first rescan of queries with more candidates than their buffers hold (with

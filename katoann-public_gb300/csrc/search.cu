@@ -351,7 +351,7 @@ struct Plan {
   bool cost;                        // the ranking CTAs split the slabs' cost, not their count
   size_t off_fq, off_qhi, off_qlo, off_qn, off_qhn, off_qh0, off_cd, off_probed, off_cnt, off_off,
       off_base, off_cur, off_work, off_ent, off_slots, off_stats,
-      off_tcitems, off_tileoff, off_qcount,  off_bound,
+      off_tcitems, off_tileoff, off_over, off_qcount, off_bound,
       off_rec, off_recn, off_qh16, off_ql16, off_qterm, off_rot,
       off_qprobes, off_z, off_qcn, off_qr16, off_share, total;
 };
@@ -439,7 +439,8 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   pl.off_qh0 = take(static_cast<size_t>(B) * 8);
   pl.off_cd = take(static_cast<size_t>(B) * L * 4);
   pl.off_probed = take(bp * 4);
-  pl.off_cnt = take(static_cast<size_t>(L) * 4);  // cleared together with qcount after it
+  pl.off_cnt = take(static_cast<size_t>(L) * 4);  // cleared together with over and qcount after it
+  pl.off_over = take(4);
   pl.off_qcount = take(static_cast<size_t>(B) * 4);
   pl.off_off = take((static_cast<size_t>(L) + 1) * 4);
   pl.off_base = take(3 * (static_cast<size_t>(L) + 1) * 4);
@@ -751,10 +752,12 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
       F.h = pl.dims;
       F.nprobe = p;
       if (static_cast<uint64_t>(p) * ix->max_list > pl.cap) {
-        // a buffer can overflow (the coarse product's terms have been read)
+        // a buffer can overflow (the coarse product's terms and distances have
+        // been read)
         F.over = reinterpret_cast<uint32_t *>(bound);
         F.over_key = reinterpret_cast<unsigned long long *>(ws + pl.off_qterm);
-        F.over_n = stats + 39;
+        F.over_list = reinterpret_cast<uint32_t *>(cd);
+        F.over_n = reinterpret_cast<uint32_t *>(ws + pl.off_over);
         if ((rc = rescan_overflows(F, qcount, nq, st))) return rc;
         g_launches += 2;
       }
