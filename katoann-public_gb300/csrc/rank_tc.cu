@@ -882,7 +882,7 @@ uint32_t rank_tc_ctas() {
 std::atomic<uint32_t> g_tc_width{0}, g_tc_beta{0};
 std::atomic<unsigned long long> g_tc_wait{0};
 
-bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s) {
+bool rank_tc_plan(uint32_t h, uint32_t dc, bool rotated, TcShape *s) {
   if (h == 0 || h % 64 || h > 1024 || h > dc || dc % 64) return false;
   TcShape t{};
   // items narrow as the queries' rows widen, so that several query buffers fit
@@ -890,7 +890,12 @@ bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s) {
   const uint32_t cap = g_tc_width.load();
   if (cap >= 16 && cap < t.N) t.N = cap;
   t.inner = h == 64 ? 64 : 128;
-  t.f = std::min(h, kTcFilterDims);
+  // without a rotation the leading dimensions are like any others: nearly every
+  // pair passes on 128 of them, and what does not fit the lists is rescanned
+  // (high bytes of 300k flat vectors, 512 queries of 33 lists, without the filter
+  // and with it: 576 dimensions 222 and 594 us, 1,024 291 and 625; where they
+  // decay as i^-1, 832 dimensions 277 and 296, 320 151 and 146)
+  t.f = rotated ? std::min(h, kTcFilterDims) : h;
   t.centred = h > 256;
   constexpr uint32_t shapes[][2] = {{4, 4}, {4, 2}, {3, 2}, {2, 2}, {1, 2}};
   for (const auto &b : shapes) {

@@ -121,7 +121,7 @@ __host__ __device__ inline TcSmem tc_smem_layout(uint32_t h, const TcShape &s) {
 inline uint32_t default_seed_rows(uint32_t S) { return std::max(1024u, 8 * std::min(S, 1u << 20)); }
 // The shape for h ranking dimensions over rows of dc bytes, or false when h
 // does not suit the pass (the caller then uses the CUDA-core pass).
-bool rank_tc_plan(uint32_t h, uint32_t dc, TcShape *s);
+bool rank_tc_plan(uint32_t h, uint32_t dc, bool rotated, TcShape *s);
 // One CTA per SM walks an equal share of all tiles.
 int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShape &s,
             cudaStream_t st);

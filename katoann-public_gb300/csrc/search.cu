@@ -384,7 +384,7 @@ int make_plan(const katoann_gpu_index *ix, uint32_t B, uint32_t k, uint32_t p, i
   // tensor-core ranking: every query's candidates within its seed bound go
   // to a buffer of `cap` entries (an overflowing query is rescanned exactly)
   pl.cap = g_candidate_cap.load();
-  pl.tc = ranking != KATO_RANK_FULL && pl.S <= pl.cap && rank_tc_plan(pl.dims, ix->dc, &pl.tcs);
+  pl.tc = ranking != KATO_RANK_FULL && pl.S <= pl.cap && rank_tc_plan(pl.dims, ix->dc, ix->rotated != 0, &pl.tcs);
   // rows per CTA of the CUDA-core pass: each of a list's parts keeps up to SC
   // candidates per query. Within kSplitEntries places for them the parts are as
   // short as they should be, beyond it so many as fit, and one per list at least.
