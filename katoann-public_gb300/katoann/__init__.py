@@ -428,11 +428,9 @@ class Index:
                     ranking_timeouts=int(s[3]), ranking_tiles=int(s[4]),
                     ranking_candidates=int(s[5]), ranking_rescans=int(s[6]),
                     ranking_max_candidates=int(s[7]), ranking_cta_max_cycles=int(s[31]),
-                    ranking_role_cycles=dict(zip(
-                        ("conv_wait_raw", "conv_wait_a", "conv_total", "mma_wait_b", "mma_wait_acc",
-                         "mma_wait_a", "mma_total", "epi_wait_b", "epi_wait_acc", "epi_total",
-                         "tma_wait_stage", "tma_total", "stage_wait_b", "stage_total",
-                         "mma_issue"), (int(v) for v in s[16:31]))),
+                    ranking_role_cycles=dict(
+                        score_wait_rows=int(s[16]), score_wait_items=int(s[17]),
+                        score_total=int(s[18]), stage_wait_buffer=int(s[28]), stage_total=int(s[29])),
                     coarse_role_cycles=dict(zip(
                         ("tma_wait", "tma_total", "mma_wait_acc", "mma_wait_stage", "mma_total",
                          "epi_wait", "epi_total"), (int(v) for v in s[32:39]))),
