@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                    const __grid_constant__ TcShape S) {
   after_previous();
   constexpr uint32_t NI = IN / 64;        // 16-byte reads per row, lane and chunk
-    constexpr uint32_t kBox = kTcBoxRows * IN, kStage = 2 * kBox;
+  constexpr uint32_t kBox = kTcBoxRows * IN, kStage = 2 * kBox;
   // row bytes enter as multiples of kScale
   constexpr float kScale = kCentred ? 1.0f : 0x1p-24f;
   extern __shared__ __align__(1024) unsigned char sm[];
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           // of an SM against all of h = 256, and completing a record costs an
           // SM about 5 ns: on while the CTA's slabs gave below 16 each, whatever
           // their items were (10M x 1,024 of one spread-out cloud: 3 per slab,
-          // 0.50 ms against 0.70; of tight clusters, 20 and more, 1.16 ms with
+          // 0.50 ms against 0.71; of tight clusters, 20 and more, 1.16 ms with
           // its records for 1.30 with 32 as the line and 1.07 without a
           // filter). The first 8 slabs go ahead, the next await their count.
           // Partial records must leave the CTA's list room (whoever's records
@@ -611,7 +611,6 @@ __device__ __forceinline__ uint32_t sketch_bin(uint32_t d) {
   return (e - 4) * 32 + ((d >> (e - 5)) & 31);
 }
 
-//
 // The sketch loads bound it: 32-byte pieces of rows h or more bytes apart. Two
 // lanes to a row halve the L1's work (2,048 rows: 148 -> 127 us for 4096 queries
 // at 1M; the squares as x (x - 2 q) by dp4a instead of a byte-wise difference
@@ -804,10 +803,14 @@ __global__ void __launch_bounds__(256, 3) rank_seed_kernel(
   }
 }
 
+constexpr uint32_t kBucketCtas = 8;
+
 // The pass's candidate records (query, xn - 2 dot, row, partial) into per-query
-// buffers of (distance bits, row); gridDim.y CTAs share each ranking CTA's
+// buffers of (distance bits, row); kBucketCtas CTAs share each ranking CTA's
 // list, so that enough records (each a global atomic and a scattered store)
-// are in flight per SM. A partial record covers the first f dimensions:
+// are in flight per SM; those without records leave after one load (2M x 768,
+// 64 lists, with eight CTAs and with one: 1 query 78.5 and 78.3 us a search, 64 142 and
+// 147, 511 226 and 243, 1,024 318 and 355). A partial record covers the first f dimensions:
 // eight lanes add the rest, 16 bytes of the row and of the query each, with
 // the loads of a warp's 32 records in flight together.
 __global__ void __launch_bounds__(256) tc_bucket_kernel(
@@ -943,11 +946,11 @@ int rank_tc(const RankTcArgs &A, const uint8_t *xhi, uint32_t npts, const TcShap
   return s.centred ? go(rank_tc_kernel<128, true>) : go(rank_tc_kernel<128, false>);
 }
 
-int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas, uint32_t nq,
+int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas,
                    const uint8_t *xhi, const uint8_t *qhi, const int2 *qcn, const int32_t *bound,
                    uint32_t dc, uint32_t f, uint32_t h, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
                    DistScale scale, unsigned long long *found, cudaStream_t st) {
-  launch(tc_bucket_kernel, dim3(ctas, nq < 512 ? 1 : 8), 256, 0, st, rec, rec_n, rec_cap, xhi, qhi, qcn, bound, dc, f, h,
+  launch(tc_bucket_kernel, dim3(ctas, kBucketCtas), 256, 0, st, rec, rec_n, rec_cap, xhi, qhi, qcn, bound, dc, f, h,
                                                   qcount, qbuf, cap, scale, found);
   KATO_LAUNCHED("tc_bucket_kernel");
   return KATO_OK;

@@ -143,7 +143,7 @@ extern std::atomic<unsigned long long> g_tc_wait;
 // Candidate records of the pass, completed over dimensions [f, h) where they
 // are partial, into per-query buffers of cap entries (distance bits, row);
 // qcount counts the candidates of each query and *found all of them.
-int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas, uint32_t nq,
+int rank_tc_bucket(const uint4 *rec, const uint32_t *rec_n, uint32_t rec_cap, uint32_t ctas,
                    const uint8_t *xhi, const uint8_t *qhi, const int2 *qcn, const int32_t *bound,
                    uint32_t dc, uint32_t f, uint32_t h, uint32_t *qcount, uint2 *qbuf, uint32_t cap,
                    DistScale scale, unsigned long long *found, cudaStream_t st);

@@ -665,7 +665,7 @@ int search_pass(const katoann_gpu_index *ix, const Plan &pl, const float *querie
     kmark(tm, 2, false, st);
     if ((rc = rank_tc(T, ix->d_hi, ix->npts, pl.tcs, st))) return rc;
     kmark(tm, 2, true, st);
-    if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, nq, ix->d_hi, qhi, T.qcn, bound, dc,
+    if ((rc = rank_tc_bucket(rec, rec_n, pl.rec_cap, pl.ctas, ix->d_hi, qhi, T.qcn, bound, dc,
                              pl.tcs.f, pl.dims, qcount, slots, pl.cap, scale, stats + 5, st)))
       return rc;
     g_launches += 3;  // seed, scan, bucket
