@@ -648,20 +648,26 @@ void validate(const void *state, uint32_t nlist, uint32_t head, const SearchPara
     throw std::invalid_argument("prefix ranking needs the rotation file (.dimc)");
 }
 
-// Whether a host buffer goes by the pinned staging: pageable memory, whose copies
-// wait for the CPU, and pinned memory of a small batch, where one copy less of
-// the results is worth more than the CPU's own. Pinned buffers of 1,024-dimensional
-// queries, direct and staged: 4 queries 109 and 107 us a search, 16 120 and 121, 113
-// (k = 100) 160 and 182.
-bool by_staging(const void *p, size_t batch_bytes) {
-  constexpr size_t kSmall = 32u << 10;
+// What a caller's buffer is. Others than host memory (null, device, managed) are
+// left to the copies, which refuse what they cannot take.
+enum class Memory { kPageable, kPinned, kOther };
+Memory memory_of(const void *p) {
   cudaPointerAttributes a{};
+  if (!p) return Memory::kOther;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return Memory::kOther;
   }
-  return a.type == cudaMemoryTypeUnregistered || (a.type == cudaMemoryTypeHost && batch_bytes <= kSmall);
+  return a.type == cudaMemoryTypeUnregistered ? Memory::kPageable
+         : a.type == cudaMemoryTypeHost       ? Memory::kPinned
+                                              : Memory::kOther;
 }
+
+// Pinned buffers of batches up to this go by the staging as pageable ones do: one
+// copy less of the results is worth more than the CPU's own (1,024-dimensional
+// queries, direct and staged: 4 queries 109 and 107 us a search, 16 120 and 121,
+// 113 with k = 100 160 and 182).
+constexpr size_t kSmallBatch = 32u << 10;
 
 // The per-query budget of a search: the device model (when the params carry
 // one and no explicit budgets) and the selection depth the workspace needs.
@@ -720,8 +726,13 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
   // the staging holds a batch of one pass: its queries, then its results
   const size_t all = qbytes + 2 * rbytes;
   const bool fits = passes == 1 && all <= State::kStageBytes;
-  unsigned char *const sq = fits && by_staging(queries, all) ? s.stage() : nullptr;
-  unsigned char *const sr = fits && (by_staging(ids, all) || by_staging(dists, all)) ? s.stage() + qbytes : nullptr;
+  auto staged = [&](Memory m) { return m == Memory::kPageable || (m == Memory::kPinned && all <= kSmallBatch); };
+  unsigned char *sq = nullptr, *sr = nullptr;
+  if (fits) {
+    const Memory mi = memory_of(ids), md = memory_of(dists);
+    if (staged(memory_of(queries))) sq = s.stage();
+    if (mi != Memory::kOther && md != Memory::kOther && (staged(mi) || staged(md))) sr = s.stage() + qbytes;
+  }
   if (sq) std::memcpy(sq, queries, qbytes);
   for (uint32_t q0 = 0; q0 < nq; q0 += mb) {
     const uint32_t nb = std::min(mb, nq - q0);
