@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   uint64_t *b_empty = b_full + kTcMaxBufs;                     // used by every scoring warp
   volatile uint32_t *err = reinterpret_cast<volatile uint32_t *>(sm + L.err);
   uint32_t *rcount = reinterpret_cast<uint32_t *>(sm + L.rcount);
-  // slabs scored, and filtered ones staged before any were
-  volatile uint32_t *slabs = rcount + 1, *fstaged = rcount + 2;
+  // slabs scored; filtered pairs staged, and those of them whose item has been left
+  uint32_t *slabs = rcount + 1, *fstaged = rcount + 2, *fpairs = rcount + 3;
   uint32_t *qids = reinterpret_cast<uint32_t *>(sm + L.qids);
   // -(bound - qn) / 2 of each query slot, in units of kScale
   float *qbv = reinterpret_cast<float *>(sm + L.qbv);
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc::mbar_init(b_full + s, 64);
       tc::mbar_init(b_empty + s, kScoreWarps);
     }
-    rcount[0] = rcount[1] = rcount[2] = 0;
+    rcount[0] = rcount[1] = rcount[2] = rcount[3] = 0;
     // the TMA swizzle pattern repeats every 1024 bytes of shared address
     *err = (tc::smem_addr(sm + L.raw) & 1023u) ? 2u : 0u;
     tc::fence_barrier_init();
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           }
         }
         if (!ok) break;
-        if (lane == 0) atomicAdd(const_cast<uint32_t *>(slabs), 1u);
+        if (lane == 0) atomicAdd(slabs, 1u);
       }
       // hand back the remaining items' buffers, so that the staging warps end
       __syncwarp();
@@ -494,6 +494,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         auto entry = [&](const TcItem &it, uint32_t j) { return j < it.ne ? A.entries[it.e0 + j] : 0u; };
         TcItem cur = item_at(sw), nxt = item_at(sw + nB);
         uint32_t s0 = slab_at(sw), s1 = slab_at(sw + 1);
+        uint32_t staged = 0;  // filtered pairs of the buffer's item
         uint32_t q0 = entry(cur, lane) / A.nprobe, q1 = entry(cur, lane + 32) / A.nprobe;
         for (uint32_t li = sw, use = 0; li < n_li; li += nB, ++use) {
           const uint32_t e0 = entry(nxt, lane), e1 = entry(nxt, lane + 32);
@@ -508,25 +509,40 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           // their items were (10M x 1,024 of one spread-out cloud: 3 per slab,
           // 0.50 ms against 0.71; of tight clusters, 20 and more, 1.16 ms with
           // its records for 1.30 with 32 as the line and 1.07 without a
-          // filter). The first 8 slabs go ahead, the next await their count.
+          // filter). The first items go ahead, those after 8 slabs await their count.
           // Partial records must leave the CTA's list room (whoever's records
           // do not fit is rescanned): an eighth of an item's pairs may pass,
           // which keeps a server's batches of a hundred or so off long lists
           // (400k searches/s at 10M: p99 8.4 -> 4.2 ms; with half the pairs, the
-          // 384-probe batches' long lists went unfiltered, 245 -> 265 us)
+          // 384-probe batches' long lists went unfiltered, 245 -> 265 us). And the
+          // pairs in the other buffers with this item's have to fit into what is left
+          // of it, but for an eighth: all of them, or at twice the records there were
+          // so far to a filtered pair (a flat spectrum, 512 queries of 16 lists,
+          // h = 512: 243 us a search, 806 with rescans)
+          const uint32_t pairs = (min(cur.nrows, (min(s1, t1) - s0) * kTcSlab) - (max(s0, t0) - s0) * kTcSlab) * cur.ne;
           bool filt = A.f < h && cur.nrows * cur.ne <= 2 * A.rec_cap;
-          uint32_t scored = 0;
-          if (filt) {
-            const uint32_t have = warp_read(rcount);
-            scored = warp_read(slabs);
-            const uint32_t ahead = warp_read(fstaged);
-            filt = (scored >= 8 ? have <= 16 * scored : ahead < 8) && have <= A.rec_cap / 4;
+          if (lane == 0) {
+            // this buffer's last item has been scored
+            const uint32_t seen = atomicAdd(fpairs, staged) + staged;
+            staged = 0;
+            if (filt) {
+              const uint32_t have = *static_cast<volatile uint32_t *>(rcount);
+              const uint32_t scored = *static_cast<volatile uint32_t *>(slabs);
+              filt = have <= min(scored >= 8 ? 16 * scored : ~0u, A.rec_cap / 4);
+              if (filt) {
+                const uint32_t ahead = atomicAdd(fstaged, pairs) + pairs - seen;
+                const uint32_t room = A.rec_cap / 8 * 7 - have;  // have is a quarter at most
+                filt = ahead <= room || (seen && 2ull * have * ahead <= static_cast<uint64_t>(room) * seen);
+                if (filt) staged = pairs;
+                else atomicSub(fstaged, pairs);
+              }
+            }
           }
+          filt = __shfl_sync(0xffffffffu, filt, 0);
           const uint32_t dims = filt ? A.f : h;
           if (lane == 0) {
             desc[sw] = Desc{s0, s1, cur.row0, cur.nrows, cur.ne, (dims + IN - 1) / IN, filt, 0};
             tc::mbar_arrive(d_full + sw);
-            if (filt && scored < 8) atomicAdd(const_cast<uint32_t *>(fstaged), s1 - s0);
           }
           // the queries' fp16 rows, `per` 16-byte units each, the ids shuffled
           const uint32_t per = (dims + IN - 1) / IN * (IN / 8), steps = (cur.ne * per + 31) / 32;

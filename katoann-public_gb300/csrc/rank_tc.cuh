@@ -106,7 +106,7 @@ __host__ __device__ inline TcSmem tc_smem_layout(uint32_t h, const TcShape &s) {
   L.desc = tc_take(o, kTcMaxBufs * kTcDesc, 16);
   L.bars = tc_take(o, (kTcScoreWarps * kTcMaxStages + 3 * kTcMaxBufs) * 8, 8);
   L.err = tc_take(o, 4, 4);
-  L.rcount = tc_take(o, 3 * 4, 4);
+  L.rcount = tc_take(o, 4 * 4, 4);
   L.total = (o + 127) / 128 * 128;
   return L;
 }

@@ -21,11 +21,12 @@ def test_ranking_kernel_reads_shared_words_as_a_warp():
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "rank_tc.cu")).read())
     at = text.index("{", text.index("rank_tc_kernel(const __grid_constant__"))
     body = text[at:_block(text, at)]
-    while (m := re.search(r"if \(tid == 0\) \{", body)):  # one thread's own decisions
-        body = body[:m.start()] + body[_block(body, m.end() - 1):]
-    words = re.findall(r"(volatile uint32_t \*\w+ = |, )?\*\s*(err|slabs|fstaged)\b(?!\s*=[^=])", body)
+    for thread in ("tid", "lane"):  # one thread's own decisions
+        while (m := re.search(r"if \(" + thread + r" == 0\) \{", body)):
+            body = body[:m.start()] + body[_block(body, m.end() - 1):]
+    words = re.findall(r"(uint32_t |, )?\*\s*(?:static_cast<volatile uint32_t \*>\()?(err|rcount|slabs|fstaged|fpairs)\b(?!\s*=[^=])", body)
     reads = [w for declared, w in words if not declared]
     assert not reads, reads
     assert "*reinterpret_cast<volatile" not in body
-    for word in ("err", "rcount", "slabs", "fstaged"):
-        assert f"warp_read({word})" in body, word
+    assert body.count("warp_read(err)") == 3
+    assert "filt = __shfl_sync(0xffffffffu, filt, 0);" in body  # what lane 0 decided
