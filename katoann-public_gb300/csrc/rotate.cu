@@ -621,9 +621,12 @@ static int encode_kmajor(CUtensorMap *map, const float *base, uint32_t ld, uint3
   return KATO_OK;
 }
 
-// Up to 64 rows the tiles of 32 would leave most of a tile empty and, at
-// d = 1,024, use 32 SMs: 16 rows took 23 us, in tiles of 8 rows 17 us.
-constexpr uint32_t kRotFewRows = 64;
+// Few rows of few dimensions: tiles of 8 rows, which need no transpose (with tiles
+// of 32 and the transpose in brackets, 16 rows: d = 128 8.5 us (9.0), 256 8.8
+// (10.4)). From 512 dimensions on the rows' slab in shared memory leaves an SM few
+// CTAs and its filling is not hidden: 64 rows of 512 12.4 us (11.8), of 1,024 18.1
+// (15.2), of 3,072 269 (44).
+constexpr uint32_t kRotFewRows = 64, kRotFewDims = 512;
 
 int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float *rot,
                        const float *rot_kmajor, void *scratch, float *out, uint32_t *timeouts,
@@ -640,7 +643,7 @@ int rotate_rows_kmajor(const float *in, uint32_t nrows, uint32_t d, const float 
   // 1 KiB of slack: the stages start on a 1 KiB boundary
   const size_t slab_smem =
       kRotStages * rot_stage_bytes<true>() + static_cast<size_t>(d16) * kSlabStride * 4 + 1024;
-  const bool few = nrows <= kRotFewRows && slab_smem <= 224 * 1024;  // d16 up to 3,728
+  const bool few = nrows <= kRotFewRows && d16 < kRotFewDims;
   if (!few) {
     transpose_pad(in, nrows, d, d16, xt, ldx, st);
     ++*launches;
