@@ -51,3 +51,23 @@ def test_rescans_by_the_grid(data, budgets, max_batch):
             assert len(bad) == 0, bad[:5]
     finally:
         assert gpu().katoann_gpu_set_candidate_cap(32768) == 0
+
+
+@pytest.mark.parametrize("S", [300, 1000, 3000])
+def test_rescans_with_many_survivors(data, S):
+    """Survivors above the 2,048 candidates that a bound looks at otherwise, and
+    counts whose eightfold lies on both sides of the buffer's size."""
+    import katoann
+    a, q = data
+    nlist = len(a["list_sizes"])
+    idx = katoann.Index()
+    idx.load_arrays(a["centroids"], a["list_sizes"], a["ids"], a["vectors"], head_dims=64)
+    kw = dict(k=10, nprobe=nlist, ranking="prefix", survivors=S)
+    rid, rd = oracle.OracleIndex(None, arrays=a).search(q[:40], **kw)
+    try:
+        assert gpu().katoann_gpu_set_candidate_cap(max(S, 512)) == 0
+        ids, dists = idx.search(q[:40], **kw)
+        assert idx.search_stats()["ranking_rescans"] > 0
+    finally:
+        assert gpu().katoann_gpu_set_candidate_cap(32768) == 0
+    assert np.array_equal(ids, rid) and np.array_equal(dists, rd)
