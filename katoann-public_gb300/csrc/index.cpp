@@ -151,10 +151,15 @@ struct Index::State {
   // pageable: its queries and results cross in one asynchronous copy each. Three
   // copies to pageable memory took a third of a one-query search.
   static constexpr size_t kStageBytes = 1u << 20;
-  mutable unsigned char *hstage = nullptr;
-  unsigned char *stage() const {
-    if (!hstage) cuda_check(cudaMallocHost(reinterpret_cast<void **>(&hstage), kStageBytes), "cudaMallocHost");
-    return hstage;
+  unsigned char *hstage = nullptr;
+
+  // What every load makes first: the stream, its event, and the pinned memory of
+  // one-pass host searches.
+  void open() {
+    cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    cuda_check(cudaEventCreateWithFlags(&done, cudaEventDisableTiming), "cudaEventCreate");
+    cuda_check(cudaMallocHost(reinterpret_cast<void **>(&hstage), kStageBytes), "cudaMallocHost");
+    wait_counts(1);
   }
 
   ~State() {
@@ -328,8 +333,7 @@ void Index::load_codes(const std::string &path, const LoadOptions &opt) {
     s.max_list = std::max(s.max_list, s.sizes[c]);
   }
   if (off[L] != n || s.max_list != h.max_list) throw std::runtime_error("bad list sizes in " + path);
-  cuda_check(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "cudaStreamCreate");
-  cuda_check(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming), "cudaEventCreate");
+  s.open();
   s.list_off.alloc((L + 1) * 4);
   cuda_check(cudaMemcpy(s.list_off.p, off.data(), (L + 1) * 4, cudaMemcpyHostToDevice), "upload");
   Pinned pin(64u << 20);
@@ -497,8 +501,7 @@ void Index::load_arrays(const IndexArrays &a, const LoadOptions &opt) {
   s.normalized = a.normalized;
   s.dc = round_up(a.dim, 64u);
   s.max_batch = std::max(1u, opt.max_batch);
-  cuda_check(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "cudaStreamCreate");
-  cuda_check(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming), "cudaEventCreate");
+  s.open();
   katoann_stream_t ks = reinterpret_cast<katoann_stream_t>(s.stream);
   const cudaMemcpyKind up = a.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const uint32_t d = s.dim, dc = s.dc, n = s.npts, L = s.nlist;
@@ -730,8 +733,8 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
   unsigned char *sq = nullptr, *sr = nullptr;
   if (fits) {
     const Memory mi = memory_of(ids), md = memory_of(dists);
-    if (staged(memory_of(queries))) sq = s.stage();
-    if (mi != Memory::kOther && md != Memory::kOther && (staged(mi) || staged(md))) sr = s.stage() + qbytes;
+    if (staged(memory_of(queries))) sq = s.hstage;
+    if (mi != Memory::kOther && md != Memory::kOther && (staged(mi) || staged(md))) sr = s.hstage + qbytes;
   }
   if (sq) std::memcpy(sq, queries, qbytes);
   for (uint32_t q0 = 0; q0 < nq; q0 += mb) {
