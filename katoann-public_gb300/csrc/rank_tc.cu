@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           }
         }
         if (!ok) break;
-        if (lane == 0) atomicAdd(slabs, 1u);
+        if (IN == 128 && lane == 0) atomicAdd(slabs, 1u);
       }
       // hand back the remaining items' buffers, so that the staging warps end
       __syncwarp();
@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           const TcItem nxt2 = item_at(li + 2 * nB);
           const int2 cn0 = A.qcn[q0], cn1 = N > 32 ? A.qcn[q1] : make_int2(0, 0);
           const int32_t bd0 = A.bound[q0], bd1 = N > 32 ? A.bound[q1] : 0;
-          bool filt = A.f < h && cur.nrows * cur.ne <= 2 * A.rec_cap;
+          // (rows of 64 dimensions are never filtered)
+          bool filt = IN == 128 && A.f < h && cur.nrows * cur.ne <= 2 * A.rec_cap;
           // pairs of the item's rows that are the CTA's
           const uint32_t rows = min(cur.nrows, (min(s1, t1) - s0) * kTcSlab) - (max(s0, t0) - s0) * kTcSlab;
           const uint32_t pairs = filt ? rows * cur.ne : 0;
@@ -523,22 +524,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           // of it, but for an eighth: all of them, or at twice the records there were
           // so far to a filtered pair (a flat spectrum, 512 queries of 16 lists,
           // h = 512: 243 us a search, 806 with rescans)
-          if (lane == 0) {
-            // (four accesses in flight together: 10M x 1,024 493.9 us, one after
-            // another 495.7; without the room's rule 490.8, and 2,000 queries of
-            // 2M x 768, whose first items do not all fit, 242 for 248)
-            const uint32_t have = *static_cast<volatile uint32_t *>(rcount);
-            const uint32_t scored = *static_cast<volatile uint32_t *>(slabs);
-            // this buffer's last item has been scored
-            const uint32_t seen = atomicAdd(fpairs, staged) + staged;
-            const uint32_t ahead = atomicAdd(fstaged, pairs) + pairs - seen;
-            const uint32_t room = A.rec_cap / 8 * 7 - have;  // have is a quarter at most
-            filt = filt && have <= min(scored >= 8 ? 16 * scored : ~0u, A.rec_cap / 4) &&
-                   (ahead <= room || (seen && 2ull * have * ahead <= static_cast<uint64_t>(room) * seen));
-            staged = filt ? pairs : 0;
-            if (pairs != staged) atomicSub(fstaged, pairs);
+          if constexpr (IN == 128) {
+            if (lane == 0) {
+              // (four accesses in flight together: 10M x 1,024 493.9 us, one after
+              // another 495.7; without the room's rule 490.8, and 2,000 queries of
+              // 2M x 768, whose first items do not all fit, 242 for 248)
+              const uint32_t have = *static_cast<volatile uint32_t *>(rcount);
+              const uint32_t scored = *static_cast<volatile uint32_t *>(slabs);
+              // this buffer's last item has been scored
+              const uint32_t seen = atomicAdd(fpairs, staged) + staged;
+              const uint32_t ahead = atomicAdd(fstaged, pairs) + pairs - seen;
+              const uint32_t room = A.rec_cap / 8 * 7 - have;  // have is a quarter at most
+              filt = filt && have <= min(scored >= 8 ? 16 * scored : ~0u, A.rec_cap / 4) &&
+                     (ahead <= room || (seen && 2ull * have * ahead <= static_cast<uint64_t>(room) * seen));
+              staged = filt ? pairs : 0;
+              if (pairs != staged) atomicSub(fstaged, pairs);
+            }
+            filt = __shfl_sync(0xffffffffu, filt, 0);
           }
-          filt = __shfl_sync(0xffffffffu, filt, 0);
           const uint32_t dims = filt ? A.f : h;
           if (lane == 0) {
             desc[sw] = Desc{s0, s1, cur.row0, cur.nrows, cur.ne, (dims + IN - 1) / IN, filt, 0};
