@@ -731,12 +731,10 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
   const bool fits = passes == 1 && all <= State::kStageBytes;
   auto staged = [&](Memory m) { return m == Memory::kPageable || (m == Memory::kPinned && all <= kSmallBatch); };
   unsigned char *sq = nullptr, *sr = nullptr;
-  if (fits) {
-    const Memory mi = memory_of(ids), md = memory_of(dists);
-    if (staged(memory_of(queries))) sq = s.hstage;
-    if (mi != Memory::kOther && md != Memory::kOther && (staged(mi) || staged(md))) sr = s.hstage + qbytes;
+  if (fits && staged(memory_of(queries))) {
+    sq = s.hstage;
+    std::memcpy(sq, queries, qbytes);
   }
-  if (sq) std::memcpy(sq, queries, qbytes);
   for (uint32_t q0 = 0; q0 < nq; q0 += mb) {
     const uint32_t nb = std::min(mb, nq - q0);
     const void *src = queries + static_cast<size_t>(q0) * s.dim;
@@ -778,6 +776,10 @@ void Index::search(const float *queries, uint32_t nq, const SearchParams &p, uin
       gpu_check(katoann_gpu_search(&s.view, s.dq.as<float>(), nb, p.k, p.nprobe, rk, p.survivors,
                                    mb, s.ws.p, s.ws.n, d_ids, d_dists,
                                    reinterpret_cast<katoann_stream_t>(s.stream)));
+    }
+    if (fits) {  // (looked up while the kernels run)
+      const Memory mi = memory_of(ids), md = memory_of(dists);
+      if (mi != Memory::kOther && md != Memory::kOther && (staged(mi) || staged(md))) sr = s.hstage + qbytes;
     }
     if (sr) {
       cuda_check(cudaMemcpyAsync(sr, d_ids, 2 * rbytes, cudaMemcpyDeviceToHost, s.stream), "copy results");
