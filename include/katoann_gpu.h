@@ -179,8 +179,9 @@ int katoann_gpu_search(const katoann_gpu_index *index, const float *d_queries, u
  * timed region is measured where it runs. Phases: 0 rotation+quantization of
  * the queries, 1 coarse product, 2 top-nprobe selection, 3 per-query probe
  * budget (empty without one), 4 inversion, 5 seed bounds of the tensor-core
- * ranking pass (empty on the CUDA-core pass), 6 ranking pass, 7 survivor
- * merge, 8 refinement. */
+ * ranking pass (empty on the CUDA-core pass), 6 ranking pass, 7 the rescans of
+ * overflowing queries by the whole grid (on the CUDA-core pass the merge of the
+ * lists' candidates), 8 survivors, exact distances and top-k. */
 #define KATO_PHASES 9
 void *katoann_gpu_timer_create(uint32_t max_passes);
 void katoann_gpu_timer_destroy(void *timer);
